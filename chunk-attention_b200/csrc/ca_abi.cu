@@ -150,6 +150,7 @@ struct ca_context {
     // The per-row path lists are read by the any-geometry kernel only: a context of the tensor-core geometry
     // builds and uploads them on the first partition = 2 request after a refresh, from this copy of the input.
     bool paths_on_device = false;
+    int max_path_tokens = 0;      // of the longest path on the device
     ca::Plan path_plan;           // infos + path_* of the current tree
     char* paths_host = nullptr;
     char* paths_dev = nullptr;
@@ -477,6 +478,7 @@ static int upload_plan(ca_context* c, const ca::Plan& pl, cudaStream_t stream) {
     c->d_tail_tokens = reinterpret_cast<const int32_t*>(c->dev_blob + parts[7].off);
     c->d_wide_chunks = reinterpret_cast<const int32_t*>(c->dev_blob + parts[8].off);
     c->paths_on_device = pl.has_paths;
+    if (pl.has_paths) c->max_path_tokens = pl.max_path_tokens;
     if (!pl.has_paths) {  // keep what a later partition = 2 request needs to build them
         c->path_plan.infos = pl.infos;
         c->path_plan.n_seqs = pl.n_seqs;
@@ -841,6 +843,7 @@ static int ensure_paths(ca_context* c, cudaStream_t stream) {
     if (c->paths_on_device) return CA_OK;
     ca::Plan& pp = c->path_plan;
     ca::build_paths(pp);
+    c->max_path_tokens = pp.max_path_tokens;
     const size_t b0 = align_up(pp.path_off.size() * 4, 256), b1 = align_up(pp.path_chunks.size() * 4, 256),
                  b2 = align_up(pp.path_tokens.size() * 4, 256);
     const size_t total = b0 + b1 + b2 + 256;
@@ -900,6 +903,7 @@ int ca_attention(ca_context* c, const void* q, void* out, int n_seqs, int partit
     g.out_width = c->geo.d_value;
     g.delta_tokens = c->delta_tokens;
     g.scale = 1.0f / std::sqrt((float)c->geo.d_head);
+    g.max_tokens = c->max_path_tokens + c->delta_tokens;
     CA_CUDA(ca::launch_attn_seq_generic(g, c->dtype, static_cast<cudaStream_t>(stream_)));
     return CA_OK;
 }
@@ -1051,6 +1055,7 @@ int ca_attention_rows(ca_context* c, const ca_rows_args* a, ca_stream stream_) {
     g.row_entry = decode ? nullptr : a->row_entry;
     g.positions = a->positions;
     g.value_freq = a->value_freq;
+    if (decode) g.max_tokens = c->max_path_tokens + c->delta_tokens;
     CA_CUDA(ca::launch_attn_seq_generic(g, c->dtype, stream));
     return CA_OK;
 }

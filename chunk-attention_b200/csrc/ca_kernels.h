@@ -148,6 +148,7 @@ struct GenericParams {
     const int32_t* row_entry = nullptr;  // path of each row; null: row r walks path r, all of it
     const int32_t* positions = nullptr;  // position of each row's token (needed with row_entry or value_freq)
     const float* value_freq = nullptr;   // radians per position of value pair i; null: values are not rotated
+    int max_tokens = 0;          // of the longest path, where the host knows it (decode)
 };
 cudaError_t launch_attn_seq_generic(const GenericParams& p, int dtype, cudaStream_t stream);
 

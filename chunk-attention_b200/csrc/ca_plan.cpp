@@ -124,6 +124,12 @@ void build_paths(Plan& plan) {
             plan.path_chunks[p] = ci.chunk_id;
             plan.path_tokens[p] = ci.n_tokens;
         }
+    plan.max_path_tokens = 0;
+    for (int s = 0; s < n_seqs; s++) {
+        int64_t n = 0;
+        for (int32_t i = plan.path_off[s]; i < plan.path_off[s + 1]; i++) n += plan.path_tokens[i];
+        plan.max_path_tokens = (int)std::min<int64_t>(INT32_MAX, std::max<int64_t>(plan.max_path_tokens, n));
+    }
     plan.has_paths = true;
 }
 

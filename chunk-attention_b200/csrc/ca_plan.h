@@ -75,6 +75,7 @@ struct Plan {
     bool has_paths = false;               // path_* are filled (build_paths)
     int window = 0;
     std::vector<int32_t> path_off, path_chunks, path_tokens;
+    int max_path_tokens = 0;              // of the longest path
     std::vector<int32_t> tail_chunk, tail_tokens;
     ca_plan_stats stats{};
 };
