@@ -7,6 +7,7 @@
 #include <torch/extension.h>
 
 #include "attention.h"
+#include "token_lists.h"
 
 namespace py = pybind11;
 using ca_host::Attention;

@@ -10,6 +10,7 @@
 
 #include "../../../include/chunk_attn_b200.h"
 #include "spans.h"
+#include "token_lists.h"
 
 namespace py = pybind11;
 
