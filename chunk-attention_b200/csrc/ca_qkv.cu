@@ -4,9 +4,10 @@
 // s of the batch into the next free row of sequence s's tail chunk; a portion of a prompt names the pool row of
 // every token, and tokens whose chunk an earlier sequence already filled are not written.
 //
-// One CTA per token: its angles go to shared memory once; then a group of lanes takes a head at a time, one 16-byte granule
-// per lane (heads whose size or alignment does not allow that: a warp per head, one rotation pair per lane and step).  All arithmetic in fp32, one rounding at the store.  Heads are padded with zeros
-// to whole 16-byte granules in the pool and in q, so that the attention kernels read granules for every head size.
+// A token's angles go to shared memory once; then a group of lanes takes a head at a time, in 16-byte granules (heads whose
+// size or alignment does not allow that: a warp per head, one rotation pair per lane and step).  All arithmetic in fp32, one
+// rounding at the store.  Heads are padded with zeros to whole 16-byte granules in the pool and in q, so that the attention
+// kernels read granules for every head size.
 #include <algorithm>
 
 #include "ca_kernels.h"
@@ -101,101 +102,186 @@ __global__ void __launch_bounds__(QKV_WARPS * 32) store_qkv_kernel(const QkvPara
     }
 }
 
-// Heads of whole granules, up to `lanes` of them (a power of two, at most 32).
-constexpr int QKV_VEC_THREADS = 256;
-template <typename T>
-__global__ void __launch_bounds__(QKV_VEC_THREADS) store_qkv_vec_kernel(const QkvParams p, int lanes) {
-    constexpr int EPG = 16 / sizeof(T), PPG = EPG / 2;
-    __shared__ float2 turn_k[QKV_MAX_D / 2], turn_v[QKV_MAX_D / 2];  // (cos, sin) of every pair
-    const int t = blockIdx.x, tid = threadIdx.x;
-    const float pos = (float)p.positions[t];
-    const int kp = p.key_freq ? p.rot_dims / 2 : 0, vp = p.value_freq ? p.d_value / 2 : 0;
-    int chunk, slot;
-    if (p.tok_slot) {
-        const int s = p.tok_slot[t];
-        chunk = s < 0 ? -1 : s / p.geo.chunk_size;
-        slot = s - chunk * p.geo.chunk_size;
-    } else {
-        chunk = p.tail_chunk[t];
-        slot = p.tail_tokens[t] + p.delta_tokens;
-        if (slot >= p.geo.chunk_size) chunk = -1;  // rejected on the host; never write past the tile
-    }
+// Heads of whole granules, at most LANES * GP of them: a group of LANES lanes takes a head at a time, lane g its granules g, g + LANES, ...
+//
+// A prompt is bound by HBM (every element read and written once), but one CTA per token with a granule per lane was bound by its
+// instructions (per granule a division, a square root, a reduction, two addresses and the weights) and by one dependent load after the
+// other: 8192 tokens of 32 + 8 + 8 heads of 128 took 77.6 us.  So a lane takes GP granules of a head, a CTA walks tokens with the next
+// pass's granules requested before the present ones are turned, a thread keeps its frequencies for all tokens, squares and weights go in
+// pairs of fp32, and 16-bit results take the hardware's reciprocal square root (relative error 2^-22): the same tokens take
+// 43.9 us (4.6 TB/s where a copy reaches 6.5).  A grid of 6 CTAs an SM: up to 888 tokens are one to a CTA.
+constexpr int QKV_VEC_THREADS = 128, QKV_VEC_CTAS = 6;
+
+__device__ __forceinline__ void widen(uint32_t v, float& lo, float& hi, __nv_bfloat16) {
+    lo = __uint_as_float(v << 16);
+    hi = __uint_as_float(v & 0xffff0000u);
+}
+__device__ __forceinline__ void widen(uint32_t v, float& lo, float& hi, __half) {
+    const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&v));
+    lo = f.x;
+    hi = f.y;
+}
+__device__ __forceinline__ uint32_t narrow(float lo, float hi, __nv_bfloat16) {
+    const __nv_bfloat162 h = __floats2bfloat162_rn(lo, hi);
+    return *reinterpret_cast<const uint32_t*>(&h);
+}
+__device__ __forceinline__ uint32_t narrow(float lo, float hi, __half) {
+    const __half2 h = __floats2half2_rn(lo, hi);
+    return *reinterpret_cast<const uint32_t*>(&h);
+}
+template <typename T> __device__ __forceinline__ float inverse_rms(float ss, float d, float eps) { return rsqrtf(__fdividef(ss, d) + eps); }
+template <> __device__ __forceinline__ float inverse_rms<float>(float ss, float d, float eps) { return 1.f / sqrtf(ss / d + eps); }
+
+template <typename T, int LANES, int GP>
+__global__ void __launch_bounds__(QKV_VEC_THREADS, QKV_VEC_CTAS) store_qkv_vec_kernel(const QkvParams p) {
+    constexpr int EPG = 16 / sizeof(T), PPG = EPG / 2, PER_PASS = QKV_VEC_THREADS / LANES;
+    __shared__ __align__(16) float2 turns[2][QKV_MAX_D];  // (cos, sin) of every pair of keys, then of values; of a token and the next
+    const int tid = threadIdx.x, g = tid & (LANES - 1), first = tid / LANES;
+    const int kp = p.key_freq ? p.rot_dims / 2 : 0, vp = p.value_freq ? p.d_value / 2 : 0, np = kp + vp;
     const int G = p.geo.n_heads, H = G * p.group, units = H + 2 * G;
-    const int g = tid & (lanes - 1), per_pass = QKV_VEC_THREADS / lanes;
-    const T* row = reinterpret_cast<const T*>(p.qkv) + (size_t)t * p.row_stride;
-    T* pool = reinterpret_cast<T*>(p.pool);
+    const int k_room = (kp + 1) & ~1;  // values' angles start at a 16-byte boundary
+    const int k_left = p.d_key - g * EPG, v_left = p.d_value - g * EPG;  // granule j of this lane exists when j * LANES * EPG is below
+    // what a later granule of a lane adds to the pool offset of its first one (LANES is a multiple of the 8 granules of a panel's line)
+    const int k_step = LANES * (p.geo.swz ? p.geo.chunk_size : 1) * 16, v_step = LANES * (p.geo.v_swz ? p.geo.chunk_size : 1) * 16;
+    const uint32_t head_bytes = (uint32_t)(p.geo.tile_elems + p.geo.v_tile_elems) * sizeof(T);
+    const int v_from = (H + G) * p.d_key;
     const Geometry v_side = tile_side(p.geo, 1);
-    constexpr int AHEAD = 1;  // heads whose granules are requested together
-    Pack<T, EPG> in[AHEAD];
-    auto source = [&](int u) { return row + (u < H + G ? u * p.d_key : (H + G) * p.d_key + (u - H - G) * p.d_value) + g * EPG; };
-    auto size_of = [&](int u) { return u < H + G ? p.d_key : p.d_value; };
-    int u = tid / lanes;
-    auto request = [&](int u) {
+
+    uint4 next[GP];
+    auto request = [&](int t, int u) {
+        const T* src = reinterpret_cast<const T*>(p.qkv) + (size_t)t * p.row_stride + g * EPG + (u < H + G ? u * p.d_key : v_from + (u - H - G) * p.d_value);
+        const int left = u < units ? (u < H + G ? k_left : v_left) : 0;
 #pragma unroll
-        for (int a = 0; a < AHEAD; a++) {
-            const int ua = u + a * per_pass;
-            if (ua < units && g * EPG < size_of(ua)) in[a] = *reinterpret_cast<const Pack<T, EPG>*>(source(ua));
+        for (int j = 0; j < GP; j++) {
+            next[j] = make_uint4(0u, 0u, 0u, 0u);
+            if (j * LANES * EPG < left) next[j] = *reinterpret_cast<const uint4*>(src + j * LANES * EPG);
         }
     };
-    request(u);
-    for (int i = tid; i < kp + vp; i += QKV_VEC_THREADS) {
-        float sn, cs;
-        sincos_for<T>(pos * (i < kp ? p.key_freq[i] : p.value_freq[i - kp]), &sn, &cs);
-        (i < kp ? turn_k[i] : turn_v[i - kp]) = make_float2(cs, sn);
-    }
-    __syncthreads();
-    auto one_head = [&](int u, const Pack<T, EPG>& in) {
-        const bool on = u < units && g * EPG < size_of(min(u, units - 1));
-        const int kind = u < H ? 0 : (u < H + G ? 1 : 2);  // q, k, v
-        float x[EPG];
-        float ss = 0.f;
-#pragma unroll
-        for (int i = 0; i < EPG; i++) {
-            x[i] = on ? to_f32(in.v[i]) : 0.f;
-            ss = fmaf(x[i], x[i], ss);
-        }
-        for (int off = lanes >> 1; off >= 1; off >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, off);
-        if (!on || (kind > 0 && chunk < 0)) return;
-        const float* w = kind == 0 ? p.q_norm : (kind == 1 ? p.k_norm : nullptr);
-        if (w) {
-            const float inv = 1.f / sqrtf(ss / p.d_key + p.eps);
-#pragma unroll
-            for (int i = 0; i < EPG; i += 4) {
-                const float4 ww = *reinterpret_cast<const float4*>(w + g * EPG + i);
-                x[i] *= inv * ww.x;
-                x[i + 1] *= inv * ww.y;
-                x[i + 2] *= inv * ww.z;
-                x[i + 3] *= inv * ww.w;
-            }
-        }
-        const float2* turn = (kind == 2 ? turn_v : turn_k) + g * PPG;
-        const int pairs = (kind == 2 ? vp : kp) - g * PPG;
-#pragma unroll
-        for (int i = 0; i < PPG; i++)
-            if (i < pairs) {
-                const float2 cs = turn[i];
-                const float a = x[2 * i], b = x[2 * i + 1];
-                x[2 * i] = a * cs.x - b * cs.y;
-                x[2 * i + 1] = b * cs.x + a * cs.y;
-            }
-        Pack<T, EPG> o;
-#pragma unroll
-        for (int i = 0; i < EPG; i++) o.v[i] = from_f32<T>(x[i]);
-        Pack<T, EPG>* dst;
-        if (kind == 0) {
-            dst = reinterpret_cast<Pack<T, EPG>*>(reinterpret_cast<T*>(p.q_out) + ((size_t)t * H + u) * p.geo.d_head) + g;
-        } else {
-            const int h = u - (kind == 1 ? H : H + G);
-            dst = reinterpret_cast<Pack<T, EPG>*>(pool + tile_base_elems(p.geo, chunk, h, kind - 1)) +
-                  tile_granule_index(kind == 2 ? v_side : p.geo, slot, g);
-        }
-        *dst = o;
+    auto place_of = [&](int t, int& a, int& b) {  // what names the token's pool row
+        a = p.tok_slot ? p.tok_slot[t] : p.tail_chunk[t];
+        b = p.tok_slot ? 0 : p.tail_tokens[t];
     };
-    for (int u0 = 0; u0 < units; u0 += AHEAD * per_pass, u += AHEAD * per_pass) {
-        if (u0 > 0) request(u);
+    int t = blockIdx.x, place_a, place_b, buf = 0;
+    if (t >= p.n_tokens) return;
+    request(t, first);
+    float pos = (float)p.positions[t];
+    place_of(t, place_a, place_b);
+    float freq[2];  // at most 256 pairs
 #pragma unroll
-        for (int a = 0; a < AHEAD; a++) one_head(u + a * per_pass, in[a]);
+    for (int i = 0; i < 2; i++) {
+        const int n = tid + i * QKV_VEC_THREADS;
+        freq[i] = n < np ? (n < kp ? p.key_freq[n] : p.value_freq[n - kp]) : 0.f;
     }
+    for (; t < p.n_tokens; t += gridDim.x, buf ^= 1) {
+        const int t2 = t + gridDim.x;
+        float2* const turn = turns[buf];
+#pragma unroll
+        for (int i = 0; i < 2; i++) {
+            const int n = tid + i * QKV_VEC_THREADS;
+            if (n < np) {
+                float sn, cs;
+                sincos_for<T>(pos * freq[i], &sn, &cs);
+                turn[n < kp ? n : n - kp + k_room] = make_float2(cs, sn);
+            }
+        }
+        int chunk = place_a, slot = place_b + p.delta_tokens;
+        if (p.tok_slot) {
+            chunk = place_a < 0 ? -1 : place_a / p.geo.chunk_size;
+            slot = place_a - chunk * p.geo.chunk_size;
+        } else if (slot >= p.geo.chunk_size) {
+            chunk = -1;  // rejected on the host; never write past the tile
+        }
+        if (t2 < p.n_tokens) {
+            pos = (float)p.positions[t2];
+            place_of(t2, place_a, place_b);
+        }
+        uint8_t* const at = static_cast<uint8_t*>(p.pool) + (size_t)max(chunk, 0) * p.geo.chunk_elems * sizeof(T);
+        uint8_t* const k_at = at + tile_granule_index(p.geo, slot, g) * 16;
+        uint8_t* const v_at = at + (p.geo.tile_elems * sizeof(T) + tile_granule_index(v_side, slot, g) * 16);
+        uint8_t* const q_at = static_cast<uint8_t*>(p.q_out) + ((size_t)t * H * p.geo.d_head + g * EPG) * sizeof(T);
+        __syncthreads();  // one a token: the other buffer is written only when every warp is past this token's angles
+        for (int u0 = 0; u0 < units; u0 += PER_PASS) {
+            const int u = u0 + first;
+            uint4 in[GP];
+#pragma unroll
+            for (int j = 0; j < GP; j++) in[j] = next[j];
+            if (u0 + PER_PASS < units) request(t, u + PER_PASS);
+            else if (t2 < p.n_tokens) request(t2, first);
+            if ((tid & ~31) / LANES + u0 >= units) continue;  // a warp without a head
+            uint64_t x[GP][PPG];
+            uint64_t s2 = 0;  // a pair of zeros
+#pragma unroll
+            for (int j = 0; j < GP; j++) {
+                const uint32_t w32[4] = {in[j].x, in[j].y, in[j].z, in[j].w};
+#pragma unroll
+                for (int i = 0; i < PPG; i++) {
+                    float lo, hi;
+                    if constexpr (sizeof(T) == 4) {
+                        lo = __uint_as_float(w32[2 * i]);
+                        hi = __uint_as_float(w32[2 * i + 1]);
+                    } else {
+                        widen(w32[i], lo, hi, T());
+                    }
+                    x[j][i] = pair_f32(lo, hi);
+                    s2 = fma_f32x2(x[j][i], x[j][i], s2);
+                }
+            }
+            const float* w = u < H ? p.q_norm : (u < H + G ? p.k_norm : nullptr);
+            uint64_t inv2 = 0;
+            if (p.q_norm || p.k_norm) {
+                float ss, ss_hi;
+                unpair_f32(s2, ss, ss_hi);
+                ss += ss_hi;
+#pragma unroll
+                for (int off = LANES >> 1; off >= 1; off >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, off);
+                const float inv = inverse_rms<T>(ss, (float)p.d_key, p.eps);
+                inv2 = pair_f32(inv, inv);
+            }
+            if (u >= units || (u >= H && chunk < 0)) continue;
+            const bool value = u >= H + G;
+            const int left = value ? v_left : k_left, pairs = (value ? vp : kp) - g * PPG;
+            const float2* turn_of = turn + (value ? k_room : 0) + g * PPG;
+            uint8_t* dst = u < H ? q_at + (size_t)((uint32_t)u * (uint32_t)(p.geo.d_head * sizeof(T)))
+                                 : (value ? v_at + (uint64_t)(uint32_t)(u - H - G) * head_bytes : k_at + (uint64_t)(uint32_t)(u - H) * head_bytes);
+            const int step = u < H ? LANES * 16 : (value ? v_step : k_step);
+#pragma unroll
+            for (int j = 0; j < GP; j++) {
+                if (j * LANES * EPG >= left) break;
+                if (w) {
+#pragma unroll
+                    for (int i = 0; i < PPG; i += 2) {
+                        const float4 ww = *reinterpret_cast<const float4*>(w + (g + j * LANES) * EPG + 2 * i);
+                        x[j][i] = mul_f32x2(x[j][i], mul_f32x2(inv2, pair_f32(ww.x, ww.y)));
+                        x[j][i + 1] = mul_f32x2(x[j][i + 1], mul_f32x2(inv2, pair_f32(ww.z, ww.w)));
+                    }
+                }
+                uint32_t o[4];
+#pragma unroll
+                for (int i = 0; i < PPG; i++) {
+                    float a, b;
+                    unpair_f32(x[j][i], a, b);
+                    if (j * LANES * PPG + i < pairs) {
+                        const float2 cs = turn_of[j * LANES * PPG + i];
+                        const float c = a;
+                        a = a * cs.x - b * cs.y;
+                        b = b * cs.x + c * cs.y;
+                    }
+                    if constexpr (sizeof(T) == 4) {
+                        o[2 * i] = __float_as_uint(a);
+                        o[2 * i + 1] = __float_as_uint(b);
+                    } else {
+                        o[i] = narrow(a, b, T());
+                    }
+                }
+                *reinterpret_cast<uint4*>(dst + j * step) = make_uint4(o[0], o[1], o[2], o[3]);
+            }
+        }
+    }
+}
+
+template <typename T, int LANES, int GP>
+void run_store_qkv_vec(const QkvParams& p, cudaStream_t stream) {
+    store_qkv_vec_kernel<T, LANES, GP><<<std::min(p.n_tokens, QKV_VEC_CTAS * 148), QKV_VEC_THREADS, 0, stream>>>(p);
 }
 template <typename T>
 void run_store_qkv(const QkvParams& p, cudaStream_t stream) {
@@ -204,9 +290,9 @@ void run_store_qkv(const QkvParams& p, cudaStream_t stream) {
     const int granules = std::max(p.d_key, p.d_value) / EPG;
     if (p.d_key % EPG == 0 && p.d_value % EPG == 0 && p.row_stride % EPG == 0 && aligned(p.qkv) && aligned(p.q_norm) && aligned(p.k_norm) &&
         granules <= 32) {
-        int lanes = 1;
-        while (lanes < granules) lanes *= 2;
-        store_qkv_vec_kernel<T><<<p.n_tokens, QKV_VEC_THREADS, 0, stream>>>(p, lanes);
+        if (granules <= 8) run_store_qkv_vec<T, 8, 1>(p, stream);
+        else if (granules <= 16) run_store_qkv_vec<T, 8, 2>(p, stream);
+        else run_store_qkv_vec<T, 16, 2>(p, stream);
     } else {
         store_qkv_kernel<T><<<p.n_tokens, QKV_WARPS * 32, 0, stream>>>(p);
     }

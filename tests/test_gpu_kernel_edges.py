@@ -39,3 +39,30 @@ def test_split_rows(dtype, d, chunk, lens):
     eng.append_token([5] * n, k1, v1)  # a token more than the work list says, some of them in a chunk of their own
     kv = [(torch.cat([k, a[None]]), torch.cat([v, b[None]])) for (k, v), a, b in zip(kv, k1, v1)]
     assert (eng.forward(q).cpu().double() - dense(q, kv, d ** -0.5)).abs().max() < tol
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("shape", [(8, 2, 64, 64, 64), (40, 8, 40, 24, 18), (2, 1, 128, 48, 128), (3, 1, 256, 256, 6), (96, 4, 16, 16, 0)])
+@pytest.mark.parametrize("lens", [[888], [889], [1, 1750, 64]])
+def test_stored_heads_of_more_tokens_than_ctas(shape, dtype, lens):
+    # The store walks tokens with a grid of at most 888 CTAs: exactly one each, one more, three for some; groups of 8 and 16
+    # lanes with one and two granules each; heads that fill a pass, a part of one, several; a rotated part that ends inside a granule.
+    import chunk_attn
+    import gagorax_oracle as oracle
+    from chunk_attn import SpanBatch
+    from test_gpu_block_ops import close, oracle_attention, rnd
+    H, G, dk, dv, rot = shape
+    eps, base, scale, dev = 1e-4, 1000.0, dk ** -0.5, torch.device("cuda:0")
+    cache = chunk_attn.Attention.shaped(n_heads=H, n_kv_heads=G, d_key=dk, d_value=dv, scale=scale, sink=True, chunk_size=64, memory_mb=64,
+                                        dtype=dtype, device=dev)
+    qn, kn = rnd(1, dk) * 0.2 + 1, rnd(2, dk) * 0.2 + 1
+    freq = lambda n: torch.from_numpy(oracle.pair_frequencies(n, base)).float().to(dev)
+    x = rnd(3, sum(lens), (H + G) * dk + G * dv).to(dtype)
+    tokens = [[10_000 * i + t for t in range(n)] for i, n in enumerate(lens)]
+    cache.extend([-1] * len(lens), tokens)
+    spans = SpanBatch(tokens, [0] * len(lens), list(range(len(lens))), dev)
+    q = cache.store_qkv(x.to(dev), spans.positions, qn.to(dev), kn.to(dev), eps, rot, freq(rot) if rot else None, freq(dv))
+    o = cache.forward_rows(q, spans.positions, freq(dv), spans.entry_of).split(lens)
+    for xs, part in zip(x.split(lens), o):
+        close(part, oracle_attention(xs.double().numpy(), shape, qn.double().numpy(), kn.double().numpy(), eps, base, scale), dtype)
+    assert cache.device_status() == 0
