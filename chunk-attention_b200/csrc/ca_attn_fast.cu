@@ -30,6 +30,7 @@
 // and unwinds instead of spinning forever.
 #include <cuda_fp16.h>
 
+#include <algorithm>
 #include <cstdlib>
 
 #include "ca_kernels.h"
@@ -782,13 +783,16 @@ __global__ void __launch_bounds__(NUM_THREADS, 2) attn_partial_kernel(const Part
 // A (sequence, head) whose private part is a single, usually partly filled, chunk is too small an item
 // for the persistent kernel (an item costs its warps the same whatever it holds).  When a batch has
 // many of them the planner puts them at the end of the item list and this kernel walks them instead:
-// one HALF-WARP per item, straight from global memory, eight tokens per round with all of a round's loads
-// (K rows and V rows) issued before any is used, so a tail of up to eight tokens costs one round trip after
-// the item's description.  Lane g of the half-warp owns granule g of every row: 16 bytes of each K row (the
+// one HALF-WARP per item, eight tokens per round.  Lane g of the half-warp owns granule g of every row: 16 bytes of each K row (the
 // products are summed over the 16 lanes with shuffles, which leaves every lane with every score, so the
 // softmax needs no further exchange) and 16 bytes = 8 output elements of each V row.  The result is an
 // ordinary partial (max and sum in log2 units, un-normalised O), combined with the row's other partials by
 // the merge kernel.
+// Bound by HBM (the tails once), if the round trips overlap: description, then tokens, then the row's other partials.  With one item
+// per half-warp and CTAs one wave after the other they did not: 1024 x 32 tails of 8 tokens (160 MB) took 44 us.  So a half-warp walks
+// items with the descriptions two items ahead and a round's tokens copied asynchronously, every lane its own granules to a place of its
+// own in shared memory, while the round before is worked on:
+// the step around it (the wide runs before it take 45 us) went from 94.6 to 78.6 us.
 // FINISH: when EVERY row of the batch has such a tail (many requests with short suffixes over shared prompts) the
 // kernel runs LAST in the step and finishes the rows itself: the half-warp keeps its partial in registers, fetches
 // the row's other partials (the shared runs', written by the kernels before it), combines, normalises and stores the
@@ -799,69 +803,95 @@ __device__ __forceinline__ void store_row8(const MergeParams& p, int row, int he
 
 constexpr int SHORT_WARPS = 4;   // small CTAs: they fit beside the wide-runs kernel's CTAs when the two overlap
 constexpr int SHORT_ITEMS_PER_CTA = 2 * SHORT_WARPS;
+constexpr int SHORT_CTAS = 4;    // per SM, by registers
 constexpr int SHORT_BLOCK = 8;   // tokens per round
 
-template <bool FINISH>
-__global__ void __launch_bounds__(SHORT_WARPS * 32, 4) attn_short_tails_kernel(const PartialParams p, const MergeParams mp) {
-    asm volatile("griddepcontrol.wait;" ::: "memory");
+// EARLY: the kernel before this one is of the same step, and had waited for all before it when this one was allowed to start; it writes
+// partials only, so tokens, queries and lists may be read before it ends.
+template <bool FINISH, bool EARLY>
+__global__ void __launch_bounds__(SHORT_WARPS * 32, SHORT_CTAS) attn_short_tails_kernel(const PartialParams p, const MergeParams mp) {
+    __shared__ __align__(16) uint4 tiles[SHORT_ITEMS_PER_CTA][2 * SHORT_BLOCK][16];  // K rows, then V rows
+    if (!EARLY) asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int g = lane & 15, half = lane >> 4;
-    const int vid = p.item_lo + ((int)blockIdx.x * SHORT_WARPS + warp) * 2 + half;  // work piece = (item, head)
-    // every lane runs every round (the shuffles below need the whole warp); a half-warp without an item, or with a
-    // rejected one, simply has no tokens
-    int nt = 0, row = 0, head = 0, chunk = 0, slot = -1;
-    if (vid < p.item_hi) {
-        const int idx = vid / p.n_heads;
-        head = vid - idx * p.n_heads;
-        const int4 d0 = __ldg(p.items + 4 * idx), d1 = __ldg(p.items + 4 * idx + 1);
-        row = d0.z;
-        chunk = d1.w;
-        slot = d1.x * p.n_heads + head;
-        if (row < 0 || d1.x < 0 || chunk < 0 || d1.z < 0 || (p.n_slots > 0 && slot >= p.n_slots) ||
-            (p.n_seqs > 0 && row >= p.n_seqs) || (p.max_chunks > 0 && chunk >= p.max_chunks)) {
+    uint4* const mine = &tiles[warp * 2 + half][0][g];
+    const uint32_t mine_u32 = smem_u32(mine);
+    const int first = p.item_lo + ((int)blockIdx.x * SHORT_WARPS + warp) * 2, stride = (int)gridDim.x * SHORT_ITEMS_PER_CTA;
+
+    struct Piece {
+        int nt, row, head, slot;  // slot < 0: nothing to do (no item, or a rejected one), and then no tokens
+        const uint8_t* tile;
+    };
+    auto fetch = [&](int v, int4& d0, int4& d1) {  // work piece v = (item, head)
+        if (v >= p.item_hi) return;
+        const int4* d = p.items + 4 * (v / p.n_heads);
+        d0 = __ldg(d);
+        d1 = __ldg(d + 1);
+    };
+    auto decode = [&](int v, const int4& d0, const int4& d1) {
+        Piece w{0, 0, 0, -1, p.pool};
+        if (v >= p.item_hi) return w;
+        w.head = v % p.n_heads;
+        w.row = d0.z;
+        const int chunk = d1.w;
+        w.slot = d1.x * p.n_heads + w.head;
+        if (w.row < 0 || d1.x < 0 || chunk < 0 || d1.z < 0 || (p.n_slots > 0 && w.slot >= p.n_slots) ||
+            (p.n_seqs > 0 && w.row >= p.n_seqs) || (p.max_chunks > 0 && chunk >= p.max_chunks)) {
             if (g == 0) report(p.status, STATUS_BAD_WORK_LIST);  // skipped
-            slot = -1;
-        } else {
-            nt = min(FAST_C, d1.z + ((d1.y & ITEM_FLAG_TAIL) ? p.delta_tokens : 0));
+            w.slot = -1;
+            w.row = 0;
+            return w;
         }
-    }
-    const int nt_warp = max(nt, __shfl_xor_sync(0xffffffffu, nt, 16));
-    // FINISH: where the row's other partials are is looked up now, in the shadow of the tail's own loads
-    constexpr int AHEAD = 4;   // lists of up to four other pieces cost one round trip after the tail
-    int lb = 0, le = 0, sl[AHEAD];
-#pragma unroll
-    for (int u = 0; u < AHEAD; u++) sl[u] = -1;
-    if (FINISH && slot >= 0) {
-        lb = __ldg(mp.merge_off + row);
-        le = __ldg(mp.merge_off + row + 1);
-        checked_bounds(mp, lb, le);
-#pragma unroll
-        for (int u = 0; u < AHEAD; u++)
-            if (lb + u < le) sl[u] = __ldg(mp.merge_slots + lb + u);   // entries; checked when they are used
-    }
-    const uint8_t* ktile = p.pool + ((size_t)chunk * p.n_heads + head) * (size_t)FAST_STAGE_BYTES;
-    const uint8_t* vtile = ktile + FAST_TILE_BYTES;
-    uint4 qraw = make_uint4(0u, 0u, 0u, 0u);
-    if (nt > 0)
-        qraw = __ldg(reinterpret_cast<const uint4*>(reinterpret_cast<const __half*>(p.q) + ((size_t)row * p.n_heads + head) * FAST_D + 8 * g));
-    float qf[8];
-    float m = NEG_BIG, l = 0.f;
-    float o[8];
-#pragma unroll
-    for (int e = 0; e < 8; e++) o[e] = 0.f;
-    for (int t0 = 0; t0 < nt_warp; t0 += SHORT_BLOCK) {
-        uint4 kr[SHORT_BLOCK], vr[SHORT_BLOCK];
+        w.nt = min(FAST_C, d1.z + ((d1.y & ITEM_FLAG_TAIL) ? p.delta_tokens : 0));
+        w.tile = p.pool + ((size_t)chunk * p.n_heads + w.head) * (size_t)FAST_STAGE_BYTES;
+        return w;
+    };
+    // tokens t0 .. t0 + 7 of one side of a piece's tile; zeros past its end
+    auto copy_side = [&](const Piece& w, int t0, int side) {
 #pragma unroll
         for (int i = 0; i < SHORT_BLOCK; i++) {
-            kr[i] = make_uint4(0u, 0u, 0u, 0u);
-            vr[i] = make_uint4(0u, 0u, 0u, 0u);
-            if (t0 + i < nt) {
-                kr[i] = __ldg(reinterpret_cast<const uint4*>(ktile + tile_off(t0 + i, g)));
-                vr[i] = __ldg(reinterpret_cast<const uint4*>(vtile + tile_off(t0 + i, g)));
-            }
+            const bool on = t0 + i < w.nt;
+            const uint8_t* src = w.tile + (on ? side * FAST_TILE_BYTES + tile_off(t0 + i, g) : 0);
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(mine_u32 + (side * SHORT_BLOCK + i) * 256), "l"(src), "r"(on ? 16 : 0)
+                         : "memory");
         }
-        if (t0 == 0) {  // the query granule of this lane, pre-scaled to log2 units
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    auto query = [&](const Piece& w) {
+        return w.nt > 0 ? __ldg(reinterpret_cast<const uint4*>(reinterpret_cast<const __half*>(p.q) + ((size_t)w.row * p.n_heads + w.head) * FAST_D + 8 * g))
+                        : make_uint4(0u, 0u, 0u, 0u);
+    };
+
+    if (first >= p.item_hi) return;
+    int4 d0 = make_int4(0, 0, 0, 0), d1 = d0;
+    fetch(first + half, d0, d1);
+    Piece cur = decode(first + half, d0, d1);
+    copy_side(cur, 0, 0);
+    copy_side(cur, 0, 1);
+    uint4 qraw = query(cur);
+    fetch(first + half + stride, d0, d1);
+    // the warp's two items are walked together: every lane runs every round, as the shuffles need the whole warp
+    for (int v = first; v < p.item_hi; v += stride) {
+        const int nt = cur.nt, row = cur.row, head = cur.head, slot = cur.slot;
+        const int nt_warp = max(nt, __shfl_xor_sync(0xffffffffu, nt, 16));
+        // FINISH: where the row's other partials are is looked up now, in the shadow of the tail's own tokens
+        constexpr int AHEAD = 4;   // lists of up to four other pieces cost one round trip after the tail
+        int lb = 0, le = 0, sl[AHEAD];
+#pragma unroll
+        for (int u = 0; u < AHEAD; u++) sl[u] = -1;
+        if (FINISH && slot >= 0) {
+            lb = __ldg(mp.merge_off + row);
+            le = __ldg(mp.merge_off + row + 1);
+            checked_bounds(mp, lb, le);
+#pragma unroll
+            for (int u = 0; u < AHEAD; u++)
+                if (lb + u < le) sl[u] = __ldg(mp.merge_slots + lb + u);   // entries; checked when they are used
+        }
+        const Piece next = decode(v + half + stride, d0, d1);
+        fetch(v + half + 2 * stride, d0, d1);
+        float qf[8];  // the query granule of this lane, pre-scaled to log2 units
+        {
             const __half2* h = reinterpret_cast<const __half2*>(&qraw);
 #pragma unroll
             for (int k = 0; k < 4; k++) {
@@ -870,101 +900,123 @@ __global__ void __launch_bounds__(SHORT_WARPS * 32, 4) attn_short_tails_kernel(c
                 qf[2 * k + 1] = f.y * p.scale_log2;
             }
         }
-        const int n_here = min(SHORT_BLOCK, nt_warp - t0);  // warp-uniform: rounds are cut short together
-        float sc[SHORT_BLOCK];
-        float mx = NEG_BIG;
+        qraw = query(next);
+        float m = NEG_BIG, l = 0.f;
+        float o[8];
 #pragma unroll
-        for (int i = 0; i < SHORT_BLOCK; i++) {
-            sc[i] = NEG_BIG;
-            if (i < n_here) {
-                const __half2* h = reinterpret_cast<const __half2*>(&kr[i]);
-                float a = 0.f;
+        for (int e = 0; e < 8; e++) o[e] = 0.f;
+        for (int t0 = 0; t0 == 0 || t0 < nt_warp; t0 += SHORT_BLOCK) {
+            const bool last = t0 + SHORT_BLOCK >= nt_warp;
+            const int n_here = min(SHORT_BLOCK, nt_warp - t0);  // warp-uniform: rounds are cut short together
+            uint4 r[SHORT_BLOCK];
+            asm volatile("cp.async.wait_group 1;" ::: "memory");  // this round's K rows are there
 #pragma unroll
-                for (int k = 0; k < 4; k++) {
-                    const float2 f = __half22float2(h[k]);
-                    a = fmaf(qf[2 * k], f.x, a);
-                    a = fmaf(qf[2 * k + 1], f.y, a);
-                }
-#pragma unroll
-                for (int off = 8; off >= 1; off >>= 1) a += __shfl_xor_sync(0xffffffffu, a, off);
-                if (t0 + i < nt) sc[i] = a;
-                mx = fmaxf(mx, sc[i]);
-            }
-        }
-        if (t0 < nt) {  // this half-warp's item still has tokens in the round
-            const float mn = fmaxf(m, mx);
-            const float alpha = fast_exp2(m - mn);
-            m = mn;
-            l *= alpha;
-#pragma unroll
-            for (int e = 0; e < 8; e++) o[e] *= alpha;
+            for (int i = 0; i < SHORT_BLOCK; i++) r[i] = mine[i * 16];
+            __syncwarp();
+            copy_side(last ? next : cur, last ? 0 : t0 + SHORT_BLOCK, 0);
+            float sc[SHORT_BLOCK];
+            float mx = NEG_BIG;
 #pragma unroll
             for (int i = 0; i < SHORT_BLOCK; i++) {
+                sc[i] = NEG_BIG;
                 if (i < n_here) {
-                    const float pw = t0 + i < nt ? fast_exp2(sc[i] - mn) : 0.f;
-                    l += pw;
-                    const __half2* h = reinterpret_cast<const __half2*>(&vr[i]);
+                    const __half2* h = reinterpret_cast<const __half2*>(&r[i]);
+                    float a = 0.f;
 #pragma unroll
                     for (int k = 0; k < 4; k++) {
                         const float2 f = __half22float2(h[k]);
-                        o[2 * k] = fmaf(pw, f.x, o[2 * k]);
-                        o[2 * k + 1] = fmaf(pw, f.y, o[2 * k + 1]);
+                        a = fmaf(qf[2 * k], f.x, a);
+                        a = fmaf(qf[2 * k + 1], f.y, a);
+                    }
+#pragma unroll
+                    for (int off = 8; off >= 1; off >>= 1) a += __shfl_xor_sync(0xffffffffu, a, off);
+                    if (t0 + i < nt) sc[i] = a;
+                    mx = fmaxf(mx, sc[i]);
+                }
+            }
+            asm volatile("cp.async.wait_group 1;" ::: "memory");  // and its V rows
+#pragma unroll
+            for (int i = 0; i < SHORT_BLOCK; i++) r[i] = mine[(SHORT_BLOCK + i) * 16];
+            __syncwarp();
+            copy_side(last ? next : cur, last ? 0 : t0 + SHORT_BLOCK, 1);
+            if (t0 < nt) {  // this half-warp's item still has tokens in the round
+                const float mn = fmaxf(m, mx);
+                const float alpha = fast_exp2(m - mn);
+                m = mn;
+                l *= alpha;
+#pragma unroll
+                for (int e = 0; e < 8; e++) o[e] *= alpha;
+#pragma unroll
+                for (int i = 0; i < SHORT_BLOCK; i++) {
+                    if (i < n_here) {
+                        const float pw = t0 + i < nt ? fast_exp2(sc[i] - mn) : 0.f;
+                        l += pw;
+                        const __half2* h = reinterpret_cast<const __half2*>(&r[i]);
+#pragma unroll
+                        for (int k = 0; k < 4; k++) {
+                            const float2 f = __half22float2(h[k]);
+                            o[2 * k] = fmaf(pw, f.x, o[2 * k]);
+                            o[2 * k + 1] = fmaf(pw, f.y, o[2 * k + 1]);
+                        }
                     }
                 }
             }
         }
-    }
-    if (slot < 0) return;
-    if (!FINISH) {
-        if (nt > 0) {
-            float4* dst = reinterpret_cast<float4*>(p.part_o + (size_t)slot * FAST_D + 8 * g);
-            dst[0] = make_float4(o[0], o[1], o[2], o[3]);
-            dst[1] = make_float4(o[4], o[5], o[6], o[7]);
+        cur = next;
+        if (EARLY && v == first) asm volatile("griddepcontrol.wait;" ::: "memory");  // from here on partials are read and written
+        if (slot >= 0 && !FINISH) {
+            if (nt > 0) {
+                float4* dst = reinterpret_cast<float4*>(p.part_o + (size_t)slot * FAST_D + 8 * g);
+                dst[0] = make_float4(o[0], o[1], o[2], o[3]);
+                dst[1] = make_float4(o[4], o[5], o[6], o[7]);
+            }
+            if (g == 0) p.part_ml[slot] = make_float2(nt > 0 ? m : NEG_BIG, l);  // an empty reserved tail: (none, 0)
         }
-        if (g == 0) p.part_ml[slot] = make_float2(nt > 0 ? m : NEG_BIG, l);  // an empty reserved tail: (none, 0)
-        return;
-    }
-    // ---- the row's other partials (no shuffles from here on: half-warps proceed on their own)
-    if (nt == 0) m = NEG_BIG;
-    for (int b = lb; b < le; b += AHEAD) {
-        if (b > lb) {
+        if (slot >= 0 && FINISH) {
+            // ---- the row's other partials (no shuffles from here on: half-warps proceed on their own)
+            if (nt == 0) m = NEG_BIG;
+            for (int b = lb; b < le; b += AHEAD) {
+                if (b > lb) {
 #pragma unroll
-            for (int u = 0; u < AHEAD; u++) sl[u] = b + u < le ? __ldg(mp.merge_slots + b + u) : -1;
-        }
-        float2 ml[AHEAD];
-        float4 v[AHEAD][2];
+                    for (int u = 0; u < AHEAD; u++) sl[u] = b + u < le ? __ldg(mp.merge_slots + b + u) : -1;
+                }
+                float2 ml[AHEAD];
+                float4 v[AHEAD][2];
 #pragma unroll
-        for (int u = 0; u < AHEAD; u++) {
-            ml[u] = make_float2(NEG_BIG, 0.f);
-            v[u][0] = v[u][1] = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (b + u < le) {
-                const int s = checked_slot(mp, sl[u], head);
-                if (s >= 0 && s != slot) {   // this half-warp's own piece is in its registers
-                    ml[u] = mp.part_ml[s];
-                    const float4* src = reinterpret_cast<const float4*>(mp.part_o + (size_t)s * FAST_D + 8 * g);
-                    v[u][0] = src[0];
-                    v[u][1] = src[1];
+                for (int u = 0; u < AHEAD; u++) {
+                    ml[u] = make_float2(NEG_BIG, 0.f);
+                    v[u][0] = v[u][1] = make_float4(0.f, 0.f, 0.f, 0.f);
+                    if (b + u < le) {
+                        const int s = checked_slot(mp, sl[u], head);
+                        if (s >= 0 && s != slot) {   // this half-warp's own piece is in its registers
+                            ml[u] = mp.part_ml[s];
+                            const float4* src = reinterpret_cast<const float4*>(mp.part_o + (size_t)s * FAST_D + 8 * g);
+                            v[u][0] = src[0];
+                            v[u][1] = src[1];
+                        }
+                    }
+                }
+#pragma unroll
+                for (int u = 0; u < AHEAD; u++) {
+                    if (!(ml[u].y > 0.f)) continue;   // no piece, this half-warp's own, or one without tokens (it has no O row)
+                    const float mn = fmaxf(m, ml[u].x);
+                    const float a = fast_exp2(m - mn), w = fast_exp2(ml[u].x - mn);
+                    m = mn;
+                    l = l * a + ml[u].y * w;
+                    o[0] = o[0] * a + v[u][0].x * w;
+                    o[1] = o[1] * a + v[u][0].y * w;
+                    o[2] = o[2] * a + v[u][0].z * w;
+                    o[3] = o[3] * a + v[u][0].w * w;
+                    o[4] = o[4] * a + v[u][1].x * w;
+                    o[5] = o[5] * a + v[u][1].y * w;
+                    o[6] = o[6] * a + v[u][1].z * w;
+                    o[7] = o[7] * a + v[u][1].w * w;
                 }
             }
-        }
-#pragma unroll
-        for (int u = 0; u < AHEAD; u++) {
-            if (!(ml[u].y > 0.f)) continue;   // no piece, this half-warp's own, or one without tokens (it has no O row)
-            const float mn = fmaxf(m, ml[u].x);
-            const float a = fast_exp2(m - mn), w = fast_exp2(ml[u].x - mn);
-            m = mn;
-            l = l * a + ml[u].y * w;
-            o[0] = o[0] * a + v[u][0].x * w;
-            o[1] = o[1] * a + v[u][0].y * w;
-            o[2] = o[2] * a + v[u][0].z * w;
-            o[3] = o[3] * a + v[u][0].w * w;
-            o[4] = o[4] * a + v[u][1].x * w;
-            o[5] = o[5] * a + v[u][1].y * w;
-            o[6] = o[6] * a + v[u][1].z * w;
-            o[7] = o[7] * a + v[u][1].w * w;
+            store_row8(mp, row, head, g, o, l > 0.f ? 1.f / l : 0.f);  // a row with no token yields zeros
         }
     }
-    store_row8(mp, row, head, g, o, l > 0.f ? 1.f / l : 0.f);  // a row with no token yields zeros
+    asm volatile("cp.async.wait_group 0;" ::: "memory");  // zeros for a piece that does not exist
 }
 
 // The un-normalised combination of the partials merge_slots[b .. e) by one warp: on return mm is their
@@ -1377,12 +1429,15 @@ cudaError_t launch_attn_partials(const PartialParams& p, int n_ctas, cudaStream_
     return err;
 }
 
-cudaError_t launch_attn_short_tails(const PartialParams& p, cudaStream_t stream, bool dependent_launch, const MergeParams* finish) {
+cudaError_t launch_attn_short_tails(const PartialParams& p, cudaStream_t stream, bool dependent_launch, const MergeParams* finish, bool early) {
     const int n = p.item_hi - p.item_lo;
     if (n <= 0) return cudaSuccess;
     static const bool pdl_disabled = std::getenv("CA_DISABLE_PDL") != nullptr;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((n + SHORT_ITEMS_PER_CTA - 1) / SHORT_ITEMS_PER_CTA);
+    int dev = 0, sms = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    cfg.gridDim = dim3(std::min((n + SHORT_ITEMS_PER_CTA - 1) / SHORT_ITEMS_PER_CTA, SHORT_CTAS * sms));
     cfg.blockDim = dim3(SHORT_WARPS * 32);
     cfg.dynamicSmemBytes = 0;
     cfg.stream = stream;
@@ -1391,7 +1446,7 @@ cudaError_t launch_attn_short_tails(const PartialParams& p, cudaStream_t stream,
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = (dependent_launch && !pdl_disabled) ? 1 : 0;
-    auto* kernel = finish ? attn_short_tails_kernel<true> : attn_short_tails_kernel<false>;
+    auto* kernel = !finish ? attn_short_tails_kernel<false, false> : (early ? attn_short_tails_kernel<true, true> : attn_short_tails_kernel<true, false>);
     const MergeParams mp = finish ? *finish : MergeParams{};
     cudaError_t err = cudaLaunchKernelEx(&cfg, kernel, p, mp);
     if (err != cudaSuccess && cfg.numAttrs == 1) {

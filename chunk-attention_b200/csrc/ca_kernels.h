@@ -61,10 +61,11 @@ struct PartialParams {
 cudaError_t launch_attn_partials(const PartialParams& p, int n_ctas, cudaStream_t stream, bool dependent_launch = false);
 // one half-warp per item over items [item_lo, item_hi): single-tile one-row items only (short private tails).
 // finish != null: every row of the batch has such an item and every other partial of the step is already in the
-// stream; the kernel then combines each row's partials itself and stores the output rows (no merge launch follows)
+// stream; the kernel then combines each row's partials itself and stores the output rows (no merge launch follows).
+// early: the launch before it is a partials or wide-runs kernel of the same step
 struct MergeParams;
 cudaError_t launch_attn_short_tails(const PartialParams& p, cudaStream_t stream, bool dependent_launch = false,
-                                    const MergeParams* finish = nullptr);
+                                    const MergeParams* finish = nullptr, bool early = false);
 cudaError_t configure_fast_kernels();  // once per device before the first launch
 
 // ---- wide shared runs on tcgen05 / TMEM (ca_attn_wide.cu): one CTA per item ---------------------------------

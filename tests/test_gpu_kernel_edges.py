@@ -66,3 +66,32 @@ def test_stored_heads_of_more_tokens_than_ctas(shape, dtype, lens):
     for xs, part in zip(x.split(lens), o):
         close(part, oracle_attention(xs.double().numpy(), shape, qn.double().numpy(), kn.double().numpy(), eps, base, scale), dtype)
     assert cache.device_status() == 0
+
+
+@pytest.mark.parametrize("n,H", [(64, 8), (310, 16)])
+@pytest.mark.parametrize("shared", [0, 256])
+def test_short_tails_walked_by_half_warps(n, H, shared):
+    # Private tails of 0 to 64 tokens (rounds of eight, both items of a warp of different lengths), fewer and more of them than the
+    # grid's half-warps; with other partials to combine and without; a token appended, into a chunk of its own for some.
+    g = torch.Generator().manual_seed(n)
+    eng = CabiEngine(H, 128, 64, torch.float16, max_chunks=4 + 2 * n)
+    sk, sv = torch.randn(shared, H, 128, generator=g).half(), torch.randn(shared, H, 128, generator=g).half()
+    kv = []
+    for i in range(n):
+        own = (7 * i) % 65 if shared else 1 + (7 * i) % 63
+        k, v = torch.randn(own, H, 128, generator=g).half(), torch.randn(own, H, 128, generator=g).half()
+        kv.append((torch.cat([sk, k]), torch.cat([sv, v])))
+        eng.add_seq(list(range(shared)) + [100_000 + 1000 * i + j for j in range(own)], *kv[-1])
+    q = torch.randn(n, H, 128, generator=g).half()
+
+    def check():
+        want = dense(q.cuda(), [(k.cuda(), v.cuda()) for k, v in kv], 128 ** -0.5)
+        # the result's rounding to fp16, 2^-11 of it, and that of a shared run's weights: 2^-11 of the mean |value|, 0.8
+        assert ((eng.forward(q).double() - want).abs() - want.abs() * 2.0 ** -11).max() < 4e-4
+
+    check()
+    check()
+    k1, v1 = torch.randn(n, H, 128, generator=g).half(), torch.randn(n, H, 128, generator=g).half()
+    eng.append_token([5] * n, k1, v1)
+    kv = [(torch.cat([k, a[None]]), torch.cat([v, b[None]])) for (k, v), a, b in zip(kv, k1, v1)]
+    check()
