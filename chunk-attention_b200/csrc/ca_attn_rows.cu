@@ -51,6 +51,13 @@ __device__ __forceinline__ void split_bf16(float a, float b, uint32_t& hi, uint3
 // byte offset of granule g of token t in a staged tile: panels of [64 tokens][128 bytes]
 __device__ __forceinline__ uint32_t staged(int t, int g) { return (g >> 3) * (R_TILE * 128) + t * 128 + (((g & 7) ^ (t & 7)) << 4); }
 
+// an 8 x 8 matrix of 16-bit elements over the warp (lane: row lane / 4, columns 2 (lane & 3) + {0, 1})
+__device__ __forceinline__ uint32_t transpose_8x8(uint32_t v) {
+    uint32_t t;
+    asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(t) : "r"(v));
+    return t;
+}
+
 // Scores, softmax and O += P V of one warp: 16 rows against 16 * NS tokens of the staged tile from token tb.
 template <int DK, int DV, int NS>
 __device__ __forceinline__ void warp_tile(uint32_t k_tile, uint32_t v_tile, int tb, int first, const uint32_t (&qf)[DK / 16][4],
@@ -123,15 +130,76 @@ __device__ __forceinline__ void warp_tile(uint32_t k_tile, uint32_t v_tile, int 
     }
 }
 
+// The same for at most 8 rows (one token's group, most decode items), with both products transposed, so that the rows are the 8
+// columns of an MMA instead of 16 of which half or more are padding: S^T = K Q^T, O^T += V^T P^T.  Half the MMAs, exponentials and
+// accumulators: a warp's chain per tile, not HBM, was what decode waited for (470 instructions per warp and tile, DRAM at 54 %).  64 rows of
+// 512 to 1024 tokens, 32 heads on 8 of 128: 44.8 -> 37.8 us (204 MB; the whole call with its merge 53.7 -> 45.1).  A lane holds the weights of rows 2 (lane & 3) + {0, 1} for tokens lane / 4 + {0, 8}; o[i] is elements 16 i + lane / 4 + {0, 8}.
+template <int DK, int DV>
+__device__ __forceinline__ void warp_tile_few(uint32_t k_tile, uint32_t v_tile, int tb, int first, const uint32_t (&qf)[DK / 16][4], int n_ctx,
+                                              float scale_log2, float (&m)[2], float (&l)[2], float (&o)[DV / 8][4], int lane) {
+    const int mat = lane >> 3, r = lane & 7;
+    float s[2][4];  // two chains
+#pragma unroll
+    for (int k = 0; k < 4; k++) s[0][k] = s[1][k] = 0.f;
+#pragma unroll
+    for (int ks = 0; ks < DK / 16; ks++) {
+        uint32_t a[4];
+        ldsm_x4(a[0], a[1], a[2], a[3], k_tile + staged(tb + (mat & 1) * 8 + r, 2 * ks + (mat >> 1)));
+        mma_bf16(s[ks & 1], a, qf[ks][0], qf[ks][2]);
+    }
+    const int token = first + tb + (lane >> 2);
+    float x[4], mx[2];
+#pragma unroll
+    for (int k = 0; k < 4; k++) x[k] = token + 8 * (k >> 1) < n_ctx ? (s[0][k] + s[1][k]) * scale_log2 : -INFINITY;
+    float alpha[2];
+#pragma unroll
+    for (int h = 0; h < 2; h++) mx[h] = fmaxf(x[h], x[2 + h]);
+#pragma unroll
+    for (int off = 4; off <= 16; off *= 2)
+#pragma unroll
+        for (int h = 0; h < 2; h++) mx[h] = fmaxf(mx[h], __shfl_xor_sync(0xffffffffu, mx[h], off));
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+        const float mn = fmaxf(m[h], mx[h]);
+        alpha[h] = fast_exp2(m[h] - mn);
+        m[h] = mn;
+        x[h] = fast_exp2(x[h] - mn);
+        x[2 + h] = fast_exp2(x[2 + h] - mn);
+        l[h] = fmaf(l[h], alpha[h], x[h] + x[2 + h]);  // this lane's tokens only: summed at the end
+    }
+    if (__any_sync(0xffffffffu, alpha[0] != 1.f || alpha[1] != 1.f)) {
+#pragma unroll
+        for (int i = 0; i < DV / 16; i++)
+#pragma unroll
+            for (int k = 0; k < 4; k++) o[i][k] *= alpha[k & 1];
+    }
+    uint32_t hi[2], lo[2];
+#pragma unroll
+    for (int t = 0; t < 2; t++) {
+        split_bf16(x[2 * t], x[2 * t + 1], hi[t], lo[t]);
+        hi[t] = transpose_8x8(hi[t]);
+        lo[t] = transpose_8x8(lo[t]);
+    }
+#pragma unroll
+    for (int dt = 0; dt < DV / 16; dt++) {
+        uint32_t a[4];
+        ldsm_x4_trans(a[0], a[1], a[2], a[3], v_tile + staged(tb + (mat >> 1) * 8 + r, 2 * dt + (mat & 1)));
+        mma_bf16(o[dt], a, hi[0], hi[1]);
+        mma_bf16(o[dt], a, lo[0], lo[1]);
+    }
+}
+
 // BULK: chunks of 64 tokens whose tiles are exactly DK and DV wide are staged verbatim (the pool's layout is the staged one)
 // by 1-D TMA bulk copies of one thread.
-template <int DK, int DV, int STAGES, bool SPAN, bool BULK>
-__global__ void __launch_bounds__(R_THREADS) rows_mma_kernel(const RowsParams p) {
+// FEW: no item has more than 8 rows.
+template <int DK, int DV, int STAGES, bool SPAN, bool BULK, bool FEW>
+__global__ void __launch_bounds__(R_THREADS, BULK && STAGES == 2 ? 3 : 1) rows_mma_kernel(const RowsParams p) {
     extern __shared__ __align__(1024) uint8_t smem[];
     constexpr int K_BYTES = R_TILE * DK * 2, STAGE_BYTES = R_TILE * (DK + DV) * 2;
     const uint32_t sbase = smem_u32(smem);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int G = p.geo.n_heads, group = p.group, H = G * group, C = p.geo.chunk_size;
+    if (!SPAN) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");  // the merge kernel may be set up; it waits for this one's end
 
     // ---- the block of rows and its chunks
     int kvh, token0, n_rows, n_ctx, slot_base = 0, row_lo = 0;
@@ -164,7 +232,7 @@ __global__ void __launch_bounds__(R_THREADS) rows_mma_kernel(const RowsParams p)
     const int splits = n_rows <= 16 ? 4 : (n_rows <= 32 ? 2 : 1);
     const int my_m = splits == 4 ? 0 : (splits == 2 ? (warp & 1) : warp);      // 16-row tile of this warp
     const int my_s = splits == 4 ? warp : (splits == 2 ? (warp >> 1) : 0);     // its share of the tokens
-    const bool busy = my_m * 16 < n_rows;
+    const bool busy = my_m * 16 < n_rows, few = FEW || (!SPAN && n_rows <= 8);
 
     // ---- staging
     const int gpr = p.geo.gpr, v_gpr = p.geo.v_gpr;
@@ -295,7 +363,8 @@ __global__ void __launch_bounds__(R_THREADS) rows_mma_kernel(const RowsParams p)
         }
         const uint32_t kt = sbase + (j % STAGES) * STAGE_BYTES, vt = kt + K_BYTES;
         if (!busy) continue;
-        if (splits == 4) warp_tile<DK, DV, 1>(kt, vt, my_s * 16, j * R_TILE, qf, limit, p.scale_log2, m, l, o, lane);
+        if (few) warp_tile_few<DK, DV>(kt, vt, my_s * 16, j * R_TILE, qf, n_ctx, p.scale_log2, m, l, o, lane);
+        else if (splits == 4) warp_tile<DK, DV, 1>(kt, vt, my_s * 16, j * R_TILE, qf, limit, p.scale_log2, m, l, o, lane);
         else if (splits == 2) warp_tile<DK, DV, 2>(kt, vt, my_s * 32, j * R_TILE, qf, limit, p.scale_log2, m, l, o, lane);
         else warp_tile<DK, DV, 4>(kt, vt, 0, j * R_TILE, qf, limit, p.scale_log2, m, l, o, lane);
     }
@@ -306,15 +375,29 @@ __global__ void __launch_bounds__(R_THREADS) rows_mma_kernel(const RowsParams p)
     constexpr int PITCH = DV + 4;
     float* stage = reinterpret_cast<float*>(smem);                  // [4 warps][16 rows][PITCH]
     float2* ml = reinterpret_cast<float2*>(stage + 4 * 16 * PITCH); // [4 warps][16 rows]
+    if (few) {
 #pragma unroll
-    for (int h = 0; h < 2; h++) {
-        l[h] += __shfl_xor_sync(0xffffffffu, l[h], 1);
-        l[h] += __shfl_xor_sync(0xffffffffu, l[h], 2);
-        const int r = warp * 16 + (lane >> 2) + 8 * h;
-        if ((lane & 3) == 0) ml[r] = make_float2(m[h], l[h]);
+        for (int h = 0; h < 2; h++) {
+            for (int off = 4; off <= 16; off *= 2) l[h] += __shfl_xor_sync(0xffffffffu, l[h], off);
+            const int r = warp * 16 + 2 * (lane & 3) + h;
+            if (lane < 4) ml[r] = make_float2(m[h], l[h]);
 #pragma unroll
-        for (int i = 0; i < DV / 8; i++)
-            *reinterpret_cast<float2*>(stage + r * PITCH + 8 * i + (lane & 3) * 2) = make_float2(o[i][2 * h], o[i][2 * h + 1]);
+            for (int i = 0; i < DV / 16; i++) {
+                stage[r * PITCH + 16 * i + (lane >> 2)] = o[i][h];
+                stage[r * PITCH + 16 * i + (lane >> 2) + 8] = o[i][2 + h];
+            }
+        }
+    } else {
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            l[h] += __shfl_xor_sync(0xffffffffu, l[h], 1);
+            l[h] += __shfl_xor_sync(0xffffffffu, l[h], 2);
+            const int r = warp * 16 + (lane >> 2) + 8 * h;
+            if ((lane & 3) == 0) ml[r] = make_float2(m[h], l[h]);
+#pragma unroll
+            for (int i = 0; i < DV / 8; i++)
+                *reinterpret_cast<float2*>(stage + r * PITCH + 8 * i + (lane & 3) * 2) = make_float2(o[i][2 * h], o[i][2 * h + 1]);
+        }
     }
     __syncthreads();
     const int m_step = splits == 1 ? 0 : (splits == 2 ? 32 : 16);  // rows between the splits of one row
@@ -378,6 +461,7 @@ __global__ void __launch_bounds__(256) rows_merge_kernel(const RowsParams p) {
     if (pair >= p.n_rows * H) return;
     const int row = pair / H, head = pair % H;
     const int b = p.merge_off[row], n = p.merge_off[row + 1] - b;
+    asm volatile("griddepcontrol.wait;" ::: "memory");  // what comes before is not written by the kernel before this one
     float M = p.sink ? 0.f : R_NEG_BIG;
     for (int i = lane; i < n; i += 32) M = fmaxf(M, p.part_ml[(size_t)p.merge_slots[b + i] * H + head].x);
     M = warp_max(M);
@@ -439,29 +523,47 @@ __global__ void __launch_bounds__(256) rows_merge_kernel(const RowsParams p) {
     }
 }
 
+// set up while the items' kernel, which allows it, still runs
+cudaError_t launch_merge(const RowsParams& p, cudaStream_t stream) {
+    const int64_t pairs = (int64_t)p.n_rows * p.geo.n_heads * p.group;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)((pairs + 7) / 8));
+    cfg.blockDim = dim3(256);
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    auto* k = p.part_width <= 64 ? rows_merge_kernel<1> : (p.part_width <= 128 ? rows_merge_kernel<2> : rows_merge_kernel<4>);
+    cudaError_t e = cudaLaunchKernelEx(&cfg, k, p);
+    if (e != cudaSuccess && cfg.numAttrs == 1) {
+        (void)cudaGetLastError();
+        cfg.numAttrs = 0;
+        e = cudaLaunchKernelEx(&cfg, k, p);
+    }
+    return e;
+}
+
 template <int DK, int DV, int STAGES, bool BULK>
 cudaError_t launch(const RowsParams& p, cudaStream_t stream) {
-    constexpr int ring = STAGES * R_TILE * (DK + DV) * 2 + (BULK ? STAGES * 8 : 0), out = 4 * 16 * (DV + 4) * 4 + 64 * 8;
-    constexpr int smem = ring > out ? ring : out;
-    auto* span = rows_mma_kernel<DK, DV, STAGES, true, BULK>;
-    auto* items = rows_mma_kernel<DK, DV, STAGES, false, BULK>;
-    auto* k = p.blocks ? span : items;
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return e;
-    if (p.blocks) {
-        k<<<dim3(p.n_blocks * p.subs, p.geo.n_heads), R_THREADS, smem, stream>>>(p);
-    } else {
-        // an item has up to ITEM_ROWS query rows except when one token's group alone has more
-        k<<<dim3(p.n_items * p.geo.n_heads, p.subs), R_THREADS, smem, stream>>>(p);
-        e = cudaGetLastError();
+    auto launch_it = [&](auto* k, int stages, dim3 grid) {
+        const int ring = stages * R_TILE * (DK + DV) * 2 + (BULK ? stages * 8 : 0), out = 4 * 16 * (DV + 4) * 4 + 64 * 8;
+        const int smem = std::max(ring, out);
+        cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
         if (e != cudaSuccess) return e;
-        const int64_t pairs = (int64_t)p.n_rows * p.geo.n_heads * p.group;
-        const unsigned grid = (unsigned)((pairs + 7) / 8);
-        if (p.part_width <= 64) rows_merge_kernel<1><<<grid, 256, 0, stream>>>(p);
-        else if (p.part_width <= 128) rows_merge_kernel<2><<<grid, 256, 0, stream>>>(p);
-        else rows_merge_kernel<4><<<grid, 256, 0, stream>>>(p);
-    }
-    return cudaGetLastError();
+        k<<<grid, R_THREADS, smem, stream>>>(p);
+        return cudaGetLastError();
+    };
+    if (p.blocks) return launch_it(rows_mma_kernel<DK, DV, STAGES, true, BULK, false>, STAGES, dim3(p.n_blocks * p.subs, p.geo.n_heads));
+    // an item has up to ITEM_ROWS query rows except when one token's group alone has more
+    const dim3 grid(p.n_items * p.geo.n_heads, p.subs);
+    // Few rows: 64 KiB of ring and three CTAs an SM instead of 96 KiB and two, the same bytes in flight and half as many warps more
+    // (with 16-row tiles that alone was 44.8 -> 41.7 us, but spilled registers); narrower heads fit three CTAs as they are.
+    constexpr int FEW_STAGES = BULK && DK + DV == 256 ? 2 : STAGES;
+    const cudaError_t e = p.item_rows <= 8 ? launch_it(rows_mma_kernel<DK, DV, FEW_STAGES, false, BULK, true>, FEW_STAGES, grid)
+                                           : launch_it(rows_mma_kernel<DK, DV, STAGES, false, BULK, false>, STAGES, grid);
+    return e != cudaSuccess ? e : launch_merge(p, stream);
 }
 
 }  // namespace

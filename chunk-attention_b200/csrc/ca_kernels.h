@@ -175,6 +175,7 @@ struct RowsParams {
     // decode: the planner's items
     const int4* items;
     int n_items;
+    int item_rows;               // most query rows (tokens x heads of a group) of an item
     int delta_tokens;
     float* part_o;               // [slots][part_width]
     float2* part_ml;             // [slots]

@@ -68,6 +68,30 @@ def test_stored_heads_of_more_tokens_than_ctas(shape, dtype, lens):
     assert cache.device_status() == 0
 
 
+@pytest.mark.parametrize("shape", [(2, 2, 128, 128), (8, 1, 64, 64), (6, 2, 128, 64), (4, 2, 80, 48), (16, 2, 256, 256), (9, 1, 64, 128)])
+@pytest.mark.parametrize("chunk", [64, 16])
+def test_decoded_rows_of_small_groups(shape, chunk):
+    # Items of at most 8 rows (groups of 1 to 8) and of 9, whose tokens end on every side of the 16 that a warp takes; tiles staged
+    # verbatim and granule by granule.
+    import chunk_attn
+    H, G, dk, dv = shape
+    lens = [1, 2, 15, 16, 17, 31, 33, 48, 63, 64, 65, 80, 127, 128, 700]
+    g = torch.Generator().manual_seed(H + dk)
+    cache = chunk_attn.Attention.shaped(n_heads=H, n_kv_heads=G, d_key=dk, d_value=dv, scale=dk ** -0.5, sink=False, chunk_size=chunk, memory_mb=64,
+                                        dtype=torch.bfloat16, device="cuda:0")
+    kv = []
+    for i, n in enumerate(lens):
+        k, v = torch.randn(n, G, dk, generator=g).bfloat16(), torch.randn(n, G, dv, generator=g).bfloat16()
+        cache.add_seq(tokens=[10_000 * i + t for t in range(n)], k=k.cuda(), v=v.cuda())
+        kv.append((k.repeat_interleave(H // G, 1), v.repeat_interleave(H // G, 1)))
+    q = torch.randn(len(lens), H, dk, generator=g).bfloat16()
+    o = cache.forward_rows(q.cuda(), torch.tensor([n - 1 for n in lens], dtype=torch.int32, device="cuda:0"))
+    want = dense(q, kv, dk ** -0.5)
+    # the result's rounding to bf16 (2^-9 of it) and that of the weights (2^-17): far below this
+    assert (o.cpu().double() - want).abs().max() < 8e-3 * max(1.0, float(want.abs().max()))
+    assert cache.device_status() == 0
+
+
 @pytest.mark.parametrize("n,H", [(64, 8), (310, 16)])
 @pytest.mark.parametrize("shared", [0, 256])
 def test_short_tails_walked_by_half_warps(n, H, shared):
