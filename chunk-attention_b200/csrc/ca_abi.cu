@@ -726,6 +726,8 @@ bool device_view_of_host(const void* host_ptr, void** dev_ptr) {
 }
 }  // namespace
 
+static constexpr int64_t kEngineMaxBytes = 64 << 10;
+
 int ca_attention_host(ca_context* c, const void* q_host, void* out_host, int n_seqs, int partition, ca_stream stream_) {
     if (!c) return fail(CA_ERR_INVALID, "context is null");
     if (!c->valid) return fail(CA_ERR_STATE, "work list is stale: call ca_refresh_kernel_context first");
@@ -755,9 +757,9 @@ int ca_attention_host(ca_context* c, const void* q_host, void* out_host, int n_s
     };
     // queries: one copy into device memory (every item re-reads its rows, so they must not stay
     // behind the bus); a pageable source goes through a pinned stand-in first
-    void* unused = nullptr;
+    void* q_dev = nullptr;
     const void* q_src = q_host;
-    if (!device_view_of_host(q_host, &unused)) {
+    if (!device_view_of_host(q_host, &q_dev)) {
         CA_CUDA(grow_host(c->host_q_stage, c->host_q_cap));
         std::memcpy(c->host_q_stage, q_host, bytes);
         q_src = c->host_q_stage;

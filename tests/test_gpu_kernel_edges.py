@@ -119,3 +119,17 @@ def test_short_tails_walked_by_half_warps(n, H, shared):
     eng.append_token([5] * n, k1, v1)
     kv = [(torch.cat([k, a[None]]), torch.cat([v, b[None]])) for (k, v), a, b in zip(kv, k1, v1)]
     check()
+
+
+def test_queries_from_host_memory_of_any_alignment():
+    # by a kernel (page-locked and aligned, one CTA or several, a part of one), and by the copy engine (an odd address)
+    import chunk_attn
+    for n, H in ((1, 1), (3, 32), (70, 32)):
+        attn = chunk_attn.Attention(n_heads=H, d_head=128, chunk_size=64, memory_mb=64, dtype=torch.float16, device="cuda:0")
+        for i in range(n):
+            k = torch.randn(5 + i % 3, H, 128).half().cuda()
+            attn.add_seq(tokens=[1000 * i + j for j in range(k.shape[0])], k=k, v=-k)
+        room = torch.randn(n * H * 128 + 8).half().pin_memory()
+        for at in (0, 4):
+            q = room[at:at + n * H * 128].view(n, H, 128)
+            assert torch.equal(attn.forward_host(q=q), attn.forward(q=q.cuda()).cpu())
