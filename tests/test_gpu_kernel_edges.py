@@ -122,10 +122,10 @@ def test_short_tails_walked_by_half_warps(n, H, shared):
 
 
 def test_queries_from_host_memory_of_any_alignment():
-    # by a kernel (page-locked and aligned, one CTA or several, a part of one), and by the copy engine (an odd address)
+    # by the copy engine (small batches, an odd address) and by a kernel (page-locked and aligned; a last CTA that is nearly empty)
     import chunk_attn
-    for n, H in ((1, 1), (3, 32), (70, 32)):
-        attn = chunk_attn.Attention(n_heads=H, d_head=128, chunk_size=64, memory_mb=64, dtype=torch.float16, device="cuda:0")
+    for n, H in ((1, 1), (3, 32), (8, 32), (33, 8), (129, 31)):
+        attn = chunk_attn.Attention(n_heads=H, d_head=128, chunk_size=64, memory_mb=256, dtype=torch.float16, device="cuda:0")
         for i in range(n):
             k = torch.randn(5 + i % 3, H, 128).half().cuda()
             attn.add_seq(tokens=[1000 * i + j for j in range(k.shape[0])], k=k, v=-k)
