@@ -1036,7 +1036,7 @@ int ca_attention_rows(ca_context* c, const ca_rows_args* a, ca_stream stream_) {
             t.blocks = a->blocks;
             t.n_blocks = a->n_blocks;
             t.n_tokens = a->n_rows;
-            t.block_tokens = a->block_rows;
+            t.block_tokens = std::max(1, 128 / c->group);  // no block that this kernel takes has more
             t.path_off = a->path_off;
             t.path_chunks = a->path_chunks;
             t.max_chunks = (int)c->max_chunks;

@@ -300,6 +300,7 @@ struct SpanAttnParams {
     const float* value_freq;
     const int32_t* blocks;       // [n_blocks][4]: span, first token, end token, 0
     int n_blocks;
+    int n_tokens, block_tokens;   // in all; at most in a block
     const int32_t* path_off;
     const int32_t* path_chunks;
     int max_chunks;

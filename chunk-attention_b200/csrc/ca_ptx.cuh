@@ -67,6 +67,12 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const void* map, int x
         "l"(map), "r"(x), "r"(y), "r"(bar)
         : "memory");
 }
+__device__ __forceinline__ void tma_load_3d(uint32_t dst, const void* map, int x, int y, int z, uint32_t bar) {
+    asm volatile(
+        "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(dst),
+        "l"(map), "r"(x), "r"(y), "r"(z), "r"(bar)
+        : "memory");
+}
 __device__ __forceinline__ void ldsm_x4(uint32_t& r0, uint32_t& r1, uint32_t& r2, uint32_t& r3, uint32_t addr) {
     asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
                  : "=r"(r0), "=r"(r1), "=r"(r2), "=r"(r3)
@@ -115,6 +121,27 @@ __device__ __forceinline__ uint32_t pack_half2(float lo, float hi) {
     return *reinterpret_cast<const uint32_t*>(&h);
 }
 
+
+// ---- cluster launch control: a running block takes over blocks of its grid that have not started
+// Ask for a block of this grid that has not started; 16 bytes of answer arrive on the barrier
+__device__ __forceinline__ void clc_try_cancel(uint32_t answer, uint32_t bar) {
+    asm volatile("clusterlaunchcontrol.try_cancel.async.shared::cta.mbarrier::complete_tx::bytes.b128 [%0], [%1];" ::"r"(answer), "r"(bar) : "memory");
+}
+// The block that was taken over, or -1
+__device__ __forceinline__ int clc_block(uint32_t answer) {
+    uint32_t got, x = 0;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t.reg .b128 r;\n\t"
+        "ld.shared.b128 r, [%2];\n\t"
+        "clusterlaunchcontrol.query_cancel.is_canceled.pred.b128 p, r;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t"
+        "mov.u32 %1, 0;\n\t"
+        "@p clusterlaunchcontrol.query_cancel.get_first_ctaid::x.b32.b128 %1, r;\n\t}"
+        : "=r"(got), "=r"(x)
+        : "r"(answer)
+        : "memory");
+    return got ? (int)x : -1;
+}
 
 // ---- tcgen05: tensor memory and the 5th-generation tensor cores ---------------------------------------------------
 // Tensor memory (TMEM) is 128 lanes x 512 columns of 32 bits per SM.  A TMEM address is (lane << 16) | column.

@@ -68,6 +68,35 @@ def test_stored_heads_of_more_tokens_than_ctas(shape, dtype, lens):
     assert cache.device_status() == 0
 
 
+@pytest.mark.parametrize("shape", [(2, 2, 64, 64), (6, 2, 128, 64), (32, 8, 128, 128), (128, 1, 64, 128)])
+@pytest.mark.parametrize("sign", [1, -1])
+@pytest.mark.parametrize("lens", [[1, 63, 64, 65, 129, 300], [40] * 80, [1] * 40])
+def test_prompts_in_pieces(shape, sign, lens):
+    # Portions on tcgen05: 1, 3, 4 and 128 query heads to a key/value head (blocks of 128, 126 and 128 rows of 128, 42, 32 and 1 tokens;
+    # angles shared by a token's rows or not), pieces of one tile, last tiles of 1 token to all of them, more pieces than CTAs, a
+    # negative scale.  What one sequence's values are must not reach another: the last one's are infinite.
+    import chunk_attn
+    import gagorax_oracle as oracle
+    from chunk_attn import SpanBatch
+    from test_gpu_block_ops import close, oracle_attention, rnd
+    H, G, dk, dv = shape
+    eps, base, scale, dev = 1e-4, 1000.0, sign * dk ** -0.5, torch.device("cuda:0")
+    cache = chunk_attn.Attention.shaped(n_heads=H, n_kv_heads=G, d_key=dk, d_value=dv, scale=scale, sink=True, chunk_size=64, memory_mb=64,
+                                        dtype=torch.bfloat16, device=dev)
+    freq = lambda n: torch.from_numpy(oracle.pair_frequencies(n, base)).float().to(dev)
+    qn, kn = rnd(1, dk) * 0.2 + 1, rnd(2, dk) * 0.2 + 1
+    x = rnd(3, sum(lens), (H + G) * dk + G * dv).to(torch.bfloat16)
+    x[-lens[-1]:, (H + G) * dk:] = float("inf")
+    tokens = [[10_000 * i + t for t in range(n)] for i, n in enumerate(lens)]
+    cache.extend([-1] * len(lens), tokens)
+    spans = SpanBatch(tokens, [0] * len(lens), list(range(len(lens))), dev)
+    q = cache.store_qkv(x.to(dev), spans.positions, qn.to(dev), kn.to(dev), eps, 32, freq(32), freq(dv))
+    o = cache.forward_rows(q, spans.positions, freq(dv), spans.entry_of).split(lens)
+    for xs, part in list(zip(x.split(lens), o))[:-1]:
+        close(part, oracle_attention(xs.double().numpy(), shape + (32,), qn.double().numpy(), kn.double().numpy(), eps, base, scale), torch.bfloat16)
+    assert cache.device_status() == 0
+
+
 @pytest.mark.parametrize("shape", [(2, 2, 128, 128), (8, 1, 64, 64), (6, 2, 128, 64), (4, 2, 80, 48), (16, 2, 256, 256), (9, 1, 64, 128)])
 @pytest.mark.parametrize("chunk", [64, 16])
 def test_decoded_rows_of_small_groups(shape, chunk):
