@@ -23,6 +23,8 @@
 
 #include "ca_kernels.h"
 #include "ca_ptx.cuh"
+#include "ca_softmax.cuh"
+#include "ca_tensor_map.h"
 #include "ca_types.cuh"
 
 namespace ca {
@@ -70,7 +72,8 @@ __global__ void __launch_bounds__(E_THREADS, 1) latent_span_kernel(const LatentS
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + Z::BODY + Z::NUM_BARS * 8);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int H = p.n_heads, head = blockIdx.x % H;
-    const int4 blk = __ldg(reinterpret_cast<const int4*>(p.blocks) + blockIdx.x / H);
+    // the last blocks of a portion see the most keys: they go first
+    const int4 blk = __ldg(reinterpret_cast<const int4*>(p.blocks) + (p.n_blocks - 1 - blockIdx.x / H));
     const int token0 = blk.y, n_tok = blk.z - blk.y;
     const int pos0 = __ldg(p.positions + token0);           // the block's tokens are consecutive positions
     const int first = __ldg(p.first + blk.x), base = __ldg(p.base + blk.x);
@@ -84,6 +87,28 @@ __global__ void __launch_bounds__(E_THREADS, 1) latent_span_kernel(const LatentS
     const int lo0 = tile_lo(0), hi0 = tile_hi(0);
     const int lo1 = group_rows(1) > 0 ? tile_lo(1) : 0, hi1 = tile_hi(1);
     const int n_tiles = max(hi0, hi1);
+
+    // The groups' queries, unrotated part as it comes, are on their way before the CTA is set up: K-major lines of 128 bytes, swizzled,
+    // eight lanes to a line; zeros past the block's rows and the head's width.  Loaded a batch after the other and held in registers they
+    // took 8 of a CTA's 70 thousand cycles (18 tiles), the rotated part, now requested ahead into L2, another 5: 16 prompts of 256 tokens,
+    // 32 heads of 128 + 64, 67.7 -> 59.4 us.
+    if (warp < 4 * E_GROUPS && group_rows(warp >> 2) > 0) {
+        const int g = warp >> 2, r = threadIdx.x & (E_ROWS - 1), n_rows = group_rows(g), width = p.dim + p.rot, gran = r & 7;
+        const uint32_t q_base = sbase + g * Z::Q_BYTES;
+        const __nv_bfloat16* const q = static_cast<const __nv_bfloat16*>(p.q) + ((size_t)(token0 + g * E_ROWS) * H + head) * width;
+        const size_t pitch = (size_t)H * width;
+#pragma unroll 2
+        for (int row = r >> 3; row < E_ROWS; row += E_ROWS / 8)
+            for (int c = 8 * gran; c < ((p.dim + 63) & ~63); c += 64) {
+                const bool on = row < n_rows && c < p.dim;
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(q_base + (c >> 6) * Z::Q_PANEL + row * 128 + ((gran ^ (row & 7)) << 4)),
+                             "l"(on ? q + row * pitch + c : q), "r"(on ? 16 : 0)
+                             : "memory");
+            }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        if (r < n_rows)
+            for (int c = 0; c < p.rot; c += 64) asm volatile("prefetch.global.L2 [%0];" ::"l"(q + r * pitch + p.dim + c));
+    }
 
     if (threadIdx.x == 0) {
         for (int i = 0; i < Z::STAGES; i++) {
@@ -217,43 +242,55 @@ __global__ void __launch_bounds__(E_THREADS, 1) latent_span_kernel(const LatentS
         const uint32_t q_base = sbase + g * Z::Q_BYTES;
         if (n_rows > 0) {
             const int tok = token0 + g * E_ROWS, gpos = pos0 + g * E_ROWS;  // the group's first token and its position
-            // ---- queries -> shared memory, K-major 128-byte-swizzled: the unrotated part as it comes, the rotated part
-            // turned by the token's position, zeros elsewhere
+            // ---- the rotated part of the queries, turned by the token's position, zeros behind it
             const int d_panels = (p.dim + 63) >> 6, width = p.dim + p.rot, half = p.rot / 2;
             const __nv_bfloat16* q = static_cast<const __nv_bfloat16*>(p.q);
             auto line = [&](int row, int gran) { return q_base + (gran >> 3) * Z::Q_PANEL + row * 128 + (((gran & 7) ^ (row & 7)) << 4); };
-            for (int i = r; i < E_ROWS * d_panels * 8; i += E_ROWS) {
-                const int row = i / (d_panels * 8), gr = i % (d_panels * 8);
-                uint4 v = make_uint4(0u, 0u, 0u, 0u);
-                if (row < n_rows && 8 * gr < p.dim)
-                    v = __ldg(reinterpret_cast<const uint4*>(q + ((size_t)(tok + row) * H + head) * width) + gr);
-                sts128(line(row, gr), (int)v.x, (int)v.y, (int)v.z, (int)v.w);
-            }
             const int rot_lines = (KP - d_panels) * 8;
             if (half % 8 == 0) {  // a unit is a granule of the first half and its partner in the second
                 const int units = half / 8, tail = rot_lines - 2 * units;
-                for (int i = r; i < E_ROWS * units; i += E_ROWS) {
-                    const int row = i / units, u = i % units;
-                    uint4 a = make_uint4(0u, 0u, 0u, 0u), b = a;
-                    if (row < n_rows) {
-                        const uint4* src = reinterpret_cast<const uint4*>(q + ((size_t)(tok + row) * H + head) * width + p.dim);
-                        a = __ldg(src + u);
-                        b = __ldg(src + units + u);
-                        const float pos = (float)(gpos + row);
-                        uint32_t* aw = reinterpret_cast<uint32_t*>(&a);
-                        uint32_t* bw = reinterpret_cast<uint32_t*>(&b);
+                int shift = 0;  // 2^shift lanes to a row: a lane keeps its unit, and the unit's frequencies
+                while ((1 << shift) < units) shift++;
+                const int u = r & ((1 << shift) - 1);
+                if (u < units) {
+                    float f[8];
 #pragma unroll
-                        for (int k = 0; k < 4; k++) {
-                            const float2 x = unpack_bf16(aw[k]), y = unpack_bf16(bw[k]);
-                            float s0, c0, s1, c1;
-                            fast_sincos(pos * __ldg(p.freq + 8 * u + 2 * k), &s0, &c0);
-                            fast_sincos(pos * __ldg(p.freq + 8 * u + 2 * k + 1), &s1, &c1);
-                            aw[k] = pack_bf16(x.x * c0 - y.x * s0, x.y * c1 - y.y * s1);
-                            bw[k] = pack_bf16(y.x * c0 + x.x * s0, y.y * c1 + x.y * s1);
+                    for (int k = 0; k < 8; k++) f[k] = __ldg(p.freq + 8 * u + k);
+                    constexpr int AHEAD = 4;  // rows whose loads are in flight together
+                    const int row_step = E_ROWS >> shift;
+#pragma unroll 1
+                    for (int row0 = r >> shift; row0 < E_ROWS; row0 += AHEAD * row_step) {
+                        uint4 a[AHEAD], b[AHEAD];
+#pragma unroll
+                        for (int j = 0; j < AHEAD; j++) {
+                            const int row = row0 + j * row_step;
+                            a[j] = b[j] = make_uint4(0u, 0u, 0u, 0u);
+                            if (row < n_rows) {
+                                const uint4* src = reinterpret_cast<const uint4*>(q + ((size_t)(tok + row) * H + head) * width + p.dim);
+                                a[j] = __ldg(src + u);
+                                b[j] = __ldg(src + units + u);
+                            }
+                        }
+#pragma unroll
+                        for (int j = 0; j < AHEAD; j++) {
+                            const int row = row0 + j * row_step;
+                            if (row >= E_ROWS) break;
+                            const float pos = (float)(gpos + row);
+                            uint32_t* aw = reinterpret_cast<uint32_t*>(&a[j]);
+                            uint32_t* bw = reinterpret_cast<uint32_t*>(&b[j]);
+#pragma unroll
+                            for (int k = 0; k < 4; k++) {
+                                const float2 x = unpack_bf16(aw[k]), y = unpack_bf16(bw[k]);
+                                float s0, c0, s1, c1;
+                                fast_sincos(pos * f[2 * k], &s0, &c0);
+                                fast_sincos(pos * f[2 * k + 1], &s1, &c1);
+                                aw[k] = pack_bf16(x.x * c0 - y.x * s0, x.y * c1 - y.y * s1);
+                                bw[k] = pack_bf16(y.x * c0 + x.x * s0, y.y * c1 + x.y * s1);
+                            }
+                            sts128(line(row, d_panels * 8 + u), (int)a[j].x, (int)a[j].y, (int)a[j].z, (int)a[j].w);
+                            sts128(line(row, d_panels * 8 + units + u), (int)b[j].x, (int)b[j].y, (int)b[j].z, (int)b[j].w);
                         }
                     }
-                    sts128(line(row, d_panels * 8 + u), (int)a.x, (int)a.y, (int)a.z, (int)a.w);
-                    sts128(line(row, d_panels * 8 + units + u), (int)b.x, (int)b.y, (int)b.z, (int)b.w);
                 }
                 for (int i = r; i < E_ROWS * tail; i += E_ROWS) sts128_zero(line(i / tail, d_panels * 8 + 2 * units + i % tail));
             } else {
@@ -275,6 +312,7 @@ __global__ void __launch_bounds__(E_THREADS, 1) latent_span_kernel(const LatentS
                     sts128(line(row, d_panels * 8 + gr), (int)pack_bf16(x[0], x[1]), (int)pack_bf16(x[2], x[3]), (int)pack_bf16(x[4], x[5]), (int)pack_bf16(x[6], x[7]));
                 }
             }
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
             fence_proxy_async();
             mbar_arrive(q_ready + 8 * g);
 
@@ -312,9 +350,7 @@ __global__ void __launch_bounds__(E_THREADS, 1) latent_span_kernel(const LatentS
                 float alpha = 1.f;
                 bool rescale = false;
                 {
-                    float mx = fmaxf(__uint_as_float(s0[0]), __uint_as_float(s1[0]));
-#pragma unroll
-                    for (int c = 1; c < 32; c++) mx = fmaxf(mx, fmaxf(__uint_as_float(s0[c]), __uint_as_float(s1[c])));
+                    float mx = tile_max(s0, s1);
                     mx = fmaxf(mx * scale, E_NEG_BIG);
                     if (i == 0) {
                         m_used = mx;
@@ -325,28 +361,12 @@ __global__ void __launch_bounds__(E_THREADS, 1) latent_span_kernel(const LatentS
                         rescale = true;
                     }
                 }
-                float sum = 0.f;
-#pragma unroll
-                for (int c = 0; c < 32; c++) {
-                    s0[c] = __float_as_uint(fast_exp2(fmaf(__uint_as_float(s0[c]), scale, -m_used)));
-                    s1[c] = __float_as_uint(fast_exp2(fmaf(__uint_as_float(s1[c]), scale, -m_used)));
-                    sum += __uint_as_float(s0[c]) + __uint_as_float(s1[c]);
-                }
-                l += sum;
-                uint32_t pk[32];
-#pragma unroll
-                for (int c = 0; c < 16; c++) {
-                    pk[c] = pack_bf16(__uint_as_float(s0[2 * c]), __uint_as_float(s0[2 * c + 1]));
-                    pk[16 + c] = pack_bf16(__uint_as_float(s1[2 * c]), __uint_as_float(s1[2 * c + 1]));
-                }
+                l += tile_weights(s0, s1, scale, m_used);
+                uint32_t pk[32], lo[32];
+                split_weights(s0, pk, lo);
+                split_weights(s1, pk + 16, lo + 16);
                 tmem_st32(lane_addr + E_COL_S + b * E_TOK, pk);
-#pragma unroll
-                for (int c = 0; c < 16; c++) {
-                    const float2 a = unpack_bf16(pk[c]), d = unpack_bf16(pk[16 + c]);
-                    pk[c] = pack_bf16(__uint_as_float(s0[2 * c]) - a.x, __uint_as_float(s0[2 * c + 1]) - a.y);
-                    pk[16 + c] = pack_bf16(__uint_as_float(s1[2 * c]) - d.x, __uint_as_float(s1[2 * c + 1]) - d.y);
-                }
-                tmem_st32(lane_addr + E_COL_S + b * E_TOK + 32, pk);
+                tmem_st32(lane_addr + E_COL_S + b * E_TOK + 32, lo);
                 if (i > 0) {
                     // O += P V of tile i - 1 is complete (every thread follows o_done phase by phase)
                     live = mbar_wait_bounded(my_o, (i - 1) & 1, p.wait_limit);
@@ -358,7 +378,7 @@ __global__ void __launch_bounds__(E_THREADS, 1) latent_span_kernel(const LatentS
                 }
                 if (__any_sync(0xffffffffu, rescale)) {
                     tc_fence_after_thread_sync();
-#pragma unroll
+#pragma unroll 1
                     for (int c = 0; c < 2 * VP; c++) {
                         uint32_t o[32];
                         tmem_ld32(lane_addr + c * 32, o);
@@ -390,7 +410,7 @@ __global__ void __launch_bounds__(E_THREADS, 1) latent_span_kernel(const LatentS
                     }
                     inv = total > 0.f ? fast_exp2(m_used - M) / total : 0.f;
                 }
-#pragma unroll
+#pragma unroll 1
                 for (int c = 0; c < 2 * VP; c++) {
                     uint32_t o[32];
                     tmem_ld32(lane_addr + c * 32, o);
@@ -402,11 +422,15 @@ __global__ void __launch_bounds__(E_THREADS, 1) latent_span_kernel(const LatentS
                 }
                 __syncwarp();
                 const int wr = (warp & 3) * 32, rows_here = min(32, n_rows - wr), grans = p.vdim >> 3;
-                __nv_bfloat16* out = static_cast<__nv_bfloat16*>(p.out);
-                for (int u = lane; u < rows_here * grans; u += 32) {
-                    const int row = wr + u / grans, gr = u % grans;
-                    const uint4 v = *reinterpret_cast<const uint4*>(q_smem + (line(row, gr) - q_base));
-                    *(reinterpret_cast<uint4*>(out + ((size_t)(tok + row) * H + head) * p.vdim) + gr) = v;
+                int shift = 0;  // 2^shift lanes to a row
+                while ((1 << shift) < grans) shift++;
+                const int gr = lane & ((1 << shift) - 1);
+                if (gr < grans) {
+                    uint4* out = reinterpret_cast<uint4*>(static_cast<__nv_bfloat16*>(p.out) + ((size_t)(tok + wr) * H + head) * p.vdim) + gr;
+                    const size_t pitch = (size_t)H * grans;
+#pragma unroll 4
+                    for (int rr = lane >> shift; rr < rows_here; rr += 32 >> shift)
+                        out[rr * pitch] = *reinterpret_cast<const uint4*>(q_smem + (line(wr + rr, gr) - q_base));
                 }
             }
         }
@@ -420,23 +444,9 @@ __global__ void __launch_bounds__(E_THREADS, 1) latent_span_kernel(const LatentS
     }
 }
 
-using EncodeTiled = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
-                                 const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-EncodeTiled encoder() {
-    static EncodeTiled fn = [] {
-        void* f = nullptr;
-        cudaDriverEntryPointQueryResult found;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &f, cudaEnableDefault, &found) != cudaSuccess || found != cudaDriverEntryPointSuccess)
-            f = nullptr;
-        return reinterpret_cast<EncodeTiled>(f);
-    }();
-    return fn;
-}
-
 // row-major bf16 [rows, cols] with `stride` elements between rows, in boxes of 64 x 64
 bool make_map(CUtensorMap* m, const void* data, int64_t rows, int64_t cols, int64_t stride) {
-    const EncodeTiled encode = encoder();
+    const TensorMapEncode encode = tensor_map_encoder();
     if (!encode) return false;
     const cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows}, strides[1] = {(cuuint64_t)stride * 2};
     const cuuint32_t box[2] = {64, E_TOK}, step[2] = {1, 1};
