@@ -559,7 +559,7 @@ cudaError_t launch(const RowsParams& p, cudaStream_t stream) {
     // an item has up to ITEM_ROWS query rows except when one token's group alone has more
     const dim3 grid(p.n_items * p.geo.n_heads, p.subs);
     // Few rows: 64 KiB of ring and three CTAs an SM instead of 96 KiB and two, the same bytes in flight and half as many warps more
-    // (with 16-row tiles that alone was 44.8 -> 41.7 us, but spilled registers); narrower heads fit three CTAs as they are.
+    // (with 16-row tiles that alone was 44.8 -> 41.7 us, but spilled registers); narrower heads keep their stages.
     constexpr int FEW_STAGES = BULK && DK + DV == 256 ? 2 : STAGES;
     const cudaError_t e = p.item_rows <= 8 ? launch_it(rows_mma_kernel<DK, DV, FEW_STAGES, false, BULK, true>, FEW_STAGES, grid)
                                            : launch_it(rows_mma_kernel<DK, DV, STAGES, false, BULK, false>, STAGES, grid);
