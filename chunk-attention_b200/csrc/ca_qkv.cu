@@ -108,8 +108,9 @@ __global__ void __launch_bounds__(QKV_WARPS * 32) store_qkv_kernel(const QkvPara
 // instructions (per granule a division, a square root, a reduction, two addresses and the weights) and by one dependent load after the
 // other: 8192 tokens of 32 + 8 + 8 heads of 128 took 77.6 us.  So a lane takes GP granules of a head, a CTA walks tokens with the next
 // pass's granules requested before the present ones are turned, a thread keeps its frequencies for all tokens, squares and weights go in
-// pairs of fp32, and 16-bit results take the hardware's reciprocal square root (relative error 2^-22): the same tokens take
-// 43.9 us (4.6 TB/s where a copy reaches 6.5).  A grid of 6 CTAs an SM: up to 888 tokens are one to a CTA.
+// pairs of fp32: the same tokens take 46.3 us (4.3 TB/s where a copy reaches 6.5).  Mean, root and reciprocal are the correctly rounded
+// ones for every type: the hardware's approximate ones take 45.1 us, but some 16-bit results then round the other way.  A grid of 6 CTAs
+// an SM: up to 888 tokens are one to a CTA.
 constexpr int QKV_VEC_THREADS = 128, QKV_VEC_CTAS = 6;
 
 __device__ __forceinline__ void widen(uint32_t v, float& lo, float& hi, __nv_bfloat16) {
@@ -129,8 +130,6 @@ __device__ __forceinline__ uint32_t narrow(float lo, float hi, __half) {
     const __half2 h = __floats2half2_rn(lo, hi);
     return *reinterpret_cast<const uint32_t*>(&h);
 }
-template <typename T> __device__ __forceinline__ float inverse_rms(float ss, float d, float eps) { return rsqrtf(__fdividef(ss, d) + eps); }
-template <> __device__ __forceinline__ float inverse_rms<float>(float ss, float d, float eps) { return 1.f / sqrtf(ss / d + eps); }
 
 template <typename T, int LANES, int GP>
 __global__ void __launch_bounds__(QKV_VEC_THREADS, QKV_VEC_CTAS) store_qkv_vec_kernel(const QkvParams p) {
@@ -234,7 +233,7 @@ __global__ void __launch_bounds__(QKV_VEC_THREADS, QKV_VEC_CTAS) store_qkv_vec_k
                 ss += ss_hi;
 #pragma unroll
                 for (int off = LANES >> 1; off >= 1; off >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, off);
-                const float inv = inverse_rms<T>(ss, (float)p.d_key, p.eps);
+                const float inv = 1.f / sqrtf(ss / (float)p.d_key + p.eps);
                 inv2 = pair_f32(inv, inv);
             }
             if (u >= units || (u >= H && chunk < 0)) continue;

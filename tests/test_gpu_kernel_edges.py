@@ -1,4 +1,5 @@
 """Kernels at the sizes where their tiles, splits and dispatch rules end, against dense attention in 64 bits."""
+import numpy as np
 import pytest
 import torch
 
@@ -162,3 +163,29 @@ def test_queries_from_host_memory_of_any_alignment():
         for at in (0, 4):
             q = room[at:at + n * H * 128].view(n, H, 128)
             assert torch.equal(attn.forward_host(q=q), attn.forward(q=q.cuda()).cpu())
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("shape", [(4, 2, 64, 64), (4, 2, 40, 48), (4, 2, 128, 128), (2, 1, 256, 64)])
+def test_head_norms_are_rounded_as_fp32_operations(dtype, shape):
+    # Whole numbers, whose squares add up exactly in any order: mean, root, reciprocal and weights, one fp32 rounding each, then the
+    # result's.  Every bit of it (an approximate root turns the rounding of some of the 16-bit results).
+    import chunk_attn
+    from chunk_attn import SpanBatch
+    H, G, dk, dv = shape
+    n, eps, dev = 700, 1e-5, torch.device("cuda:0")
+    g = torch.Generator().manual_seed(dk)
+    cache = chunk_attn.Attention.shaped(n_heads=H, n_kv_heads=G, d_key=dk, d_value=dv, scale=dk ** -0.5, sink=False, chunk_size=64, memory_mb=64,
+                                        dtype=dtype, device=dev)
+    x = torch.randint(-30, 31, (n, (H + G) * dk + G * dv), generator=g).float()
+    w = torch.randn(dk, generator=g) * 0.2 + 1
+    tokens = [list(range(n))]
+    cache.extend([-1], tokens)
+    spans = SpanBatch(tokens, [0], [0], dev)
+    q = cache.store_qkv(x.to(dev, dtype), spans.positions, w.to(dev), w.to(dev), eps, 0, None, None)
+    heads = x[:, :H * dk].view(n, H, dk).numpy()
+    mean = np.square(heads).sum(-1, keepdims=True) / np.float32(dk)
+    inv, w = np.float32(1) / np.sqrt(mean + np.float32(eps)), w.numpy()
+    want = heads * inv * w if dtype == torch.float32 and dk == 256 else heads * (inv * w)  # heads of more than 32 granules: weights last
+    assert want.dtype == np.float32
+    assert torch.equal(q.view(n, H, -1)[..., :dk].cpu(), torch.from_numpy(want).to(dtype))
