@@ -192,8 +192,17 @@ __device__ __forceinline__ void warp_tile_few(uint32_t k_tile, uint32_t v_tile, 
 // BULK: chunks of 64 tokens whose tiles are exactly DK and DV wide are staged verbatim (the pool's layout is the staged one)
 // by 1-D TMA bulk copies of one thread.
 // FEW: no item has more than 8 rows.
+//
+// CTAs of an SM that the registers leave room for: as many as the stages in shared memory do, and within that the compiler may use what
+// helps.  With a bound of 1 for all, 64-wide heads staged granule by granule took 187 registers (135 with no bound) and lost the third
+// CTA: 64 rows of 500 shared and 500 own tokens, 32 heads on 8 of 64, chunks of 32: 42.9 us with no bound, 49.6 with 1, 41.1 so; 8
+// prompts of 1000 tokens 290, 313, 273.  128-wide ones, 2 CTAs, 64 x 700 own tokens: 86.6 with no bound, 82.5 so.  Portions with keys
+// of 64 and values of 128 would spill too much for a third CTA (a prompt of 4000: 356 with no bound, 377 with 3, 317 with 1).
+constexpr int min_ctas(int dk, int dv, int stages, bool span) {
+    return span && dk < dv ? 1 : 233472 / (stages * R_TILE * (dk + dv) * 2 + stages * 8 + 1024);
+}
 template <int DK, int DV, int STAGES, bool SPAN, bool BULK, bool FEW>
-__global__ void __launch_bounds__(R_THREADS, BULK && STAGES == 2 ? 3 : 1) rows_mma_kernel(const RowsParams p) {
+__global__ void __launch_bounds__(R_THREADS, min_ctas(DK, DV, STAGES, SPAN)) rows_mma_kernel(const RowsParams p) {
     extern __shared__ __align__(1024) uint8_t smem[];
     constexpr int K_BYTES = R_TILE * DK * 2, STAGE_BYTES = R_TILE * (DK + DV) * 2;
     const uint32_t sbase = smem_u32(smem);
@@ -232,7 +241,9 @@ __global__ void __launch_bounds__(R_THREADS, BULK && STAGES == 2 ? 3 : 1) rows_m
     const int splits = n_rows <= 16 ? 4 : (n_rows <= 32 ? 2 : 1);
     const int my_m = splits == 4 ? 0 : (splits == 2 ? (warp & 1) : warp);      // 16-row tile of this warp
     const int my_s = splits == 4 ? warp : (splits == 2 ? (warp >> 1) : 0);     // its share of the tokens
-    const bool busy = my_m * 16 < n_rows, few = FEW || (!SPAN && n_rows <= 8);
+    // Small items between wide ones take the small tile too, but not beside the widest heads' other tiles, which spill as it is (76 bytes,
+    // 188 with it: 64 rows of 500 shared and 500 own tokens, 8 heads of 256: 166.5 us, 191.2 with it).
+    const bool busy = my_m * 16 < n_rows, few = FEW || (!SPAN && DK + DV < 512 && n_rows <= 8);
 
     // ---- staging
     const int gpr = p.geo.gpr, v_gpr = p.geo.v_gpr;
