@@ -726,8 +726,6 @@ bool device_view_of_host(const void* host_ptr, void** dev_ptr) {
 }
 }  // namespace
 
-static constexpr int64_t kEngineMaxBytes = 64 << 10;
-
 int ca_attention_host(ca_context* c, const void* q_host, void* out_host, int n_seqs, int partition, ca_stream stream_) {
     if (!c) return fail(CA_ERR_INVALID, "context is null");
     if (!c->valid) return fail(CA_ERR_STATE, "work list is stale: call ca_refresh_kernel_context first");
@@ -757,23 +755,17 @@ int ca_attention_host(ca_context* c, const void* q_host, void* out_host, int n_s
     };
     // queries: one copy into device memory (every item re-reads its rows, so they must not stay
     // behind the bus); a pageable source goes through a pinned stand-in first
-    void* q_dev = nullptr;
+    void* unused = nullptr;
     const void* q_src = q_host;
-    if (!device_view_of_host(q_host, &q_dev)) {
+    if (!device_view_of_host(q_host, &unused)) {
         CA_CUDA(grow_host(c->host_q_stage, c->host_q_cap));
         std::memcpy(c->host_q_stage, q_host, bytes);
         q_src = c->host_q_stage;
-        if (!device_view_of_host(c->host_q_stage, &q_dev)) q_dev = nullptr;
     }
-    // The driver sends up to 64 KiB along with the copy's command; above that the copy engine takes its turn, and a kernel brings the rows
-    // over the bus sooner, while the attention kernel sets itself up.  Whole calls, 32 heads, engine against kernel: 1 row (8 KiB) 21.0
-    // and 24.8 us, 8 rows 25.9 and 26.4, 32 rows 55.7 and 42.2, 128 rows 170 and 99, 512 rows (4 MiB) 558 and 334.
-    void* q_end = nullptr;
-    if (q_dev && (int64_t)bytes > kEngineMaxBytes && bytes % 16 == 0 && reinterpret_cast<uintptr_t>(q_dev) % 16 == 0 &&
-        device_view_of_host(static_cast<const char*>(q_src) + bytes - 1, &q_end) && q_end == static_cast<char*>(q_dev) + bytes - 1)
-        CA_CUDA(ca::launch_fetch_host(c->q_stage, q_dev, (int64_t)bytes, stream));
-    else
-        CA_CUDA(cudaMemcpyAsync(c->q_stage, q_src, bytes, cudaMemcpyHostToDevice, stream));
+    // By the copy engine: the driver checks the range of a copy, while a kernel that read past its page-locked part would fault.  What a
+    // kernel brings does not show from box to box (32 heads of 128, 1024 shared and 64 own tokens, two boxes: 32 rows 46.4 and 48.9 us a
+    // call, 47.2 and 45.5 by a kernel; 64 rows 69.2 and 68.8, 71.8 and 70.3; 128 rows 118.1 and 118.8, 120.2 and 118.4)
+    CA_CUDA(cudaMemcpyAsync(c->q_stage, q_src, bytes, cudaMemcpyHostToDevice, stream));
     // output: the last kernel stores its rows straight into the caller's page-locked buffer
     void* out_dev = nullptr;
     const bool direct = device_view_of_host(out_host, &out_dev) && reinterpret_cast<uintptr_t>(out_dev) % 16 == 0;

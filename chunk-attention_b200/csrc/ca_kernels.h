@@ -368,9 +368,6 @@ struct AppendParams {
 // vec16: rows are whole 16-byte granules and k, v are 16-byte aligned
 cudaError_t launch_append_kv(const AppendParams& p, bool vec16, cudaStream_t stream);
 
-// src: device address of page-locked host memory; both 16-byte aligned, bytes a multiple of 16
-cudaError_t launch_fetch_host(void* dst, const void* src, int64_t bytes, cudaStream_t stream);
-
 constexpr int SCATTER_MAX_CHUNKS = 512;
 struct ScatterParams {
     void* pool;

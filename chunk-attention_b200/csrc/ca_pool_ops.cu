@@ -128,20 +128,6 @@ __global__ void read_chunk_kernel(const ReadChunkParams p) {
 
 inline int blocks_for(int64_t total, int threads) { return (int)((total + threads - 1) / threads); }
 
-// Queries in page-locked host memory -> device memory, in 16-byte units, four a thread in flight together over the bus.
-constexpr int FETCH_THREADS = 128, FETCH_AHEAD = 4;
-__global__ void __launch_bounds__(FETCH_THREADS) fetch_host_kernel(uint4* dst, const uint4* src, int64_t n) {
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");  // the next kernel sets itself up; it waits for this one's end
-    const int64_t i0 = (int64_t)blockIdx.x * (FETCH_THREADS * FETCH_AHEAD) + threadIdx.x;
-    uint4 v[FETCH_AHEAD];
-#pragma unroll
-    for (int k = 0; k < FETCH_AHEAD; k++)
-        if (i0 + k * FETCH_THREADS < n) v[k] = src[i0 + k * FETCH_THREADS];
-#pragma unroll
-    for (int k = 0; k < FETCH_AHEAD; k++)
-        if (i0 + k * FETCH_THREADS < n) dst[i0 + k * FETCH_THREADS] = v[k];
-}
-
 }  // namespace
 
 cudaError_t launch_append_kv(const AppendParams& p, bool vec16, cudaStream_t stream) {
@@ -211,13 +197,6 @@ cudaError_t launch_read_chunk(const ReadChunkParams& p, cudaStream_t stream) {
     } else {
         read_chunk_kernel<uint32_t><<<grid, 256, 0, stream>>>(p);
     }
-    return cudaGetLastError();
-}
-
-cudaError_t launch_fetch_host(void* dst, const void* src, int64_t bytes, cudaStream_t stream) {
-    const int64_t n = bytes / 16, per_cta = FETCH_THREADS * FETCH_AHEAD;
-    if (n <= 0) return cudaSuccess;
-    fetch_host_kernel<<<(unsigned)((n + per_cta - 1) / per_cta), FETCH_THREADS, 0, stream>>>(static_cast<uint4*>(dst), static_cast<const uint4*>(src), n);
     return cudaGetLastError();
 }
 

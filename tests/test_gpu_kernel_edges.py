@@ -152,7 +152,7 @@ def test_short_tails_walked_by_half_warps(n, H, shared):
 
 
 def test_queries_from_host_memory_of_any_alignment():
-    # by the copy engine (small batches, an odd address) and by a kernel (page-locked and aligned; a last CTA that is nearly empty)
+    # from 256 bytes to a megabyte, from an address that is a multiple of 16 bytes and from one of 8
     import chunk_attn
     for n, H in ((1, 1), (3, 32), (8, 32), (33, 8), (129, 31)):
         attn = chunk_attn.Attention(n_heads=H, d_head=128, chunk_size=64, memory_mb=256, dtype=torch.float16, device="cuda:0")
