@@ -1034,6 +1034,7 @@ int ca_attention_rows(ca_context* c, const ca_rows_args* a, ca_stream stream_) {
             t.max_chunks = (int)c->max_chunks;
             t.status = c->status;
             t.wait_limit = c->opt_wait_limit;
+            t.withhold_item = c->opt_withhold_item;
             CA_CUDA(ca::launch_span_attn(t, c->geo.d_head, c->geo.d_value, stream));
             return CA_OK;
         }

@@ -59,6 +59,7 @@ struct alignas(16) Work {
     int tail;   // tokens of the last tile
     int open;   // tokens every row of the block sees
     int kvh;
+    int withheld;  // failure-path tests: the producer stops here
     const int32_t* list;
 };
 
@@ -154,6 +155,7 @@ __global__ void __launch_bounds__(A_THREADS, 2) span_attn_kernel(const SpanAttnP
                     w.tail = n_ctx - (w.n_tiles - 1) * A_TOK;
                     w.open = __ldg(p.positions + blk.y) + 1;
                     w.kvh = item % G;
+                    w.withheld = item == p.withhold_item;
                     w.list = p.path_chunks + __ldg(p.path_off + blk.x);
                 }
                 work[n & 1] = w;
@@ -162,7 +164,7 @@ __global__ void __launch_bounds__(A_THREADS, 2) span_attn_kernel(const SpanAttnP
             }
         } else if (warp == 4 && lane == 0) {
             // ---- producer: slot i & 3 takes K of tile i / 2 (even i) or its V (odd i), i counted over all pieces
-            int issued = 0, n = 0;
+            int issued = 0, q_issued = 0, n = 0;
             for (bool live = true; live; n++) {
                 if (!wait(work_full + 8 * (n & 1), (n >> 1) & 1, STATUS_FULL_WAIT_TIMEOUT)) break;
                 const Work w = work[n & 1];
@@ -195,13 +197,14 @@ __global__ void __launch_bounds__(A_THREADS, 2) span_attn_kernel(const SpanAttnP
                         issued++;
                         if (j == 0 && side == 0) {
                             // the queries follow the first K tile.  Rows past the block are other tokens' or zeros: nobody reads theirs
-                            if (!wait(q_empty, (n & 1) ^ 1, STATUS_EMPTY_WAIT_TIMEOUT)) {
+                            if (w.withheld || !wait(q_empty, (n & 1) ^ 1, STATUS_EMPTY_WAIT_TIMEOUT)) {
                                 live = false;
                                 break;
                             }
                             mbar_arrive_expect_tx(q_full, (DK / 64) * p.block_tokens * group * 128);
 #pragma unroll
                             for (int pn = 0; pn < DK / 64; pn++) tma_load_3d(sbase + pn * Z::Q_PANEL, &q_map, 64 * pn, w.kvh * group, w.token0, q_full);
+                            q_issued++;
                         }
                     }
                     chunk = next;
@@ -209,7 +212,7 @@ __global__ void __launch_bounds__(A_THREADS, 2) span_attn_kernel(const SpanAttnP
             }
             for (int f = issued > A_SLOTS ? issued - A_SLOTS : 0; f < issued; f++)
                 if (!wait(full_bar + 8 * (f & (A_SLOTS - 1)), (f / A_SLOTS) & 1, STATUS_DRAIN_TIMEOUT)) break;
-            if (n > 0) wait(q_full, (n - 1) & 1, STATUS_DRAIN_TIMEOUT);
+            if (q_issued > 0) wait(q_full, (q_issued - 1) & 1, STATUS_DRAIN_TIMEOUT);  // pieces begun may be one more
         } else if (warp == 5 && elect_one()) {
             // ---- MMA issuer: one thread; t counts tiles over all pieces
             constexpr uint32_t DESC_HI = umma_desc_sw128_hi(1024);

@@ -306,6 +306,7 @@ struct SpanAttnParams {
     int max_chunks;
     int* status;
     long long wait_limit;
+    int withhold_item;           // failure-path tests only: the producer stops before the queries of this piece
 };
 bool span_attn_serves(const Geometry& g, int d_value, int block_query_rows);
 cudaError_t launch_span_attn(const SpanAttnParams& p, int d_key, int d_value, cudaStream_t stream);

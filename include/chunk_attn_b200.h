@@ -151,8 +151,9 @@ CA_API int ca_context_create_shaped(ca_context** out, int device, const ca_head_
 /* Contexts with a head shape, portions of prompts in bf16 with 64-token chunks and heads of 64 or 128 elements: 1 (default)
  * the tcgen05 kernel, softmax weights as two bf16 numbers; 2 the same with one bf16 number; 0 the mma.sync kernel. */
 #define CA_OPT_SPAN_TENSOR 11
-/* Failure-path tests only: the CTA that draws item `value` of the next launches stops feeding its consumer
- * warps, whose bounded wait then runs out (status 1).  -1 (default) switches it off. */
+/* Failure-path tests only: the CTA that draws item `value` of the next launches (portions of prompts on tcgen05: piece
+ * `value`, key/value heads fastest) stops feeding its consumer warps, whose bounded wait then runs out (status 1; portions:
+ * 1 or 2).  -1 (default) switches it off. */
 #define CA_OPT_TEST_WITHHOLD_ITEM 8
 CA_API int ca_context_set_option(ca_context* ctx, int option, int64_t value);
 

@@ -48,6 +48,40 @@ def test_wait_that_runs_out_is_reported_and_the_context_survives():
     assert eng.ctx.status() == 0
 
 
+@pytest.mark.parametrize("piece", [0, 700, 1279])
+@pytest.mark.parametrize("span_tensor", [1, 2])
+def test_prompts_whose_producer_stops_end_with_a_status(piece, span_tensor):
+    # 1280 pieces of prompts on tcgen05, more than CTAs, so that the later ones are taken over by CTAs that have worked on others.  In
+    # front of one piece's queries its CTA's producer stops: the other roles' waits run out, no copy is still awaited (status 3), and
+    # the kernel returns by itself.  Then the same call gives the same rows as before, to the bit.
+    import chunk_attn
+    from chunk_attn import SpanBatch
+    H, G, d, n, dev = 32, 8, 128, 80, torch.device("cuda:0")
+    cache = chunk_attn.Attention.shaped(n_heads=H, n_kv_heads=G, d_key=d, d_value=d, scale=d ** -0.5, sink=True, chunk_size=64, memory_mb=128,
+                                        dtype=torch.bfloat16, device=dev)
+    cache.set_option(cabi.CA_OPT_SPAN_TENSOR, span_tensor)
+    tokens = [[1000 * i + t for t in range(40)] for i in range(n)]
+    cache.extend([-1] * n, tokens)
+    spans = SpanBatch(tokens, [0] * n, list(range(n)), dev)
+    x = torch.randn(40 * n, (H + 2 * G) * d, generator=torch.Generator().manual_seed(piece)).to(dev, torch.bfloat16)
+    q = cache.store_qkv(x, spans.positions, None, None, 1e-5, 0, None, None)
+    run = lambda: cache.forward_rows(q, spans.positions, None, spans.entry_of)
+    want = run()
+    assert cache.device_status() == 0
+    cache.set_option(cabi.CA_OPT_WAIT_LIMIT_CYCLES, 2_000_000)
+    cache.set_option(cabi.CA_OPT_TEST_WITHHOLD_ITEM, piece)
+    t0, t1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+    t0.record()
+    run()
+    t1.record()
+    torch.cuda.synchronize()
+    assert t0.elapsed_time(t1) < 500.0            # ms
+    assert cache.device_status() in (cabi.STATUS_FULL_WAIT_TIMEOUT, cabi.STATUS_EMPTY_WAIT_TIMEOUT)
+    cache.set_option(cabi.CA_OPT_TEST_WITHHOLD_ITEM, -1)
+    cache.set_option(cabi.CA_OPT_WAIT_LIMIT_CYCLES, 4_000_000_000)
+    assert torch.equal(run(), want)
+
+
 def test_option_ranges():
     eng = CabiEngine(2, 128, 64, torch.float16, max_chunks=8)
     with pytest.raises(cabi.CAError):

@@ -189,3 +189,41 @@ def test_head_norms_are_rounded_as_fp32_operations(dtype, shape):
     want = heads * inv * w if dtype == torch.float32 and dk == 256 else heads * (inv * w)  # heads of more than 32 granules: weights last
     assert want.dtype == np.float32
     assert torch.equal(q.view(n, H, -1)[..., :dk].cpu(), torch.from_numpy(want).to(dtype))
+
+
+@pytest.mark.parametrize("shape", [(6, 2, 64, 64), (32, 8, 128, 128), (2, 2, 128, 64), (8, 1, 64, 128)])
+@pytest.mark.parametrize("lens", [[1, 63, 64, 65, 129, 300], [40] * 80])
+def test_prompts_on_each_kernel(shape, lens):
+    # The weights of the softmax as one bf16 number (each within 2^-9 of itself, so a row within 2^-9 of the largest value) and as
+    # two, and the mma.sync kernel; every result is rounded to bf16, another 2^-9 of it.
+    import chunk_attn
+    from chunk_attn import SpanBatch, cabi
+    H, G, dk, dv = shape
+    dev, n = torch.device("cuda:0"), len(lens)
+    cache = chunk_attn.Attention.shaped(n_heads=H, n_kv_heads=G, d_key=dk, d_value=dv, scale=dk ** -0.5, sink=True, chunk_size=64, memory_mb=128,
+                                        dtype=torch.bfloat16, device=dev)
+    tokens = [[10_000 * i + t for t in range(x)] for i, x in enumerate(lens)]
+    cache.extend([-1] * n, tokens)
+    spans = SpanBatch(tokens, [0] * n, list(range(n)), dev)
+    x = torch.randn(sum(lens), (H + G) * dk + G * dv, generator=torch.Generator().manual_seed(dk)).to(dev, torch.bfloat16)
+    q = cache.store_qkv(x, spans.positions, None, None, 1e-5, 0, None, None)
+    out = []
+    for option in (0, 1, 2):
+        cache.set_option(cabi.CA_OPT_SPAN_TENSOR, option)
+        out.append(cache.forward_rows(q, spans.positions, None, spans.entry_of).double())
+    start, at = 0, (H + G) * dk
+    for length in lens:
+        xs = x[start:start + length].double()
+        kk = xs[:, H * dk:at].view(length, G, dk).repeat_interleave(H // G, 1)
+        vv = xs[:, at:].view(length, G, dv).repeat_interleave(H // G, 1)
+        s = torch.einsum("ihd,jhd->hij", xs[:, :H * dk].view(length, H, dk), kk) * dk ** -0.5
+        s = s.masked_fill(torch.ones(length, length, dtype=torch.bool, device=dev).triu(1), float("-inf"))
+        m = s.amax(-1, keepdim=True).clamp(min=0)  # the unit term: a score of zero without a value
+        e = torch.exp(s - m)
+        want = torch.einsum("hij,jhd->ihd", e / (e.sum(-1, keepdim=True) + torch.exp(-m)), vv)
+        for o, weights in zip(out, (2.0 ** -16, 2.0 ** -16, 2.0 ** -9)):
+            # the fast exponentials and the scores' fp32 sums: 2^-14 of the largest value
+            bound = want.abs() * 2.0 ** -8 + (weights + 2.0 ** -14) * vv.abs().max()
+            assert ((o[start:start + length].view_as(want) - want).abs() <= bound).all()
+        start += length
+    assert cache.device_status() == 0
