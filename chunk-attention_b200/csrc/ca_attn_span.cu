@@ -28,6 +28,8 @@
 // columns are freed there.
 #include <cuda.h>
 
+#include <atomic>
+
 #include "ca_kernels.h"
 #include "ca_ptx.cuh"
 #include "ca_softmax.cuh"
@@ -456,9 +458,16 @@ cudaError_t launch(const SpanAttnParams& p, cudaStream_t stream) {
     static_assert(2 * (smem + 1024) <= 233472, "two CTAs do not fit in one SM's shared memory");
     CUtensorMap queries;
     if (!make_query_map(&queries, p, DK)) return cudaErrorInvalidValue;
-    cudaFuncAttributes have;
-    cudaError_t e = cudaFuncGetAttributes(&have, k);
-    if (e == cudaSuccess && 2 * have.numRegs < A_SOFTMAX_REGS + A_OTHER_REGS) e = cudaErrorInvalidConfiguration;  // the warps would wait for registers for good
+    // With fewer registers the warps would wait for them for good.  What the compiler gave the kernel does not change: asking on every
+    // launch made a call on a short prompt wait 1.1 us longer for its host part (40 tokens: 9.6 us a call, 8.5 so).
+    static std::atomic<bool> enough[2];
+    cudaError_t e = cudaSuccess;
+    if (!enough[p.split_weights ? 1 : 0]) {
+        cudaFuncAttributes have;
+        e = cudaFuncGetAttributes(&have, k);
+        if (e == cudaSuccess && 2 * have.numRegs < A_SOFTMAX_REGS + A_OTHER_REGS) e = cudaErrorInvalidConfiguration;
+        if (e == cudaSuccess) enough[p.split_weights ? 1 : 0] = true;
+    }
     if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
     if (e != cudaSuccess) return e;
