@@ -275,17 +275,19 @@ __global__ void __launch_bounds__(E_THREADS, 1) latent_span_kernel(const LatentS
                         for (int j = 0; j < AHEAD; j++) {
                             const int row = row0 + j * row_step;
                             if (row >= E_ROWS) break;
-                            const float pos = (float)(gpos + row);
-                            uint32_t* aw = reinterpret_cast<uint32_t*>(&a[j]);
-                            uint32_t* bw = reinterpret_cast<uint32_t*>(&b[j]);
+                            if (row < n_rows) {
+                                const float pos = (float)(gpos + row);
+                                uint32_t* aw = reinterpret_cast<uint32_t*>(&a[j]);
+                                uint32_t* bw = reinterpret_cast<uint32_t*>(&b[j]);
 #pragma unroll
-                            for (int k = 0; k < 4; k++) {
-                                const float2 x = unpack_bf16(aw[k]), y = unpack_bf16(bw[k]);
-                                float s0, c0, s1, c1;
-                                fast_sincos(pos * f[2 * k], &s0, &c0);
-                                fast_sincos(pos * f[2 * k + 1], &s1, &c1);
-                                aw[k] = pack_bf16(x.x * c0 - y.x * s0, x.y * c1 - y.y * s1);
-                                bw[k] = pack_bf16(y.x * c0 + x.x * s0, y.y * c1 + x.y * s1);
+                                for (int k = 0; k < 4; k++) {
+                                    const float2 x = unpack_bf16(aw[k]), y = unpack_bf16(bw[k]);
+                                    float s0, c0, s1, c1;
+                                    fast_sincos(pos * f[2 * k], &s0, &c0);
+                                    fast_sincos(pos * f[2 * k + 1], &s1, &c1);
+                                    aw[k] = pack_bf16(x.x * c0 - y.x * s0, x.y * c1 - y.y * s1);
+                                    bw[k] = pack_bf16(y.x * c0 + x.x * s0, y.y * c1 + x.y * s1);
+                                }
                             }
                             sts128(line(row, d_panels * 8 + u), (int)a[j].x, (int)a[j].y, (int)a[j].z, (int)a[j].w);
                             sts128(line(row, d_panels * 8 + units + u), (int)b[j].x, (int)b[j].y, (int)b[j].z, (int)b[j].w);
