@@ -3,6 +3,7 @@ import numpy as np
 import pytest
 import torch
 
+from chunk_attn import cabi
 from gpu_helpers import CabiEngine
 
 pytestmark = pytest.mark.gpu
@@ -122,17 +123,20 @@ def test_decoded_rows_of_small_groups(shape, chunk):
     assert cache.device_status() == 0
 
 
-@pytest.mark.parametrize("n,H", [(64, 8), (310, 16)])
-@pytest.mark.parametrize("shared", [0, 256])
-def test_short_tails_walked_by_half_warps(n, H, shared):
-    # Private tails of 0 to 64 tokens (rounds of eight, both items of a warp of different lengths), fewer and more of them than the
-    # grid's half-warps; with other partials to combine and without; a token appended, into a chunk of its own for some.
+@pytest.mark.parametrize("n,H", [(64, 8), (310, 16), (700, 16)])
+@pytest.mark.parametrize("shared,most", [(0, 63), (256, 63), (256, 64)])
+def test_short_tails_walked_by_half_warps(n, H, shared, most):
+    # Private tails of up to 64 tokens (rounds of eight, both items of a warp of different lengths): 512 of them for the grid's 4736
+    # half-warps, 4960 (a second item for some), 11200 (a third for some); with other partials to combine and without; a token appended,
+    # into a chunk of its own for some.  Tails of 64 have a next chunk already and are not short: where there are some the merge kernel
+    # finishes the rows, else the kernel itself does.
     g = torch.Generator().manual_seed(n)
     eng = CabiEngine(H, 128, 64, torch.float16, max_chunks=4 + 2 * n)
+    eng.ctx.set_option(cabi.CA_OPT_NUM_CTAS, 8)  # the tails are many by comparison and take their own kernel
     sk, sv = torch.randn(shared, H, 128, generator=g).half(), torch.randn(shared, H, 128, generator=g).half()
     kv = []
     for i in range(n):
-        own = (7 * i) % 65 if shared else 1 + (7 * i) % 63
+        own = (7 * i) % (most + 1) if shared else 1 + (7 * i) % 63
         k, v = torch.randn(own, H, 128, generator=g).half(), torch.randn(own, H, 128, generator=g).half()
         kv.append((torch.cat([sk, k]), torch.cat([sv, v])))
         eng.add_seq(list(range(shared)) + [100_000 + 1000 * i + j for j in range(own)], *kv[-1])
@@ -144,6 +148,12 @@ def test_short_tails_walked_by_half_warps(n, H, shared):
         assert ((eng.forward(q).double() - want).abs() - want.abs() * 2.0 ** -11).max() < 4e-4
 
     check()
+    rows = sum(k.shape[0] < shared + 64 for k, _ in kv)
+    launches = []
+    for finish in (0, 1):
+        eng.ctx.set_option(cabi.CA_OPT_FINISH_IN_TAILS, finish)
+        launches.append(eng.ctx.stats()["kernels_per_step"])
+    assert eng.ctx.stats()["n_items_short"] == rows * H and launches[0] - launches[1] == (rows == n)
     check()
     k1, v1 = torch.randn(n, H, 128, generator=g).half(), torch.randn(n, H, 128, generator=g).half()
     eng.append_token([5] * n, k1, v1)
@@ -197,7 +207,7 @@ def test_prompts_on_each_kernel(shape, lens):
     # The weights of the softmax as one bf16 number (each within 2^-9 of itself, so a row within 2^-9 of the largest value) and as
     # two, and the mma.sync kernel; every result is rounded to bf16, another 2^-9 of it.
     import chunk_attn
-    from chunk_attn import SpanBatch, cabi
+    from chunk_attn import SpanBatch
     H, G, dk, dv = shape
     dev, n = torch.device("cuda:0"), len(lens)
     cache = chunk_attn.Attention.shaped(n_heads=H, n_kv_heads=G, d_key=dk, d_value=dv, scale=dk ** -0.5, sink=True, chunk_size=64, memory_mb=128,
