@@ -34,7 +34,7 @@ constexpr int GEN_WARPS = 4;
 constexpr int GEN_MAX_D = 256;
 // CTAs up to which a row's cluster grows.  Measured at 1, 2 and 4 times this (16 x 500 + 256 tokens, 8 fp32 heads of 64):
 // 9.5 / 14.2 / 14.2 us, 16 x 833 fp16: 11.7 / 12.3 / 14.9: more CTAs of a cluster only wait for each other.
-constexpr int64_t GEN_SPLIT_CTAS = 148 * 4;
+constexpr int64_t GEN_SPLIT_CTAS = B200_SMS * 4;
 
 // A finished row leaves: value(e) is element e of it.  Values that were cached turned by their own position are turned
 // back by the row's.

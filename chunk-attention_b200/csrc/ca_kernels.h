@@ -21,6 +21,8 @@ constexpr int STATUS_BAD_WORK_LIST = 4;       // an item or merge entry named a 
 constexpr int STATUS_BAD_POSITION = 5;        // rotary embedding: a position outside the cos/sin table: row skipped
 constexpr long long DEFAULT_WAIT_LIMIT_CYCLES = 4000000000LL;  // about two seconds of SM clock
 
+constexpr int B200_SMS = 148;  // sizes grids and splits; no result depends on it
+
 // ---- fast path: fp16, d_head 128, chunk_size 64 -----------------------------------------------
 constexpr int FAST_D = 128;
 constexpr int FAST_C = 64;

@@ -280,7 +280,7 @@ __global__ void __launch_bounds__(QKV_VEC_THREADS, QKV_VEC_CTAS) store_qkv_vec_k
 
 template <typename T, int LANES, int GP>
 void run_store_qkv_vec(const QkvParams& p, cudaStream_t stream) {
-    store_qkv_vec_kernel<T, LANES, GP><<<std::min(p.n_tokens, QKV_VEC_CTAS * 148), QKV_VEC_THREADS, 0, stream>>>(p);
+    store_qkv_vec_kernel<T, LANES, GP><<<std::min(p.n_tokens, QKV_VEC_CTAS * B200_SMS), QKV_VEC_THREADS, 0, stream>>>(p);
 }
 template <typename T>
 void run_store_qkv(const QkvParams& p, cudaStream_t stream) {

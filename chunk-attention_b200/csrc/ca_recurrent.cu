@@ -413,7 +413,7 @@ int scan_run(const ca_spans& sp, int channels, int n_states) {
     const int per_block = SCAN_THREADS / scan_lanes(n_states, 8);
     const int64_t blocks = (channels + per_block - 1) / per_block;
     if (sp.n_work == sp.n_entries || blocks * sp.n_entries >= 444) return 0;
-    const int64_t run = (blocks * sp.n_work + 148 * 7 - 1) / (148 * 7);  // one wave of about seven CTAs per SM
+    const int64_t run = (blocks * sp.n_work + B200_SMS * 7 - 1) / (B200_SMS * 7);  // one wave of about seven CTAs per SM
     const int longest = (sp.max_tokens + sp.work_len - 1) / sp.work_len;
     return run >= longest ? 0 : (int)run;
 }
@@ -440,7 +440,7 @@ template <typename T, int L>
 void launch_scan_step(const ScanParams& p, cudaStream_t stream) {
     constexpr int per_block = SCAN_THREADS / L;
     const int blocks = (p.C + per_block - 1) / per_block;
-    const dim3 grid(blocks, std::min(p.sp.n_entries, std::max(1, 148 * 64 / blocks)));
+    const dim3 grid(blocks, std::min(p.sp.n_entries, std::max(1, B200_SMS * 64 / blocks)));
     if (p.N % 4 == 0) scan_step_kernel<T, L, true><<<grid, SCAN_THREADS, 0, stream>>>(p);
     else scan_step_kernel<T, L, false><<<grid, SCAN_THREADS, 0, stream>>>(p);
 }
@@ -645,7 +645,7 @@ int selective_scan(const ScanParams& p, cudaStream_t stream) {
 int decay_run(const ca_spans& sp, int heads) {
     const int longest = (sp.max_tokens + sp.work_len - 1) / sp.work_len;
     if (longest <= 1) return 0;
-    auto waves = [](int64_t ctas) { return (double)((ctas + 147) / 148); };
+    auto waves = [](int64_t ctas) { return (double)((ctas + B200_SMS - 1) / B200_SMS); };
     double best = waves((int64_t)sp.n_entries * heads) * longest;
     int best_run = 0;
     for (int run = 2; run < longest; run += 2) {
