@@ -18,10 +18,11 @@ CA_DTYPE_F16, CA_DTYPE_F32, CA_DTYPE_BF16 = 0, 1, 2
 CA_OPT_SPLIT_PHASES, CA_OPT_NUM_CTAS, CA_OPT_SEQ_FIRST_TENSOR, CA_OPT_TRACE, CA_OPT_DEPENDENT_LAUNCH = 1, 2, 3, 4, 5
 CA_OPT_WIDE_RUNS, CA_OPT_WAIT_LIMIT_CYCLES, CA_OPT_TEST_WITHHOLD_ITEM, CA_OPT_OVERLAP_KERNELS, CA_OPT_FINISH_IN_TAILS = 6, 7, 8, 9, 10
 CA_OPT_SPAN_TENSOR = 11
+CA_OPT_DIRECT = 12
 STATUS_FULL_WAIT_TIMEOUT, STATUS_EMPTY_WAIT_TIMEOUT, STATUS_DRAIN_TIMEOUT, STATUS_BAD_WORK_LIST, STATUS_BAD_POSITION = 1, 2, 3, 4, 5
 PLAN_ITEMS = 0
 (PLAN_MERGE_OFF, PLAN_MERGE_SLOTS, PLAN_PATH_OFF, PLAN_PATH_CHUNKS, PLAN_PATH_TOKENS, PLAN_TAIL_CHUNK,
- PLAN_TAIL_TOKENS, PLAN_WIDE_CHUNKS) = range(3, 11)
+ PLAN_TAIL_TOKENS, PLAN_WIDE_CHUNKS, PLAN_DIRECT_ENTRIES, PLAN_DIRECT_RANGES, PLAN_DIRECT_BLOCKS) = range(3, 14)
 
 # every symbol include/chunk_attn_b200.h declares
 EXPORTED = [
@@ -36,7 +37,7 @@ EXPORTED = [
     "ca_norm_rows", "ca_embed_rows", "ca_gelu_tanh", "ca_conv_silu", "ca_scan_scratch_floats", "ca_selective_scan", "ca_decay_scratch_floats", "ca_block_status", "ca_decay_attention",
     "ca_scaled_norm", "ca_clamped_glu", "ca_softcap", "ca_latent_store", "ca_latent_block", "ca_latent_attention", "ca_latent_decodes", "ca_latent_gather",
     "ca_latent_expands", "ca_latent_expanded_block", "ca_latent_expanded",
-    "ca_plan_build_windowed",
+    "ca_plan_build_windowed", "ca_plan_direct",
 ]
 CA_STATIC_MAX_SLOTS = 16384
 
@@ -96,6 +97,7 @@ def _load():
         "ca_plan_build_windowed": (i32, [C.POINTER(vp), C.POINTER(ChunkInfo), i32, i32, i32, i32, i32, i64, i32, i32]),
         "ca_plan_build_for_context": (i32, [vp, C.POINTER(vp), C.POINTER(ChunkInfo), i32, i32]),
         "ca_refresh_from_plan": (i32, [vp, vp, vp]),
+        "ca_plan_direct": (i32, [vp, i32, i32, i32, C.POINTER(i32)]),
         "ca_plan_array": (i32, [vp, i32, C.POINTER(C.POINTER(C.c_int32)), C.POINTER(i64)]),
         "ca_plan_stats_get": (i32, [vp, C.POINTER(PlanStats)]),
         "ca_plan_destroy": (None, [vp]),
@@ -162,6 +164,13 @@ class Plan:
         if cnt.value == 0:
             return np.zeros(0, np.int32)
         return np.ctypeslib.as_array(ptr, shape=(cnt.value,)).copy()
+
+    def direct(self, mode, d_head, against_items=True):
+        """CTAs per block of rows and head of the one-launch kernel (0: the step goes another way); its lists are then in
+        `array(PLAN_DIRECT_...)`."""
+        cluster = C.c_int()
+        check(lib.ca_plan_direct(self._h, mode, d_head, int(against_items), C.byref(cluster)))
+        return cluster.value
 
     def items(self):
         return self.array(PLAN_ITEMS).reshape(-1, 16)

@@ -84,6 +84,7 @@ struct ca_plan {
     int d_head = ca::FAST_D;
     int esize = 2;
     int window = 0, group = 1;
+    int direct = 0;
 };
 
 namespace {
@@ -117,6 +118,7 @@ struct ca_context {
     unsigned long long* trace = nullptr;  // [kTraceCtas][4], allocated when tracing is switched on
     int trace_ctas = 0;                   // CTAs of the last traced launch
     int trace_cycles = 0;                 // CA_OPT_TRACE = 2: the tcgen05 kernel accounts for cycles per role instead
+    int opt_direct = 1;                   // CA_OPT_DIRECT
     int opt_finish_in_tails = 1;          // CA_OPT_FINISH_IN_TAILS: the short-tails kernel finishes the rows when it can
     bool out_is_host = false;             // set by ca_attention_host around its launches: the rows go to host memory
 
@@ -128,6 +130,7 @@ struct ca_context {
         int64_t n_merge_slots = 0;  // entries of merge_slots
         int max_merge_len = 0;
         bool split_phases = false;
+        int direct_cluster = 0, direct_blocks = 0, direct_rows = 0;  // Plan::direct_*
         ca_plan_stats stats{};
     } meta;
     bool valid = false;
@@ -147,6 +150,8 @@ struct ca_context {
     const int32_t *d_path_off = nullptr, *d_path_chunks = nullptr, *d_path_tokens = nullptr;
     const int32_t *d_tail_chunk = nullptr, *d_tail_tokens = nullptr;
     const int32_t* d_wide_chunks = nullptr;
+    const int4 *d_direct_entries = nullptr, *d_direct_ranges = nullptr;
+    const int2* d_direct_blocks = nullptr;
     // The per-row path lists are read by the any-geometry kernel only: a context of the tensor-core geometry
     // builds and uploads them on the first partition = 2 request after a refresh, from this copy of the input.
     bool paths_on_device = false;
@@ -312,6 +317,9 @@ int ca_context_set_option(ca_context* c, int option, int64_t value) {
     } else if (option == CA_OPT_WIDE_RUNS) {
         if (value < 0 || value > 2) return fail(CA_ERR_INVALID, "wide-runs mode must be 0, 1 or 2");
         c->opt_wide = (int)value;
+    } else if (option == CA_OPT_DIRECT) {
+        if (value < 0 || value > 2) return fail(CA_ERR_INVALID, "CA_OPT_DIRECT takes 0, 1 or 2");
+        c->opt_direct = (int)value;
     } else if (option == CA_OPT_OVERLAP_KERNELS) {
         c->opt_overlap = value != 0;
         return CA_OK;
@@ -359,11 +367,20 @@ static int upload_plan(ca_context* c, const ca::Plan& pl, cudaStream_t stream);
 // CTAs the work list is cut for: the latent kernel's fill an SM each
 static int ctas_of(const ca_context* c) { return c->opt_ctas > 0 ? c->opt_ctas : c->num_sms * (c->shape.latent ? 1 : ca::FAST_CTAS_PER_SM); }
 
+// CA_OPT_DIRECT as it counts for this context: options that choose among the kernels of the item lists choose those kernels
+static int direct_mode(const ca_context* c) {
+    if (c->shaped || !ca::attn_direct_serves(c->geo) || c->opt_split || c->opt_ctas > 0 || !c->opt_sf_tensor || c->opt_wide != 1) return 0;
+    return c->opt_direct;
+}
+
 static std::string plan_for(const ca_context* c, ca::Plan& plan, const ca_chunk_info* infos, int n_infos, int n_seqs, int n_ctas) {
-    if (!c->shaped)
-        return ca::build_plan(plan, infos, n_infos, n_seqs, c->geo.n_heads, c->geo.chunk_size, c->tpp_threshold, n_ctas,
-                              c->max_chunks, c->opt_split, c->geo.d_head, c->geo.esize, c->fast, c->opt_sf_tensor, c->opt_wide,
-                              /*want_paths=*/!c->fast);
+    if (!c->shaped) {
+        const std::string err = ca::build_plan(plan, infos, n_infos, n_seqs, c->geo.n_heads, c->geo.chunk_size, c->tpp_threshold, n_ctas,
+                                               c->max_chunks, c->opt_split, c->geo.d_head, c->geo.esize, c->fast, c->opt_sf_tensor, c->opt_wide,
+                                               /*want_paths=*/!c->fast);
+        if (err.empty()) ca::build_direct(plan, direct_mode(c), c->geo.d_head, c->fast);
+        return err;
+    }
     const int d_mean = c->shape.latent ? c->geo.d_head / 2 : (c->geo.d_head + c->geo.d_value) / 2;
     // items of up to 64 query rows (a sequence brings `group` of them), one partial per row; no kernel of their own for
     // short tails or wide runs
@@ -403,6 +420,7 @@ int ca_plan_build_for_context(const ca_context* c, ca_plan** out, const ca_chunk
     p->esize = c->geo.esize;
     p->window = c->shape.window;
     p->group = c->group;
+    p->direct = direct_mode(c);
     *out = p;
     return CA_OK;
 }
@@ -419,14 +437,16 @@ int ca_refresh_from_plan(ca_context* c, const ca_plan* plan, ca_stream stream_) 
     DeviceGuard guard(c->device);
     if (guard.err != cudaSuccess) return fail_cuda(guard.err, "cudaSetDevice");
     c->valid = false;
-    return upload_plan(c, pl, static_cast<cudaStream_t>(stream_));
+    const int rc = upload_plan(c, pl, static_cast<cudaStream_t>(stream_));
+    if (plan->direct != direct_mode(c)) c->meta.direct_cluster = 0;  // its items serve any options
+    return rc;
 }
 
 static int upload_plan(ca_context* c, const ca::Plan& pl, cudaStream_t stream) {
 
     // pack every table into one staging buffer
     struct Part { const void* src; size_t bytes; size_t off; };
-    Part parts[9] = {
+    Part parts[12] = {
         {pl.items.data(), pl.items.size() * sizeof(ca::PlanItem), 0},
         {pl.merge_off.data(), pl.merge_off.size() * 4, 0},
         {pl.merge_slots.data(), pl.merge_slots.size() * 4, 0},
@@ -436,6 +456,9 @@ static int upload_plan(ca_context* c, const ca::Plan& pl, cudaStream_t stream) {
         {pl.tail_chunk.data(), pl.tail_chunk.size() * 4, 0},
         {pl.tail_tokens.data(), pl.tail_tokens.size() * 4, 0},
         {pl.wide_chunks.data(), pl.wide_chunks.size() * 4, 0},
+        {pl.direct_entries.data(), pl.direct_entries.size() * 4, 0},
+        {pl.direct_ranges.data(), pl.direct_ranges.size() * 4, 0},
+        {pl.direct_blocks.data(), pl.direct_blocks.size() * 4, 0},
     };
     size_t total = 0;
     for (Part& p : parts) {
@@ -477,6 +500,9 @@ static int upload_plan(ca_context* c, const ca::Plan& pl, cudaStream_t stream) {
     c->d_tail_chunk = reinterpret_cast<const int32_t*>(c->dev_blob + parts[6].off);
     c->d_tail_tokens = reinterpret_cast<const int32_t*>(c->dev_blob + parts[7].off);
     c->d_wide_chunks = reinterpret_cast<const int32_t*>(c->dev_blob + parts[8].off);
+    c->d_direct_entries = reinterpret_cast<const int4*>(c->dev_blob + parts[9].off);
+    c->d_direct_ranges = reinterpret_cast<const int4*>(c->dev_blob + parts[10].off);
+    c->d_direct_blocks = reinterpret_cast<const int2*>(c->dev_blob + parts[11].off);
     c->paths_on_device = pl.has_paths;
     if (pl.has_paths) c->max_path_tokens = pl.max_path_tokens;
     if (!pl.has_paths) {  // keep what a later partition = 2 request needs to build them
@@ -521,6 +547,9 @@ static int upload_plan(ca_context* c, const ca::Plan& pl, cudaStream_t stream) {
     c->meta.n_merge_slots = (int64_t)pl.merge_slots.size();
     c->meta.max_merge_len = pl.max_merge_len;
     c->meta.split_phases = pl.split_phases;
+    c->meta.direct_cluster = pl.direct_cluster;
+    c->meta.direct_rows = pl.direct_rows;
+    c->meta.direct_blocks = (int)(pl.direct_blocks.size() / 2);
     c->meta.stats = pl.stats;
     c->valid = true;
     return CA_OK;
@@ -813,6 +842,50 @@ int ca_peer_barrier(void* const* flag_arrays, int n_peers, int rank, uint32_t ep
     return CA_OK;
 }
 
+// The step goes to the one-launch kernel: the work list has its form, no option looks at the kernels of the item lists, and rows
+// can be moved in whole granules.
+static bool goes_direct(const ca_context* c, const void* q = nullptr, const void* out = nullptr) {
+    return c->meta.direct_cluster > 0 && c->opt_withhold_item < 0 && !c->trace && !c->opt_overlap &&
+           (reinterpret_cast<uintptr_t>(c->pool) | reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(out)) % 16 == 0;
+}
+
+// peers: the rows go into the outputs it names instead of `out`
+static int run_direct(ca_context* c, const void* q, void* out, const ca::MergeParams* peers, ca_stream stream_) {
+    DeviceGuard guard(c->device);
+    if (guard.err != cudaSuccess) return fail_cuda(guard.err, "cudaSetDevice");
+    ca::DirectParams d;
+    d.pool = static_cast<const uint8_t*>(c->pool);
+    d.n_heads = c->geo.n_heads;
+    d.chunk_size = c->geo.chunk_size;
+    d.d = c->geo.d_head;
+    d.gpr = c->geo.gpr;
+    d.v_offset = (size_t)c->geo.tile_elems * c->geo.esize;
+    d.pair_bytes = 2 * d.v_offset;
+    d.q = q;
+    d.out = out;
+    d.entries = c->d_direct_entries;
+    d.ranges = c->d_direct_ranges;
+    d.blocks = c->d_direct_blocks;
+    d.n_blocks = c->meta.direct_blocks;
+    d.cluster = c->meta.direct_cluster;
+    d.block_rows = c->meta.direct_rows;
+    d.delta_tokens = c->delta_tokens;
+    d.scale_log2 = 1.4426950408889634f / std::sqrt((float)c->geo.d_head);
+    d.zero_if_none = c->fast;
+    d.one_weight = c->fast;
+    d.max_chunks = (int)(c->max_chunks < INT32_MAX ? c->max_chunks : INT32_MAX);
+    d.status = c->status;
+    if (peers) {
+        d.n_peers = peers->n_peers;
+        d.total_heads = peers->total_heads;
+        d.head_offset = peers->head_offset;
+        d.mc_out = peers->mc_out;
+        for (int i = 0; i < d.n_peers; i++) d.peer_out[i] = peers->peer_out[i];
+    }
+    CA_CUDA(ca::launch_attn_direct(d, c->geo.swz != 0, static_cast<cudaStream_t>(stream_)));
+    return CA_OK;
+}
+
 int ca_attention_to_peers(ca_context* c, const void* q, void* const* peer_out, int n_peers, void* multicast_out,
                           int total_heads, int head_offset, int n_seqs, ca_stream stream_) {
     int rc = check_attention_args(c, q, n_seqs);
@@ -830,6 +903,7 @@ int ca_attention_to_peers(ca_context* c, const void* q, void* const* peer_out, i
     m.head_offset = head_offset;
     for (int i = 0; i < n_peers; i++) m.peer_out[i] = peer_out[i];
     m.mc_out = multicast_out;
+    if (goes_direct(c, q)) return run_direct(c, q, nullptr, &m, stream_);
     bool finished = false;
     rc = run_partials(c, q, n_seqs, 3, stream_, &m, &finished);
     if (rc != CA_OK) return rc;
@@ -883,6 +957,7 @@ int ca_attention(ca_context* c, const void* q, void* out, int n_seqs, int partit
     if (partition < 0 || partition > 2) return fail(CA_ERR_INVALID, "Unsupported partition type");
     if (n_seqs == 0) return CA_OK;
     if (!out) return fail(CA_ERR_INVALID, "out is null");
+    if (partition != CA_PARTITION_SEQ_FIRST && goes_direct(c, q, out)) return run_direct(c, q, out, nullptr, stream_);
     if (c->fast && partition != CA_PARTITION_SEQ_FIRST) {
         const ca::MergeParams m = merge_params_of(c, out, n_seqs);
         bool finished = false;
@@ -1414,7 +1489,8 @@ int ca_context_stats(const ca_context* c, ca_plan_stats* out) {
     if (!c || !out) return fail(CA_ERR_INVALID, "null argument");
     if (!c->valid) return fail(CA_ERR_STATE, "work list is stale");
     *out = c->meta.stats;
-    if (tails_can_finish(c)) out->kernels_per_step -= 1;  // the short-tails kernel stores the rows: no merge launch
+    if (goes_direct(c)) out->kernels_per_step = 1;
+    else if (tails_can_finish(c)) out->kernels_per_step -= 1;  // the short-tails kernel stores the rows: no merge launch
     else if (c->meta.short_all_empty && c->delta_tokens == 0) out->kernels_per_step -= 1;  // nothing to do for empty tails
     return CA_OK;
 }
@@ -1456,6 +1532,15 @@ int ca_plan_build_windowed(ca_plan** out, const ca_chunk_info* infos, int n_info
     return CA_OK;
 }
 
+int ca_plan_direct(ca_plan* plan, int mode, int d_head, int against_items, int* cluster) {
+    if (!plan || !cluster) return fail(CA_ERR_INVALID, "null argument");
+    if (mode < 0 || mode > 2 || d_head < 1 || d_head > 128) return fail(CA_ERR_INVALID, "mode must be 0, 1 or 2, d_head at most 128");
+    if (!plan->plan.has_paths) ca::build_paths(plan->plan);
+    ca::build_direct(plan->plan, mode, d_head, against_items != 0);
+    *cluster = plan->plan.direct_cluster;
+    return CA_OK;
+}
+
 int ca_plan_array(const ca_plan* plan, int which, const int32_t** data, int64_t* count) {
     if (!plan || !data || !count) return fail(CA_ERR_INVALID, "null argument");
     const ca::Plan& pl = plan->plan;
@@ -1475,6 +1560,9 @@ int ca_plan_array(const ca_plan* plan, int which, const int32_t** data, int64_t*
         case CA_PLAN_TAIL_CHUNK: v = &pl.tail_chunk; break;
         case CA_PLAN_TAIL_TOKENS: v = &pl.tail_tokens; break;
         case CA_PLAN_WIDE_CHUNKS: v = &pl.wide_chunks; break;
+        case CA_PLAN_DIRECT_ENTRIES: v = &pl.direct_entries; break;
+        case CA_PLAN_DIRECT_RANGES: v = &pl.direct_ranges; break;
+        case CA_PLAN_DIRECT_BLOCKS: v = &pl.direct_blocks; break;
         default: return fail(CA_ERR_INVALID, "unknown plan array");
     }
     *data = v->data();

@@ -21,8 +21,6 @@ constexpr int STATUS_BAD_WORK_LIST = 4;       // an item or merge entry named a 
 constexpr int STATUS_BAD_POSITION = 5;        // rotary embedding: a position outside the cos/sin table: row skipped
 constexpr long long DEFAULT_WAIT_LIMIT_CYCLES = 4000000000LL;  // about two seconds of SM clock
 
-constexpr int B200_SMS = 148;  // sizes grids and splits; no result depends on it
-
 // ---- fast path: fp16, d_head 128, chunk_size 64 -----------------------------------------------
 constexpr int FAST_D = 128;
 constexpr int FAST_C = 64;
@@ -132,6 +130,31 @@ struct PeerBarrierParams {
     int* status;                       // may be null
 };
 cudaError_t launch_peer_barrier(const PeerBarrierParams& p, cudaStream_t stream);
+
+// ---- small steps in one launch (ca_attn_direct.cu): fp16, rows of whole granules, d_head <= 128 ----------------
+struct DirectParams {
+    const uint8_t* pool;
+    int n_heads, chunk_size, d, gpr;
+    size_t pair_bytes, v_offset; // of a (chunk, head): K and V tile; where V starts
+    const void* q;               // fp16 [n_seqs, n_heads, d]
+    void* out;                   // the same
+    const int4* entries;         // Plan::direct_entries
+    const int4* ranges;          // Plan::direct_ranges
+    const int2* blocks;          // Plan::direct_blocks
+    int n_blocks, cluster;       // CTAs per block and head
+    int block_rows;              // of the longest block
+    int delta_tokens;
+    float scale_log2;
+    int zero_if_none;            // rows whose scores are all -inf: 1 zeros, 0 NaN
+    int one_weight;              // softmax weights enter the second product as one fp16 number (else as two)
+    int max_chunks;
+    int* status;
+    int n_peers = 0, total_heads = 0, head_offset = 0;  // as in MergeParams
+    void* peer_out[MERGE_MAX_PEERS] = {};
+    void* mc_out = nullptr;
+};
+bool attn_direct_serves(const Geometry& g);
+cudaError_t launch_attn_direct(const DirectParams& p, bool panels, cudaStream_t stream);
 
 // ---- generic path: any d_head <= 256, any chunk size, fp16, bf16 or fp32 -----------------------------
 struct GenericParams {

@@ -29,6 +29,8 @@
 
 namespace ca {
 
+constexpr int B200_SMS = 148;  // sizes grids, splits and estimates; no result depends on it
+
 struct Geometry {
     int n_heads;  // key/value heads
     int d_head;

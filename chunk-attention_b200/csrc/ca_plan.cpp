@@ -5,6 +5,8 @@
 #include <cstdio>
 #include <unordered_map>
 
+#include "ca_layout.h"
+
 namespace ca {
 namespace {
 
@@ -106,6 +108,162 @@ std::vector<int32_t> first_positions(const ca_chunk_info* infos, int n_infos) {
 }
 
 }  // namespace
+
+// ---- the one-launch kernel's work ----------------------------------------------------------------------------------------
+namespace {
+
+// A chunk counts as the steps it holds now, a tail as at least one: tokens appended later lengthen the range that holds its end.
+int direct_steps(const Plan& plan, const ca_chunk_info& ci, bool* tail = nullptr) {
+    const bool t = ci.seq_end - ci.seq_begin == 1 && plan.tail_chunk[ci.seq_begin] == ci.chunk_id;
+    if (tail) *tail = t;
+    const int n = (ci.n_tokens + DIRECT_STEP - 1) / DIRECT_STEP;
+    return t ? std::max(1, n) : n;
+}
+
+// Per block of rows the chunks that any of them sees, in depth-first order, and the ranges of steps that the warps of the
+// block's CTAs take.
+void cut_direct(Plan& plan, int rows_per_block, int cluster) {
+    const int n_seqs = plan.n_seqs, n_blocks = (n_seqs + rows_per_block - 1) / rows_per_block, warps = cluster * DIRECT_WARPS;
+    std::vector<int32_t> first((size_t)n_blocks + 1, 0);
+    std::vector<int64_t> steps((size_t)n_blocks, 0);
+    auto each = [&](auto f) {  // f(block, chunk, its steps, whether it is a tail)
+        for (const ca_chunk_info& ci : plan.infos) {
+            bool tail;
+            const int s = direct_steps(plan, ci, &tail);
+            if (s > 0)
+                for (int b = ci.seq_begin / rows_per_block; b <= (ci.seq_end - 1) / rows_per_block; b++) f(b, ci, s, tail);
+        }
+    };
+    each([&](int b, const ca_chunk_info&, int s, bool) {
+        first[b + 1]++;
+        steps[b] += s;
+    });
+    for (int b = 0; b < n_blocks; b++) first[b + 1] += first[b];
+    plan.direct_entries.resize((size_t)first[n_blocks] * 4);
+    std::vector<int32_t> at(first.begin(), first.end() - 1), length((size_t)first[n_blocks]);
+    each([&](int b, const ca_chunk_info& ci, int s, bool tail) {
+        const int r0 = b * rows_per_block, lo = std::max(0, ci.seq_begin - r0), hi = std::min(rows_per_block, ci.seq_end - r0);
+        length[at[b]] = s;
+        int32_t* e = plan.direct_entries.data() + 4 * (size_t)at[b]++;
+        e[0] = ci.chunk_id;
+        e[1] = ci.n_tokens;
+        e[2] = ((1 << hi) - 1) & ~((1 << lo) - 1);
+        e[3] = tail ? 1 : 0;
+    });
+    plan.direct_blocks.resize((size_t)n_blocks * 2);
+    plan.direct_ranges.resize((size_t)n_blocks * warps * 4);
+    for (int b = 0; b < n_blocks; b++) {
+        plan.direct_blocks[2 * b] = b * rows_per_block;
+        plan.direct_blocks[2 * b + 1] = std::min(rows_per_block, n_seqs - b * rows_per_block);
+        int64_t before = 0;  // steps of the block ahead of entry e
+        int e = first[b];
+        for (int w = 0; w < warps; w++) {
+            int32_t* r = plan.direct_ranges.data() + 4 * ((size_t)b * warps + w);
+            const int64_t lo = steps[b] * w / warps, hi = steps[b] * (w + 1) / warps;
+            r[0] = 1;  // nothing
+            r[1] = r[2] = r[3] = 0;
+            if (lo == hi) continue;
+            while (before + length[e] <= lo) before += length[e++];
+            r[0] = e;
+            r[1] = (int32_t)(lo - before);
+            while (before + length[e] < hi) before += length[e++];
+            r[2] = e;
+            r[3] = before + length[e] == hi ? DIRECT_TO_THE_END : (int32_t)(hi - before);
+        }
+    }
+    plan.direct_cluster = cluster;
+    plan.direct_rows = std::min(rows_per_block, n_seqs);
+}
+
+// Waves of CTAs: a second one costs as much as the first, many follow each other without a gap.
+double waves(double ctas, double slots) {
+    const double w = ctas / slots;
+    return w <= 1 ? 1 : (w <= 2 ? 2 : w + 0.5);
+}
+
+}  // namespace
+
+// Which way a step goes, by estimates of its time in us.  Their constants are fits to steps back to back on a B200, 340 of them
+// (heads of 32 to 128, 1 to 256 rows, 0 to 2048 shared and 4 to 4000 own tokens, every shape of blocks and clusters): the shape they
+// pick is 1 % from the best one in the mean, and the way they pick loses at most a few per cent.
+// Some of them, items or any-geometry kernel -> here: 8 heads of 128, 4 rows of 200 tokens 8.1 -> 5.8; 32 heads, 1 row of 1500
+// 12.1 -> 8.4, of 4000 16.9 -> 14.1; 32 heads, 4 rows of 256 shared and 200 own 10.9 -> 8.7; 16 rows over 256 shared 11.7 -> 9.0;
+// 12 heads of 64, 16 rows of 500 shared and 250 own 11.5 -> 8.1.  Larger steps belong to the items: 64 rows of 1100 tokens, 8 heads,
+// 52 against 59 (CTAs of units that differ cannot take over from each other), 16 rows of 2048 shared and 1100 own, 32 heads, 62 against 69.
+void build_direct(Plan& plan, int mode, int d_head, bool items) {
+    plan.direct_cluster = 0;
+    plan.direct_entries.clear();
+    plan.direct_ranges.clear();
+    plan.direct_blocks.clear();
+    // planning costs time at every change of the tree, too: about 1 us per 1000 chunks
+    constexpr int MAX_INFOS = 8192;
+    constexpr int64_t MAX_ITEM_BYTES = 70000000;
+    if (mode == 0 || plan.n_seqs == 0) return;
+    const int64_t H = plan.n_heads, pairs = H * plan.n_seqs;
+    if (mode == 1 && ((int64_t)plan.infos.size() > MAX_INFOS || (items && (plan.n_items_short > 0 || plan.stats.unique_kv_bytes > MAX_ITEM_BYTES)))) return;
+    const bool small = d_head <= 64;  // the instances of up to 64 elements: more CTAs on an SM
+    const double step_us = 2.0 * DIRECT_STEP * d_head * 2 / 15.6e6;  // bytes of a step at the rate of the L2
+    double best = 0;
+    int rows = 1, cluster = 1;
+    // steps of every block of 1, 2, 4 and 8 rows: differences of what several rows share, and what one row has alone
+    constexpr int SIZES = 4;
+    static_assert(1 << (SIZES - 1) == DIRECT_ROWS, "block sizes");
+    std::vector<int64_t> own((size_t)plan.n_seqs, 0), diff[SIZES], steps;
+    bool any_shared = false;
+    for (int k = 0; k < SIZES; k++) diff[k].assign((size_t)((plan.n_seqs - 1) >> k) + 2, 0);
+    for (const ca_chunk_info& ci : plan.infos) {
+        const int s = direct_steps(plan, ci);
+        if (ci.seq_end - ci.seq_begin == 1) {
+            own[ci.seq_begin] += s;
+        } else {
+            any_shared = true;
+            for (int k = 0; k < SIZES; k++) {
+                diff[k][ci.seq_begin >> k] += s;
+                diff[k][((ci.seq_end - 1) >> k) + 1] -= s;
+            }
+        }
+    }
+    for (int k = 0; k < SIZES; k++) {
+        const int R = 1 << k;
+        if (R > 1 && R / 2 >= plan.n_seqs) break;
+        const int n_blocks = (plan.n_seqs + R - 1) / R;
+        steps.assign((size_t)n_blocks, 0);
+        int64_t shared = 0;
+        for (int b = 0; b < n_blocks; b++) steps[b] = shared += diff[k][b];
+        for (int s = 0; s < plan.n_seqs; s++) steps[s >> k] += own[s];
+        int64_t total = 0, longest = 0;
+        for (int64_t s : steps) {
+            total += s;
+            longest = std::max(longest, s);
+        }
+        for (int c = 1; c <= DIRECT_MAX_CLUSTER; c *= 2) {
+            // clusters do not fill every SM
+            const double W = waves((double)n_blocks * H * c, B200_SMS * (small ? 4 : 3) * (c == 8 ? 0.9 : c == 4 ? 0.95 : 1.0));
+            const double per_warp = (double)((longest + c * DIRECT_WARPS - 1) / (c * DIRECT_WARPS));
+            const double t = W * ((small ? 3.2 : 3.3) + (small ? 0.48 : 0.61) * per_warp) + (c > 1 ? 1.5 : 0.0) + (double)(total * H) * step_us;
+            if ((R == 1 && c == 1) || t < best) {
+                best = t;
+                rows = R;
+                cluster = c;
+            }
+        }
+    }
+    double other;
+    double margin = 0.95;
+    if (items) {  // two launches, K/V at HBM rate; shared runs bring a partial result per row and piece
+        other = 7.8 + (double)plan.stats.unique_kv_bytes / 6.9e6 + (plan.stats.n_runs > 0 ? 3.5e-3 * (double)pairs + 0.03 * plan.max_merge_len : 0.0);
+    } else {      // the any-geometry kernel: every row walks its whole path
+        const int block = d_head <= 32 ? 32 : 16;
+        int64_t c = 1, total = 0;
+        while (c < 8 && pairs * c * 2 <= 4 * B200_SMS && c * 4 * block < plan.max_path_tokens) c *= 2;
+        for (int32_t n : plan.path_tokens) total += n;
+        const double per_warp = (double)(((plan.max_path_tokens + block - 1) / block + 4 * c - 1) / (4 * c));
+        const double W = waves((double)(pairs * c), B200_SMS * (small ? 7.0 : 4.0));
+        if (d_head > 32) margin = small ? 1.3 : (any_shared ? 1.05 : 0.95);
+        other = 3.0 + W * (1.0 + (small ? 0.5 : 1.1) * per_warp) + (c > 1 ? 0.7 : 0.0) + (double)(total * H) * d_head * 4 / 20e6;
+    }
+    if (mode == 2 || best < margin * other) cut_direct(plan, rows, cluster);
+}
 
 // The root-to-leaf chunk list of every row (CSR), read by the any-geometry kernel only.
 void build_paths(Plan& plan) {

@@ -47,6 +47,13 @@ constexpr int WIDE_MIN_ROWS = 32;
 constexpr double WIDE_MMA_SYNC_FLOPS = 200e12;
 constexpr double WIDE_HBM_BYTES_PER_S = 6.4e12;
 
+// The one-launch kernel (ca_attn_direct.cu) works on blocks of rows instead of items.
+constexpr int DIRECT_ROWS = 8;        // rows of a block at most: the columns of mma.sync
+constexpr int DIRECT_WARPS = 4;       // warps of a CTA
+constexpr int DIRECT_STEP = 16;       // tokens a warp takes at a time
+constexpr int DIRECT_MAX_CLUSTER = 8; // CTAs that share a block of rows
+constexpr int DIRECT_TO_THE_END = 1 << 20;  // end of a range that takes all of its last chunk, tokens appended since included
+
 struct PlanItem {
     int32_t n_tiles;      // 1 .. MAX_TILES_PER_ITEM
     int32_t first;        // position of the item's first token (plans with a window; else 0)
@@ -77,6 +84,12 @@ struct Plan {
     std::vector<int32_t> path_off, path_chunks, path_tokens;
     int max_path_tokens = 0;              // of the longest path
     std::vector<int32_t> tail_chunk, tail_tokens;
+    // the one-launch kernel's form of the work; direct_cluster == 0: the step goes by items
+    int direct_cluster = 0;                // CTAs per (block of rows, head)
+    int direct_rows = 0;                   // rows of the longest block
+    std::vector<int32_t> direct_entries;   // [4]: chunk, tokens, rows of the block that see it (bits), 1 for a tail; block by block
+    std::vector<int32_t> direct_ranges;    // [blocks][cluster * DIRECT_WARPS][4]: first entry and step, last entry and its end step
+    std::vector<int32_t> direct_blocks;    // [blocks][2]: first row, rows
     ca_plan_stats stats{};
 };
 
@@ -94,6 +107,9 @@ std::string build_plan(Plan& plan, const ca_chunk_info* infos, int n_infos, int 
                        bool one_partial_per_row = false,   // items of shared runs do not emit a partial per token split
                        int window = 0,  // > 0: chunks that lie before the window of every row they serve are left out
                        bool even_items = false);  // items of about equal size, as many as fill whole waves of n_ctas CTAs
+// Fills Plan::direct_* where the one-launch kernel is the faster way (mode 1) or always (mode 2).  items: else the step goes by
+// items, not by the any-geometry kernel.
+void build_direct(Plan& plan, int mode, int d_head, bool items);
 // The per-row path lists (path_off / path_chunks / path_tokens) from plan.infos, for a plan built without them.
 void build_paths(Plan& plan);
 

@@ -151,6 +151,9 @@ CA_API int ca_context_create_shaped(ca_context** out, int device, const ca_head_
 /* Contexts with a head shape, portions of prompts in bf16 with 64-token chunks and heads of 64 or 128 elements: 1 (default)
  * the tcgen05 kernel, softmax weights as two bf16 numbers; 2 the same with one bf16 number; 0 the mma.sync kernel. */
 #define CA_OPT_SPAN_TENSOR 11
+/* Steps of fp16 caches with d_head <= 128 in one launch instead of partial results and their combination: 1 (default) where
+ * that is faster, 0 never, 2 always. */
+#define CA_OPT_DIRECT 12
 /* Failure-path tests only: the CTA that draws item `value` of the next launches (portions of prompts on tcgen05: piece
  * `value`, key/value heads fastest) stops feeding its consumer warps, whose bounded wait then runs out (status 1; portions:
  * 1 or 2).  -1 (default) switches it off. */
@@ -592,6 +595,11 @@ CA_API int ca_attention_static_status(int32_t* status, ca_stream stream);
 #define CA_PLAN_TAIL_TOKENS 9    /* int32[n_seqs]                                                */
 #define CA_PLAN_WIDE_CHUNKS 10   /* int32[]: chunk lists of the wide items (an item's first chunk entry
                                     is its offset here); empty when wide_runs is 0               */
+#define CA_PLAN_DIRECT_ENTRIES 11 /* int32[][4], block of rows by block: chunk, tokens, rows of the block that see it
+                                    (bits), 1 for a tail                                          */
+#define CA_PLAN_DIRECT_RANGES 12 /* int32[blocks][warps][4]: first entry and 16-token step of a warp's range, last entry
+                                    and the step it ends before (1 << 20: the entry's end); first > last: nothing */
+#define CA_PLAN_DIRECT_BLOCKS 13 /* int32[blocks][2]: first row, rows                            */
 /* wide_runs: the meaning of CA_OPT_WIDE_RUNS (0 never, 1 by cost, 2 every shared run) */
 CA_API int ca_plan_build(ca_plan** out, const ca_chunk_info* infos, int n_infos, int n_seqs,
                          int n_heads, int chunk_size, int tpp_threshold, int n_ctas,
@@ -601,6 +609,10 @@ CA_API int ca_plan_build(ca_plan** out, const ca_chunk_info* infos, int n_infos,
  * position of its first token. */
 CA_API int ca_plan_build_windowed(ca_plan** out, const ca_chunk_info* infos, int n_infos, int n_seqs, int chunk_size,
                                   int tpp_threshold, int n_ctas, int64_t max_chunks, int rows_per_item, int window);
+/* Adds the form of the work that the one-launch kernel takes (CA_OPT_DIRECT; mode: its meaning), for heads of d_head elements;
+ * against_items: the alternative is the list of items (else the any-geometry kernel).  Returns in *cluster the CTAs per block of
+ * rows and head, 0 when the step does not go that way. */
+CA_API int ca_plan_direct(ca_plan* plan, int mode, int d_head, int against_items, int* cluster);
 CA_API int ca_plan_array(const ca_plan* plan, int which, const int32_t** data, int64_t* count);
 CA_API int ca_plan_stats_get(const ca_plan* plan, ca_plan_stats* out);
 /* One work list for several contexts.  The caches of a model's layers see the same tree at every step, so

@@ -1,0 +1,135 @@
+"""The one-launch kernel against dense attention in 64 bits, and against the kernels it stands in for."""
+import numpy as np
+import pytest
+import torch
+
+from chunk_attn import cabi
+from gpu_helpers import CabiEngine
+from test_gpu_kernel_edges import dense
+
+pytestmark = pytest.mark.gpu
+
+
+def engine(H, d, chunk, max_chunks, mode=2):
+    eng = CabiEngine(H, d, chunk, torch.float16, max_chunks=max_chunks)
+    eng.ctx.set_option(cabi.CA_OPT_DIRECT, mode)
+    return eng
+
+
+def fill(eng, g, shared, lens, scale=1.0):
+    """Sequences of `lens` own tokens over `shared` common ones; their contexts by row."""
+    H, d = eng.H, eng.d
+    rnd = lambda n: (torch.randn(n, H, d, generator=g) * scale).half()
+    pk, pv = rnd(shared), rnd(shared)
+    ctx = []
+    for i, n in enumerate(lens):
+        k, v = torch.cat([pk, rnd(n)]), torch.cat([pv, rnd(n)])
+        row = eng.add_seq(list(range(shared)) + [10_000 * (i + 1) + j for j in range(n)], k, v)
+        ctx.insert(row, (k, v))
+    return ctx
+
+
+# Scores and sums are fp32, weights have 22 bits (or fp16's 11 with 64-token chunks of 128, where they had them before); what is
+# left is the rounding of the result: 2^-11 of values that are below 2 here, and the repository's bar for fp16 above it.
+TOL = 1e-3
+
+
+@pytest.mark.parametrize("d,chunk", [(128, 64), (128, 32), (64, 64), (64, 16), (96, 40), (72, 24), (40, 64), (32, 16), (8, 17), (120, 64)])
+@pytest.mark.parametrize("shared,lens", [(0, [1]), (0, [15, 16, 17]), (0, [700]), (64, [1, 63, 64, 65]), (130, [5, 5, 5, 5, 5]), (200, [33] * 8),
+                                         (100, [7] * 9), (64, [300, 1, 20] * 6)])
+def test_edges(d, chunk, shared, lens):
+    # instances of every width, 1 to 8 rows a block and several blocks, clusters of every size, ranges that end inside a chunk.
+    # The pool's unused rows hold NaN.
+    H = 3
+    g = torch.Generator().manual_seed(d + chunk + shared)
+    eng = engine(H, d, chunk, max_chunks=sum(n // chunk + 3 for n in lens) + shared // chunk + 4)
+    ctx = fill(eng, g, shared, lens)
+    q = torch.randn(len(lens), H, d, generator=g).half()
+    for step in range(3):  # tokens beyond what the work list says
+        got = eng.forward(q).cpu().double()
+        assert eng.ctx.stats()["kernels_per_step"] == 1
+        assert (got - dense(q, ctx, d ** -0.5)).abs().max() < TOL
+        k1, v1 = torch.randn(len(lens), H, d, generator=g).half(), torch.randn(len(lens), H, d, generator=g).half()
+        eng.append_token([7] * len(lens), k1, v1)
+        ctx = [(torch.cat([k, a[None]]), torch.cat([v, b[None]])) for (k, v), a, b in zip(ctx, k1, v1)]
+
+
+@pytest.mark.parametrize("d,chunk", [(128, 64), (64, 32)])
+def test_two_levels_and_scores_that_rise(d, chunk):
+    # groups of rows over prompts of their own: the rows that see a chunk change along a warp's range; scores that grow by
+    # more than the step in which the reference follows them, and by less
+    H, g = 2, torch.Generator().manual_seed(5)
+    eng = engine(H, d, chunk, max_chunks=200)
+    root = (torch.randn(2 * chunk, H, d, generator=g).half(), torch.randn(2 * chunk, H, d, generator=g).half())
+    ctx = []
+    for i in range(11):
+        grp = torch.Generator().manual_seed(i // 3)
+        gk, gv = torch.randn(chunk, H, d, generator=grp).half() * 2, torch.randn(chunk, H, d, generator=grp).half()
+        own = 20 + 13 * i
+        k = torch.cat([root[0], gk, torch.randn(own, H, d, generator=g).half() * torch.linspace(0.5, 6, own)[:, None, None]]).half()
+        v = torch.cat([root[1], gv, torch.randn(own, H, d, generator=g).half()])
+        row = eng.add_seq(list(range(2 * chunk)) + [500 * (i // 3 + 1) + j for j in range(chunk)] + [10_000 * (i + 1) + j for j in range(own)], k, v)
+        ctx.insert(row, (k, v))
+    q = torch.randn(11, H, d, generator=g).half()
+    assert (eng.forward(q).cpu().double() - dense(q, ctx, d ** -0.5)).abs().max() < 2 * TOL  # values up to 4
+
+
+@pytest.mark.parametrize("d,chunk", [(128, 64), (64, 64)])
+def test_a_row_with_infinities_stays_alone(d, chunk):
+    H, g, lens = 2, torch.Generator().manual_seed(9), [50, 90, 20, 64]
+    eng = engine(H, d, chunk, max_chunks=40)
+    rnd = lambda n: torch.randn(n, H, d, generator=g).half()
+    pk, pv = rnd(chunk), rnd(chunk)
+    ctx = []
+    for i, n in enumerate(lens):
+        k, v = torch.cat([pk, rnd(n)]), torch.cat([pv, rnd(n)])
+        if i == 1:
+            v[chunk + 3], k[chunk + 5] = float("inf"), float("nan")
+        eng.add_seq(list(range(chunk)) + [1000 * (i + 1) + j for j in range(n)], k, v)
+        ctx.append((k, v))
+    q = rnd(4)
+    got, want = eng.forward(q).cpu().double(), dense(q, ctx, d ** -0.5)
+    assert torch.isnan(got[1]).all()
+    keep = [0, 2, 3]
+    assert (got[keep] - want[keep]).abs().max() < TOL
+
+
+def test_the_same_as_the_other_kernels():
+    # one switch between them, the same tree: results differ by roundings only, and a row without tokens is zero both ways
+    for d, chunk in ((128, 64), (80, 32)):
+        H, g = 4, torch.Generator().manual_seed(3)
+        eng = engine(H, d, chunk, max_chunks=80)
+        fill(eng, g, 2 * chunk, [30, 1, 77, 64, 5])
+        q = torch.randn(5, H, d, generator=g).half()
+        out = {}
+        for mode in (0, 1, 2):
+            eng.ctx.set_option(cabi.CA_OPT_DIRECT, mode)
+            eng.valid = False
+            out[mode] = eng.forward(q).float()
+        assert (out[0] - out[2]).abs().max() < TOL and (out[0] - out[1]).abs().max() < TOL
+        # queries that do not lie on 16 bytes: what was taken before is taken still, by the any-geometry kernel
+        if d != 128:
+            odd = torch.empty(q.numel() + 1, dtype=torch.float16, device="cuda")[1:].view(q.shape).copy_(q)
+            res = torch.empty_like(q, device="cuda")
+            eng.ctx.attention(odd, res, 0)
+            assert (res.float() - out[0]).abs().max() < TOL
+
+
+def test_captured_and_replayed():
+    H, d, chunk, g = 4, 64, 32, torch.Generator().manual_seed(1)
+    eng = engine(H, d, chunk, max_chunks=40)
+    ctx = fill(eng, g, 40, [20, 50])
+    q = torch.randn(2, H, d, generator=g).half().cuda()
+    out = torch.empty_like(q)
+    eng.refresh()
+    torch.cuda.synchronize()
+    stream = torch.cuda.Stream()
+    with torch.cuda.stream(stream):
+        eng.ctx.attention(q, out, 0)
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=stream):
+            eng.ctx.attention(q, out, 0)
+    q.copy_(torch.randn(2, H, d, generator=g).half())
+    graph.replay()
+    torch.cuda.synchronize()
+    assert (out.cpu().double() - dense(q.cpu(), ctx, d ** -0.5)).abs().max() < TOL
