@@ -119,6 +119,7 @@ struct ca_context {
     int trace_ctas = 0;                   // CTAs of the last traced launch
     int trace_cycles = 0;                 // CA_OPT_TRACE = 2: the tcgen05 kernel accounts for cycles per role instead
     int opt_direct = 1;                   // CA_OPT_DIRECT
+    int opt_finish_in_wide = 1;           // CA_OPT_FINISH_IN_WIDE
     int opt_finish_in_tails = 1;          // CA_OPT_FINISH_IN_TAILS: the short-tails kernel finishes the rows when it can
     bool out_is_host = false;             // set by ca_attention_host around its launches: the rows go to host memory
 
@@ -130,6 +131,9 @@ struct ca_context {
         int64_t n_merge_slots = 0;  // entries of merge_slots
         int max_merge_len = 0;
         bool split_phases = false;
+        int wide_pieces = 0;           // Plan::wide_pieces
+        int32_t short_slot_base = 0;
+        int64_t tail_rounds = 0;       // 8-token rounds of all tails at the refresh
         int direct_cluster = 0, direct_blocks = 0, direct_rows = 0;  // Plan::direct_*
         ca_plan_stats stats{};
     } meta;
@@ -337,6 +341,10 @@ int ca_context_set_option(ca_context* c, int option, int64_t value) {
     } else if (option == CA_OPT_FINISH_IN_TAILS) {
         if (value != 0 && value != 1) return fail(CA_ERR_INVALID, "CA_OPT_FINISH_IN_TAILS takes 0 or 1");
         c->opt_finish_in_tails = (int)value;
+        return CA_OK;
+    } else if (option == CA_OPT_FINISH_IN_WIDE) {
+        if (value < 0 || value > 2) return fail(CA_ERR_INVALID, "CA_OPT_FINISH_IN_WIDE takes 0, 1 or 2");
+        c->opt_finish_in_wide = (int)value;
         return CA_OK;
     } else if (option == CA_OPT_SPAN_TENSOR) {
         if (value < 0 || value > 2) return fail(CA_ERR_INVALID, "CA_OPT_SPAN_TENSOR takes 0, 1 or 2");
@@ -547,6 +555,10 @@ static int upload_plan(ca_context* c, const ca::Plan& pl, cudaStream_t stream) {
     c->meta.n_merge_slots = (int64_t)pl.merge_slots.size();
     c->meta.max_merge_len = pl.max_merge_len;
     c->meta.split_phases = pl.split_phases;
+    c->meta.wide_pieces = pl.wide_pieces;
+    c->meta.short_slot_base = pl.short_slot_base;
+    c->meta.tail_rounds = 0;
+    for (int32_t t : pl.tail_tokens) c->meta.tail_rounds += (t + 7) / 8;
     c->meta.direct_cluster = pl.direct_cluster;
     c->meta.direct_rows = pl.direct_rows;
     c->meta.direct_blocks = (int)(pl.direct_blocks.size() / 2);
@@ -607,6 +619,21 @@ static bool tails_can_finish(const ca_context* c) {
                                !(c->meta.short_all_empty && c->delta_tokens == 0)));
 }
 
+// True when the wide-runs kernel does the whole step: all rows are in one run, cut into at most two pieces, and have nothing
+// beside it but a short tail; and where that is faster.  A CTA's tails are walked by few warps, so they must be few beside its tiles, and
+// every SM needs its CTAs.  32 heads, steps back to back, two or three kernels -> one, in us: 1000 rows of 2048 shared and 4 / 20 / 40 own
+// tokens 67 / 105 / 153 -> 58 / 93 / 153; of 512 shared and 4 / 20 (8 tiles a CTA, 3 rounds of 8 tokens a row) 41 / 78 -> 36 / 79; 560 rows of
+// 2048 and 20 (160 CTAs on 148 SMs) 68 -> 76; 830 (224 CTAs) 92 -> 85; 400 of 512 and 4 (4 tiles) 23 -> 25.
+static bool wide_can_finish(const ca_context* c) {
+    if (!c->fast || !c->opt_finish_in_tails || !c->opt_finish_in_wide || c->opt_overlap || c->trace || c->meta.split_phases || c->meta.n_items_wide == 0 ||
+        c->meta.n_items_short != c->meta.n_seqs || c->meta.n_items_short + c->meta.n_items_wide != c->meta.n_items || c->meta.wide_pieces < 1 ||
+        c->meta.wide_pieces > 2)
+        return false;
+    const double H = c->geo.n_heads, ctas = c->meta.n_items_wide * H, tiles = (double)c->meta.n_wide_chunks / c->meta.wide_pieces,
+                 rounds = (c->meta.tail_rounds + c->meta.n_seqs * (c->delta_tokens / 8.0)) * H / (128 * ctas);
+    return c->opt_finish_in_wide == 2 || (tiles >= 8 && tiles >= 4 * rounds && (ctas >= 1.46 * c->num_sms));
+}
+
 // The partial results of a step.  finish != null and tails_can_finish(): the short-tails kernel goes LAST and stores the
 // output rows described by *finish; *finished tells the caller that no merge is needed.
 static int run_partials(ca_context* c, const void* q, int n_seqs, int phases, ca_stream stream_, const ca::MergeParams* finish,
@@ -659,8 +686,9 @@ static int run_partials(ca_context* c, const void* q, int n_seqs, int phases, ca
     // first (the short tails before the wide runs, whose set-up then overlaps them) so that the persistent kernel's
     // tail leads straight into the merge.
     const int n_items = c->meta.n_items - c->meta.n_items_short - c->meta.n_items_wide;
-    const bool finish_in_tails = finish && finished && phases == 3 && tails_can_finish(c);
-    const bool run_short = !finish_in_tails && c->meta.n_items_short > 0 && (phases & 2) &&
+    const bool finish_in_wide = finish && finished && phases == 3 && wide_can_finish(c);
+    const bool finish_in_tails = !finish_in_wide && finish && finished && phases == 3 && tails_can_finish(c);
+    const bool run_short = !finish_in_tails && !finish_in_wide && c->meta.n_items_short > 0 && (phases & 2) &&
                            !(c->meta.short_all_empty && c->delta_tokens == 0);
     const bool run_wide = c->meta.n_items_wide > 0 && (phases & 1);
     // The short tails are bound by memory, the wide runs by the tensor and special-function pipes, and they touch
@@ -702,6 +730,18 @@ static int run_partials(ca_context* c, const void* q, int n_seqs, int phases, ca
         w.trace_cycles = c->trace_cycles;
         c->trace_ctas = (w.item_hi - w.item_lo) < kTraceCtas ? (w.item_hi - w.item_lo) : 0;
         if (c->trace_ctas == 0) w.trace = nullptr;
+        if (finish_in_wide) {
+            ca::WideFinish f;
+            f.pieces = c->meta.wide_pieces;
+            f.tail_chunk = c->d_tail_chunk;
+            f.tail_tokens = c->d_tail_tokens;
+            f.delta_tokens = c->delta_tokens;
+            f.slot0 = c->meta.short_slot_base;
+            f.out = *finish;
+            CA_CUDA(ca::launch_attn_wide(w, stream, (c->opt_pdl & 2) != 0, &f));
+            *finished = true;
+            return CA_OK;
+        }
         CA_CUDA(ca::launch_attn_wide(w, stream, (c->opt_pdl & 2) != 0));
     }
     if (beside) CA_CUDA(cudaStreamWaitEvent(stream, c->ev_join, 0));
@@ -1489,7 +1529,7 @@ int ca_context_stats(const ca_context* c, ca_plan_stats* out) {
     if (!c || !out) return fail(CA_ERR_INVALID, "null argument");
     if (!c->valid) return fail(CA_ERR_STATE, "work list is stale");
     *out = c->meta.stats;
-    if (goes_direct(c)) out->kernels_per_step = 1;
+    if (goes_direct(c) || wide_can_finish(c)) out->kernels_per_step = 1;
     else if (tails_can_finish(c)) out->kernels_per_step -= 1;  // the short-tails kernel stores the rows: no merge launch
     else if (c->meta.short_all_empty && c->delta_tokens == 0) out->kernels_per_step -= 1;  // nothing to do for empty tails
     return CA_OK;

@@ -91,8 +91,6 @@ struct WideParams {
                                           // S, [5] that thread from S ready to P handed over, [7] bits 0-47 the MMA thread
                                           // waiting for the K tile, bits 48-63 the SM the CTA ran on
 };
-cudaError_t launch_attn_wide(const WideParams& p, cudaStream_t stream, bool dependent_launch = false);
-cudaError_t configure_wide_kernel();  // once per device before the first launch
 
 constexpr int MERGE_MAX_PEERS = 8;
 struct MergeParams {
@@ -117,6 +115,19 @@ struct MergeParams {
     int* status = nullptr;       // and STATUS_BAD_WORK_LIST recorded here (0 / null: unchecked)
 };
 cudaError_t launch_attn_merge(const MergeParams& p, cudaStream_t stream, bool dependent_launch);
+
+// The wide items of a step whose rows are all in one run and have nothing beside it but a short private tail: the kernel
+// walks the tails, too, and stores finished rows.
+struct WideFinish {
+    int pieces = 1;              // of a block of rows: 1 or 2, the CTAs of a cluster; every block has that many
+    const int32_t* tail_chunk = nullptr;   // [n_seqs]
+    const int32_t* tail_tokens = nullptr;  // [n_seqs], when the plan was built
+    int delta_tokens = 0;
+    int slot0 = 0;               // partial row of row 0's tail, as numbered per item
+    MergeParams out;             // where the rows go
+};
+cudaError_t launch_attn_wide(const WideParams& p, cudaStream_t stream, bool dependent_launch = false, const WideFinish* finish = nullptr);
+cudaError_t configure_wide_kernel();  // once per device before the first launch
 
 constexpr int STATUS_PEER_WAIT_TIMEOUT = 6;   // a peer did not reach the barrier within the time allowed
 // One-phase barrier among the ranks of a node over flag words in each other's memory: rank r stores `epoch` into

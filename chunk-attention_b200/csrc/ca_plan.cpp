@@ -301,6 +301,7 @@ std::string build_plan(Plan& plan, const ca_chunk_info* infos, int n_infos, int 
     plan.items.clear();
     plan.wide_chunks.clear();
     plan.n_items_wide = 0;
+    plan.wide_pieces = 0;
     plan.merge_slots.clear();
     plan.path_chunks.clear();
     plan.path_tokens.clear();
@@ -539,6 +540,7 @@ std::string build_plan(Plan& plan, const ca_chunk_info* infos, int n_infos, int 
             // pieces of 2 .. 32 chunks, equal up to one
             int n_pieces = std::min(pieces_wanted, std::max(1, n_chunks / 2));
             n_pieces = std::max(n_pieces, (n_chunks + WIDE_MAX_TILES - 1) / WIDE_MAX_TILES);
+            if (runs.size() == 1 && n == n_seqs) plan.wide_pieces = n_pieces;
             const int32_t list_off = (int32_t)plan.wide_chunks.size();
             plan.wide_chunks.insert(plan.wide_chunks.end(), r.chunks.begin(), r.chunks.end());
             for (int blk = 0; blk < n_blocks; blk++) {

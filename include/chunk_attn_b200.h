@@ -151,6 +151,9 @@ CA_API int ca_context_create_shaped(ca_context** out, int device, const ca_head_
 /* Contexts with a head shape, portions of prompts in bf16 with 64-token chunks and heads of 64 or 128 elements: 1 (default)
  * the tcgen05 kernel, softmax weights as two bf16 numbers; 2 the same with one bf16 number; 0 the mma.sync kernel. */
 #define CA_OPT_SPAN_TENSOR 11
+/* Steps whose rows are all in one wide run and have nothing beside it but a short tail: the wide-runs kernel walks the tails, too,
+ * and stores finished rows (needs CA_OPT_FINISH_IN_TAILS): 1 (default) where that is faster, 0 never, 2 always. */
+#define CA_OPT_FINISH_IN_WIDE 13
 /* Steps of fp16 caches with d_head <= 128 in one launch instead of partial results and their combination: 1 (default) where
  * that is faster, 0 never, 2 always. */
 #define CA_OPT_DIRECT 12
