@@ -120,6 +120,7 @@ struct ca_context {
     int trace_cycles = 0;                 // CA_OPT_TRACE = 2: the tcgen05 kernel accounts for cycles per role instead
     int opt_direct = 1;                   // CA_OPT_DIRECT
     int opt_finish_in_wide = 1;           // CA_OPT_FINISH_IN_WIDE
+    int opt_latent_rows = 1;              // CA_OPT_LATENT_ROWS
     int opt_finish_in_tails = 1;          // CA_OPT_FINISH_IN_TAILS: the short-tails kernel finishes the rows when it can
     bool out_is_host = false;             // set by ca_attention_host around its launches: the rows go to host memory
 
@@ -132,6 +133,7 @@ struct ca_context {
         int max_merge_len = 0;
         bool split_phases = false;
         int wide_pieces = 0;           // Plan::wide_pieces
+        int max_item_tiles = 0;
         int32_t short_slot_base = 0;
         int64_t tail_rounds = 0;       // 8-token rounds of all tails at the refresh
         int direct_cluster = 0, direct_blocks = 0, direct_rows = 0;  // Plan::direct_*
@@ -346,6 +348,10 @@ int ca_context_set_option(ca_context* c, int option, int64_t value) {
         if (value < 0 || value > 2) return fail(CA_ERR_INVALID, "CA_OPT_FINISH_IN_WIDE takes 0, 1 or 2");
         c->opt_finish_in_wide = (int)value;
         return CA_OK;
+    } else if (option == CA_OPT_LATENT_ROWS) {
+        if (value < 0 || value > 2) return fail(CA_ERR_INVALID, "CA_OPT_LATENT_ROWS takes 0, 1 or 2");
+        c->opt_latent_rows = (int)value;
+        return CA_OK;
     } else if (option == CA_OPT_SPAN_TENSOR) {
         if (value < 0 || value > 2) return fail(CA_ERR_INVALID, "CA_OPT_SPAN_TENSOR takes 0, 1 or 2");
         c->opt_span_tensor = (int)value;
@@ -394,7 +400,7 @@ static std::string plan_for(const ca_context* c, ca::Plan& plan, const ca_chunk_
     // short tails or wide runs
     return ca::build_plan(plan, infos, n_infos, n_seqs, c->geo.n_heads, c->geo.chunk_size, c->tpp_threshold, n_ctas, c->max_chunks,
                           false, d_mean, c->geo.esize, c->items, /*seq_first_tensor=*/false,
-                          /*wide_mode=*/0, /*want_paths=*/!c->items, 64 / c->group, /*one_partial_per_row=*/true, c->shape.window,
+                          /*wide_mode=*/0, /*want_paths=*/!c->items || c->shape.latent, 64 / c->group, /*one_partial_per_row=*/true, c->shape.window,
                           /*even_items=*/c->shape.latent != 0);
 }
 
@@ -556,6 +562,8 @@ static int upload_plan(ca_context* c, const ca::Plan& pl, cudaStream_t stream) {
     c->meta.max_merge_len = pl.max_merge_len;
     c->meta.split_phases = pl.split_phases;
     c->meta.wide_pieces = pl.wide_pieces;
+    c->meta.max_item_tiles = 0;
+    for (const ca::PlanItem& it : pl.items) c->meta.max_item_tiles = std::max(c->meta.max_item_tiles, (int)it.n_tiles);
     c->meta.short_slot_base = pl.short_slot_base;
     c->meta.tail_rounds = 0;
     for (int32_t t : pl.tail_tokens) c->meta.tail_rounds += (t + 7) / 8;
@@ -1230,6 +1238,30 @@ int ca_latent_store(ca_context* c, const ca_latent_store_args* a, ca_stream stre
     return CA_OK;
 }
 
+// CTAs that take a sequence's decode (0: the step goes by items, whose partials a second kernel combines), by estimates in us of
+// which way is faster.  Measured, items -> sequences: 32 heads, 148 sequences of 40 / 200 tokens 14.3 / 20.2 -> 10.7 / 15.5, 110 of 1000
+// 39.9 -> 36.6, 74 of 1000 (two CTAs each) 27.1 -> 24.9; not for 37 of 1000 (three CTAs each) 16.9 -> 19.7, 8 of 4000 16.7 -> 23.4.
+static int latent_pieces(const ca_context* c, int delta_tokens) {
+    if (!c->opt_latent_rows || !c->paths_on_device || c->meta.n_items_cf > 0 || c->meta.n_seqs == 0 || !ca::latent_rows_finishes(c->geo, c->shape.n_heads))
+        return 0;
+    const double n = c->meta.n_seqs, H = c->shape.n_heads, split = std::ceil(H / 64);  // CTAs take up to 64 heads
+    int longest = c->max_path_tokens + delta_tokens;
+    if (c->shape.window > 0) longest = std::min(longest, c->shape.window + 63);
+    const double tiles = (longest + 63) / 64, sms = c->num_sms;
+    const double items = 7 + std::ceil(c->meta.n_items * split / sms) * (2 + 1.4 * c->meta.max_item_tiles) + 0.03 * n * H / 32 + (c->meta.n_items > n ? 0.03 * n : 0);
+    double best = 1e30;
+    int pieces = 0;
+    for (int P = 1; P <= ca::LATENT_MAX_PIECES; P++) {
+        if (P > 1 && n * P * split > sms) break;
+        const double t = 2 + std::ceil(n * P * split / sms) * (7 + 1.4 * std::ceil(tiles / P)) + (P > 1 ? 1.5 : 0) + (H > 32 ? 1 : 0);
+        if (t < best) {
+            best = t;
+            pieces = P;
+        }
+    }
+    return c->opt_latent_rows == 2 || best < 0.97 * items ? pieces : 0;
+}
+
 int ca_latent_attention(ca_context* c, const ca_latent_args* a, ca_stream stream_) {
     if (!c || !a) return fail(CA_ERR_INVALID, "null argument");
     if (!c->shape.latent) return fail(CA_ERR_INVALID, "latent_attention needs a latent context");
@@ -1284,6 +1316,12 @@ int ca_latent_attention(ca_context* c, const ca_latent_args* a, ca_stream stream
         p.part_width = c->geo.d_value;
         p.merge_off = c->d_merge_off;
         p.merge_slots = c->d_merge_slots;
+        p.pieces = latent_pieces(c, p.delta_tokens);
+        if (p.pieces > 0) {
+            p.path_off = c->d_path_off;
+            p.path_chunks = c->d_path_chunks;
+            p.tail_tokens = c->d_tail_tokens;
+        }
     }
     cudaStream_t stream = static_cast<cudaStream_t>(stream_);
     if (c->items) CA_CUDA(ca::launch_latent_rows(p, stream));

@@ -245,6 +245,7 @@ struct LatentStoreParams {
 };
 cudaError_t launch_latent_store(const LatentStoreParams& p, int dtype, cudaStream_t stream);
 
+constexpr int LATENT_MAX_PIECES = 2;
 struct LatentParams {
     const void* pool;
     Geometry geo;
@@ -275,12 +276,16 @@ struct LatentParams {
     int part_width;
     const int32_t* merge_off;
     const int32_t* merge_slots;
+    // decode by sequences: a cluster of `pieces` CTAs (up to LATENT_MAX_PIECES) each, over path_off / path_chunks; 0: the items
+    int pieces = 0;
+    const int32_t* tail_tokens;
     int max_chunks;
     int* status;
     long long wait_limit;
 };
 cudaError_t launch_latent_generic(const LatentParams& p, int dtype, cudaStream_t stream);  // portions, any geometry
 bool latent_rows_serves(const Geometry& g);
+bool latent_rows_finishes(const Geometry& g, int n_heads);  // decode by sequences
 cudaError_t launch_latent_rows(const LatentParams& p, cudaStream_t stream);                // bf16, 64-token chunks
 
 // portions of prompts on tcgen05, keys and values expanded (ca_latent_span.cu)

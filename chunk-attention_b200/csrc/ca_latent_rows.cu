@@ -14,11 +14,18 @@
 //                 side in one product; 64: one after the other); A = the same staged rows read the other way
 // Cache rows arrive by 1-D TMA bulk copies, verbatim (the pool's lines are the swizzled operand layout), in a ring of
 // 16 KiB units: two 64-element panels of a 64-token chunk, released one by one as the second product has used them.  Decode
-// emits one partial per row and item, combined by a merge kernel; portions emit finished rows.
+// emits one partial per row and item, combined by a merge kernel; or, where sequences share nothing and are many, a CTA or a
+// cluster of two takes a sequence, results meet in distributed shared memory and the rows are finished (ROWS; the rule is in
+// ca_abi.cu).  Portions emit finished rows.
+// What sets the pace of decode: a tile takes 1.4 us of a CTA (32 heads, 576 elements a token), whether it comes from HBM or the L2: 36
+// products of 128 x 64 x 16 from shared memory and the softmax between them; a CTA's start (set-up, queries, first scores) 4 to 5 us, its
+// end 2 to 4.
 // Warp roles: 0-7 softmax and epilogue, 8 TMA producer, 9 TMEM and the first product's issue, 10 the second one's.
 //
 // Every wait is bounded: on expiry a status code is recorded, every role runs out without waiting further, nothing is
 // stored, and the TMEM columns are freed at the common exit.
+#include <cooperative_groups.h>
+
 #include <algorithm>
 
 #include "ca_kernels.h"
@@ -62,8 +69,76 @@ template <int N> __host__ __device__ inline Layout layout_of(int gpr, int units)
     return l;
 }
 
-template <int N, bool SPAN>
-__global__ void __launch_bounds__(L_THREADS) latent_rows_kernel(const LatentParams p, int units) {
+// What a block of query rows is: rows of the decode items' token ranges, consecutive tokens of a portion, or all heads of a sequence's
+// last token, whose chunks the CTAs of a cluster share.
+enum { ITEMS, PORTIONS, ROWS };
+
+// ROWS: the softmax warps combine the cluster's results for the rows (heads) that are this CTA's, rank, rank + P, ..., with the sink, and
+// store bf16: factors of every result first, then sums, a thread for four elements of every second row, four rows under way.
+__device__ __forceinline__ void finish_rows(const LatentParams& p, int P, const cooperative_groups::cluster_group& cl, const uint8_t* stage, const float2* ml_s, float* factor_s,
+                                            int rank, int n_rows, int head0, __nv_bfloat16* out, int tid) {
+    const int mine = (n_rows - rank + P - 1) / P, width = p.geo.d_value;
+    if (tid < mine) {
+        const int row = rank + tid * P;
+        float2 ml[LATENT_MAX_PIECES];
+        float M = p.sink ? p.sink[head0 + row] * L_LOG2E : L_NEG_BIG, sink = M;
+#pragma unroll
+        for (int q = 0; q < LATENT_MAX_PIECES; q++) {
+            ml[q] = make_float2(L_NEG_BIG, 0.f);
+            if (q < P) ml[q] = (P > 1 ? cl.map_shared_rank(ml_s, q) : ml_s)[row];
+        }
+#pragma unroll
+        for (int q = 0; q < LATENT_MAX_PIECES; q++) M = fmaxf(M, ml[q].x);
+        float L = p.sink ? fast_exp2(sink - M) : 0.f;
+#pragma unroll
+        for (int q = 0; q < LATENT_MAX_PIECES; q++) {
+            ml[q].x = fast_exp2(ml[q].x - M);
+            L = fmaf(ml[q].x, ml[q].y, L);
+        }
+        const float inv = L > 0.f ? 1.f / L : 0.f;
+#pragma unroll
+        for (int q = 0; q < LATENT_MAX_PIECES; q++) factor_s[tid * LATENT_MAX_PIECES + q] = ml[q].x * inv;
+    }
+    softmax_warps_sync();
+    constexpr int AHEAD = 4;
+    for (int e = 4 * (tid & 127); e < width; e += 512)
+        for (int i0 = tid >> 7; i0 < mine; i0 += 2 * AHEAD) {
+            float4 acc[AHEAD];
+#pragma unroll
+            for (int u = 0; u < AHEAD; u++) acc[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+            for (int q = 0; q < P; q++) {
+                const float* from = reinterpret_cast<const float*>(P > 1 ? cl.map_shared_rank(stage, q) : stage) + e;
+                float4 v[AHEAD];
+#pragma unroll
+                for (int u = 0; u < AHEAD; u++) v[u] = i0 + 2 * u < mine ? *reinterpret_cast<const float4*>(from + (rank + (i0 + 2 * u) * P) * width) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+                for (int u = 0; u < AHEAD; u++) {
+                    const float w = i0 + 2 * u < mine ? factor_s[(i0 + 2 * u) * LATENT_MAX_PIECES + q] : 0.f;
+                    acc[u].x = fmaf(w, v[u].x, acc[u].x);
+                    acc[u].y = fmaf(w, v[u].y, acc[u].y);
+                    acc[u].z = fmaf(w, v[u].z, acc[u].z);
+                    acc[u].w = fmaf(w, v[u].w, acc[u].w);
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < AHEAD; u++) {
+                if (i0 + 2 * u >= mine) break;
+                __nv_bfloat16* dst = out + (size_t)(rank + (i0 + 2 * u) * P) * p.kv_rank + e;
+                if (p.kv_rank % 4 == 0) {
+                    if (e < p.kv_rank) *reinterpret_cast<uint2*>(dst) = make_uint2(pack_bf16(acc[u].x, acc[u].y), pack_bf16(acc[u].z, acc[u].w));
+                } else {
+                    const float x[4] = {acc[u].x, acc[u].y, acc[u].z, acc[u].w};
+#pragma unroll
+                    for (int k = 0; k < 4; k++)
+                        if (e + k < p.kv_rank) dst[k] = __float2bfloat16_rn(x[k]);
+                }
+            }
+        }
+}
+
+template <int N, int MODE>
+__global__ void __launch_bounds__(L_THREADS) latent_rows_kernel(const __grid_constant__ LatentParams p, int units) {
+    constexpr bool SPAN = MODE == PORTIONS;
     extern __shared__ __align__(1024) uint8_t smem[];
     constexpr int TPR = L_SOFT / N, PER = L_TOK / TPR;  // threads of a row, tokens of a thread
     constexpr int CH = N < 32 ? N : 32;              // TMEM columns read at a time
@@ -79,11 +154,28 @@ __global__ void __launch_bounds__(L_THREADS) latent_rows_kernel(const LatentPara
     const uint32_t full = smem_u32(bar_mem), empty = full + 8 * L_MAX_UNITS, s_full = empty + 8 * L_MAX_UNITS, p_full = s_full + 16,
                    o_done = p_full + 8, q_ready = o_done + 8, s_empty = q_ready + 8;
     float* const alpha_s = reinterpret_cast<float*>(bar_mem + 2 * L_MAX_UNITS + 7);  // [N]
-    int* const flag_s = reinterpret_cast<int*>(alpha_s + L_MAX_ROWS);                 // [2]
-    uint32_t* const tmem_slot = reinterpret_cast<uint32_t*>(flag_s + 2);
+    int* const flag_s = reinterpret_cast<int*>(alpha_s + L_MAX_ROWS);                 // [2], and warps that staged their results
+    uint32_t* const tmem_slot = reinterpret_cast<uint32_t*>(flag_s + 3);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int H = p.n_heads;
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");  // the merge kernel may be set up; it waits for this one's end
+    if (tid == 0) {
+        for (int i = 0; i < units; i++) {
+            mbar_init(full + 8 * i, 1);
+            mbar_init(empty + 8 * i, 1);
+        }
+        mbar_init(s_full, 1);
+        mbar_init(s_full + 8, 1);
+        mbar_init(p_full, L_SOFT);
+        mbar_init(o_done, 1);
+        mbar_init(q_ready, L_SOFT);
+        mbar_init(s_empty, L_SOFT / 32);
+        mbar_init(s_empty + 8, L_SOFT / 32);
+        flag_s[0] = flag_s[1] = flag_s[2] = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    // launched as a programmatic dependent: set up while the kernel ahead drains, nothing in global memory is touched before it is complete
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
     // ---- the block of rows and its tokens: [start, end) relative to position `first` of list[0]
     int token0, n_rows, first, end, low, row_lo = (int)blockIdx.y * N, slot_base = 0;
@@ -98,6 +190,14 @@ __global__ void __launch_bounds__(L_THREADS) latent_rows_kernel(const LatentPara
         list = p.path_chunks + p.path_off[b.x];
         end = p.positions[token0 + (row_lo + n_rows - 1) / H] + 1;
         low = p.positions[token0 + row_lo / H];
+    } else if (MODE == ROWS) {
+        token0 = blockIdx.x / p.pieces;
+        n_rows = min(N, H - row_lo);
+        first = 0;
+        const int begin = p.path_off[token0], chunks = p.path_off[token0 + 1] - begin;
+        list = p.path_chunks + begin;
+        end = max(0, chunks - 1) * L_TOK + min(L_TOK, p.tail_tokens[token0] + p.delta_tokens);
+        low = p.positions[token0];
     } else {
         const int4* it = p.items + 4 * blockIdx.x;
         const int4 a = __ldg(it), b = __ldg(it + 1);  // tiles, first, row, rows | slot, flags, last, chunks ...
@@ -112,25 +212,15 @@ __global__ void __launch_bounds__(L_THREADS) latent_rows_kernel(const LatentPara
         low = p.positions[token0];
         for (int i = 1; i < a.w; i++) low = min(low, p.positions[token0 + i]);
     }
-    const int start = p.window > 0 ? max(0, low - p.window + 1 - first) / L_TOK * L_TOK : 0;
+    int start = p.window > 0 ? max(0, low - p.window + 1 - first) / L_TOK * L_TOK : 0;
+    if (MODE == ROWS && end > start) {  // this CTA's share of the tiles
+        const int all = (end - start + L_TOK - 1) / L_TOK, piece = blockIdx.x % p.pieces, to = start + all * (piece + 1) / p.pieces * L_TOK;
+        start += all * piece / p.pieces * L_TOK;
+        end = min(end, to);
+    }
     const int n_tiles = end > start ? (end - start + L_TOK - 1) / L_TOK : 0;
     const int tail = end - start - (n_tiles - 1) * L_TOK;  // tokens of the last tile
 
-    if (tid == 0) {
-        for (int i = 0; i < units; i++) {
-            mbar_init(full + 8 * i, 1);
-            mbar_init(empty + 8 * i, 1);
-        }
-        mbar_init(s_full, 1);
-        mbar_init(s_full + 8, 1);
-        mbar_init(p_full, L_SOFT);
-        mbar_init(o_done, 1);
-        mbar_init(q_ready, L_SOFT);
-        mbar_init(s_empty, L_SOFT / 32);
-        mbar_init(s_empty + 8, L_SOFT / 32);
-        flag_s[0] = flag_s[1] = 0;
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
     // Only the stored tokens of the last tile are copied.  The lines behind them meet weights of zero, so they only have to be
     // finite: they are cleared in the units that tile will use (what earlier tiles bring there is finite, too).
     if (n_tiles > 0 && tail < L_TOK) {
@@ -159,10 +249,12 @@ __global__ void __launch_bounds__(L_THREADS) latent_rows_kernel(const LatentPara
         if (lane == 0) {
             int issued = 0, slot = 0, parity = 1;
             bool live = true;
+            int next = n_tiles > 0 ? __ldg(list + start / L_TOK) : 0;  // a tile ahead: the lookup would hold up every tile's copies
             for (int j = 0; j < n_tiles && live; j++) {
                 const int at = start + j * L_TOK;
                 const uint32_t bytes = min(L_TOK, end - at) * 128;
-                int chunk = __ldg(list + at / L_TOK);
+                int chunk = next;
+                if (j + 1 < n_tiles) next = __ldg(list + at / L_TOK + 1);
                 if (chunk < 0 || chunk >= p.max_chunks) {
                     report(p.status, STATUS_BAD_WORK_LIST);
                     chunk = 0;
@@ -505,6 +597,8 @@ __global__ void __launch_bounds__(L_THREADS) latent_rows_kernel(const LatentPara
                     total = l * fast_exp2(m_used - M) + fast_exp2(sk - M);
                 }
                 f = total > 0.f ? fast_exp2(m_used - M) / total : 0.f;
+            } else if (MODE == ROWS) {
+                reinterpret_cast<float2*>(sc)[row] = make_float2(m_used, l);  // the scores' place
             } else if (row < n_rows && live) {
                 p.part_ml[((size_t)slot_base + rr / H) * H + head] = make_float2(m_used, l);
             }
@@ -539,6 +633,10 @@ __global__ void __launch_bounds__(L_THREADS) latent_rows_kernel(const LatentPara
 #pragma unroll
                             for (int i = 0; i < CH; i++, out += p.kv_rank)
                                 if (c + i < n_rows) *out = __float2bfloat16_rn(__uint_as_float(o[i]) * alpha_s[c + i]);
+                    } else if (MODE == ROWS) {  // the ring is free: every product is complete
+                        if (e < p.geo.d_value)
+#pragma unroll
+                            for (int i = 0; i < CH; i++) reinterpret_cast<uint32_t*>(smem)[(c + i) * p.geo.d_value + e] = o[i];
                     } else if (e < p.part_width) {
 #pragma unroll
                         for (int i = 0; i < CH; i++, part_o += p.part_width)
@@ -546,7 +644,21 @@ __global__ void __launch_bounds__(L_THREADS) latent_rows_kernel(const LatentPara
                     }
                 }
             }
+            if (MODE == ROWS && lane == 0) atomicAdd(flag_s + 2, 1);
         }
+    }
+    if (MODE == ROWS) {
+        const cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
+        __syncwarp();
+        if (p.pieces > 1) cl.sync();
+        else __syncthreads();
+        bool valid = warp < L_SOFT / 32;
+        for (int q = 0; q < p.pieces; q++) valid = valid && (p.pieces > 1 ? cl.map_shared_rank(flag_s, q) : flag_s)[2] == L_SOFT / 32;
+        if (valid)  // else a wait ran out: the status says so, the rows keep what they held
+            finish_rows(p, p.pieces, cl, smem, reinterpret_cast<const float2*>(sc), sc + 2 * N, blockIdx.x % p.pieces, n_rows, row_lo,
+                        static_cast<__nv_bfloat16*>(p.out) + ((size_t)token0 * H + row_lo) * p.kv_rank, tid);
+        __syncwarp();
+        if (p.pieces > 1) cl.sync();  // the other CTAs' shared memory is read until here
     }
     // ---- common exit: nobody touches TMEM after this barrier, then the allocating warp frees it
     tc_fence_before_thread_sync();
@@ -614,21 +726,41 @@ __global__ void __launch_bounds__(128) latent_merge_kernel(const LatentParams p)
 constexpr int L_SMEM_LIMIT = 227 * 1024;
 constexpr int L_CONTROL = (2 * L_MAX_UNITS + 7) * 8 + L_MAX_ROWS * 4 + 16;  // barriers, row factors, flags, TMEM address
 
-template <int N> cudaError_t launch(const LatentParams& p, cudaStream_t stream) {
-    const int tile_units = ((p.geo.gpr >> 3) + 1) / 2, fixed = layout_of<N>(p.geo.gpr, 0).end + L_CONTROL;
+template <int N> int units_for(const Geometry& g) {
     // three tiles keep the copies ahead of the products; more would only keep other CTAs off the SM
-    const int units = std::min({L_MAX_UNITS, 3 * tile_units, (L_SMEM_LIMIT - fixed) / L_UNIT});
-    if (units < tile_units + 1) return cudaErrorInvalidValue;
+    const int tile_units = ((g.gpr >> 3) + 1) / 2, fixed = layout_of<N>(g.gpr, 0).end + L_CONTROL;
+    return std::min({L_MAX_UNITS, 3 * tile_units, (L_SMEM_LIMIT - fixed) / L_UNIT});
+}
+// ROWS stages O in the ring's place
+template <int N> bool stages(const Geometry& g) { return (size_t)N * g.d_value * 4 <= (size_t)std::max(0, units_for<N>(g)) * L_UNIT; }
+
+template <int N, int MODE> cudaError_t launch(const LatentParams& p, cudaStream_t stream) {
+    const int tile_units = ((p.geo.gpr >> 3) + 1) / 2, fixed = layout_of<N>(p.geo.gpr, 0).end + L_CONTROL;
+    const int units = units_for<N>(p.geo);
+    if (units < tile_units + 1 || (MODE == ROWS && !stages<N>(p.geo))) return cudaErrorInvalidValue;
     const int smem = units * L_UNIT + fixed;
-    const int rows = p.path_off ? p.block_rows * p.n_heads : std::max(p.n_heads, p.item_rows);
-    auto* span = latent_rows_kernel<N, true>;
-    auto* items = latent_rows_kernel<N, false>;
-    auto* k = p.path_off ? span : items;
+    const int rows = MODE == PORTIONS ? p.block_rows * p.n_heads : (MODE == ROWS ? p.n_heads : std::max(p.n_heads, p.item_rows));
+    auto* k = latent_rows_kernel<N, MODE>;
     cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
     if (e != cudaSuccess) return e;
-    k<<<dim3(p.path_off ? p.n_blocks : p.n_items, (rows + N - 1) / N), L_THREADS, smem, stream>>>(p, units);
-    return cudaGetLastError();
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(MODE == PORTIONS ? p.n_blocks : (MODE == ROWS ? p.n_rows * p.pieces : p.n_items), (rows + N - 1) / N);
+    cfg.blockDim = dim3(L_THREADS);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = MODE == ROWS ? p.pieces : 1;
+    attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = MODE == ROWS && p.pieces > 1 ? 2 : 1;
+    return cudaLaunchKernelEx(&cfg, k, p, units);
+}
+template <int MODE> cudaError_t launch_mode(const LatentParams& p, int rows, cudaStream_t stream) {
+    return rows <= 16 ? launch<16, MODE>(p, stream) : (rows <= 32 ? launch<32, MODE>(p, stream) : launch<64, MODE>(p, stream));
 }
 
 }  // namespace
@@ -637,10 +769,15 @@ bool latent_rows_serves(const Geometry& g) {
     return g.esize == 2 && g.chunk_size == L_TOK && g.swz && g.d_head <= 640 && g.d_value <= 512;
 }
 
+bool latent_rows_finishes(const Geometry& g, int n_heads) {
+    return latent_rows_serves(g) && (n_heads <= 16 ? stages<16>(g) : (n_heads <= 32 ? stages<32>(g) : stages<64>(g)));
+}
+
 cudaError_t launch_latent_rows(const LatentParams& p, cudaStream_t stream) {
-    const int rows = p.path_off ? p.block_rows * p.n_heads : std::max(p.n_heads, p.item_rows);
-    cudaError_t e = rows <= 16 ? launch<16>(p, stream) : (rows <= 32 ? launch<32>(p, stream) : launch<64>(p, stream));
-    if (e != cudaSuccess || p.path_off) return e;
+    if (p.pieces > 0) return launch_mode<ROWS>(p, p.n_heads, stream);
+    if (p.path_off) return launch_mode<PORTIONS>(p, p.block_rows * p.n_heads, stream);
+    const cudaError_t e = launch_mode<ITEMS>(p, std::max(p.n_heads, p.item_rows), stream);
+    if (e != cudaSuccess) return e;
     const int64_t pairs = (int64_t)p.n_rows * p.n_heads;
     if (pairs > 0x7fffffff) return cudaErrorInvalidValue;
     cudaLaunchConfig_t cfg{};

@@ -154,6 +154,9 @@ CA_API int ca_context_create_shaped(ca_context** out, int device, const ca_head_
 /* Steps whose rows are all in one wide run and have nothing beside it but a short tail: the wide-runs kernel walks the tails, too,
  * and stores finished rows (needs CA_OPT_FINISH_IN_TAILS): 1 (default) where that is faster, 0 never, 2 always. */
 #define CA_OPT_FINISH_IN_WIDE 13
+/* Decode steps of latent caches whose sequences share nothing: a CTA or two for every sequence, one launch, instead of items whose
+ * partial results a second kernel combines: 1 (default) where that is faster, 0 never, 2 always. */
+#define CA_OPT_LATENT_ROWS 14
 /* Steps of fp16 caches with d_head <= 128 in one launch instead of partial results and their combination: 1 (default) where
  * that is faster, 0 never, 2 always. */
 #define CA_OPT_DIRECT 12
