@@ -383,7 +383,9 @@ static int ctas_of(const ca_context* c) { return c->opt_ctas > 0 ? c->opt_ctas :
 
 // CA_OPT_DIRECT as it counts for this context: options that choose among the kernels of the item lists choose those kernels
 static int direct_mode(const ca_context* c) {
-    if (c->shaped || !ca::attn_direct_serves(c->geo) || c->opt_split || c->opt_ctas > 0 || !c->opt_sf_tensor || c->opt_wide != 1) return 0;
+    if (c->opt_split || c->opt_ctas > 0 || !c->opt_sf_tensor || c->opt_wide != 1) return 0;
+    if (c->shaped ? c->shape.latent || c->dtype != CA_DTYPE_BF16 || !ca::attn_direct_serves_grouped(c->geo, c->shape, c->group) : !ca::attn_direct_serves(c->geo))
+        return 0;
     return c->opt_direct;
 }
 
@@ -398,10 +400,12 @@ static std::string plan_for(const ca_context* c, ca::Plan& plan, const ca_chunk_
     const int d_mean = c->shape.latent ? c->geo.d_head / 2 : (c->geo.d_head + c->geo.d_value) / 2;
     // items of up to 64 query rows (a sequence brings `group` of them), one partial per row; no kernel of their own for
     // short tails or wide runs
-    return ca::build_plan(plan, infos, n_infos, n_seqs, c->geo.n_heads, c->geo.chunk_size, c->tpp_threshold, n_ctas, c->max_chunks,
+    const std::string err = ca::build_plan(plan, infos, n_infos, n_seqs, c->geo.n_heads, c->geo.chunk_size, c->tpp_threshold, n_ctas, c->max_chunks,
                           false, d_mean, c->geo.esize, c->items, /*seq_first_tensor=*/false,
                           /*wide_mode=*/0, /*want_paths=*/!c->items || c->shape.latent, 64 / c->group, /*one_partial_per_row=*/true, c->shape.window,
                           /*even_items=*/c->shape.latent != 0);
+    if (err.empty()) ca::build_direct(plan, direct_mode(c), c->geo.d_head, /*items=*/true, c->group);
+    return err;
 }
 
 int ca_refresh_kernel_context(ca_context* c, const ca_chunk_info* infos, int n_infos, int n_seqs, ca_stream stream_) {
@@ -897,8 +901,8 @@ static bool goes_direct(const ca_context* c, const void* q = nullptr, const void
            (reinterpret_cast<uintptr_t>(c->pool) | reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(out)) % 16 == 0;
 }
 
-// peers: the rows go into the outputs it names instead of `out`
-static int run_direct(ca_context* c, const void* q, void* out, const ca::MergeParams* peers, ca_stream stream_) {
+// peers: the rows go into the outputs it names instead of `out`.  rows: the step of a context with a head shape
+static int run_direct(ca_context* c, const void* q, void* out, const ca::MergeParams* peers, const ca_rows_args* rows, ca_stream stream_) {
     DeviceGuard guard(c->device);
     if (guard.err != cudaSuccess) return fail_cuda(guard.err, "cudaSetDevice");
     ca::DirectParams d;
@@ -923,6 +927,14 @@ static int run_direct(ca_context* c, const void* q, void* out, const ca::MergePa
     d.one_weight = c->fast;
     d.max_chunks = (int)(c->max_chunks < INT32_MAX ? c->max_chunks : INT32_MAX);
     d.status = c->status;
+    if (rows) {
+        d.group = c->group;
+        d.scale_log2 = c->shape.scale * 1.4426950408889634f;
+        d.sink = c->shape.sink;
+        d.positions = rows->positions;
+        d.value_freq = rows->value_freq;
+        d.zero_if_none = 1;
+    }
     if (peers) {
         d.n_peers = peers->n_peers;
         d.total_heads = peers->total_heads;
@@ -951,7 +963,7 @@ int ca_attention_to_peers(ca_context* c, const void* q, void* const* peer_out, i
     m.head_offset = head_offset;
     for (int i = 0; i < n_peers; i++) m.peer_out[i] = peer_out[i];
     m.mc_out = multicast_out;
-    if (goes_direct(c, q)) return run_direct(c, q, nullptr, &m, stream_);
+    if (goes_direct(c, q)) return run_direct(c, q, nullptr, &m, nullptr, stream_);
     bool finished = false;
     rc = run_partials(c, q, n_seqs, 3, stream_, &m, &finished);
     if (rc != CA_OK) return rc;
@@ -1005,7 +1017,7 @@ int ca_attention(ca_context* c, const void* q, void* out, int n_seqs, int partit
     if (partition < 0 || partition > 2) return fail(CA_ERR_INVALID, "Unsupported partition type");
     if (n_seqs == 0) return CA_OK;
     if (!out) return fail(CA_ERR_INVALID, "out is null");
-    if (partition != CA_PARTITION_SEQ_FIRST && goes_direct(c, q, out)) return run_direct(c, q, out, nullptr, stream_);
+    if (partition != CA_PARTITION_SEQ_FIRST && goes_direct(c, q, out)) return run_direct(c, q, out, nullptr, nullptr, stream_);
     if (c->fast && partition != CA_PARTITION_SEQ_FIRST) {
         const ca::MergeParams m = merge_params_of(c, out, n_seqs);
         bool finished = false;
@@ -1101,6 +1113,7 @@ int ca_attention_rows(ca_context* c, const ca_rows_args* a, ca_stream stream_) {
     DeviceGuard guard(c->device);
     if (guard.err != cudaSuccess) return fail_cuda(guard.err, "cudaSetDevice");
     cudaStream_t stream = static_cast<cudaStream_t>(stream_);
+    if (decode && goes_direct(c, a->q, a->out)) return run_direct(c, a->q, a->out, nullptr, a, stream_);
     if (c->dtype == CA_DTYPE_BF16) {
         ca::RowsParams r{};
         r.pool = c->pool;

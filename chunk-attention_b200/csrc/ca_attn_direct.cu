@@ -1,15 +1,16 @@
-// Decode attention of small steps in ONE launch (fp16 caches, rows of whole 16-byte granules, d_head <= 128).
+// Decode attention of small steps in ONE launch: fp16 caches with rows of whole 16-byte granules and d_head <= 128, and bf16 caches of
+// grouped heads (1, 2, 4 or 8 query heads to a key/value head) of 64 or 128 elements.
 //
-// A unit is a key/value head and a block of up to 8 consecutive rows; its work is the list of chunks that any of the rows
-// sees, each with the set of rows that see it, so a shared chunk is read once for the block.  The list is cut into steps of 16
+// A unit is a key/value head and a block of up to 8 columns: consecutive rows, each with the query heads of the group; its work is the list of chunks that any of the rows
+// sees, each with the set of columns that see it, so a shared chunk is read once for the block.  The list is cut into steps of 16
 // tokens, dealt in consecutive ranges to the warps of a CLUSTER of 1 to 8 CTAs per unit (cut by the host, ca_plan.h).  A
 // warp takes K and V from global memory straight into registers, as the operands of mma.sync:
 //   S^T = K Q^T          lane (g, c) = (lane / 4, lane % 4) holds granules 4 j + c of tokens g and g + 8: their four registers are
 //                        the A operands of two MMAs (the contraction's order is free as long as q follows it)
 //   O^T += V^T P^T       lane (g, c) holds granules 8 i + g of tokens 2 c, 2 c + 1, 2 c + 8, 2 c + 9; byte permutes of two tokens'
 //                        registers give the A operands.  P goes from the one layout to the other by movmatrix, as the sum of two
-//                        fp16 numbers (22 bits of the fp32 weight)
-// The 8 columns of both products are the rows of the block.  When the set of rows changes along a warp's range, what it has
+//                        numbers of the cache's type (22 bits of the fp32 weight in fp16, 16 in bf16)
+// The 8 columns of both products are those of the block.  When the set of columns changes along a warp's range, what it has
 // is combined into the warp's own area of shared memory, for the rows that saw it only: what the other columns hold is
 // dropped, so a row's infinities never meet another row.  Areas are combined per CTA, and the CTAs' results through
 // distributed shared memory: no partial results in global memory, no second launch.
@@ -26,6 +27,7 @@
 #include <cuda_fp16.h>
 
 #include <cstdlib>
+#include <type_traits>
 
 #include "ca_kernels.h"
 #include "ca_plan.h"
@@ -43,19 +45,32 @@ __device__ __forceinline__ uint32_t transpose_8x8(uint32_t v) {
     asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(t) : "r"(v));
     return t;
 }
-__device__ __forceinline__ void mma_f16(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
-    asm volatile(
-        "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-        : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+template <typename T> __device__ __forceinline__ void mma_16bit(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+    if constexpr (std::is_same_v<T, __half>)
+        asm volatile(
+            "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+            : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+            : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+    else
+        asm volatile(
+            "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+            : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+            : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
-// weights as fp16 hi + lo pairs (column, column + 1)
-__device__ __forceinline__ void split_f16(float a, float b, uint32_t& hi, uint32_t& lo) {
-    const __half2 h = __floats2half2_rn(a, b);
-    const float2 f = __half22float2(h);
-    const __half2 r = __floats2half2_rn(a - f.x, b - f.y);
-    hi = *reinterpret_cast<const uint32_t*>(&h);
-    lo = *reinterpret_cast<const uint32_t*>(&r);
+template <typename T> __device__ __forceinline__ uint32_t pack_pair(float a, float b) {
+    if constexpr (std::is_same_v<T, __half>) return pack_half2(a, b);
+    const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
+    return *reinterpret_cast<const uint32_t*>(&h);
+}
+// weights as hi + lo pairs (column, column + 1)
+template <typename T> __device__ __forceinline__ void split_pair(float a, float b, uint32_t& hi, uint32_t& lo) {
+    hi = pack_pair<T>(a, b);
+    if constexpr (std::is_same_v<T, __half>) {
+        const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&hi));
+        lo = pack_pair<T>(a - f.x, b - f.y);
+    } else {
+        lo = pack_pair<T>(a - __uint_as_float(hi << 16), b - __uint_as_float(hi & 0xffff0000u));
+    }
 }
 
 constexpr float D_RESCALE_STEP = 8.f;  // a row's reference follows its maximum in steps of at least 2^8
@@ -70,7 +85,8 @@ template <int VG> struct DirectSmem {
 // KQ: groups of 4 granules of a K row; VG: groups of 8 granules of a V row; PANELS: the pool's swizzled layout (ca_layout.h).
 // LO: 0 weights as one fp16 number; 1 hi and lo in two products; 2 blocks of up to 4 rows, columns 4 .. 7 repeat the rows and take
 // the lo parts, so that one product does both.
-template <int KQ, int VG, bool PANELS, int LO, bool PEERS>
+// T bf16: grouped heads, with the sink and the values' turn of their layers.
+template <typename T, int KQ, int VG, bool PANELS, int LO, bool PEERS>
 __global__ void __launch_bounds__(D_WARPS * 32, VG == 2 ? 3 : 4) attn_direct_kernel(const DirectParams p) {
     using Smem = DirectSmem<VG>;
     constexpr int DV = Smem::DV, PITCH = Smem::PITCH;
@@ -87,8 +103,14 @@ __global__ void __launch_bounds__(D_WARPS * 32, VG == 2 ? 3 : 4) attn_direct_ker
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, c = lane & 3;
     const int4 range = __ldg(p.ranges + (size_t)block * (p.cluster * D_WARPS) + rank * D_WARPS + warp);  // entry, step | entry, step (end)
     const int2 rows = __ldg(p.blocks + block);
-    const int row_begin = rows.x, n_rows = rows.y;
+    constexpr bool GROUPED = std::is_same_v<T, __nv_bfloat16>;
+    const int row_begin = rows.x, n_rows = GROUPED ? rows.y * p.group : rows.y;  // from here on a row is a column: a row's query head
     const int C = p.chunk_size;
+    // (row, query head) of column n, numbered as in q and out
+    auto pair_of = [&](int n) {
+        if (!GROUPED) return (size_t)(row_begin + n) * p.n_heads + head;
+        return ((size_t)(row_begin + n / p.group) * p.n_heads + head) * p.group + n % p.group;
+    };
 
     // byte offsets of this lane's granules inside a tile, from token t0 on (a multiple of 16)
     const int row_bytes = PANELS ? 128 : p.gpr * 16;
@@ -164,7 +186,7 @@ __global__ void __launch_bounds__(D_WARPS * 32, VG == 2 ? 3 : 4) attn_direct_ker
     for (int j = 0; j < KQ; j++) {
         const int G = 4 * j + c, r = LO == 2 ? g & 3 : g;
         q[j] = make_uint4(0u, 0u, 0u, 0u);
-        if (r < n_rows && G < p.gpr) q[j] = __ldg(reinterpret_cast<const uint4*>(p.q) + ((size_t)(row_begin + r) * p.n_heads + head) * p.gpr + G);
+        if (r < n_rows && G < p.gpr) q[j] = __ldg(reinterpret_cast<const uint4*>(p.q) + pair_of(r) * p.gpr + G);
     }
 
     float o[VG * 4][4], m[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f};
@@ -180,8 +202,8 @@ __global__ void __launch_bounds__(D_WARPS * 32, VG == 2 ? 3 : 4) attn_direct_ker
         for (int k = 0; k < 4; k++) s2[0][k] = s2[1][k] = 0.f;
 #pragma unroll
         for (int j = 0; j < KQ; j++) {
-            mma_f16(s2[0], kr[j][0].x, kr[j][1].x, kr[j][0].y, kr[j][1].y, q[j].x, q[j].y);
-            mma_f16(s2[1], kr[j][0].z, kr[j][1].z, kr[j][0].w, kr[j][1].w, q[j].z, q[j].w);
+            mma_16bit<T>(s2[0], kr[j][0].x, kr[j][1].x, kr[j][0].y, kr[j][1].y, q[j].x, q[j].y);
+            mma_16bit<T>(s2[1], kr[j][0].z, kr[j][1].z, kr[j][0].w, kr[j][1].w, q[j].z, q[j].w);
         }
         advance();
         if (left > 0) load_k();
@@ -214,8 +236,8 @@ __global__ void __launch_bounds__(D_WARPS * 32, VG == 2 ? 3 : 4) attn_direct_ker
             l[h] += s[h] + s[2 + h];  // this lane's tokens
         }
         uint32_t hi0, lo0, hi1, lo1;
-        split_f16(s[0], s[1], hi0, lo0);
-        split_f16(s[2], s[3], hi1, lo1);
+        split_pair<T>(s[0], s[1], hi0, lo0);
+        split_pair<T>(s[2], s[3], hi1, lo1);
         if (LO == 2 && c >= 2) {
             hi0 = lo0;
             hi1 = lo1;
@@ -233,8 +255,8 @@ __global__ void __launch_bounds__(D_WARPS * 32, VG == 2 ? 3 : 4) attn_direct_ker
                 const uint32_t t0 = (&vr[i][0].x)[r], t1 = (&vr[i][1].x)[r], t8 = (&vr[i][2].x)[r], t9 = (&vr[i][3].x)[r];
                 const uint32_t a0 = __byte_perm(t0, t1, 0x5410), a1 = __byte_perm(t0, t1, 0x7632);
                 const uint32_t a2 = __byte_perm(t8, t9, 0x5410), a3 = __byte_perm(t8, t9, 0x7632);
-                mma_f16(o[i * 4 + r], a0, a1, a2, a3, hi0, hi1);
-                if (LO == 1) mma_f16(o[i * 4 + r], a0, a1, a2, a3, lo0, lo1);
+                mma_16bit<T>(o[i * 4 + r], a0, a1, a2, a3, hi0, hi1);
+                if (LO == 1) mma_16bit<T>(o[i * 4 + r], a0, a1, a2, a3, lo0, lo1);
             }
         if (left > 0) load_v();
         if (left <= 0 || mask != rows_here) {
@@ -351,46 +373,59 @@ __global__ void __launch_bounds__(D_WARPS * 32, VG == 2 ? 3 : 4) attn_direct_ker
     const cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
     if (p.cluster > 1) cl.sync();
     else __syncthreads();
-    // ---- the CTAs of the unit: the rows are dealt to them; eight lanes side by side hold eight elements of a row, each of another
-    // CTA's result, so that all are on their way at once
-    const int r = threadIdx.x & 7, mine = (n_rows - rank + p.cluster - 1) / p.cluster;
-    const float* from = p.cluster > 1 && r < p.cluster ? cl.map_shared_rank(area, r) : area;
+    // ---- the CTAs of the unit: the rows are dealt to them; as many lanes side by side as CTAs hold eight elements of a row, each of
+    // another CTA's result, so that all are on their way at once
+    const int r = threadIdx.x & (p.cluster - 1), mine = (n_rows - rank + p.cluster - 1) / p.cluster;
+    const float* from = p.cluster > 1 ? cl.map_shared_rank(area, r) : area;
     const float* from_m = from + (area_m - area);
-    for (int i = threadIdx.x >> 3; i < mine * (DV / 8); i += D_WARPS * 4) {
+    const uint32_t group = ((1u << p.cluster) - 1) << (lane - r);  // the lanes of a row's other elements may have left the loop
+    for (int i = threadIdx.x / p.cluster; i < mine * (DV / 8); i += D_WARPS * 32 / p.cluster) {
         const int n = rank + (i / (DV / 8)) * p.cluster, d = 8 * (i % (DV / 8));
-        float m_r = -INFINITY, sum = 0.f, v[8];
-        int seen = 0;
+        const float4 v0 = *reinterpret_cast<const float4*>(from + n * PITCH + d), v1 = *reinterpret_cast<const float4*>(from + n * PITCH + d + 4);
+        const float m_r = from_m[n];
+        float sum = from_m[D_WARPS * p.block_rows + n], mm = m_r, v[8] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w};
+        int seen = reinterpret_cast<const int*>(from_m)[2 * D_WARPS * p.block_rows];
+        if (p.cluster > 1) {
 #pragma unroll
-        for (int k = 0; k < 8; k++) v[k] = 0.f;
-        if (r < p.cluster) {
-            const float4 v0 = *reinterpret_cast<const float4*>(from + n * PITCH + d), v1 = *reinterpret_cast<const float4*>(from + n * PITCH + d + 4);
-            m_r = from_m[n];
-            sum = from_m[D_WARPS * p.block_rows + n];
-            seen = reinterpret_cast<const int*>(from_m)[2 * D_WARPS * p.block_rows];
-            v[0] = v0.x, v[1] = v0.y, v[2] = v0.z, v[3] = v0.w, v[4] = v1.x, v[5] = v1.y, v[6] = v1.z, v[7] = v1.w;
-        }
-        const uint32_t group = 0xffu << (threadIdx.x & 24);  // the lanes of a row's other elements may have left the loop
-        float mm = m_r;
+            for (int off = 1; off < DIRECT_MAX_CLUSTER; off <<= 1)
+                if (off < p.cluster) mm = fmaxf(mm, __shfl_xor_sync(group, mm, off));
+            const float a = fast_exp2(m_r - (mm == -INFINITY ? 0.f : mm));
+            sum *= a;
 #pragma unroll
-        for (int off = 1; off < 8; off <<= 1) mm = fmaxf(mm, __shfl_xor_sync(group, mm, off));
-        const float a = fast_exp2(m_r - (mm == -INFINITY ? 0.f : mm));
-        sum *= a;
+            for (int k = 0; k < 8; k++) v[k] *= a;
 #pragma unroll
-        for (int k = 0; k < 8; k++) v[k] *= a;
+            for (int off = 1; off < DIRECT_MAX_CLUSTER; off <<= 1) {
+                if (off >= p.cluster) break;
+                sum += __shfl_xor_sync(group, sum, off);
+                seen |= __shfl_xor_sync(group, seen, off);
 #pragma unroll
-        for (int off = 1; off < 8; off <<= 1) {
-            sum += __shfl_xor_sync(group, sum, off);
-            seen |= __shfl_xor_sync(group, seen, off);
-#pragma unroll
-            for (int k = 0; k < 8; k++) v[k] += __shfl_xor_sync(group, v[k], off);
+                for (int k = 0; k < 8; k++) v[k] += __shfl_xor_sync(group, v[k], off);
+            }
         }
         // a row with no token yields zeros; one whose scores are all -inf has no softmax (zeros where the work lists of items say so)
-        const float inv = mm == -INFINITY ? (((seen >> n) & 1) && !p.zero_if_none ? nanf("") : 0.f) : 1.f / sum;
+        float inv;
+        if (GROUPED && p.sink) {  // one more entry of score zero
+            const float top = fmaxf(mm, 0.f), keep = fast_exp2(mm - top);
+            inv = keep / (sum * keep + fast_exp2(-top));
+        } else {
+            inv = mm == -INFINITY ? (((seen >> n) & 1) && !p.zero_if_none ? nanf("") : 0.f) : 1.f / sum;
+        }
         if (r > 0 || d >= p.d) continue;
-        const uint4 packed = make_uint4(pack_half2(v[0] * inv, v[1] * inv), pack_half2(v[2] * inv, v[3] * inv), pack_half2(v[4] * inv, v[5] * inv),
-                                        pack_half2(v[6] * inv, v[7] * inv));
+        if (GROUPED && p.value_freq) {  // values were cached turned by their position: back by the row's
+            const float pos = (float)__ldg(p.positions + row_begin + n / p.group);
+#pragma unroll
+            for (int k = 0; k < 8; k += 2) {
+                float sn, cs;
+                fast_sincos(pos * __ldg(p.value_freq + (d + k) / 2), &sn, &cs);
+                const float x = v[k] * cs + v[k + 1] * sn;
+                v[k + 1] = v[k + 1] * cs - v[k] * sn;
+                v[k] = x;
+            }
+        }
+        const uint4 packed = make_uint4(pack_pair<T>(v[0] * inv, v[1] * inv), pack_pair<T>(v[2] * inv, v[3] * inv), pack_pair<T>(v[4] * inv, v[5] * inv),
+                                        pack_pair<T>(v[6] * inv, v[7] * inv));
         if (!PEERS) {
-            *reinterpret_cast<uint4*>(static_cast<__half*>(p.out) + ((size_t)(row_begin + n) * p.n_heads + head) * p.d + d) = packed;
+            *reinterpret_cast<uint4*>(static_cast<T*>(p.out) + pair_of(n) * p.d + d) = packed;
         } else {  // head-sharded: into every rank's full-width output, by the switch or by plain stores over NVLink
             const size_t to = ((size_t)(row_begin + n) * p.total_heads + p.head_offset + head) * p.d + d;
             if (p.mc_out) {
@@ -405,8 +440,8 @@ __global__ void __launch_bounds__(D_WARPS * 32, VG == 2 ? 3 : 4) attn_direct_ker
     if (p.cluster > 1) cl.sync();  // the other CTAs' shared memory is read until here
 }
 
-template <int KQ, int VG, bool PANELS, int LO, bool PEERS = false> cudaError_t launch(const DirectParams& p, cudaStream_t stream) {
-    auto* const kernel = attn_direct_kernel<KQ, VG, PANELS, LO, PEERS>;
+template <typename T, int KQ, int VG, bool PANELS, int LO, bool PEERS = false> cudaError_t launch(const DirectParams& p, cudaStream_t stream) {
+    auto* const kernel = attn_direct_kernel<T, KQ, VG, PANELS, LO, PEERS>;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)((int64_t)p.n_blocks * p.n_heads * p.cluster));
     cfg.blockDim = dim3(D_WARPS * 32);
@@ -436,14 +471,22 @@ template <int KQ, int VG, bool PANELS, int LO, bool PEERS = false> cudaError_t l
 bool attn_direct_serves(const Geometry& g) {
     return g.esize == 2 && g.epg == 8 && g.d_head == g.d_value && g.d_head <= 128 && g.chunk_size >= D_STEP;
 }
+bool attn_direct_serves_grouped(const Geometry& g, const ca_head_shape& shape, int group) {
+    return attn_direct_serves(g) && g.swz != 0 && shape.d_key == g.d_head && shape.d_value == g.d_head && group <= D_ROWS && (group & (group - 1)) == 0;
+}
 
 template <int KQ, int VG, bool PANELS> static cudaError_t launch_rows(const DirectParams& p, cudaStream_t stream) {
-    if constexpr (PANELS && VG == 2) {  // the geometry of the item lists
-        if (p.n_peers > 0) return p.block_rows <= 4 ? launch<KQ, VG, PANELS, 2, true>(p, stream) : launch<KQ, VG, PANELS, 0, true>(p, stream);
-        if (p.block_rows > 4 && p.one_weight) return launch<KQ, VG, PANELS, 0>(p, stream);
+    if constexpr (PANELS) {
+        if (p.group > 0)
+            return p.n_peers > 0 ? cudaErrorInvalidValue
+                                 : (p.block_rows <= 4 ? launch<__nv_bfloat16, KQ, VG, PANELS, 2>(p, stream) : launch<__nv_bfloat16, KQ, VG, PANELS, 1>(p, stream));
     }
-    if (p.n_peers > 0) return cudaErrorInvalidValue;
-    return p.block_rows <= 4 ? launch<KQ, VG, PANELS, 2>(p, stream) : launch<KQ, VG, PANELS, 1>(p, stream);
+    if constexpr (PANELS && VG == 2) {  // the geometry of the item lists
+        if (p.n_peers > 0) return p.block_rows <= 4 ? launch<__half, KQ, VG, PANELS, 2, true>(p, stream) : launch<__half, KQ, VG, PANELS, 0, true>(p, stream);
+        if (p.block_rows > 4 && p.one_weight) return launch<__half, KQ, VG, PANELS, 0>(p, stream);
+    }
+    if (p.n_peers > 0 || p.group > 0) return cudaErrorInvalidValue;
+    return p.block_rows <= 4 ? launch<__half, KQ, VG, PANELS, 2>(p, stream) : launch<__half, KQ, VG, PANELS, 1>(p, stream);
 }
 
 cudaError_t launch_attn_direct(const DirectParams& p, bool panels, cudaStream_t stream) {

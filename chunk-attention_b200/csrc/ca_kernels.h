@@ -142,7 +142,7 @@ struct PeerBarrierParams {
 };
 cudaError_t launch_peer_barrier(const PeerBarrierParams& p, cudaStream_t stream);
 
-// ---- small steps in one launch (ca_attn_direct.cu): fp16, rows of whole granules, d_head <= 128 ----------------
+// ---- small steps in one launch (ca_attn_direct.cu): fp16, rows of whole granules, d_head <= 128; bf16 grouped heads of 64 or 128 ----
 struct DirectParams {
     const uint8_t* pool;
     int n_heads, chunk_size, d, gpr;
@@ -153,7 +153,11 @@ struct DirectParams {
     const int4* ranges;          // Plan::direct_ranges
     const int2* blocks;          // Plan::direct_blocks
     int n_blocks, cluster;       // CTAs per block and head
-    int block_rows;              // of the longest block
+    int block_rows;              // columns (rows times heads of a group) of the longest block
+    int group = 0;               // bf16 caches: query heads per key/value head; 0: fp16
+    int sink = 0;                // bf16: one is added to the softmax denominator
+    const int32_t* positions = nullptr;  // bf16: [n_seqs], with value_freq
+    const float* value_freq = nullptr;   // bf16: null: values are not rotated
     int delta_tokens;
     float scale_log2;
     int zero_if_none;            // rows whose scores are all -inf: 1 zeros, 0 NaN
@@ -165,6 +169,7 @@ struct DirectParams {
     void* mc_out = nullptr;
 };
 bool attn_direct_serves(const Geometry& g);
+bool attn_direct_serves_grouped(const Geometry& g, const ca_head_shape& shape, int group);
 cudaError_t launch_attn_direct(const DirectParams& p, bool panels, cudaStream_t stream);
 
 // ---- generic path: any d_head <= 256, any chunk size, fp16, bf16 or fp32 -----------------------------

@@ -122,7 +122,7 @@ int direct_steps(const Plan& plan, const ca_chunk_info& ci, bool* tail = nullptr
 
 // Per block of rows the chunks that any of them sees, in depth-first order, and the ranges of steps that the warps of the
 // block's CTAs take.
-void cut_direct(Plan& plan, int rows_per_block, int cluster) {
+void cut_direct(Plan& plan, int rows_per_block, int cluster, int group) {
     const int n_seqs = plan.n_seqs, n_blocks = (n_seqs + rows_per_block - 1) / rows_per_block, warps = cluster * DIRECT_WARPS;
     std::vector<int32_t> first((size_t)n_blocks + 1, 0);
     std::vector<int64_t> steps((size_t)n_blocks, 0);
@@ -147,7 +147,7 @@ void cut_direct(Plan& plan, int rows_per_block, int cluster) {
         int32_t* e = plan.direct_entries.data() + 4 * (size_t)at[b]++;
         e[0] = ci.chunk_id;
         e[1] = ci.n_tokens;
-        e[2] = ((1 << hi) - 1) & ~((1 << lo) - 1);
+        e[2] = ((1 << hi * group) - 1) & ~((1 << lo * group) - 1);
         e[3] = tail ? 1 : 0;
     });
     plan.direct_blocks.resize((size_t)n_blocks * 2);
@@ -172,7 +172,7 @@ void cut_direct(Plan& plan, int rows_per_block, int cluster) {
         }
     }
     plan.direct_cluster = cluster;
-    plan.direct_rows = std::min(rows_per_block, n_seqs);
+    plan.direct_rows = std::min(rows_per_block, n_seqs) * group;
 }
 
 // Waves of CTAs: a second one costs as much as the first, many follow each other without a gap.
@@ -190,7 +190,8 @@ double waves(double ctas, double slots) {
 // 12.1 -> 8.4, of 4000 16.9 -> 14.1; 32 heads, 4 rows of 256 shared and 200 own 10.9 -> 8.7; 16 rows over 256 shared 11.7 -> 9.0;
 // 12 heads of 64, 16 rows of 500 shared and 250 own 11.5 -> 8.1.  Larger steps belong to the items: 64 rows of 1100 tokens, 8 heads,
 // 52 against 59 (CTAs of units that differ cannot take over from each other), 16 rows of 2048 shared and 1100 own, 32 heads, 62 against 69.
-void build_direct(Plan& plan, int mode, int d_head, bool items) {
+void build_direct(Plan& plan, int mode, int d_head, bool items, int group) {
+    const int columns = std::max(1, group);  // of a row
     plan.direct_cluster = 0;
     plan.direct_entries.clear();
     plan.direct_ranges.clear();
@@ -200,7 +201,7 @@ void build_direct(Plan& plan, int mode, int d_head, bool items) {
     constexpr int64_t MAX_ITEM_BYTES = 70000000;
     if (mode == 0 || plan.n_seqs == 0) return;
     const int64_t H = plan.n_heads, pairs = H * plan.n_seqs;
-    if (mode == 1 && ((int64_t)plan.infos.size() > MAX_INFOS || (items && (plan.n_items_short > 0 || plan.stats.unique_kv_bytes > MAX_ITEM_BYTES)))) return;
+    if (mode == 1 && ((int64_t)plan.infos.size() > MAX_INFOS || (items && group == 0 && (plan.n_items_short > 0 || plan.stats.unique_kv_bytes > MAX_ITEM_BYTES)))) return;
     const bool small = d_head <= 64;  // the instances of up to 64 elements: more CTAs on an SM
     const double step_us = 2.0 * DIRECT_STEP * d_head * 2 / 15.6e6;  // bytes of a step at the rate of the L2
     double best = 0;
@@ -225,7 +226,7 @@ void build_direct(Plan& plan, int mode, int d_head, bool items) {
     }
     for (int k = 0; k < SIZES; k++) {
         const int R = 1 << k;
-        if (R > 1 && R / 2 >= plan.n_seqs) break;
+        if (R > 1 && (R / 2 >= plan.n_seqs || R * columns > DIRECT_ROWS || (columns > 1 && !any_shared))) break;
         const int n_blocks = (plan.n_seqs + R - 1) / R;
         steps.assign((size_t)n_blocks, 0);
         int64_t shared = 0;
@@ -250,7 +251,15 @@ void build_direct(Plan& plan, int mode, int d_head, bool items) {
     }
     double other;
     double margin = 0.95;
-    if (items) {  // two launches, K/V at HBM rate; shared runs bring a partial result per row and piece
+    if (group > 0) {
+        // Grouped heads: their items cost more (every row of a group is a partial row), and large steps go this way, too, at 4.6 MB per us
+        // with values of 128 and 6 with 64, where the items reach 6.2 behind a longer start. Items -> here with 32 heads on 8 of 128: 1 row of
+        // 4000 tokens 22 -> 11.6 us, 16 rows of 200 10.4 -> 6.9, of 1000 22.4 -> 17.4, 256 of 200 47 -> 41; 64 of 1000 stay (45 against 47).
+        // 16 heads of 64, alone: 64 rows of 200 18.9 -> 11.9, of 1000 42.8 -> 37.2.
+        const double mb = (double)plan.stats.unique_kv_bytes * 1e-6;
+        best = std::max(best, 4.0 + mb / (small ? 6.0 : 4.6));
+        other = 9.0 + 0.16 * mb + 2.2e-3 * (double)(pairs * group) + 0.13 * plan.max_merge_len;
+    } else if (items) {  // two launches, K/V at HBM rate; shared runs bring a partial result per row and piece
         other = 7.8 + (double)plan.stats.unique_kv_bytes / 6.9e6 + (plan.stats.n_runs > 0 ? 3.5e-3 * (double)pairs + 0.03 * plan.max_merge_len : 0.0);
     } else {      // the any-geometry kernel: every row walks its whole path
         const int block = d_head <= 32 ? 32 : 16;
@@ -262,7 +271,7 @@ void build_direct(Plan& plan, int mode, int d_head, bool items) {
         if (d_head > 32) margin = small ? 1.3 : (any_shared ? 1.05 : 0.95);
         other = 3.0 + W * (1.0 + (small ? 0.5 : 1.1) * per_warp) + (c > 1 ? 0.7 : 0.0) + (double)(total * H) * d_head * 4 / 20e6;
     }
-    if (mode == 2 || best < margin * other) cut_direct(plan, rows, cluster);
+    if (mode == 2 || best < margin * other) cut_direct(plan, rows, cluster, columns);
 }
 
 // The root-to-leaf chunk list of every row (CSR), read by the any-geometry kernel only.

@@ -87,8 +87,8 @@ struct Plan {
     std::vector<int32_t> tail_chunk, tail_tokens;
     // the one-launch kernel's form of the work; direct_cluster == 0: the step goes by items
     int direct_cluster = 0;                // CTAs per (block of rows, head)
-    int direct_rows = 0;                   // rows of the longest block
-    std::vector<int32_t> direct_entries;   // [4]: chunk, tokens, rows of the block that see it (bits), 1 for a tail; block by block
+    int direct_rows = 0;                   // columns of the longest block
+    std::vector<int32_t> direct_entries;   // [4]: chunk, tokens, columns of the block that see it (bits), 1 for a tail; block by block
     std::vector<int32_t> direct_ranges;    // [blocks][cluster * DIRECT_WARPS][4]: first entry and step, last entry and its end step
     std::vector<int32_t> direct_blocks;    // [blocks][2]: first row, rows
     ca_plan_stats stats{};
@@ -109,8 +109,8 @@ std::string build_plan(Plan& plan, const ca_chunk_info* infos, int n_infos, int 
                        int window = 0,  // > 0: chunks that lie before the window of every row they serve are left out
                        bool even_items = false);  // items of about equal size, as many as fill whole waves of n_ctas CTAs
 // Fills Plan::direct_* where the one-launch kernel is the faster way (mode 1) or always (mode 2).  items: else the step goes by
-// items, not by the any-geometry kernel.
-void build_direct(Plan& plan, int mode, int d_head, bool items);
+// items, not by the any-geometry kernel.  group: of grouped heads, the query heads per key/value head, each a column (0: fp16 caches).
+void build_direct(Plan& plan, int mode, int d_head, bool items, int group = 0);
 // The per-row path lists (path_off / path_chunks / path_tokens) from plan.infos, for a plan built without them.
 void build_paths(Plan& plan);
 

@@ -133,3 +133,43 @@ def test_captured_and_replayed():
     graph.replay()
     torch.cuda.synchronize()
     assert (out.cpu().double() - dense(q.cpu(), ctx, d ** -0.5)).abs().max() < TOL
+
+
+@pytest.mark.parametrize("heads,kv,d", [(4, 4, 64), (6, 3, 128), (16, 4, 128), (12, 3, 64), (16, 2, 128), (8, 1, 64)])
+@pytest.mark.parametrize("sink,scale", [(True, None), (False, -0.07)])
+@pytest.mark.parametrize("chunk,lens", [(64, [1, 15, 16, 17, 63, 64, 65, 129]), (32, [700]), (64, [33] * 20), (48, [5, 300])])
+def test_grouped_heads(heads, kv, d, sink, scale, chunk, lens):
+    # 1 to 8 query heads to a key/value head, with and without the sink, a scale that turns the order of scores round, values turned back;
+    # the items' kernels, the rule's choice and this kernel against the oracle
+    import chunk_attn
+    import gagorax_oracle as oracle
+    from chunk_attn import SpanBatch
+    from test_gpu_block_ops import close, rnd
+    dev, base, eps, dt = torch.device("cuda:0"), 500.0, 1e-5, torch.bfloat16
+    scale = d ** -0.5 if scale is None else scale
+    cache = chunk_attn.Attention.shaped(n_heads=heads, n_kv_heads=kv, d_key=d, d_value=d, scale=scale, sink=sink, chunk_size=chunk, memory_mb=64, dtype=dt, device=dev)
+    qn, kn = rnd(1, d) * 0.2 + 1, rnd(2, d) * 0.2 + 1
+    kf = torch.from_numpy((base ** (-2.0 * np.arange(d // 2) / d)).astype(np.float32)).to(dev)
+    width, want, last = (heads + 2 * kv) * d, [], []
+    for i, n in enumerate(lens):
+        x = rnd(10 + i, n + 1, width).to(dt)
+        tokens = [10_000 * (i + 1) + j for j in range(n)]
+        cache.extend([-1], [tokens])
+        cache.store_qkv(x[:n].to(dev), SpanBatch([tokens], [0], [i], dev).positions, qn.to(dev), kn.to(dev), eps, d, kf, kf)
+        last.append(x[n:])
+        z, pos = x.double().numpy(), np.arange(n + 1)
+        q, k, v = (z[:, a:b].reshape(n + 1, -1, d) for a, b in ((0, heads * d), (heads * d, (heads + kv) * d), ((heads + kv) * d, width)))
+        q = oracle.rotary(oracle.rms_norm(q, qn.double().numpy(), eps), pos, d, base)[-1]
+        k, v = oracle.rotary(oracle.rms_norm(k, kn.double().numpy(), eps), pos, d, base), oracle.rotary(v, pos, d, base)
+        s = np.einsum("hd,thd->ht", q, np.repeat(k, heads // kv, 1)) * scale
+        top = np.maximum(s.max(1, keepdims=True), 0.0) if sink else s.max(1, keepdims=True)
+        p = np.exp(s - top)
+        o = np.einsum("ht,thd->hd", p / (p.sum(1, keepdims=True) + (np.exp(-top) if sink else 0.0)), np.repeat(v, heads // kv, 1))
+        want.append(oracle.rotary(o[None], np.array([-n]), d, base))
+    spans = SpanBatch([[7]] * len(lens), lens, list(range(len(lens))), dev)
+    q = cache.store_qkv(torch.cat(last).to(dev), spans.positions, qn.to(dev), kn.to(dev), eps, d, kf, kf, append_tokens=[7] * len(lens))
+    for mode in (0, 1, 2):
+        cache.set_option(cabi.CA_OPT_DIRECT, mode)
+        got = cache.forward_rows(q, spans.positions, kf)
+        close(got, np.concatenate(want), dt, "mode %d" % mode)
+    assert cache.plan_stats()["kernels_per_step"] == 1 and cache.device_status() == 0
