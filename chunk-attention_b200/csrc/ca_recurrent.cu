@@ -7,6 +7,7 @@
 // all single pieces runs a recurrence in one launch; otherwise the scan takes three: local end state of every piece
 // from zero, a sweep over the pieces of each sequence that turns them into initial states, and the outputs.
 #include <algorithm>
+#include <cmath>
 #include <type_traits>
 
 #include "../../include/chunk_attn_b200.h"
@@ -123,136 +124,214 @@ struct ScanParams {
     float* piece_dt;         // [pieces, C]: sum of dt over the piece
     int C, N;
     int run;                 // pieces a CTA takes (0: whole spans)
+    bool bc_vec;             // rows of bc can be read 16 bytes at a time
+    bool x_vec;              // and those of x, z and dt
     ca_spans sp;
 };
 constexpr int SCAN_THREADS = 128;
-constexpr int SCAN_TOKENS = 32;  // tokens whose B and C are staged at a time (two buffers)
+// Tokens that are staged at a time (two buffers): of fp32 rows fewer, for as many CTAs on an SM
+template <typename T> constexpr int scan_tokens() { return sizeof(T) == 4 ? 16 : 32; }
+// CTAs of an SM with NS states per lane, by registers
+constexpr int scan_blocks(int ns) { return ns >= 16 ? 4 : ns >= 8 ? 4 : 6; }
 
 
-// L lanes share a channel, NS states each.  Of a group of tokens, lane i of a channel reads the inputs of tokens i, i + L,
-// ... and evaluates their step size and, at the end, their output; dt and dt x travel by shuffles.
-// PHASE 0: whole spans: state in, outputs, state out (spans in turn per CTA column).  1: end state of the run from zero, and
+// What a stage holds: B and C, zero past N, and the rows of a CTA's channels
+template <typename T, int L, int NS> struct ScanStage {
+    static constexpr int TOKENS = scan_tokens<T>();
+    static constexpr int CHANNELS = SCAN_THREADS / L;
+    static constexpr int DT = TOKENS * 2 * L * NS * 4, X = DT + TOKENS * CHANNELS * 4, GATE = X + TOKENS * CHANNELS * (int)sizeof(T);
+    static constexpr int BYTES = GATE + TOKENS * CHANNELS * (int)sizeof(T);
+};
+// n rows of ROW bytes, of which `valid` exist, 16 bytes at a time by all threads of the CTA
+template <int ROW> __device__ __forceinline__ void scan_copy(uint8_t* to, const uint8_t* from, size_t stride, int n, int valid) {
+    static_assert(ROW % 16 == 0, "16-byte parts");
+    constexpr int PARTS = ROW / 16;
+    const uint32_t dst = (uint32_t)__cvta_generic_to_shared(to);
+    for (int i = threadIdx.x; i < n * PARTS; i += SCAN_THREADS) {
+        const int row = i / PARTS, b = i % PARTS * 16;
+        if (b < valid) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + row * ROW + b), "l"(from + row * stride + b) : "memory");
+    }
+}
+
+// L lanes share a channel, NS states each, in quads: lane ln has states 4 (ln + L i) .. + 3, so that the lanes' reads of B and C meet
+// different banks.  Of a group of tokens, lane i of a channel evaluates the step size and, at the end, the output of tokens i, i + L, ...;
+// dt and dt x travel by shuffles, the lanes' parts of the outputs by halving exchanges of the whole group.
+// PHASE 0: whole spans, in turn where a CTA has several: state in, outputs, state out.  1: end state of the run from zero, and
 // sum of dt.  2: outputs from the run's initial state.
 template <typename T, int L, int NS, int PHASE>
-__global__ void __launch_bounds__(SCAN_THREADS, 8) scan_kernel(const ScanParams p) {
-    extern __shared__ __align__(16) float bc_s[];  // 2 x [SCAN_TOKENS][B: L * NS | C: L * NS], zero past N
-    constexpr int GROUP = L <= 8 ? 8 : L;  // tokens whose x, dt, z are requested together, one group ahead
-    constexpr int NP = L * NS, OWN = (GROUP + L - 1) / L, BUF = SCAN_TOKENS * 2 * NP;
-    const int c = blockIdx.x * (SCAN_THREADS / L) + threadIdx.x / L;
-    const int ln = threadIdx.x & (L - 1), base = (threadIdx.x & 31) & ~(L - 1), n0 = ln * NS, N = p.N;
+__global__ void __launch_bounds__(SCAN_THREADS, scan_blocks(NS)) scan_kernel(const ScanParams p) {
+    extern __shared__ __align__(16) uint8_t scan_s[];  // two stages
+    using Z = ScanStage<T, L, NS>;
+    constexpr int GROUP = L <= 8 ? 8 : L;  // tokens of one exchange
+    constexpr int NP = L * NS, OWN = GROUP / L, CB = Z::CHANNELS, TOKENS = Z::TOKENS;
+    static_assert(TOKENS % GROUP == 0, "groups of the staged tokens");
+    const int c0 = blockIdx.x * CB, ch = threadIdx.x / L, c = c0 + ch;
+    const int ln = threadIdx.x & (L - 1), base = (threadIdx.x & 31) & ~(L - 1), N = p.N;
     const bool on = c < p.C;
     const int cc = on ? c : p.C - 1;
+    // Copies of B and C: 16 bytes each where rows allow it.  Thread i takes parts i, i + SCAN_THREADS, ... of the rows laid end to end
+    const int width = p.bc_vec ? 4 : 1, parts = 2 * N / width;
+    const int row0 = threadIdx.x / parts, part0 = threadIdx.x % parts, row_step = SCAN_THREADS / parts, part_step = SCAN_THREADS % parts;
+    auto stage = [&](int tb, int t1, int buf) {  // the next tokens, asynchronously; B and C are zero for what a group has behind the last
+        uint8_t* to = scan_s + buf * Z::BYTES;
+        const int nt = min(TOKENS, t1 - tb), rows = (nt + GROUP - 1) / GROUP * GROUP;
+        for (int row = row0, part = part0; row < rows;) {
+            const int r = part * width;
+            const uint32_t dst = (uint32_t)__cvta_generic_to_shared(to + (row * 2 * NP + (r < N ? r : r - N + NP)) * 4);
+            const float* src = p.bc + (size_t)(tb + min(row, nt - 1)) * p.bc_stride + r;
+            if (p.bc_vec)
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(row < nt ? 16 : 0) : "memory");
+            else
+                asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(row < nt ? 4 : 0) : "memory");
+            row += row_step;
+            part += part_step;
+            if (part >= parts) {
+                part -= parts;
+                row++;
+            }
+        }
+        if (p.x_vec) {
+            scan_copy<4 * CB>(to + Z::DT, reinterpret_cast<const uint8_t*>(p.dt + (size_t)tb * p.C + c0), (size_t)p.C * 4, nt, (p.C - c0) * 4);
+            constexpr int ROW = CB * (int)sizeof(T);
+            const int valid = (p.C - c0) * (int)sizeof(T);
+            scan_copy<ROW>(to + Z::X, reinterpret_cast<const uint8_t*>(static_cast<const T*>(p.x) + (size_t)tb * p.C + c0), (size_t)p.C * sizeof(T), nt, valid);
+            if (PHASE != 1)
+                scan_copy<ROW>(to + Z::GATE, reinterpret_cast<const uint8_t*>(static_cast<const T*>(p.z) + (size_t)tb * p.z_stride + c0), (size_t)p.z_stride * sizeof(T), nt, valid);
+        } else {
+            for (int i = threadIdx.x; i < nt * CB; i += SCAN_THREADS) {
+                const int t = tb + i / CB, k = c0 + i % CB;
+                if (k >= p.C) continue;
+                reinterpret_cast<float*>(to + Z::DT)[i] = p.dt[(size_t)t * p.C + k];
+                reinterpret_cast<T*>(to + Z::X)[i] = static_cast<const T*>(p.x)[(size_t)t * p.C + k];
+                if (PHASE != 1) reinterpret_cast<T*>(to + Z::GATE)[i] = static_cast<const T*>(p.z)[(size_t)t * p.z_stride + k];
+            }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    int unit = blockIdx.y;
+    if (PHASE == 0 && gridDim.y == p.sp.n_entries && p.sp.n_entries <= SCAN_THREADS) {  // the longest spans first
+        __shared__ int ranked;
+        const int E = p.sp.n_entries, e = threadIdx.x;
+        if (e < E) {
+            const int len = p.sp.cu[e + 1] - p.sp.cu[e];
+            int rank = 0;
+            for (int k = 0; k < E; k++) {
+                const int other = p.sp.cu[k + 1] - p.sp.cu[k];
+                rank += other > len || (other == len && k < e);
+            }
+            if (rank == unit) ranked = e;
+        }
+        __syncthreads();
+        unit = ranked;
+    }
+    int e = unit, t0, t1;
+    if (PHASE == 0) {
+        t0 = p.sp.cu[e];
+        t1 = p.sp.cu[e + 1];
+    } else {
+        const int4 wk = reinterpret_cast<const int4*>(p.sp.work)[unit];
+        if (wk.w % p.run) return;  // a run starts at every run-th piece
+        e = wk.x;
+        t0 = wk.y;
+        t1 = min(p.sp.cu[e + 1], t0 + p.run * p.sp.work_len);
+    }
+    int buf = 0;
+    stage(t0, t1, 0);
     uint64_t A2[NS / 2];  // pairs of states
+    auto rate = [&](int n) {  // finite where A is not NaN: a step of no length must leave the state as it is
+        if (n >= N) return 0.f;
+        const float a = p.A[(size_t)cc * N + n] * LOG2E;
+        return isinf(a) ? copysignf(3.402823466e38f, a) : a;
+    };
 #pragma unroll
     for (int i = 0; i < NS; i += 2) {
-        const float* a = p.A + (size_t)cc * N + n0 + i;
-        A2[i / 2] = pair_f32(n0 + i < N ? a[0] * LOG2E : 0.f, n0 + i + 1 < N ? a[1] * LOG2E : 0.f);
+        const int n = 4 * (ln + L * (i / 4)) + i % 4;
+        A2[i / 2] = pair_f32(rate(n), rate(n + 1));
     }
     const float bias = p.dt_bias[cc], D = PHASE == 1 ? 0.f : p.D[cc];
-    const T* X = static_cast<const T*>(p.x) + cc;
-    const T* Z = static_cast<const T*>(p.z) + cc;
     T* Y = static_cast<T*>(p.y) + cc;
-    const float* DT = p.dt + cc;
-    // the padding past N is never copied into
-    for (int i = threadIdx.x; i < 2 * BUF; i += SCAN_THREADS)
-        if (i % NP >= N) bc_s[i] = 0.f;
-    for (int unit = blockIdx.y; unit < (PHASE == 0 ? p.sp.n_entries : p.sp.n_work); unit += gridDim.y) {
-        int e = unit, t0, t1;
-        if (PHASE == 0) {
-            t0 = p.sp.cu[e];
-            t1 = p.sp.cu[e + 1];
-        } else {
-            const int4 wk = reinterpret_cast<const int4*>(p.sp.work)[unit];
-            if (wk.w % p.run) continue;  // a run starts at every run-th piece
-            e = wk.x;
-            t0 = wk.y;
-            t1 = min(p.sp.cu[e + 1], t0 + p.run * p.sp.work_len);
-        }
+    if (N < NP)  // the padding past N is never copied into
+        for (int i = threadIdx.x; i < TOKENS * 2 * NP; i += SCAN_THREADS)
+            if (i % NP >= N) reinterpret_cast<float*>(scan_s)[i] = reinterpret_cast<float*>(scan_s + Z::BYTES)[i] = 0.f;
+    const bool vec = N % 4 == 0;
+    float sum_dt = 0.f;
+    for (bool first = true;;) {
+        const int after = unit + gridDim.y;  // this CTA's next span
+        const bool more = PHASE == 0 && after < p.sp.n_entries;
+        const int a0 = more ? p.sp.cu[after] : 0, a1 = more ? p.sp.cu[after + 1] : 0;
         float S[NS];
-        float* slot = p.state + ((size_t)p.sp.slot[e] * p.C + cc) * N + n0;
-        float* piece = PHASE == 0 ? nullptr : p.piece_state + ((size_t)unit * p.C + cc) * N + n0;
-        const bool live = p.sp.start[e] > 0;
-        const bool vec = N % 4 == 0;
+        float* slot = p.state + ((size_t)p.sp.slot[e] * p.C + cc) * N;
+        float* piece = PHASE == 0 ? nullptr : p.piece_state + ((size_t)unit * p.C + cc) * N;
         const float* from = PHASE == 0 ? slot : piece;
 #pragma unroll
         for (int i = 0; i < NS; i++) S[i] = 0.f;
-        if (PHASE == 2 || (PHASE == 0 && live)) {
-            if (vec) {
+        if (PHASE == 2 || (PHASE == 0 && p.sp.start[e] > 0)) {
 #pragma unroll
-                for (int i = 0; i < NS; i += 4)
-                    if (n0 + i < N) {
-                        const float4 v = *reinterpret_cast<const float4*>(from + i);
+            for (int i = 0; i < NS; i += 4) {
+                const int n = 4 * (ln + L * (i / 4));
+                if (vec) {
+                    if (n < N) {
+                        const float4 v = *reinterpret_cast<const float4*>(from + n);
                         S[i] = v.x; S[i + 1] = v.y; S[i + 2] = v.z; S[i + 3] = v.w;
                     }
-            } else {
+                } else {
 #pragma unroll
-                for (int i = 0; i < NS; i++)
-                    if (n0 + i < N) S[i] = from[i];
+                    for (int j = 0; j < 4; j++)
+                        if (n + j < N) S[i + j] = from[n + j];
+                }
             }
         }
         uint64_t S2[NS / 2];
 #pragma unroll
         for (int i = 0; i < NS; i += 2) S2[i / 2] = pair_f32(S[i], S[i + 1]);
-        float sum_dt = 0.f;
-        auto stage = [&](int tb, int buf) {  // B and C of the next tokens, asynchronously
-            const int nt = min(SCAN_TOKENS, t1 - tb);
-            for (int i = threadIdx.x; i < nt * 2 * N; i += SCAN_THREADS) {
-                const int tt = i / (2 * N), r = i - tt * 2 * N;
-                const uint32_t dst = (uint32_t)__cvta_generic_to_shared(bc_s + buf * BUF + tt * 2 * NP + (r < N ? r : r - N + NP));
-                asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(p.bc + (size_t)(tb + tt) * p.bc_stride + r) : "memory");
+        for (int tb = t0; tb < t1; tb += TOKENS, buf ^= 1, first = false) {
+            const int nt = min(TOKENS, t1 - tb);
+            if (!first) __syncthreads();  // the other buffer is free
+            const bool same = tb + TOKENS < t1;
+            if (same || more) {
+                stage(same ? tb + TOKENS : a0, same ? t1 : a1, buf ^ 1);
+                asm volatile("cp.async.wait_group 1;" ::: "memory");
+            } else {
+                asm volatile("cp.async.wait_group 0;" ::: "memory");
             }
-        };
-        float xs[OWN], ds[OWN], zs[OWN], nd[OWN];
-        T nx[OWN], nz[OWN];  // as they come: a conversion here would wait for the loads
-        auto request = [&](int t) {  // this lane's tokens of the group that starts at t
-#pragma unroll
-            for (int k = 0; k < OWN; k++) {
-                const int tk = ln + k * L;
-                nd[k] = 0.f;
-                nx[k] = nz[k] = from_f32<T>(0.f);
-                if (tk < GROUP && t + tk < t1) {
-                    nx[k] = X[(size_t)(t + tk) * p.C];
-                    nd[k] = DT[(size_t)(t + tk) * p.C];
-                    if (PHASE != 1) nz[k] = Z[(size_t)(t + tk) * p.z_stride];
-                }
-            }
-        };
-        __syncthreads();  // nobody reads the buffers of the span before any more
-        stage(t0, 0);
-        asm volatile("cp.async.commit_group;" ::: "memory");
-        request(t0);
-        int buf = 0;
-        for (int tb = t0; tb < t1; tb += SCAN_TOKENS, buf ^= 1) {
-            const int nt = min(SCAN_TOKENS, t1 - tb);
-            if (tb > t0) __syncthreads();  // the other buffer is free
-            if (tb + SCAN_TOKENS < t1) stage(tb + SCAN_TOKENS, buf ^ 1);
-            asm volatile("cp.async.commit_group;" ::: "memory");
-            asm volatile("cp.async.wait_group 1;" ::: "memory");
             __syncthreads();
+            const uint8_t* now = scan_s + buf * Z::BYTES;
             for (int g = 0; g < nt; g += GROUP) {
-                float us[OWN], ys[OWN];
-#pragma unroll
-                for (int k = 0; k < OWN; k++) {
-                    xs[k] = to_f32(nx[k]);
-                    zs[k] = to_f32(nz[k]);
-                    ds[k] = softplus_f(nd[k] + bias);
+                float xs[OWN], ds[OWN], us[OWN], ys[GROUP];
+                const int t = tb + g + ln, at = (g + ln) * CB + ch;  // this lane's tokens: t + k * L
+                T* const y_row = Y + (size_t)(tb + g) * p.C;
+                auto inputs = [&](int k) {
+                    const bool valid = t + k * L < t1;
+                    xs[k] = valid ? to_f32(reinterpret_cast<const T*>(now + Z::X)[at + k * L * CB]) : 0.f;
+                    const float raw = reinterpret_cast<const float*>(now + Z::DT)[at + k * L * CB] + bias;
+                    ds[k] = softplus_for<T>(valid ? raw : -1e30f);  // a step of no length, exactly 0, leaves the state as it is
                     us[k] = ds[k] * xs[k];
-                    ys[k] = 0.f;
+                    if (PHASE == 1) sum_dt += ds[k];
+                };
+                constexpr int HALF = (OWN + 1) / 2;  // the tokens of a lane in the first half of a group
+                const bool both = OWN == 1 || nt - g > HALF * L;
+#pragma unroll
+                for (int k = 0; k < HALF; k++) inputs(k);
+                if (both) {
+#pragma unroll
+                    for (int k = HALF; k < OWN; k++) inputs(k);
+                } else {
+#pragma unroll
+                    for (int k = HALF; k < OWN; k++) xs[k] = ds[k] = us[k] = 0.f;
                 }
-                if (tb + g + GROUP < t1) request(tb + g + GROUP);
+                const float* rows = reinterpret_cast<const float*>(now) + g * 2 * NP + 4 * ln;
                 auto token = [&](int k) {
-                    const int own = k % L;
                     float dt = ds[k / L], u = us[k / L];
                     if (L > 1) {
-                        dt = __shfl_sync(0xffffffffu, dt, base + own);
-                        u = __shfl_sync(0xffffffffu, u, base + own);
+                        dt = __shfl_sync(0xffffffffu, dt, base + k % L);
+                        u = __shfl_sync(0xffffffffu, u, base + k % L);
                     }
-                    const float* B = bc_s + buf * BUF + (g + k) * 2 * NP + n0;
                     const uint64_t dt2 = pair_f32(dt, dt), u2 = pair_f32(u, u);
-                    uint64_t y2 = 0;
+                    uint64_t y2;
 #pragma unroll
                     for (int i = 0; i < NS; i += 4) {
-                        const ulonglong2 b4 = *reinterpret_cast<const ulonglong2*>(B + i), c4 = *reinterpret_cast<const ulonglong2*>(B + NP + i);
+                        const float* B = rows + k * 2 * NP + L * i;
+                        const ulonglong2 b4 = *reinterpret_cast<const ulonglong2*>(B), c4 = *reinterpret_cast<const ulonglong2*>(B + NP);
                         const uint64_t bb[2] = {b4.x, b4.y}, cc2[2] = {c4.x, c4.y};
 #pragma unroll
                         for (int j = 0; j < 2; j++) {
@@ -260,53 +339,79 @@ __global__ void __launch_bounds__(SCAN_THREADS, 8) scan_kernel(const ScanParams 
                             float lo, hi;
                             unpair_f32(mul_f32x2(dt2, A2[i / 2 + j]), lo, hi);
                             s2 = fma_f32x2(pair_f32(exp2_approx(lo), exp2_approx(hi)), s2, mul_f32x2(u2, bb[j]));
-                            if (PHASE != 1) y2 = fma_f32x2(s2, cc2[j], y2);
+                            if (PHASE != 1) y2 = i + j == 0 ? mul_f32x2(s2, cc2[j]) : fma_f32x2(s2, cc2[j], y2);
                         }
                     }
-                    float y, y_hi;
-                    unpair_f32(y2, y, y_hi);
-                    y += y_hi;
-                    if (PHASE == 1) {
-                        sum_dt += dt;
-                    } else {
-#pragma unroll
-                        for (int off = L >> 1; off >= 1; off >>= 1) y += __shfl_xor_sync(0xffffffffu, y, off);
-                        if (own == ln) ys[k / L] = y;
+                    if (PHASE != 1) {
+                        float y, y_hi;
+                        unpair_f32(y2, y, y_hi);
+                        ys[k] = y + y_hi;
                     }
                 };
-                if (nt - g >= GROUP) {
+                // four at a time: short spans end there, and four are enough to cover one another's latencies
 #pragma unroll
-                    for (int k = 0; k < GROUP; k++) token(k);
-                } else {
+                for (int q = 0; q < GROUP; q += 4) {
+                    if (q == 0 || nt - g > q) {
 #pragma unroll
-                    for (int k = 0; k < GROUP; k++)
-                        if (g + k < nt) token(k);
+                        for (int k = q; k < q + 4; k++) token(k);
+                    } else if (PHASE != 1) {
+#pragma unroll
+                        for (int k = q; k < q + 4; k++) ys[k] = 0.f;
+                    }
                 }
                 if (PHASE != 1) {
+                    // the lanes' parts: a lane gives up half of the tokens it still has, for the other half of its partner's
 #pragma unroll
-                    for (int k = 0; k < OWN; k++) {
-                        const int tk = ln + k * L;
-                        if (on && tk < GROUP && g + tk < nt)
-                            Y[(size_t)(tb + g + tk) * p.C] = from_f32<T>(fmaf(D, xs[k], ys[k]) * silu_for<T>(zs[k]));
+                    for (int off = L / 2; off >= 1; off >>= 1) {
+                        const bool upper = ln & off;
+#pragma unroll
+                        for (int k = 0; k < GROUP; k++)
+                            if (k % L < off) {
+                                const float got = __shfl_xor_sync(0xffffffffu, upper ? ys[k] : ys[k + off], off);
+                                ys[k] = (upper ? ys[k + off] : ys[k]) + got;
+                            }
                     }
+                    // the gates of all tokens at once: behind a branch each, they waited for one another
+                    auto outputs = [&](auto first_k, auto end_k) {
+                        constexpr int from = decltype(first_k)::value, to = decltype(end_k)::value;
+                        float o[to - from + 1];
+#pragma unroll
+                        for (int k = from; k < to; k++)
+                            o[k - from] = fmaf(D, xs[k], ys[k * L]) * silu_for<T>(to_f32(reinterpret_cast<const T*>(now + Z::GATE)[at + k * L * CB]));
+#pragma unroll
+                        for (int k = from; k < to; k++)
+                            if (on && t + k * L < t1) y_row[(ln + k * L) * p.C] = from_f32<T>(o[k - from]);
+                    };
+                    outputs(std::integral_constant<int, 0>(), std::integral_constant<int, HALF>());
+                    if (both) outputs(std::integral_constant<int, HALF>(), std::integral_constant<int, OWN>());
                 }
             }
         }
 #pragma unroll
         for (int i = 0; i < NS; i += 2) unpair_f32(S2[i / 2], S[i], S[i + 1]);
+        if (PHASE == 1) {
+#pragma unroll
+            for (int off = L / 2; off >= 1; off >>= 1) sum_dt += __shfl_xor_sync(0xffffffffu, sum_dt, off);
+        }
         if (PHASE != 2 && on) {
             float* dst = PHASE == 0 ? slot : piece;
-            if (vec) {
 #pragma unroll
-                for (int i = 0; i < NS; i += 4)
-                    if (n0 + i < N) *reinterpret_cast<float4*>(dst + i) = make_float4(S[i], S[i + 1], S[i + 2], S[i + 3]);
-            } else {
+            for (int i = 0; i < NS; i += 4) {
+                const int n = 4 * (ln + L * (i / 4));
+                if (vec) {
+                    if (n < N) *reinterpret_cast<float4*>(dst + n) = make_float4(S[i], S[i + 1], S[i + 2], S[i + 3]);
+                } else {
 #pragma unroll
-                for (int i = 0; i < NS; i++)
-                    if (n0 + i < N) dst[i] = S[i];
+                    for (int j = 0; j < 4; j++)
+                        if (n + j < N) dst[n + j] = S[i + j];
+                }
             }
             if (PHASE == 1 && ln == 0) p.piece_dt[(size_t)unit * p.C + c] = sum_dt;
         }
+        if (!more) break;
+        unit = e = after;
+        t0 = a0;
+        t1 = a1;
     }
 }
 
@@ -360,7 +465,7 @@ __global__ void __launch_bounds__(SCAN_THREADS) scan_step_kernel(const ScanParam
     for (int e = blockIdx.y; e < p.sp.n_entries; e += gridDim.y) {
         Inputs now = in;
         request(e + gridDim.y);
-        const float x = to_f32(now.x), dt = softplus_f(now.dt + bias), u = dt * x;
+        const float x = to_f32(now.x), dt = softplus_for<T>(now.dt + bias), u = dt * x;
         float y = 0.f;
 #pragma unroll
         for (int i = 0; i < NS; i++) {
@@ -401,35 +506,87 @@ __global__ void scan_sweep_kernel(const ScanParams p) {
     *slot = S;
 }
 
-// Lanes per channel: eight states each in the scan, whose inner loop then is bound by the exponentials and not by shuffles
-// and shared memory; four in the decode step, where the state's way through memory is what counts.
+// Lanes per channel with per_lane states each
 int scan_lanes(int n_states, int per_lane) {
     int lanes = 1;
     while (lanes < 32 && lanes * per_lane < n_states) lanes *= 2;
     return lanes;
 }
-// Pieces per CTA.  Sequential over whole spans (0) when spans and channels alone fill the GPU; else runs that do.
-int scan_run(const ca_spans& sp, int channels, int n_states) {
-    const int per_block = SCAN_THREADS / scan_lanes(n_states, 8);
-    const int64_t blocks = (channels + per_block - 1) / per_block;
-    if (sp.n_work == sp.n_entries || blocks * sp.n_entries >= 444) return 0;
-    const int64_t run = (blocks * sp.n_work + B200_SMS * 7 - 1) / (B200_SMS * 7);  // one wave of about seven CTAs per SM
-    const int longest = (sp.max_tokens + sp.work_len - 1) / sp.work_len;
-    return run >= longest ? 0 : (int)run;
+// instances of the scan: the others are slower at every size, or their lanes have no states
+constexpr bool scan_instance(int lanes, int per_lane) { return per_lane == 4 ? lanes <= 4 : per_lane == 8 ? lanes <= 16 : lanes >= 4 && lanes <= 16; }
+struct ScanShape {
+    int per_lane;  // states
+    int run;       // pieces of a CTA, 0: whole spans
+};
+// States per lane and, where whole spans leave the GPU idle, the length of runs, by estimates of the time: a token costs a warp alone
+// `alone` ns, and each warp of an SM's quarter `busy` ns where many share it (8 tokens a group, bf16).  Runs are two passes and a sweep.
+// 8192 channels of 16 states, 4 | 8 | 16 states a lane: 64 spans of 128 tokens 478 | 398 | 387 us, 8 of 596 to 1000 361 | 306 | 355,
+// one of 4096 356 | 363 | 617 (in runs 440), one of 2048 channels 280 | 363 | 613 (in runs 134).  4096 channels, 8 spans: 64 states
+// 694 | 567 | 526, 128 states - | 1192 | 978.
+ScanShape scan_shape(const ca_spans& sp, int channels, int n_states) {
+    constexpr double SWEEP_NS = 8000.0;
+    const int pieces = (sp.max_tokens + sp.work_len - 1) / sp.work_len;
+    ScanShape best{n_states > 128 ? 16 : 8, 0};
+    double best_t = 0;
+    for (int ns = 4; ns <= 16; ns *= 2) {
+        const int L = scan_lanes(n_states, ns);
+        if (!scan_instance(L, ns) || L * ns < n_states || (ns > 4 && L == 1 && n_states <= ns / 2)) continue;
+        const double alone = ns == 4 ? (L == 1 ? 116 : L == 2 ? 85 : 70) : ns == 8 ? (L == 1 ? 130 : 88) : 150;
+        const double busy = ns == 4 ? (L == 1 ? 46 : L == 2 ? 38 : 34) : ns == 8 ? (L == 1 ? 62 : 56) : 104;
+        const int64_t blocks = ((int64_t)channels * L + SCAN_THREADS - 1) / SCAN_THREADS;
+        // CTAs of equal lengths on every SM; a few more on some of them are a longer time
+        auto pass = [&](double tokens_each, double ctas, double longest) {
+            const double per_sm = ctas / B200_SMS, uneven = per_sm > scan_blocks(ns) ? per_sm + 0.3 : std::ceil(per_sm);
+            const double chain = longest * alone, work = tokens_each * uneven * busy;
+            return std::max(chain, work) + 0.26 * std::min(chain, work);
+        };
+        for (int run = 0; run < pieces; run = run == 0 ? 1 : run + std::max(1, run / 4)) {
+            double t;
+            if (run == 0) {
+                t = pass((double)sp.n_tokens / sp.n_entries, (double)blocks * sp.n_entries, sp.max_tokens);
+            } else {
+                const double runs = (double)sp.n_work / run + 0.5 * sp.n_entries * (run - 1) / run;
+                t = SWEEP_NS + 2.0 * pass((double)sp.n_tokens / runs, blocks * runs, (double)run * sp.work_len);
+            }
+            if (best_t == 0 || t < best_t) {
+                best_t = t;
+                best = ScanShape{ns, run};
+            }
+        }
+    }
+    return best;
 }
 
-template <typename T, int L>
+// CTAs that share the spans.  One each, or, of short spans, several: a CTA's beginning costs as much as about 7 tokens (200 spans of 3
+// tokens, 8192 channels: 133 us with one each, 90 so; 64 of 20: 107 and 81), and the next span's rows arrive under the present one.
+int scan_rows(const ca_spans& sp, int blocks, int resident) {
+    constexpr int SHORT = 40, BEGIN = 7;
+    const int E = sp.n_entries;
+    if (sp.max_tokens > SHORT) return E;
+    auto time = [&](int rows) {  // a few CTAs behind the last full wave take most of another one
+        const double waves = (double)blocks * rows / resident, full = std::floor(waves), each = (E + rows - 1) / rows;
+        return (waves <= 1.0 ? 1.0 : full + (waves > full ? std::max(waves - full, 0.7) : 0.0)) * (each * sp.n_tokens / E + BEGIN);
+    };
+    int best = E;
+    for (int rows = std::min(E, 4 * resident / blocks + 1); rows >= 1; rows--)
+        if (time(rows) < time(best)) best = rows;
+    return best;
+}
+
+template <typename T, int L, int NS>
 void launch_scan(const ScanParams& p, cudaStream_t stream) {
-    constexpr int NS = 8, per_block = SCAN_THREADS / L;
+    constexpr int per_block = SCAN_THREADS / L;
     const int blocks = (p.C + per_block - 1) / per_block;
-    const size_t smem = (size_t)2 * SCAN_TOKENS * 2 * L * NS * sizeof(float);  // at most 128 KiB (256 states)
-    if (smem > 48 * 1024) {
-        cudaFuncSetAttribute(scan_kernel<T, L, NS, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        cudaFuncSetAttribute(scan_kernel<T, L, NS, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        cudaFuncSetAttribute(scan_kernel<T, L, NS, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    constexpr int smem = 2 * ScanStage<T, L, NS>::BYTES;
+    static_assert(smem <= 227 * 1024 - 1024, "two stages");
+    if (smem > 40 * 1024) {
+        cudaFuncSetAttribute(scan_kernel<T, L, NS, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        cudaFuncSetAttribute(scan_kernel<T, L, NS, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        cudaFuncSetAttribute(scan_kernel<T, L, NS, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     }
     if (p.run == 0) {
-        scan_kernel<T, L, NS, 0><<<dim3(blocks, p.sp.n_entries), SCAN_THREADS, smem, stream>>>(p);
+        const int rows = scan_rows(p.sp, blocks, B200_SMS * std::min(scan_blocks(NS), 227 * 1024 / (smem + 1024)));
+        scan_kernel<T, L, NS, 0><<<dim3(blocks, rows), SCAN_THREADS, smem, stream>>>(p);
     } else {
         scan_kernel<T, L, NS, 1><<<dim3(blocks, p.sp.n_work), SCAN_THREADS, smem, stream>>>(p);
         scan_sweep_kernel<<<dim3((unsigned)(((int64_t)p.C * p.N + 255) / 256), p.sp.n_entries), 256, 0, stream>>>(p);
@@ -632,11 +789,19 @@ int conv_silu(void* out, const void* x, int64_t x_stride, const float* taps, con
 }
 
 template <typename T>
-int selective_scan(const ScanParams& p, cudaStream_t stream) {
+int selective_scan(const ScanParams& p, int per_lane, cudaStream_t stream) {
     if (p.sp.max_tokens == 1 && p.N <= 128)
         by_lanes(scan_lanes(p.N, 4), [&](auto l) { launch_scan_step<T, decltype(l)::value>(p, stream); });
     else
-        by_lanes(scan_lanes(p.N, 8), [&](auto l) { launch_scan<T, decltype(l)::value>(p, stream); });
+        by_lanes(scan_lanes(p.N, per_lane), [&](auto l) {
+            constexpr int L = decltype(l)::value;
+            if constexpr (scan_instance(L, 4))
+                if (per_lane == 4) launch_scan<T, L, 4>(p, stream);
+            if constexpr (scan_instance(L, 8))
+                if (per_lane == 8) launch_scan<T, L, 8>(p, stream);
+            if constexpr (scan_instance(L, 16))
+                if (per_lane == 16) launch_scan<T, L, 16>(p, stream);
+        });
     return done();
 }
 
@@ -711,7 +876,7 @@ int ca_conv_silu(void* out, const void* x, int64_t x_stride, const float* taps, 
 }
 
 int64_t ca_scan_scratch_floats(const ca_spans* sp, int channels, int n_states) {
-    if (!sp || channels <= 0 || n_states <= 0 || scan_run(*sp, channels, n_states) == 0) return 0;
+    if (!sp || channels <= 0 || n_states <= 0 || scan_shape(*sp, channels, n_states).run == 0) return 0;
     return (int64_t)sp->n_work * channels * ((int64_t)n_states + 1);
 }
 
@@ -722,15 +887,19 @@ int ca_selective_scan(void* y, const void* x, const void* z, int64_t z_stride, c
     if (channels <= 0 || n_states < 1 || n_states > 256) return fail("selective_scan: 1 to 256 states per channel");
     if (!y || !x || !z || !dt || !dt_bias || !A || !bc || !D || !state) return fail("selective_scan: null pointer");
     ScanParams p;
-    p.run = scan_run(*sp, channels, n_states);
+    const ScanShape shape = scan_shape(*sp, channels, n_states);
+    const size_t es = dtype == CA_DTYPE_F32 ? 4 : 2;
+    p.run = shape.run;
+    p.x_vec = channels * es % 16 == 0 && z_stride * es % 16 == 0 && aligned16(x) && aligned16(z) && aligned16(dt);
+    p.bc_vec = n_states % 4 == 0 && bc_stride % 4 == 0 && aligned16(bc);
     if (p.run > 0 && !scratch) return fail("selective_scan: this batch needs scratch");
     p.y = y; p.x = x; p.z = z; p.z_stride = z_stride; p.dt = dt; p.dt_bias = dt_bias; p.A = A; p.bc = bc; p.bc_stride = bc_stride;
     p.D = D; p.state = state; p.piece_state = scratch;
     p.piece_dt = scratch ? scratch + (size_t)sp->n_work * channels * n_states : nullptr;
     p.C = channels; p.N = n_states; p.sp = *sp;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    if (dtype == CA_DTYPE_BF16) return selective_scan<__nv_bfloat16>(p, s);
-    if (dtype == CA_DTYPE_F32) return selective_scan<float>(p, s);
+    if (dtype == CA_DTYPE_BF16) return selective_scan<__nv_bfloat16>(p, shape.per_lane, s);
+    if (dtype == CA_DTYPE_F32) return selective_scan<float>(p, shape.per_lane, s);
     return fail("selective_scan: unknown element type");
 }
 

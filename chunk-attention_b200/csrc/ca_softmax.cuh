@@ -3,7 +3,7 @@
 // The tcgen05 attention kernels keep two softmax warps on a scheduler, too few to hide a chain of dependent operations or to issue
 // every cycle, so what counts is the length of a tile's chain and its instructions: maxima and sums go in four chains of 3-operand
 // maxima and of pairs, products and differences in pairs of fp32 (two results per instruction, each rounded as the scalar one).
-// 8192 tokens of one prompt, 32 heads on 8 of 128: 601 -> 586 us; nothing for the kernel of wide shared runs, which keeps its own.
+// 8192 tokens of one prompt, 32 heads on 8 of 128: 601 -> 586 us; the kernel of wide shared runs is as fast either way.
 #pragma once
 #include "ca_ptx.cuh"
 #include "ca_types.cuh"

@@ -1,0 +1,59 @@
+"""The selective scan over its whole range of shapes: every number of states per lane, spans and runs of them, rows that can and
+cannot be copied 16 bytes at a time, against the recurrence in 64 bits."""
+import numpy as np
+import pytest
+import torch
+
+import gagorax_oracle as oracle
+from chunk_attn import SpanBatch, ops
+from test_gpu_block_ops import close, rnd
+
+pytestmark = pytest.mark.gpu
+DEV = torch.device("cuda:0")
+# spans end before, at and behind the groups of 8 tokens and the 32 that are staged together
+EDGES = [1, 7, 8, 9, 31, 32, 33, 65]
+
+
+def scan(lens, channels, states, dtype, A=None):
+    n, E = sum(lens), len(lens)
+    x, z = rnd(1, n, channels).to(dtype), rnd(2, n, channels).to(dtype)
+    dt, bc = rnd(3, n, channels), rnd(4, n, 2 * states)
+    A = -torch.exp(rnd(5, channels, states)) if A is None else A
+    D, bias = rnd(6, channels), rnd(7, channels) - 2
+    state = torch.full((E + 1, channels, states), 7.0, device=DEV)
+    spans = SpanBatch([[1] * k for k in lens], [0] * E, list(range(E, 0, -1)), DEV)
+    y = ops.selective_scan(x.to(DEV), z.to(DEV), dt.to(DEV), bias.to(DEV), A.to(DEV), bc.to(DEV), D.to(DEV), state, spans)
+    at, want, ends = 0, [], []
+    num = lambda t: t.double().numpy()
+    for k in lens:
+        s = slice(at, at + k)
+        o, S = oracle.selective_scan(num(x[s]), oracle.softplus(num(dt[s]) + num(bias)), num(A), num(bc[s])[:, :states], num(bc[s])[:, states:], num(D))
+        want.append(o * oracle.silu(num(z[s])))
+        ends.append(S)
+        at += k
+    return y, state, want, ends
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("lens,channels,states", [
+    (EDGES, 40, 3), (EDGES, 33, 6), (EDGES, 136, 8), (EDGES, 72, 16), (EDGES, 72, 18), (EDGES, 40, 64), (EDGES, 17, 129), (EDGES, 24, 256),
+    ([40] * 20, 4096, 16), ([33] * 8, 4096, 64), ([300, 257], 200, 4), ([300, 257], 200, 16), ([400], 136, 128), ([400, 31], 130, 160),
+    ([33] * 130, 64, 16),  # more spans than are put into order
+    ([3, 32, 1, 9] * 60, 1024, 16), ([3, 32, 1, 9] * 60, 264, 100)])  # short ones: several by a CTA
+def test_scan_shapes(lens, channels, states, dtype):
+    y, state, want, ends = scan(lens, channels, states, dtype)
+    close(y, np.concatenate(want), dtype)
+    state = state.cpu()
+    for e, S in enumerate(ends):
+        close(state[len(lens) - e], S, torch.float32, "state")
+    assert bool((state[0] == 7.0).all())
+
+
+def test_rates_without_bound():
+    """A state that is forgotten at once: nothing of it may come back with the tokens that fill up a span's last group."""
+    A = -torch.exp(rnd(5, 48, 16))
+    A[:, 3] = -float("inf")
+    y, state, want, ends = scan([5, 12, 32], 48, 16, torch.float32, A)
+    close(y, np.concatenate(want), torch.float32)
+    for e, S in enumerate(ends):
+        close(state[3 - e], S, torch.float32, "state")
