@@ -94,6 +94,39 @@ def test_a_row_with_infinities_stays_alone(d, chunk):
     assert (got[keep] - want[keep]).abs().max() < TOL
 
 
+@pytest.mark.parametrize("d,chunk", [(128, 64), (64, 64), (128, 32), (96, 40), (40, 64), (8, 17)])
+@pytest.mark.parametrize("shared,lens", [(0, [1]), (0, [900]), (64, [50, 90, 20, 64]), (130, [5, 70, 1, 200, 33, 16, 17, 40]), (64, [30] * 11)])
+@pytest.mark.parametrize("where", ["own", "shared"])
+def test_infinite_values(d, chunk, shared, lens, where):
+    # weights of 1 (a single token) down to 2^-20, blocks of 1 to 8 rows: an infinite value comes out as it is, infinities of both signs as
+    # NaN, and neither reaches another element or, from a row's own tokens, another row
+    if where == "shared" and not shared:
+        pytest.skip("no shared tokens")
+    H, g, n = 2, torch.Generator().manual_seed(d + chunk + len(lens)), len(lens)
+    eng = engine(H, d, chunk, max_chunks=sum(x // chunk + 3 for x in lens) + shared // chunk + 4)
+    rnd = lambda k, scale=1.0: (torch.randn(k, H, d, generator=g) * scale).half()
+    pk, pv = rnd(shared, 2.0), rnd(shared)
+    if where == "shared":
+        pv[3, :, 0], pv[40, :, 1], pv[5, 0, 2] = float("inf"), float("-inf"), float("inf")
+    ctx = []
+    for i, length in enumerate(lens):
+        k, v = rnd(length, 2.0), rnd(length)
+        if where == "own" and i == n // 2:
+            v[length // 2, :, 0], v[-1, :, 1], v[0, 1, 2] = float("inf"), float("-inf"), float("inf")
+            if length > 2:
+                v[1, :, 3], v[2, :, 3] = float("inf"), float("-inf")
+        k, v = torch.cat([pk, k]), torch.cat([pv, v])
+        row = eng.add_seq(list(range(shared)) + [10_000 * (i + 1) + j for j in range(length)], k, v)
+        ctx.insert(row, (k, v))
+    q = rnd(n)
+    got, want = eng.forward(q).cpu().double(), dense(q, ctx, d ** -0.5)
+    finite = torch.isfinite(want)
+    assert ((got[finite] - want[finite]).abs() < TOL * want[finite].abs().clamp(min=1)).all()  # values are up to 4
+    assert torch.equal(torch.isnan(got), torch.isnan(want)) and torch.equal(torch.isposinf(got), torch.isposinf(want)) and torch.equal(torch.isneginf(got), torch.isneginf(want))
+    if where == "own":
+        assert (~finite.flatten(1).all(1)).sum() == 1
+
+
 def test_the_same_as_the_other_kernels():
     # one switch between them, the same tree: results differ by roundings only, and a row without tokens is zero both ways
     for d, chunk in ((128, 64), (80, 32)):
