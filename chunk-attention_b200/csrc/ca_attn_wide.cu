@@ -287,7 +287,7 @@ __device__ __forceinline__ void finish_rows(const WideParams& p, const WideFinis
             if (r >= end) break;
             float m = ml[u].x, l = ml[u].y;
             float4 acc = v[u];
-            if (!(l > 0.f)) {  // no token: its O row holds what was there before
+            if (l == 0.f) {  // no token: its O row holds what was there before.  A sum that is NaN stays: so must the row be
                 m = W_NEG_BIG;
                 l = 0.f;
                 acc = make_float4(0.f, 0.f, 0.f, 0.f);

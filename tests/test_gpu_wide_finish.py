@@ -11,8 +11,9 @@ pytestmark = pytest.mark.gpu
 C = 64
 
 
-def build(H, n, shared, tails, n_ctas, seed):
-    """n rows over `shared` common tokens (whole chunks), row i with tails[i % len(tails)] tokens of its own."""
+def build(H, n, shared, tails, n_ctas, seed, bad=None):
+    """n rows over `shared` common tokens (whole chunks), row i with tails[i % len(tails)] tokens of its own.  bad: a row and what is
+    wrong with its last token."""
     g = torch.Generator().manual_seed(seed)
     rnd = lambda k: (torch.randn(k, H, 128, generator=g)).half()
     eng = CabiEngine(H, 128, C, torch.float16, max_chunks=shared // C + 2 * n + 4)
@@ -24,6 +25,9 @@ def build(H, n, shared, tails, n_ctas, seed):
     for i in range(n):
         t = tails[i % len(tails)]
         k, v = torch.cat([pk, rnd(t)]), torch.cat([pv, rnd(t)])
+        if bad and bad[0] == i:
+            side, value = bad[1].split()
+            (k if side == "key" else v)[-1, :, 5] = float(value)
         row = eng.add_seq(list(range(shared)) + [10_000 * (i + 1) + j for j in range(t)], k, v)
         ctx.insert(row, (k, v))
     return eng, ctx, rnd(n)
@@ -54,12 +58,35 @@ def test_one_kernel(H, n, pieces, n_ctas, shared, tails):
         want = dense(q[some].cuda(), [(ctx[r][0].cuda(), ctx[r][1].cuda()) for r in some], 128 ** -0.5)
         assert (got[some].double() - want).abs().max() < TOL
         assert (got.float() - off(eng, q).float()).abs().max() < TOL  # every row
-        k1, v1 = torch.randn(n, H, 128, generator=torch.Generator().manual_seed(step)).half(), torch.randn(n, H, 128).half()
+        g1 = torch.Generator().manual_seed(step)
+        k1, v1 = torch.randn(n, H, 128, generator=g1).half(), torch.randn(n, H, 128, generator=g1).half()
         if max(tails) + step >= C - 1:
             break
         eng.append_token([5] * n, k1, v1)
         ctx = [(torch.cat([k, a[None]]), torch.cat([v, b[None]])) for (k, v), a, b in zip(ctx, k1, v1)]
     assert eng.ctx.status() == 0
+
+
+@pytest.mark.parametrize("n_ctas,pieces", [(4, 1), (8, 2)])
+@pytest.mark.parametrize("tails", [[1], [9, 3]])
+@pytest.mark.parametrize("what", ["key nan", "key inf", "value nan", "value inf"])
+def test_a_row_with_no_number_stays_alone(n_ctas, pieces, tails, what):
+    # a row's own token that is not a number, or infinite, shows in that row as it does in dense attention, not in the others (the
+    # next row is walked by the same warp)
+    H, n, bad = 2, 130, 41
+    eng, ctx, q = build(H, n, 8 * C, tails, n_ctas, 7, bad=(bad, what))
+    got = eng.forward(q)
+    st = eng.ctx.stats()
+    assert st["n_items_wide"] == 2 * H * pieces and st["kernels_per_step"] == 1
+    want = dense(q.cuda(), [(k.cuda(), v.cuda()) for k, v in ctx], 128 ** -0.5)
+    others = [r for r in range(n) if r != bad]
+    assert (got[others].double() - want[others]).abs().max() < TOL
+    if what.startswith("value"):
+        assert torch.equal(got[bad, :, 5].isnan(), want[bad, :, 5].isnan()) and torch.equal(got[bad, :, 5].isinf(), want[bad, :, 5].isinf())
+        got[bad, :, 5] = want[bad, :, 5] = 0
+    number = ~torch.isnan(want[bad])   # an infinite key is a score of +inf, or one of -inf and then a weight of zero
+    assert torch.equal(number, ~torch.isnan(got[bad])) and bool((got[bad].double() - want[bad])[number].abs().lt(TOL).all())
+    assert bool(number.all()) == what.startswith("value") and not (what == "key nan" and bool(number.any()))
 
 
 def test_empty_tails_and_peers():
