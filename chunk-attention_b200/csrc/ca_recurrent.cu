@@ -284,6 +284,7 @@ __global__ void __launch_bounds__(SCAN_THREADS, scan_blocks(NS)) scan_kernel(con
         uint64_t S2[NS / 2];
 #pragma unroll
         for (int i = 0; i < NS; i += 2) S2[i / 2] = pair_f32(S[i], S[i + 1]);
+        if (t0 == t1 && more) stage(a0, a1, buf);  // a span without tokens: nothing below requests the next one's
         for (int tb = t0; tb < t1; tb += TOKENS, buf ^= 1, first = false) {
             const int nt = min(TOKENS, t1 - tb);
             if (!first) __syncthreads();  // the other buffer is free

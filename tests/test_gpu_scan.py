@@ -1,11 +1,13 @@
 """The selective scan over its whole range of shapes: every number of states per lane, spans and runs of them, rows that can and
 cannot be copied 16 bytes at a time, against the recurrence in 64 bits."""
+import ctypes as C
+
 import numpy as np
 import pytest
 import torch
 
 import gagorax_oracle as oracle
-from chunk_attn import SpanBatch, ops
+from chunk_attn import SpanBatch, cabi, ops
 from test_gpu_block_ops import close, rnd
 
 pytestmark = pytest.mark.gpu
@@ -57,3 +59,44 @@ def test_rates_without_bound():
     close(y, np.concatenate(want), torch.float32)
     for e, S in enumerate(ends):
         close(state[3 - e], S, torch.float32, "state")
+
+
+class Spans(C.Structure):
+    _fields_ = [(n, C.c_int32) for n in ("n_entries", "n_tokens", "max_tokens", "n_work", "work_len")] + \
+               [(n, C.c_void_p) for n in ("cu", "start", "slot", "entry_of", "work", "work_off")]
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("lens,channels", [([3, 0, 5] * 100, 8192), ([0, 0, 9, 33, 0] * 25, 4096), ([0, 40], 64)])
+def test_spans_without_tokens(lens, channels, dtype):
+    # batches that the C interface takes: a CTA that has several spans goes on behind one without tokens, whose state stays (or, at a
+    # sequence's beginning, becomes zero).  Compared with the batch without those spans, bit by bit
+    N, E, n = 16, len(lens), sum(lens)
+    bf16 = dtype == torch.bfloat16
+    x, z, dt, bc = rnd(1, n, channels).to(dtype).to(DEV), rnd(2, n, channels).to(dtype).to(DEV), rnd(3, n, channels).to(DEV), rnd(4, n, 2 * N).to(DEV)
+    A, D, bias = (-torch.exp(rnd(5, channels, N))).to(DEV), rnd(6, channels).to(DEV), (rnd(7, channels) - 2).to(DEV)
+    state0 = rnd(8, E, channels, N).to(DEV)
+    scan = cabi.lib.ca_selective_scan
+    scan.argtypes = [C.c_void_p] * 3 + [C.c_int64] + [C.c_void_p] * 4 + [C.c_int64] + [C.c_void_p] * 3 + [C.POINTER(Spans)] + [C.c_int] * 3 + [C.c_void_p]
+
+    def run(entries):
+        ints = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)
+        length = [lens[e] for e in entries]
+        cu = ints([0] + list(np.cumsum(length)))
+        pieces = [[i, int(c), int(c) + k, 0] for i, (k, c) in enumerate(zip(length, np.cumsum([0] + length)))]
+        starts = ints([e % 2 for e in entries])  # every other one has a past
+        slots, of = ints(entries), ints([i for i, k in enumerate(length) for _ in range(k)])
+        work, off = ints(pieces), ints(list(range(len(entries) + 1)))
+        sp = Spans(len(entries), n, max(lens), len(pieces), 64, cu.data_ptr(), starts.data_ptr(), slots.data_ptr(), of.data_ptr(), work.data_ptr(), off.data_ptr())
+        y, state = torch.full((n, channels), float("nan"), dtype=dtype, device=DEV), state0.clone()
+        assert scan(y.data_ptr(), x.data_ptr(), z.data_ptr(), channels, dt.data_ptr(), bias.data_ptr(), A.data_ptr(), bc.data_ptr(), 2 * N, D.data_ptr(),
+                    state.data_ptr(), None, C.byref(sp), channels, N, cabi.CA_DTYPE_BF16 if bf16 else cabi.CA_DTYPE_F32, None) == 0
+        torch.cuda.synchronize()
+        return y, state
+
+    y, state = run(list(range(E)))
+    want_y, want = run([e for e in range(E) if lens[e]])
+    for e in range(E):
+        if not lens[e] and e % 2 == 0:
+            want[e] = 0
+    assert torch.equal(y, want_y) and torch.equal(state, want)
