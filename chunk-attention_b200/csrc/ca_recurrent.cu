@@ -305,7 +305,7 @@ __global__ void __launch_bounds__(SCAN_THREADS, scan_blocks(NS)) scan_kernel(con
                     const bool valid = t + k * L < t1;
                     xs[k] = valid ? to_f32(reinterpret_cast<const T*>(now + Z::X)[at + k * L * CB]) : 0.f;
                     const float raw = reinterpret_cast<const float*>(now + Z::DT)[at + k * L * CB] + bias;
-                    ds[k] = softplus_for<T>(valid ? raw : -1e30f);  // a step of no length, exactly 0, leaves the state as it is
+                    ds[k] = softplus_f(valid ? raw : -1e30f);  // a step of no length, exactly 0, leaves the state as it is
                     us[k] = ds[k] * xs[k];
                     if (PHASE == 1) sum_dt += ds[k];
                 };
@@ -466,7 +466,7 @@ __global__ void __launch_bounds__(SCAN_THREADS) scan_step_kernel(const ScanParam
     for (int e = blockIdx.y; e < p.sp.n_entries; e += gridDim.y) {
         Inputs now = in;
         request(e + gridDim.y);
-        const float x = to_f32(now.x), dt = softplus_for<T>(now.dt + bias), u = dt * x;
+        const float x = to_f32(now.x), dt = softplus_f(now.dt + bias), u = dt * x;
         float y = 0.f;
 #pragma unroll
         for (int i = 0; i < NS; i++) {

@@ -105,17 +105,10 @@ template <typename T> __device__ __forceinline__ float silu_for(float z) { retur
 template <> __device__ __forceinline__ float silu_for<float>(float z) { return silu_f(z); }
 
 // log(1 + exp(z)) = max(z, 0) + log(1 + e), e = exp(-|z|) in (0, 1], with log(1 + e) = 2 artanh(s), s = e / (2 + e) <= 1/3,
-// by its power series up to s^13 (the rest is below 2^-25 of the sum).  Kernels of 16-bit types take e and s by the hardware's approximations
-template <typename T> __device__ __forceinline__ float softplus_for(float z) {
-    float e, s;
-    if constexpr (sizeof(T) == 2) {
-        e = exp2_approx(-1.4426950408889634f * fabsf(z));
-        s = e * rcp_approx(2.f + e);
-    } else {
-        e = exp2f(-1.4426950408889634f * fabsf(z));
-        s = __fdividef(e, 2.f + e);
-    }
-    const float q = s * s;
+// by its power series up to s^13 (the rest is below 2^-25 of the sum)
+__device__ __forceinline__ float softplus_f(float z) {
+    const float e = exp2f(-1.4426950408889634f * fabsf(z));
+    const float s = __fdividef(e, 2.f + e), q = s * s;
     float a = fmaf(q, 1.f / 13.f, 1.f / 11.f);
     a = fmaf(q, a, 1.f / 9.f);
     a = fmaf(q, a, 1.f / 7.f);

@@ -61,6 +61,22 @@ def test_rates_without_bound():
         close(state[3 - e], S, torch.float32, "state")
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("lens", [[5, 33], [1, 1, 1]])
+def test_smallest_steps(lens, dtype):
+    # steps of exp(-88), which is below 2^-126, are steps: inputs of 1e38 bring them back into sight.  Spans and single tokens
+    n, E, channels, states = sum(lens), len(lens), 40, 16
+    x, z = torch.full((n, channels), 1e38).to(dtype), torch.ones(n, channels).to(dtype)
+    dt, bias, bc = torch.full((n, channels), -88.0), torch.zeros(channels), torch.ones(n, 2 * states)
+    state = torch.zeros(E, channels, states, device=DEV)
+    spans = SpanBatch([[1] * k for k in lens], [0] * E, list(range(E)), DEV)
+    ops.selective_scan(x.to(DEV), z.to(DEV), dt.to(DEV), bias.to(DEV), torch.full((channels, states), -1.0, device=DEV), bc.to(DEV),
+                       torch.zeros(channels, device=DEV), state, spans)
+    for e, k in enumerate(lens):  # every token adds the same; numbers below 2^-126 have 20 bits there
+        want = k * float(np.exp(-88.0)) * x[0, 0].item()
+        assert bool((state[e] / want - 1).abs().lt(1e-5).all())
+
+
 class Spans(C.Structure):
     _fields_ = [(n, C.c_int32) for n in ("n_entries", "n_tokens", "max_tokens", "n_work", "work_len")] + \
                [(n, C.c_void_p) for n in ("cu", "start", "slot", "entry_of", "work", "work_off")]
