@@ -84,7 +84,6 @@ struct ca_plan {
     int d_head = ca::FAST_D;
     int esize = 2;
     int window = 0, group = 1;
-    int direct = 0;
 };
 
 namespace {
@@ -438,7 +437,6 @@ int ca_plan_build_for_context(const ca_context* c, ca_plan** out, const ca_chunk
     p->esize = c->geo.esize;
     p->window = c->shape.window;
     p->group = c->group;
-    p->direct = direct_mode(c);
     *out = p;
     return CA_OK;
 }
@@ -456,7 +454,9 @@ int ca_refresh_from_plan(ca_context* c, const ca_plan* plan, ca_stream stream_) 
     if (guard.err != cudaSuccess) return fail_cuda(guard.err, "cudaSetDevice");
     c->valid = false;
     const int rc = upload_plan(c, pl, static_cast<cudaStream_t>(stream_));
-    if (plan->direct != direct_mode(c)) c->meta.direct_cluster = 0;  // its items serve any options
+    // its items serve any options; the one-launch kernel takes lists that were cut for it, for columns of this context's rows
+    const int direct = direct_mode(c);
+    if (direct == 0 || pl.direct_mode != direct || pl.direct_dim != c->geo.d_head || pl.direct_group != (c->shaped ? c->group : 0)) c->meta.direct_cluster = 0;
     return rc;
 }
 

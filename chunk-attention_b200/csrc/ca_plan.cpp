@@ -193,6 +193,9 @@ double waves(double ctas, double slots) {
 void build_direct(Plan& plan, int mode, int d_head, bool items, int group) {
     const int columns = std::max(1, group);  // of a row
     plan.direct_cluster = 0;
+    plan.direct_mode = mode;
+    plan.direct_dim = d_head;
+    plan.direct_group = group;
     plan.direct_entries.clear();
     plan.direct_ranges.clear();
     plan.direct_blocks.clear();

@@ -87,6 +87,7 @@ struct Plan {
     std::vector<int32_t> tail_chunk, tail_tokens;
     // the one-launch kernel's form of the work; direct_cluster == 0: the step goes by items
     int direct_cluster = 0;                // CTAs per (block of rows, head)
+    int direct_mode = 0, direct_dim = 0, direct_group = 0;  // what build_direct was asked for: other kernels than that must not get the lists
     int direct_rows = 0;                   // columns of the longest block
     std::vector<int32_t> direct_entries;   // [4]: chunk, tokens, columns of the block that see it (bits), 1 for a tail; block by block
     std::vector<int32_t> direct_ranges;    // [blocks][cluster * DIRECT_WARPS][4]: first entry and step, last entry and its end step

@@ -617,7 +617,8 @@ CA_API int ca_plan_build_windowed(ca_plan** out, const ca_chunk_info* infos, int
                                   int tpp_threshold, int n_ctas, int64_t max_chunks, int rows_per_item, int window);
 /* Adds the form of the work that the one-launch kernel takes (CA_OPT_DIRECT; mode: its meaning), for heads of d_head elements;
  * against_items: the alternative is the list of items (else the any-geometry kernel).  Returns in *cluster the CTAs per block of
- * rows and head, 0 when the step does not go that way. */
+ * rows and head, 0 when the step does not go that way.  The form is that of contexts without a head shape; a refresh from the plan
+ * leaves it aside where the context's kernel, mode or head size is another one. */
 CA_API int ca_plan_direct(ca_plan* plan, int mode, int d_head, int against_items, int* cluster);
 CA_API int ca_plan_array(const ca_plan* plan, int which, const int32_t** data, int64_t* count);
 CA_API int ca_plan_stats_get(const ca_plan* plan, ca_plan_stats* out);

@@ -1,4 +1,6 @@
 """The one-launch kernel against dense attention in 64 bits, and against the kernels it stands in for."""
+import ctypes as C
+
 import numpy as np
 import pytest
 import torch
@@ -206,3 +208,84 @@ def test_grouped_heads(heads, kv, d, sink, scale, chunk, lens):
         got = cache.forward_rows(q, spans.positions, kf)
         close(got, np.concatenate(want), dt, "mode %d" % mode)
     assert cache.plan_stats()["kernels_per_step"] == 1 and cache.device_status() == 0
+
+
+class Shape(C.Structure):
+    _fields_ = [(n, C.c_int32) for n in ("n_heads", "n_kv_heads", "d_key", "d_value", "sink")] + [("scale", C.c_float), ("latent", C.c_int32), ("window", C.c_int32)]
+
+
+class RowsArgs(C.Structure):
+    _fields_ = [("q", C.c_void_p), ("out", C.c_void_p), ("n_rows", C.c_int32)] + [(n, C.c_void_p) for n in ("positions", "value_freq", "row_entry", "path_off", "path_chunks", "blocks")] + \
+               [("n_blocks", C.c_int32), ("block_rows", C.c_int32)]
+
+
+def stream_now():
+    return C.c_void_p(torch.cuda.current_stream().cuda_stream)
+
+
+def rewritten_plan(handle, infos, n_seqs, d):
+    """A plan built for the context, whose one-launch lists are then cut again, for single rows and heads of d elements."""
+    arr, n = cabi.make_infos(infos)
+    plan, cluster = C.c_void_p(), C.c_int()
+    cabi.check(cabi.lib.ca_plan_build_for_context(handle, C.byref(plan), arr, n, n_seqs))
+    cabi.check(cabi.lib.ca_plan_direct(plan, 2, d, 1, C.byref(cluster)))
+    assert cluster.value > 0
+    cabi.check(cabi.lib.ca_refresh_from_plan(handle, plan, stream_now()))
+    cabi.lib.ca_plan_destroy(plan)
+
+
+@pytest.mark.parametrize("dtype,d,off", [(torch.float32, 64, False), (torch.float16, 64, True), (torch.float16, 128, True)])
+def test_lists_that_are_not_this_contexts(dtype, d, off):
+    # lists cut for other kernels than a context's (fp32 caches, the option switched off) are left aside; its own way is taken
+    g = torch.Generator().manual_seed(2)
+    eng = CabiEngine(4, d, 64, dtype, max_chunks=40)
+    if off:
+        eng.ctx.set_option(cabi.CA_OPT_DIRECT, 0)
+    rnd = lambda n: torch.randn(n, 4, d, generator=g).to(dtype)
+    ctx = []
+    for i, n in enumerate([70, 5, 200]):
+        k, v = rnd(n), rnd(n)
+        ctx.insert(eng.add_seq([1000 * i + j for j in range(n)], k, v), (k, v))
+    q = rnd(3)
+    want = eng.forward(q)
+    kernels = eng.ctx.stats()["kernels_per_step"]
+    rewritten_plan(eng.ctx._h, eng.tree.get_chunks(), 3, d)
+    assert torch.equal(eng.forward(q), want) and eng.ctx.stats()["kernels_per_step"] == kernels
+    assert (want.cpu().double() - dense(q, ctx, d ** -0.5)).abs().max() < TOL
+
+
+def test_lists_of_rows_for_grouped_heads():
+    # blocks of 8 rows are blocks of 32 columns where four query heads share a key/value head: such lists are left aside
+    n, d, heads, kv = 8, 64, 16, 4
+    shape = Shape(heads, kv, d, d, 1, 0.1, 0, 0)
+    size = cabi.lib.ca_chunk_bytes_shaped(C.byref(shape), 64, cabi.CA_DTYPE_BF16)
+    g = torch.Generator(device="cuda").manual_seed(4)
+    pool = torch.randn(12 * size // 2, generator=g, device="cuda").bfloat16()
+    handle = C.c_void_p()
+    cabi.check(cabi.lib.ca_context_create_shaped(C.byref(handle), 0, C.byref(shape), 64, cabi.CA_DTYPE_BF16, C.c_void_p(pool.data_ptr()), C.c_int64(12), 1))
+    try:
+        infos = [(0, 64, 0, n)] + [(1 + i, 20 + i, i, i + 1) for i in range(n)]
+        q = torch.randn(n, heads, d, generator=g, device="cuda").bfloat16()
+        positions = torch.tensor([64 + 19 + i for i in range(n)], dtype=torch.int32, device="cuda")
+        stats = cabi.PlanStats()
+
+        def run():
+            out = torch.empty_like(q)
+            args = RowsArgs(q.data_ptr(), out.data_ptr(), n, positions.data_ptr(), None, None, None, None, None, 0, 0)
+            cabi.check(cabi.lib.ca_attention_rows(handle, C.byref(args), stream_now()))
+            cabi.check(cabi.lib.ca_context_stats(handle, C.byref(stats)))
+            torch.cuda.synchronize()
+            return out, stats.as_dict()["kernels_per_step"]
+
+        arr, m = cabi.make_infos(infos)
+        cabi.check(cabi.lib.ca_context_set_option(handle, cabi.CA_OPT_DIRECT, 0))
+        cabi.check(cabi.lib.ca_refresh_kernel_context(handle, arr, m, n, stream_now()))
+        want, kernels = run()
+        cabi.check(cabi.lib.ca_context_set_option(handle, cabi.CA_OPT_DIRECT, 2))
+        rewritten_plan(handle, infos, n, d)
+        got, now = run()
+        assert torch.equal(got, want) and now == kernels > 1
+        status = C.c_int32()
+        assert cabi.lib.ca_status_read(handle, stream_now(), C.byref(status)) == 0
+    finally:
+        cabi.lib.ca_context_destroy(handle)
