@@ -927,6 +927,7 @@ static int run_direct(ca_context* c, const void* q, void* out, const ca::MergePa
     d.one_weight = c->fast;
     d.max_chunks = (int)(c->max_chunks < INT32_MAX ? c->max_chunks : INT32_MAX);
     d.status = c->status;
+    d.dependent = c->opt_pdl;
     if (rows) {
         d.group = c->group;
         d.scale_log2 = c->shape.scale * 1.4426950408889634f;
@@ -1040,6 +1041,7 @@ int ca_attention(ca_context* c, const void* q, void* out, int n_seqs, int partit
     g.n_rows = n_seqs;
     g.out_width = c->geo.d_value;
     g.delta_tokens = c->delta_tokens;
+    g.dependent = c->opt_pdl;
     g.scale = 1.0f / std::sqrt((float)c->geo.d_head);
     g.max_tokens = c->max_path_tokens + c->delta_tokens;
     CA_CUDA(ca::launch_attn_seq_generic(g, c->dtype, static_cast<cudaStream_t>(stream_)));
@@ -1130,6 +1132,7 @@ int ca_attention_rows(ca_context* c, const ca_rows_args* a, ca_stream stream_) {
         r.max_chunks = (int)c->max_chunks;
         r.status = c->status;
         r.wait_limit = c->opt_wait_limit;
+        r.dependent = c->opt_pdl;
         if (decode) {
             r.items = c->d_items;
             r.n_items = c->meta.n_items;
@@ -1191,6 +1194,7 @@ int ca_attention_rows(ca_context* c, const ca_rows_args* a, ca_stream stream_) {
     g.path_tokens = decode ? c->d_path_tokens : nullptr;
     g.n_rows = a->n_rows;
     g.delta_tokens = c->delta_tokens;
+    g.dependent = c->opt_pdl;
     g.scale = c->shape.scale;
     g.group = c->group;
     g.out_width = c->shape.d_value;
@@ -1319,6 +1323,7 @@ int ca_latent_attention(ca_context* c, const ca_latent_args* a, ca_stream stream
     p.max_chunks = (int)c->max_chunks;
     p.status = c->status;
     p.wait_limit = c->opt_wait_limit;
+    p.dependent = c->opt_pdl;
     if (decode) {
         p.items = c->d_items;
         p.n_items = c->meta.n_items;

@@ -29,10 +29,10 @@
 #include <cooperative_groups.h>
 #include <cuda_fp16.h>
 
-#include <cstdlib>
 #include <type_traits>
 
 #include "ca_kernels.h"
+#include "ca_launch.cuh"
 #include "ca_plan.h"
 #include "ca_ptx.cuh"
 #include "ca_types.cuh"
@@ -542,28 +542,8 @@ __global__ void __launch_bounds__(D_WARPS * 32, VG == 2 ? 3 : 4) attn_direct_ker
 
 template <typename T, int KQ, int VG, bool PANELS, int LO, bool PEERS = false> cudaError_t launch(const DirectParams& p, cudaStream_t stream) {
     auto* const kernel = attn_direct_kernel<T, KQ, VG, PANELS, LO, PEERS>;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)((int64_t)p.n_blocks * p.n_heads * p.cluster));
-    cfg.blockDim = dim3(D_WARPS * 32);
-    cfg.dynamicSmemBytes = DirectSmem<VG>::bytes(p.block_rows);
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[2];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = p.cluster;
-    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
-    const int n = p.cluster > 1 ? 1 : 0;
-    attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[n].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    static const bool pdl_disabled = std::getenv("CA_DISABLE_PDL") != nullptr;
-    cfg.numAttrs = pdl_disabled ? n : n + 1;
-    cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, p);
-    if (e != cudaSuccess && cfg.numAttrs > n) {
-        (void)cudaGetLastError();
-        cfg.numAttrs = n;
-        e = cudaLaunchKernelEx(&cfg, kernel, p);
-    }
-    return e;
+    return launch_kernel(kernel, dim3((unsigned)((int64_t)p.n_blocks * p.n_heads * p.cluster)), D_WARPS * 32, DirectSmem<VG>::bytes(p.block_rows), p.cluster,
+                         (p.dependent & DEPENDENT_ATTENTION) != 0, stream, p);
 }
 
 }  // namespace

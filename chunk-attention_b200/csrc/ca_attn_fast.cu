@@ -31,9 +31,9 @@
 #include <cuda_fp16.h>
 
 #include <algorithm>
-#include <cstdlib>
 
 #include "ca_kernels.h"
+#include "ca_launch.cuh"
 #include "ca_plan.h"
 #include "ca_ptx.cuh"
 #include "ca_rows_out.cuh"
@@ -1329,23 +1329,7 @@ __global__ void peer_barrier_kernel(const PeerBarrierParams p) {
 }  // namespace
 
 cudaError_t launch_peer_barrier(const PeerBarrierParams& p, cudaStream_t stream) {
-    static const bool pdl_disabled = std::getenv("CA_DISABLE_PDL") != nullptr;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(1);
-    cfg.blockDim = dim3(32);
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = pdl_disabled ? 0 : 1;
-    cudaError_t err = cudaLaunchKernelEx(&cfg, peer_barrier_kernel, p);
-    if (err != cudaSuccess && cfg.numAttrs == 1) {
-        (void)cudaGetLastError();
-        cfg.numAttrs = 0;
-        err = cudaLaunchKernelEx(&cfg, peer_barrier_kernel, p);
-    }
-    return err;
+    return launch_kernel(peer_barrier_kernel, dim3(1), 32, 0, 1, true, stream, p);
 }
 
 cudaError_t configure_fast_kernels() {
@@ -1358,93 +1342,35 @@ cudaError_t configure_fast_kernels() {
 
 cudaError_t launch_attn_partials(const PartialParams& p, int n_ctas, cudaStream_t stream, bool dependent_launch) {
     if (n_ctas <= 0) return cudaSuccess;
-    static const bool pdl_disabled = std::getenv("CA_DISABLE_PDL") != nullptr;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(n_ctas);
-    cfg.blockDim = dim3(NUM_THREADS);
-    cfg.dynamicSmemBytes = SMEM_BYTES;
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = (dependent_launch && !pdl_disabled) ? 1 : 0;
-    cudaError_t err = cudaLaunchKernelEx(&cfg, attn_partial_kernel, p);
-    if (err != cudaSuccess && cfg.numAttrs == 1) {
-        (void)cudaGetLastError();
-        cfg.numAttrs = 0;
-        err = cudaLaunchKernelEx(&cfg, attn_partial_kernel, p);
-    }
-    return err;
+    return launch_kernel(attn_partial_kernel, dim3(n_ctas), NUM_THREADS, SMEM_BYTES, 1, dependent_launch, stream, p);
 }
 
 cudaError_t launch_attn_short_tails(const PartialParams& p, cudaStream_t stream, bool dependent_launch, const MergeParams* finish, bool early) {
     const int n = p.item_hi - p.item_lo;
     if (n <= 0) return cudaSuccess;
-    static const bool pdl_disabled = std::getenv("CA_DISABLE_PDL") != nullptr;
-    cudaLaunchConfig_t cfg = {};
     int dev = 0, sms = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cfg.gridDim = dim3(std::min((n + SHORT_ITEMS_PER_CTA - 1) / SHORT_ITEMS_PER_CTA, SHORT_CTAS * sms));
-    cfg.blockDim = dim3(SHORT_WARPS * 32);
-    cfg.dynamicSmemBytes = 0;
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = (dependent_launch && !pdl_disabled) ? 1 : 0;
+    const dim3 grid(std::min((n + SHORT_ITEMS_PER_CTA - 1) / SHORT_ITEMS_PER_CTA, SHORT_CTAS * sms));
     auto* kernel = !finish ? attn_short_tails_kernel<false, false> : (early ? attn_short_tails_kernel<true, true> : attn_short_tails_kernel<true, false>);
-    const MergeParams mp = finish ? *finish : MergeParams{};
-    cudaError_t err = cudaLaunchKernelEx(&cfg, kernel, p, mp);
-    if (err != cudaSuccess && cfg.numAttrs == 1) {
-        (void)cudaGetLastError();
-        cfg.numAttrs = 0;
-        err = cudaLaunchKernelEx(&cfg, kernel, p, mp);
-    }
-    return err;
+    return launch_kernel(kernel, grid, SHORT_WARPS * 32, 0, 1, dependent_launch, stream, p, finish ? *finish : MergeParams{});
 }
 
 cudaError_t launch_attn_merge(const MergeParams& p, cudaStream_t stream, bool dependent_launch) {
     if (p.n_pairs <= 0) return cudaSuccess;
-    static const bool pdl_disabled = std::getenv("CA_DISABLE_PDL") != nullptr;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((p.n_pairs + 3) / 4);
-    cfg.blockDim = dim3(128);
-    cfg.dynamicSmemBytes = 0;
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = (dependent_launch && !pdl_disabled) ? 1 : 0;
     // pick the instance whose single wave holds the grid
     int dev = 0, sms = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const int grid = (int)cfg.gridDim.x;
+    const int grid = (p.n_pairs + 3) / 4;
+    auto launch = [&](auto* kernel, int ctas) { return launch_kernel(kernel, dim3(ctas), 128, 0, 1, dependent_launch, stream, p); };
     // long lists under few rows: a CTA per row instead of a warp per row (a couple of waves at most)
-    const bool wide = p.n_pairs <= 8 * sms && p.n_merge_entries * (long long)p.n_heads > 48LL * p.n_pairs;
-    if (wide) cfg.gridDim = dim3(p.n_pairs);
+    if (p.n_pairs <= 8 * sms && p.n_merge_entries * (long long)p.n_heads > 48LL * p.n_pairs) return launch(attn_merge_wide_kernel, p.n_pairs);
     // many rows of at most four pieces each: eight lanes per row instead of a warp
-    const bool small = !wide && p.max_list > 0 && p.max_list <= SMALL_MAX_LIST && grid > 3 * sms;
-    if (small) cfg.gridDim = dim3((p.n_pairs + 15) / 16);
-    auto launch = [&]() {
-        if (wide) return cudaLaunchKernelEx(&cfg, attn_merge_wide_kernel, p);
-        if (small) return cudaLaunchKernelEx(&cfg, attn_merge_small_kernel, p);
-        if (grid <= 3 * sms) return cudaLaunchKernelEx(&cfg, attn_merge_kernel<16, 3>, p);
-        if (grid <= 5 * sms) return cudaLaunchKernelEx(&cfg, attn_merge_kernel<8, 5>, p);
-        return cudaLaunchKernelEx(&cfg, attn_merge_kernel<0, 7>, p);
-    };
-    cudaError_t err = launch();
-    if (err != cudaSuccess && cfg.numAttrs == 1) {
-        // the stream or driver refused the programmatic launch: fall back to a plain ordered launch
-        (void)cudaGetLastError();
-        cfg.numAttrs = 0;
-        err = launch();
-    }
-    return err;
+    if (p.max_list > 0 && p.max_list <= SMALL_MAX_LIST && grid > 3 * sms) return launch(attn_merge_small_kernel, (p.n_pairs + 15) / 16);
+    if (grid <= 3 * sms) return launch(attn_merge_kernel<16, 3>, grid);
+    if (grid <= 5 * sms) return launch(attn_merge_kernel<8, 5>, grid);
+    return launch(attn_merge_kernel<0, 7>, grid);
 }
 
 }  // namespace ca

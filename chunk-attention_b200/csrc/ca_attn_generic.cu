@@ -24,9 +24,8 @@
 // (the output row is turned back) are parameters of the walk.
 #include <cooperative_groups.h>
 
-#include <cstdlib>
-
 #include "ca_kernels.h"
+#include "ca_launch.cuh"
 #include "ca_types.cuh"
 
 namespace ca {
@@ -356,45 +355,18 @@ __global__ void __launch_bounds__(GEN_WARPS * 32) attn_split_kernel(const Generi
     if (cluster > 1) cl.sync();  // the other CTAs' shared memory is read until here
 }
 
-// As a programmatic dependent: the CTAs are set up while the kernel ahead of them drains (4 x 288 tokens, 8 fp32 heads of 64,
-// steps back to back: 7.2 -> 5.8 us; 16 x 833, 12 fp16 heads of 64: 13.2 -> 11.4).  Where that is refused, an ordinary launch.
-template <typename... P, typename... A>
-cudaError_t launch_dependent(void (*kernel)(P...), unsigned ctas, int cluster, cudaStream_t stream, const A&... args) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(ctas);
-    cfg.blockDim = dim3(GEN_WARPS * 32);
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[2];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = cluster;
-    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
-    const int n = cluster > 1 ? 1 : 0;
-    attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[n].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    static const bool pdl_disabled = std::getenv("CA_DISABLE_PDL") != nullptr;
-    cfg.numAttrs = pdl_disabled ? n : n + 1;
-    cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, args...);
-    if (e != cudaSuccess && cfg.numAttrs > n) {
-        (void)cudaGetLastError();
-        cfg.numAttrs = n;
-        e = cudaLaunchKernelEx(&cfg, kernel, args...);
-    }
-    return e;
-}
-
+// Dependent launches: 4 x 288 tokens, 8 fp32 heads of 64, steps back to back: 7.2 -> 5.8 us.
 template <typename T, int LPT, int GPL, int U> cudaError_t launch_split(const GenericParams& p, unsigned pairs, cudaStream_t stream) {
     // as many CTAs per row as still run beside each other and have a block of tokens for each of their warps
     int cluster = 1;
     while (cluster < 8 && (int64_t)pairs * cluster * 2 <= GEN_SPLIT_CTAS && (p.max_tokens == 0 || cluster * GEN_WARPS * (32 / LPT * U) < p.max_tokens)) cluster *= 2;
-    return launch_dependent(attn_split_kernel<T, LPT, GPL, U>, pairs * cluster, cluster, stream, p, cluster);
+    return launch_kernel(attn_split_kernel<T, LPT, GPL, U>, dim3(pairs * cluster), GEN_WARPS * 32, 0, cluster, (p.dependent & DEPENDENT_ATTENTION) != 0, stream, p, cluster);
 }
 
 template <typename T> cudaError_t launch_generic(const GenericParams& p, unsigned pairs, cudaStream_t stream) {
     // 16-byte granule reads need the pool base aligned (rows and tiles then are, too)
-    if (p.geo.epg == 1 || reinterpret_cast<uintptr_t>(p.pool) % 16 != 0) {
-        return launch_dependent(attn_elem_kernel<T>, pairs, 1, stream, p);
-    }
+    if (p.geo.epg == 1 || reinterpret_cast<uintptr_t>(p.pool) % 16 != 0)
+        return launch_kernel(attn_elem_kernel<T>, dim3(pairs), GEN_WARPS * 32, 0, 1, (p.dependent & DEPENDENT_ATTENTION) != 0, stream, p);
     const int g = p.geo.gpr > p.geo.v_gpr ? p.geo.gpr : p.geo.v_gpr;
     if (g <= 4) return launch_split<T, 4, 1, 4>(p, pairs, stream);
     if (g <= 8) return launch_split<T, 8, 1, 4>(p, pairs, stream);

@@ -15,6 +15,7 @@
 #include <algorithm>
 
 #include "ca_kernels.h"
+#include "ca_launch.cuh"
 #include "ca_plan.h"
 #include "ca_ptx.cuh"
 #include "ca_types.cuh"
@@ -537,23 +538,8 @@ __global__ void __launch_bounds__(256) rows_merge_kernel(const RowsParams p) {
 // set up while the items' kernel, which allows it, still runs
 cudaError_t launch_merge(const RowsParams& p, cudaStream_t stream) {
     const int64_t pairs = (int64_t)p.n_rows * p.geo.n_heads * p.group;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)((pairs + 7) / 8));
-    cfg.blockDim = dim3(256);
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
     auto* k = p.part_width <= 64 ? rows_merge_kernel<1> : (p.part_width <= 128 ? rows_merge_kernel<2> : rows_merge_kernel<4>);
-    cudaError_t e = cudaLaunchKernelEx(&cfg, k, p);
-    if (e != cudaSuccess && cfg.numAttrs == 1) {
-        (void)cudaGetLastError();
-        cfg.numAttrs = 0;
-        e = cudaLaunchKernelEx(&cfg, k, p);
-    }
-    return e;
+    return launch_kernel(k, dim3((unsigned)((pairs + 7) / 8)), 256, 0, 1, (p.dependent & DEPENDENT_MERGE) != 0, stream, p);
 }
 
 template <int DK, int DV, int STAGES, bool BULK>

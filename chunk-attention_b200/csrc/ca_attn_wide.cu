@@ -36,9 +36,8 @@
 #include <cooperative_groups.h>
 #include <cuda_fp16.h>
 
-#include <cstdlib>
-
 #include "ca_kernels.h"
+#include "ca_launch.cuh"
 #include "ca_plan.h"
 #include "ca_ptx.cuh"
 #include "ca_rows_out.cuh"
@@ -668,30 +667,9 @@ cudaError_t configure_wide_kernel() {
 cudaError_t launch_attn_wide(const WideParams& p, cudaStream_t stream, bool dependent_launch, const WideFinish* finish) {
     const int n = p.item_hi - p.item_lo;
     if (n <= 0) return cudaSuccess;
-    static const bool pdl_disabled = std::getenv("CA_DISABLE_PDL") != nullptr;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(n);
-    cfg.blockDim = dim3(finish ? W_FINISH_THREADS : W_THREADS);
-    cfg.dynamicSmemBytes = finish ? W_FINISH_BYTES : W_SMEM_BYTES;
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[2];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = finish ? finish->pieces : 1;
-    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
-    const int n_attr = finish && finish->pieces > 1 ? 1 : 0;
-    attr[n_attr].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[n_attr].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = n_attr + ((dependent_launch && !pdl_disabled) ? 1 : 0);
-    auto* kernel = finish ? attn_wide_kernel<false, true> : ((p.trace && p.trace_cycles) ? attn_wide_kernel<true, false> : attn_wide_kernel<false, false>);
-    const WideFinish f = finish ? *finish : WideFinish{};
-    cudaError_t err = cudaLaunchKernelEx(&cfg, kernel, p, f);
-    if (err != cudaSuccess && cfg.numAttrs > n_attr) {
-        (void)cudaGetLastError();
-        cfg.numAttrs = n_attr;
-        err = cudaLaunchKernelEx(&cfg, kernel, p, f);
-    }
-    return err;
+    if (finish) return launch_kernel(attn_wide_kernel<false, true>, dim3(n), W_FINISH_THREADS, W_FINISH_BYTES, finish->pieces, dependent_launch, stream, p, *finish);
+    auto* kernel = (p.trace && p.trace_cycles) ? attn_wide_kernel<true, false> : attn_wide_kernel<false, false>;
+    return launch_kernel(kernel, dim3(n), W_THREADS, W_SMEM_BYTES, 1, dependent_launch, stream, p, WideFinish{});
 }
 
 }  // namespace ca

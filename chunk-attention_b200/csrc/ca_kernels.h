@@ -167,6 +167,7 @@ struct DirectParams {
     int n_peers = 0, total_heads = 0, head_offset = 0;  // as in MergeParams
     void* peer_out[MERGE_MAX_PEERS] = {};
     void* mc_out = nullptr;
+    int dependent = 3;           // CA_OPT_DEPENDENT_LAUNCH
 };
 bool attn_direct_serves(const Geometry& g);
 bool attn_direct_serves_grouped(const Geometry& g, const ca_head_shape& shape, int group);
@@ -191,6 +192,7 @@ struct GenericParams {
     const int32_t* positions = nullptr;  // position of each row's token (needed with row_entry or value_freq)
     const float* value_freq = nullptr;   // radians per position of value pair i; null: values are not rotated
     int max_tokens = 0;          // of the longest path, where the host knows it (decode)
+    int dependent = 3;           // CA_OPT_DEPENDENT_LAUNCH
 };
 cudaError_t launch_attn_seq_generic(const GenericParams& p, int dtype, cudaStream_t stream);
 
@@ -226,6 +228,7 @@ struct RowsParams {
     int max_chunks;
     int* status;
     long long wait_limit;
+    int dependent = 3;           // CA_OPT_DEPENDENT_LAUNCH
 };
 cudaError_t launch_attn_rows(const RowsParams& p, cudaStream_t stream);
 
@@ -287,6 +290,7 @@ struct LatentParams {
     int max_chunks;
     int* status;
     long long wait_limit;
+    int dependent = 3;           // CA_OPT_DEPENDENT_LAUNCH
 };
 cudaError_t launch_latent_generic(const LatentParams& p, int dtype, cudaStream_t stream);  // portions, any geometry
 bool latent_rows_serves(const Geometry& g);

@@ -29,6 +29,7 @@
 #include <algorithm>
 
 #include "ca_kernels.h"
+#include "ca_launch.cuh"
 #include "ca_plan.h"
 #include "ca_ptx.cuh"
 #include "ca_types.cuh"
@@ -744,20 +745,8 @@ template <int N, int MODE> cudaError_t launch(const LatentParams& p, cudaStream_
     cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
     if (e != cudaSuccess) return e;
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(MODE == PORTIONS ? p.n_blocks : (MODE == ROWS ? p.n_rows * p.pieces : p.n_items), (rows + N - 1) / N);
-    cfg.blockDim = dim3(L_THREADS);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[2];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    attr[1].id = cudaLaunchAttributeClusterDimension;
-    attr[1].val.clusterDim.x = MODE == ROWS ? p.pieces : 1;
-    attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = MODE == ROWS && p.pieces > 1 ? 2 : 1;
-    return cudaLaunchKernelEx(&cfg, k, p, units);
+    const dim3 grid(MODE == PORTIONS ? p.n_blocks : (MODE == ROWS ? p.n_rows * p.pieces : p.n_items), (rows + N - 1) / N);
+    return launch_kernel(k, grid, L_THREADS, smem, MODE == ROWS ? p.pieces : 1, (p.dependent & DEPENDENT_ATTENTION) != 0, stream, p, units);
 }
 template <int MODE> cudaError_t launch_mode(const LatentParams& p, int rows, cudaStream_t stream) {
     return rows <= 16 ? launch<16, MODE>(p, stream) : (rows <= 32 ? launch<32, MODE>(p, stream) : launch<64, MODE>(p, stream));
@@ -780,16 +769,7 @@ cudaError_t launch_latent_rows(const LatentParams& p, cudaStream_t stream) {
     if (e != cudaSuccess) return e;
     const int64_t pairs = (int64_t)p.n_rows * p.n_heads;
     if (pairs > 0x7fffffff) return cudaErrorInvalidValue;
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3((unsigned)pairs);
-    cfg.blockDim = dim3(128);
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, latent_merge_kernel, p);
+    return launch_kernel(latent_merge_kernel, dim3((unsigned)pairs), 128, 0, 1, (p.dependent & DEPENDENT_MERGE) != 0, stream, p);
 }
 
 }  // namespace ca
