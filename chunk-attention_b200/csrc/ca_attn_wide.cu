@@ -349,7 +349,8 @@ __global__ void __launch_bounds__(FINISH ? W_FINISH_THREADS : W_THREADS, 2) attn
         tmem_relinquish_alloc_permit();
     }
     // as a programmatic dependent launch the CTA has set itself up while the kernel before it was finishing;
-    // nothing in global memory has been touched so far
+    // nothing in global memory has been touched so far.  Tensor memory is held already: a kernel that uses it, too, must have allocated
+    // its own before it lets this one in
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 

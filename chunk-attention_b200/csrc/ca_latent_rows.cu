@@ -176,7 +176,6 @@ __global__ void __launch_bounds__(L_THREADS) latent_rows_kernel(const __grid_con
     }
     // launched as a programmatic dependent: set up while the kernel ahead drains, nothing in global memory is touched before it is complete
     asm volatile("griddepcontrol.wait;" ::: "memory");
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
     // ---- the block of rows and its tokens: [start, end) relative to position `first` of list[0]
     int token0, n_rows, first, end, low, row_lo = (int)blockIdx.y * N, slot_base = 0;
@@ -244,6 +243,9 @@ __global__ void __launch_bounds__(L_THREADS) latent_rows_kernel(const __grid_con
     __syncthreads();
     tc_fence_after_thread_sync();
     const uint32_t tmem_base = *tmem_slot;
+    // The next kernel may be set up only now: one that allocates tensor memory before it waits for this one (ca_attn_wide.cu) could
+    // otherwise hold what a CTA of this one still has to be given, and each would wait for the other.
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
     if (warp == 8) {
         // ---- producer

@@ -47,11 +47,11 @@ def filled(dtype, d, lens, direct):
     return eng.ctx.set_option, lambda: eng.ctx.attention(q, out, 0)
 
 
-def latent(rows):
+def latent(rows, H=32, lens=(70, 130)):
     import chunk_attn
     from chunk_attn import SpanBatch
     from test_gpu_latent_rows import EPS, frequencies
-    dev, lens, H, R, rot = torch.device("cuda:0"), [70, 130], 32, 512, 64
+    dev, lens, R, rot = torch.device("cuda:0"), list(lens), 512, 64
     cache = chunk_attn.Attention.latent(n_heads=H, latent=R, rotated=rot, scale=(R + rot) ** -0.5, window=0, chunk_size=64, memory_mb=64, dtype=torch.bfloat16, device=dev)
     cache.set_option(cabi.CA_OPT_LATENT_ROWS, rows)
     freq = frequencies(rot)[1]
@@ -106,3 +106,28 @@ def test_option(name):
         # the first step's attention kernel has none ahead of it
         want = (attention if mask & 2 else 0) + (2 * merge if mask & 1 else 0)
         assert (count, edges) == (2 * kernels, want), (mask, count, edges)
+
+
+@pytest.mark.parametrize("heads", [16, 32, 64])
+def test_tensor_memory_of_two_kernels(heads):
+    # A latent step and, behind it on the stream, one over wide runs, whose kernel holds tensor memory while it waits for the kernel
+    # ahead: results are those of steps alone.  (The latent kernel has its own before it lets the next one in.)
+    from test_gpu_wide_finish import build
+    for rows in (2, 0):
+        _, step = latent(rows, heads, [70, 130] * 100)
+        eng, _, q = build(4, 130, 8 * 64, [3], 8, 5)
+        q, out = q.cuda(), torch.empty_like(q).cuda()
+        wide = lambda: eng.ctx.attention(q, out, 0)
+        eng.refresh()
+        want_latent, _ = step().clone(), wide()
+        torch.cuda.synchronize()
+        want = out.clone()
+        for _ in range(20):
+            got = step()
+            out.zero_()
+            step()
+            wide()
+            step()
+            wide()
+        torch.cuda.synchronize()
+        assert torch.equal(out, want) and torch.equal(got, want_latent) and eng.ctx.status() == 0
