@@ -133,6 +133,7 @@ struct ca_context {
         bool split_phases = false;
         int wide_pieces = 0;           // Plan::wide_pieces
         int max_item_tiles = 0;
+        bool gaps = false;             // Plan::gaps
         int32_t short_slot_base = 0;
         int64_t tail_rounds = 0;       // 8-token rounds of all tails at the refresh
         int direct_cluster = 0, direct_blocks = 0, direct_rows = 0;  // Plan::direct_*
@@ -566,6 +567,7 @@ static int upload_plan(ca_context* c, const ca::Plan& pl, cudaStream_t stream) {
     c->meta.max_merge_len = pl.max_merge_len;
     c->meta.split_phases = pl.split_phases;
     c->meta.wide_pieces = pl.wide_pieces;
+    c->meta.gaps = pl.gaps;
     c->meta.max_item_tiles = 0;
     for (const ca::PlanItem& it : pl.items) c->meta.max_item_tiles = std::max(c->meta.max_item_tiles, (int)it.n_tiles);
     c->meta.short_slot_base = pl.short_slot_base;
@@ -1259,7 +1261,7 @@ int ca_latent_store(ca_context* c, const ca_latent_store_args* a, ca_stream stre
 // which way is faster.  Measured, items -> sequences: 32 heads, 148 sequences of 40 / 200 tokens 14.3 / 20.2 -> 10.7 / 15.5, 110 of 1000
 // 39.9 -> 36.6, 74 of 1000 (two CTAs each) 27.1 -> 24.9; not for 37 of 1000 (three CTAs each) 16.9 -> 19.7, 8 of 4000 16.7 -> 23.4.
 static int latent_pieces(const ca_context* c, int delta_tokens) {
-    if (!c->opt_latent_rows || !c->paths_on_device || c->meta.n_items_cf > 0 || c->meta.n_seqs == 0 || !ca::latent_rows_finishes(c->geo, c->shape.n_heads))
+    if (!c->opt_latent_rows || !c->paths_on_device || c->meta.gaps || c->meta.n_items_cf > 0 || c->meta.n_seqs == 0 || !ca::latent_rows_finishes(c->geo, c->shape.n_heads))
         return 0;
     const double n = c->meta.n_seqs, H = c->shape.n_heads, split = std::ceil(H / 64);  // CTAs take up to 64 heads
     int longest = c->max_path_tokens + delta_tokens;

@@ -314,6 +314,7 @@ std::string build_plan(Plan& plan, const ca_chunk_info* infos, int n_infos, int 
     plan.wide_chunks.clear();
     plan.n_items_wide = 0;
     plan.wide_pieces = 0;
+    plan.gaps = false;
     plan.merge_slots.clear();
     plan.path_chunks.clear();
     plan.path_tokens.clear();
@@ -388,6 +389,7 @@ std::string build_plan(Plan& plan, const ca_chunk_info* infos, int n_infos, int 
             for (int s = ci.seq_begin; s < ci.seq_end; s++) shortest = std::min(shortest, first[leaf[s]] + infos[leaf[s]].n_tokens);
             if (leaf[ci.seq_begin] != i && first[i] + ci.n_tokens <= (int64_t)shortest - window) {
                 dropped[i] = 1;
+                if (ci.n_tokens != chunk_size) plan.gaps = true;
                 unique_tokens -= ci.n_tokens;
             }
         }

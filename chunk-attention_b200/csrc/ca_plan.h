@@ -76,6 +76,7 @@ struct Plan {
     int32_t short_slot_base = 0;          // first partial row (per-item numbering) of the short tails
     int n_items_wide = 0;                 // how many at the END of the list are wide items for the tcgen05 kernel
     std::vector<int32_t> wide_chunks;     // chunk lists of the wide items
+    bool gaps = false;                    // a chunk left out ahead of the windows was not full: path lists do not give positions
     int wide_pieces = 0;                  // pieces of every block of rows when ONE wide run holds all rows, else 0
     std::vector<int32_t> merge_off, merge_slots;
     int max_merge_len = 0;                // pieces of the row that has most

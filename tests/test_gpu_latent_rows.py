@@ -1,5 +1,7 @@
 """Decode of latent caches by sequences (a CTA or a cluster of two for each, one launch) against attention in 64 bits, and where it is
 taken."""
+import ctypes as C
+
 import numpy as np
 import pytest
 import torch
@@ -69,3 +71,45 @@ def test_sequences(H, R, rot, window, lens):
     assert cache.device_status() == 0
     with pytest.raises(RuntimeError):
         cache.set_option(cabi.CA_OPT_LATENT_ROWS, 3)
+
+
+class Shape(C.Structure):
+    _fields_ = [(n, C.c_int32) for n in ("n_heads", "n_kv_heads", "d_key", "d_value", "sink")] + [("scale", C.c_float), ("latent", C.c_int32), ("window", C.c_int32)]
+
+
+class LatentArgs(C.Structure):
+    _fields_ = [("q_lat", C.c_void_p), ("q_rot", C.c_void_p), ("q_rot_row", C.c_int64), ("q_rot_head", C.c_int64), ("out", C.c_void_p), ("n_rows", C.c_int32)] + \
+               [(n, C.c_void_p) for n in ("positions", "freq", "sink", "row_entry", "path_off", "path_chunks", "blocks")] + \
+               [(n, C.c_int32) for n in ("n_blocks", "block_rows", "delta_tokens")]
+
+
+@pytest.mark.parametrize("head", [30, 64])
+def test_chunks_ahead_of_the_window_that_are_not_full(head):
+    # lists that the C interface takes: a sequence begins with a chunk of `head` tokens, which no window reaches any more.  Positions do
+    # not follow from the number of chunks then; the step's result is that of its items, whatever the option says
+    n, H, R, rot, window = 3, 16, 128, 64, 60
+    shape = Shape(H, 1, R + rot, R, 0, 0.1, 1, window)
+    size = cabi.lib.ca_chunk_bytes_shaped(C.byref(shape), 64, cabi.CA_DTYPE_BF16)
+    g = torch.Generator(device="cuda").manual_seed(4)
+    pool = torch.randn(4 * n * size // 2, generator=g, device="cuda").bfloat16()
+    handle, stream = C.c_void_p(), C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    cabi.check(cabi.lib.ca_context_create_shaped(C.byref(handle), 0, C.byref(shape), 64, cabi.CA_DTYPE_BF16, C.c_void_p(pool.data_ptr()), C.c_int64(4 * n), 1))
+    try:
+        tokens = [head, 64, 64, 20]
+        arr, m = cabi.make_infos([(4 * s + i, t, s, s + 1) for s in range(n) for i, t in enumerate(tokens)])
+        q_lat, q_rot = (torch.randn(n, H, w, generator=g, device="cuda").bfloat16() for w in (R, rot))
+        positions = torch.full((n,), sum(tokens) - 1, dtype=torch.int32, device="cuda")
+        freq = frequencies(rot)[1]
+        out = {}
+        for mode in (0, 1, 2):
+            cabi.check(cabi.lib.ca_context_set_option(handle, cabi.CA_OPT_LATENT_ROWS, mode))
+            cabi.check(cabi.lib.ca_refresh_kernel_context(handle, arr, m, n, stream))
+            out[mode] = torch.empty_like(q_lat)
+            args = LatentArgs(q_lat.data_ptr(), q_rot.data_ptr(), H * rot, rot, out[mode].data_ptr(), n, positions.data_ptr(), freq.data_ptr(), None, None, None, None,
+                              None, 0, 0, -1)
+            cabi.check(cabi.lib.ca_latent_attention(handle, C.byref(args), stream))
+            torch.cuda.synchronize()
+        for mode in (1, 2):  # the two ways differ by the rounding of a bf16 result
+            assert (out[mode].float() - out[0].float()).norm() < 2 ** -7 * out[0].float().norm()
+    finally:
+        cabi.lib.ca_context_destroy(handle)
