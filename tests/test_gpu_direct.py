@@ -129,6 +129,32 @@ def test_infinite_values(d, chunk, shared, lens, where):
         assert (~finite.flatten(1).all(1)).sum() == 1
 
 
+@pytest.mark.parametrize("d,chunk", [(64, 64), (128, 32), (128, 64), (32, 16)])
+@pytest.mark.parametrize("rows", [1, 4, 8])
+def test_many_small_weights(d, chunk, rows):
+    # one token of large weight and no value, 4000 of 2^-26 to 2^-30 of it with values of up to 60000, rows alone and over shared tokens:
+    # the small ones are the result.  Values to 1 %: its distance from their weights' last bit is what is looked at
+    H, n = 2, 4000
+    eng = engine(H, d, chunk, max_chunks=(n + 64) // chunk + 3 * rows + 4)
+    k, v = torch.zeros(n, H, d), torch.full((n, H, d), 60000.0)
+    k[:, :, 0] = -torch.linspace(0, 2.8, n)[:, None]
+    k[7, :, 0], v[7] = 18.0, 0.0
+    own = torch.full((1, H, d), -10.0).half()
+    ctx = []
+    for i in range(rows):
+        kk, vv = torch.cat([k.half(), own]), torch.cat([v.half(), own])
+        row = eng.add_seq(list(range(n)) + [10_000 * (i + 1)], kk, vv)
+        ctx.insert(row, (kk, vv))
+    q = torch.zeros(rows, H, d)
+    q[:, :, 0] = d ** 0.5
+    want = dense(q.half(), ctx, d ** -0.5)
+    for mode in (0, 2) if (d, chunk) != (128, 64) else (2,):  # the items' kernels have weights of 11 bits
+        eng.ctx.set_option(cabi.CA_OPT_DIRECT, mode)
+        eng.valid = False
+        got = eng.forward(q.half()).cpu().double()
+        assert want.abs().min() > 0.5 and ((got - want).abs() < 0.01 * want.abs()).all(), mode
+
+
 def test_the_same_as_the_other_kernels():
     # one switch between them, the same tree: results differ by roundings only, and a row without tokens is zero both ways
     for d, chunk in ((128, 64), (80, 32)):
