@@ -13,7 +13,7 @@ class CabiEngine:
     """Prefix tree on the host (the compiled PrefixTree) + every device operation through the C ABI:
     ca_scatter_prefill, ca_refresh_kernel_context, ca_append_kv, ca_attention, ca_copy_chunks."""
 
-    def __init__(self, n_heads, d_head, chunk_size, dtype, max_chunks=256, tpp_threshold=1, device=0):
+    def __init__(self, n_heads, d_head, chunk_size, dtype, max_chunks=256, tpp_threshold=1, device=0, direct=None):
         self.H, self.d, self.C, self.dtype = n_heads, d_head, chunk_size, dtype
         self.device = torch.device("cuda", device)
         nbytes = cabi.lib.ca_chunk_bytes(n_heads, d_head, chunk_size, DT[dtype])
@@ -21,6 +21,8 @@ class CabiEngine:
         self.pool = torch.full((max_chunks * nbytes,), 0xFF, dtype=torch.uint8, device=self.device)
         self.tree = PrefixTree(chunk_size, max_chunks)
         self.ctx = cabi.Context(n_heads, d_head, chunk_size, DT[dtype], self.pool, max_chunks, tpp_threshold, device)
+        if direct is not None:
+            self.ctx.set_option(cabi.CA_OPT_DIRECT, direct)
         self.valid = False
 
     def add_seq(self, tokens, k, v):

@@ -50,7 +50,14 @@ def test_edges(d, chunk, shared, lens):
     for step in range(3):  # tokens beyond what the work list says
         got = eng.forward(q).cpu().double()
         assert eng.ctx.stats()["kernels_per_step"] == 1
-        assert (got - dense(q, ctx, d ** -0.5)).abs().max() < TOL
+        want = dense(q, ctx, d ** -0.5)
+        assert (got - want).abs().max() < TOL
+        if step == 0:  # and the kernels it stands in for
+            eng.ctx.set_option(cabi.CA_OPT_DIRECT, 0)
+            eng.valid = False
+            assert (eng.forward(q).cpu().double() - want).abs().max() < TOL
+            eng.ctx.set_option(cabi.CA_OPT_DIRECT, 2)
+            eng.valid = False
         k1, v1 = torch.randn(len(lens), H, d, generator=g).half(), torch.randn(len(lens), H, d, generator=g).half()
         eng.append_token([7] * len(lens), k1, v1)
         ctx = [(torch.cat([k, a[None]]), torch.cat([v, b[None]])) for (k, v), a, b in zip(ctx, k1, v1)]

@@ -22,12 +22,16 @@ def dense(q, contexts, scale):
                                      (torch.float16, 256), (torch.float32, 4), (torch.float32, 36), (torch.float32, 68), (torch.float32, 256),
                                      (torch.float16, 20), (torch.float32, 30)])
 @pytest.mark.parametrize("chunk,lens", [(7, [1, 2, 6, 7, 8, 50]), (64, [1, 15, 16, 17, 63, 64, 65, 700]), (32, [33, 512]), (16, [9] * 70)])
-def test_split_rows(dtype, d, chunk, lens):
+@pytest.mark.parametrize("direct", [0, 1])
+def test_split_rows(dtype, d, chunk, lens, direct):
     # every lane layout (4 or 8 lanes per token, 1 to 8 granules each; the last two have rows of no whole granules), blocks that
-    # end inside a chunk, clusters of 1 to 8 CTAs, warps without a block.  The pool's unused rows hold NaN.
+    # end inside a chunk, clusters of 1 to 8 CTAs, warps without a block; by default, fp16 rows of up to 128 elements may go to the
+    # one-launch kernel instead.  The pool's unused rows hold NaN.
+    if direct and (dtype == torch.float32 or d > 128 or d % 8 or chunk < 16):
+        pytest.skip("these have one kernel")
     H, n = 3, len(lens)
     g = torch.Generator().manual_seed(d + chunk)
-    eng = CabiEngine(H, d, chunk, dtype, max_chunks=sum(x // chunk + 2 for x in lens))
+    eng = CabiEngine(H, d, chunk, dtype, max_chunks=sum(x // chunk + 2 for x in lens), direct=direct)
     kv = [(torch.randn(x, H, d, generator=g).to(dtype), torch.randn(x, H, d, generator=g).to(dtype)) for x in lens]
     for i, (k, v) in enumerate(kv):
         eng.add_seq([1000 * i + j for j in range(lens[i])], k, v)
@@ -101,7 +105,8 @@ def test_prompts_in_pieces(shape, sign, lens):
 
 @pytest.mark.parametrize("shape", [(2, 2, 128, 128), (8, 1, 64, 64), (6, 2, 128, 64), (4, 2, 80, 48), (16, 2, 256, 256), (9, 1, 64, 128)])
 @pytest.mark.parametrize("chunk", [64, 16])
-def test_decoded_rows_of_small_groups(shape, chunk):
+@pytest.mark.parametrize("direct", [0, 1])
+def test_decoded_rows_of_small_groups(shape, chunk, direct):
     # Items of at most 8 rows (groups of 1 to 8) and of 9, whose tokens end on every side of the 16 that a warp takes; tiles staged
     # verbatim and granule by granule.
     import chunk_attn
@@ -110,6 +115,7 @@ def test_decoded_rows_of_small_groups(shape, chunk):
     g = torch.Generator().manual_seed(H + dk)
     cache = chunk_attn.Attention.shaped(n_heads=H, n_kv_heads=G, d_key=dk, d_value=dv, scale=dk ** -0.5, sink=False, chunk_size=chunk, memory_mb=64,
                                         dtype=torch.bfloat16, device="cuda:0")
+    cache.set_option(cabi.CA_OPT_DIRECT, direct)
     kv = []
     for i, n in enumerate(lens):
         k, v = torch.randn(n, G, dk, generator=g).bfloat16(), torch.randn(n, G, dv, generator=g).bfloat16()
@@ -120,7 +126,7 @@ def test_decoded_rows_of_small_groups(shape, chunk):
     want = dense(q, kv, dk ** -0.5)
     # the result's rounding to bf16 (2^-9 of it) and that of the weights (2^-17): far below this
     assert (o.cpu().double() - want).abs().max() < 8e-3 * max(1.0, float(want.abs().max()))
-    assert cache.device_status() == 0
+    assert cache.device_status() == 0 and (direct or cache.plan_stats()["kernels_per_step"] == 2)
 
 
 @pytest.mark.parametrize("n,H", [(64, 8), (310, 16), (700, 16)])

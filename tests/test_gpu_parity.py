@@ -142,73 +142,84 @@ def test_reference_forward_case_fp32():
 
 
 # ---- tensor-core / TMA path ------------------------------------------------------------------------------
+# small steps may go to the one-launch kernel by default: the kernels of the item lists are looked at with that off, too
+by_items_and_by_default = pytest.mark.parametrize("direct", [0, 1])
+
+
 def fast_engine(H=4, max_chunks=512, **kw):
     return CabiEngine(H, 128, 64, torch.float16, max_chunks=max_chunks, **kw)
 
 
-def test_reference_cuda_test_case():
+@by_items_and_by_default
+def test_reference_cuda_test_case(direct):
     # tests/test_chunk_attn_cuda.py:19-72: 32 x 2000 tokens, 1000 shared, H2 d128 chunk 64 fp16
     # (2000 % 64 = 16 exercises tail masking; 1000 % 64 = 40 leaves the last shared chunk private)
     w = W.single_level("refcuda", 2, 128, 64, torch.float16, 32, 1000, 1000, 21, 1.0)
-    eng = fast_engine(H=2, max_chunks=32 * 17 + 32)
+    eng = fast_engine(direct=direct, H=2, max_chunks=32 * 17 + 32)
     check_against_oracle(w, eng, TOL_F16)
     st = eng.ctx.stats()
     assert st["fast_path"] == 1 and st["n_shared_chunks"] == 15
 
 
 @pytest.mark.parametrize("n_seqs", [1, 2, 3, 15, 16, 17, 33, 64, 70, 130])
-def test_sharer_counts(n_seqs):
+@by_items_and_by_default
+def test_sharer_counts(n_seqs, direct):
     w = W.single_level("n%d" % n_seqs, 2, 128, 64, torch.float16, n_seqs, 3 * 64, 64 + 9, 30 + n_seqs, 0.5)
-    eng = fast_engine(H=2, max_chunks=3 + n_seqs * 3)
+    eng = fast_engine(direct=direct, H=2, max_chunks=3 + n_seqs * 3)
     check_against_oracle(w, eng, TOL_F16)
 
 
 @pytest.mark.parametrize("tensor_tails", [1, 0])
 @pytest.mark.parametrize("unique", [0, 1, 7, 8, 9, 17, 63, 64, 65])
-def test_partial_and_empty_tails(unique, tensor_tails):
+@by_items_and_by_default
+def test_partial_and_empty_tails(unique, tensor_tails, direct):
     # both ways of walking a private tail: tensor cores (default) and CUDA cores
     w = W.single_level("u%d" % unique, 3, 128, 64, torch.float16, 5, 2 * 64, unique, 40 + unique, 0.5)
-    eng = fast_engine(H=3)
+    eng = fast_engine(direct=direct, H=3)
     eng.ctx.set_option(cabi.CA_OPT_SEQ_FIRST_TENSOR, tensor_tails)
     check_against_oracle(w, eng, TOL_F16)
 
 
-def test_no_prefix_and_full_prefix():
+@by_items_and_by_default
+def test_no_prefix_and_full_prefix(direct):
     for shared, unique in ((0, 5 * 64 + 3), (4 * 64, 0)):
         w = W.single_level("x", 2, 128, 64, torch.float16, 6, shared, unique, 50, 0.5)
-        eng = fast_engine(H=2)
+        eng = fast_engine(direct=direct, H=2)
         check_against_oracle(w, eng, TOL_F16)
 
 
-def test_peaky_scores_and_many_pieces():
+@by_items_and_by_default
+def test_peaky_scores_and_many_pieces(direct):
     # q scaled x8 makes the softmax concentrate: exercises the running max and the merge weights.
     # A small CTA count forces long per-CTA item lists; a large one cuts runs into many pieces.
     w = W.single_level("peaky", 4, 128, 64, torch.float16, 9, 6 * 64, 3 * 64 + 5, 60, 0.5)
     w.q = w.q * 8
     for n_ctas in (1, 5, 148):
         for split, tensor_tails in ((0, 1), (1, 1), (0, 0), (1, 0)):
-            eng = fast_engine(H=4)
+            eng = fast_engine(direct=direct, H=4)
             eng.ctx.set_option(cabi.CA_OPT_NUM_CTAS, n_ctas)
             eng.ctx.set_option(cabi.CA_OPT_SPLIT_PHASES, split)
             eng.ctx.set_option(cabi.CA_OPT_SEQ_FIRST_TENSOR, tensor_tails)
             check_against_oracle(w, eng, TOL_F16, partitions=(0,))
 
 
-def test_tpp_threshold_semantics():
+@by_items_and_by_default
+def test_tpp_threshold_semantics(direct):
     w = W.single_level("tpp", 2, 128, 64, torch.float16, 3, 2 * 64, 10, 70, 0.5)
-    eng = fast_engine(H=2, tpp_threshold=3)
+    eng = fast_engine(direct=direct, H=2, tpp_threshold=3)
     check_against_oracle(w, eng, TOL_F16)
     assert eng.ctx.stats()["n_shared_chunks"] == 0
 
 
 @pytest.mark.parametrize("tensor_tails", [1, 0])
-def test_decode_trace_with_churn(tensor_tails):
+@by_items_and_by_default
+def test_decode_trace_with_churn(tensor_tails, direct):
     # scaled-down two-level tree with incremental decode: append every step, churn every 4 steps,
     # the oracle mirrors every operation; tails cross chunk boundaries during the trace
     cfg = W.Config4(n_heads=2, n_groups=3, per_group=4, root_len=128, group_len=64, unique_len=60, steps=14,
                     churn_every=4, churn=2)
     from chunk_attn_oracle import Attention as OracleAttention
-    eng = fast_engine(H=2, max_chunks=256)
+    eng = fast_engine(direct=direct, H=2, max_chunks=256)
     eng.ctx.set_option(cabi.CA_OPT_SEQ_FIRST_TENSOR, tensor_tails)
     ora = OracleAttention(2, 128, 64)
     seqs = []
@@ -255,10 +266,11 @@ def test_config2_full_size_vs_oracle():
     assert st["n_shared_chunks"] == 32 and st["n_runs"] == 1 and st["kernels_per_step"] == 2
 
 
-def test_rows_written_into_peer_outputs():
+@by_items_and_by_default
+def test_rows_written_into_peer_outputs(direct):
     # ca_attention_to_peers on one GPU: two local buffers stand in for two ranks' full-width outputs
     w = W.single_level("peers", 4, 128, 64, torch.float16, 9, 3 * 64, 64 + 30, 95, 0.5)
-    eng = fast_engine(H=4)
+    eng = fast_engine(direct=direct, H=4)
     rows = W.populate(eng, w)
     q = w.q[rows].to("cuda", torch.float16).contiguous()
     expected = eng.forward(q)
