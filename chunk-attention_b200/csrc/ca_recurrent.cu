@@ -153,6 +153,12 @@ template <int ROW> __device__ __forceinline__ void scan_copy(uint8_t* to, const 
     }
 }
 
+// a state's rate in powers of two, finite where A is not NaN: a step of no length must leave the state as it is
+__device__ __forceinline__ float scan_rate(float A) {
+    const float a = A * LOG2E;
+    return isinf(a) ? copysignf(3.402823466e38f, a) : a;
+}
+
 // L lanes share a channel, NS states each, in quads: lane ln has states 4 (ln + L i) .. + 3, so that the lanes' reads of B and C meet
 // different banks.  Of a group of tokens, lane i of a channel evaluates the step size and, at the end, the output of tokens i, i + L, ...;
 // dt and dt x travel by shuffles, the lanes' parts of the outputs by halving exchanges of the whole group.
@@ -238,11 +244,7 @@ __global__ void __launch_bounds__(SCAN_THREADS, scan_blocks(NS)) scan_kernel(con
     int buf = 0;
     stage(t0, t1, 0);
     uint64_t A2[NS / 2];  // pairs of states
-    auto rate = [&](int n) {  // finite where A is not NaN: a step of no length must leave the state as it is
-        if (n >= N) return 0.f;
-        const float a = p.A[(size_t)cc * N + n] * LOG2E;
-        return isinf(a) ? copysignf(3.402823466e38f, a) : a;
-    };
+    auto rate = [&](int n) { return n < N ? scan_rate(p.A[(size_t)cc * N + n]) : 0.f; };
 #pragma unroll
     for (int i = 0; i < NS; i += 2) {
         const int n = 4 * (ln + L * (i / 4)) + i % 4;
@@ -416,6 +418,160 @@ __global__ void __launch_bounds__(SCAN_THREADS, scan_blocks(NS)) scan_kernel(con
     }
 }
 
+// Short spans: eight states a lane, inputs straight to registers, so that eight CTAs share an SM and one's beginning and end hide under the
+// others' tokens.  Of a group of eight tokens, lane i of a channel reads the inputs of tokens i, i + L, ... and evaluates their step size
+// and, at the end, their output; dt and dt x travel by shuffles, B and C through shared memory.
+constexpr int SHORT_TOKENS = 32;  // whose B and C are staged at a time (two buffers)
+template <typename T, int L>
+__global__ void __launch_bounds__(SCAN_THREADS, L == 1 ? 6 : 8) scan_short_kernel(const ScanParams p) {
+    constexpr int NS = 8, GROUP = 8, NP = L * NS, OWN = GROUP / L, BUF = SHORT_TOKENS * 2 * NP;
+    __shared__ __align__(16) float bc_s[2 * BUF];  // 2 x [SHORT_TOKENS][B: L * NS | C: L * NS], zero past N
+    const int c = blockIdx.x * (SCAN_THREADS / L) + threadIdx.x / L;
+    const int ln = threadIdx.x & (L - 1), base = (threadIdx.x & 31) & ~(L - 1), n0 = ln * NS, N = p.N;
+    const bool on = c < p.C, vec = N % 4 == 0;
+    const int cc = on ? c : p.C - 1;
+    uint64_t A2[NS / 2];  // pairs of states
+#pragma unroll
+    for (int i = 0; i < NS; i += 2) {
+        const float* a = p.A + (size_t)cc * N + n0 + i;
+        A2[i / 2] = pair_f32(n0 + i < N ? scan_rate(a[0]) : 0.f, n0 + i + 1 < N ? scan_rate(a[1]) : 0.f);
+    }
+    const float bias = p.dt_bias[cc], D = p.D[cc];
+    const T* X = static_cast<const T*>(p.x) + cc;
+    const T* Z = static_cast<const T*>(p.z) + cc;
+    T* Y = static_cast<T*>(p.y) + cc;
+    const float* DT = p.dt + cc;
+    if (N < NP)  // the padding past N is never copied into
+        for (int i = threadIdx.x; i < 2 * BUF; i += SCAN_THREADS)
+            if (i % NP >= N) bc_s[i] = 0.f;
+    const int e = blockIdx.y, t0 = p.sp.cu[e], t1 = p.sp.cu[e + 1];
+    float S[NS];
+    float* slot = p.state + ((size_t)p.sp.slot[e] * p.C + cc) * N + n0;
+#pragma unroll
+    for (int i = 0; i < NS; i++) S[i] = 0.f;
+    if (p.sp.start[e] > 0) {
+        if (vec) {
+#pragma unroll
+            for (int i = 0; i < NS; i += 4)
+                if (n0 + i < N) {
+                    const float4 v = *reinterpret_cast<const float4*>(slot + i);
+                    S[i] = v.x; S[i + 1] = v.y; S[i + 2] = v.z; S[i + 3] = v.w;
+                }
+        } else {
+#pragma unroll
+            for (int i = 0; i < NS; i++)
+                if (n0 + i < N) S[i] = slot[i];
+        }
+    }
+    uint64_t S2[NS / 2];
+#pragma unroll
+    for (int i = 0; i < NS; i += 2) S2[i / 2] = pair_f32(S[i], S[i + 1]);
+    auto stage = [&](int tb, int buf) {  // B and C of the next tokens, asynchronously
+        const int nt = min(SHORT_TOKENS, t1 - tb);
+        for (int i = threadIdx.x; i < nt * 2 * N; i += SCAN_THREADS) {
+            const int tt = i / (2 * N), r = i - tt * 2 * N;
+            const uint32_t dst = (uint32_t)__cvta_generic_to_shared(bc_s + buf * BUF + tt * 2 * NP + (r < N ? r : r - N + NP));
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(p.bc + (size_t)(tb + tt) * p.bc_stride + r) : "memory");
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    float nd[OWN];
+    T nx[OWN], nz[OWN];  // as they come: a conversion here would wait for the loads
+    auto request = [&](int t) {  // this lane's tokens of the group that starts at t
+#pragma unroll
+        for (int k = 0; k < OWN; k++) {
+            const int tk = ln + k * L;
+            nd[k] = 0.f;
+            nx[k] = nz[k] = from_f32<T>(0.f);
+            if (t + tk < t1) {
+                nx[k] = X[(size_t)(t + tk) * p.C];
+                nd[k] = DT[(size_t)(t + tk) * p.C];
+                nz[k] = Z[(size_t)(t + tk) * p.z_stride];
+            }
+        }
+    };
+    stage(t0, 0);
+    request(t0);
+    int buf = 0;
+    for (int tb = t0; tb < t1; tb += SHORT_TOKENS, buf ^= 1) {
+        const int nt = min(SHORT_TOKENS, t1 - tb);
+        if (tb > t0) __syncthreads();  // the other buffer is free
+        if (tb + SHORT_TOKENS < t1) {
+            stage(tb + SHORT_TOKENS, buf ^ 1);
+            asm volatile("cp.async.wait_group 1;" ::: "memory");
+        } else {
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
+        }
+        __syncthreads();
+        for (int g = 0; g < nt; g += GROUP) {
+            float xs[OWN], ds[OWN], us[OWN], ys[OWN], zs[OWN];
+#pragma unroll
+            for (int k = 0; k < OWN; k++) {
+                xs[k] = to_f32(nx[k]);
+                zs[k] = to_f32(nz[k]);
+                ds[k] = softplus_f(nd[k] + bias);
+                us[k] = ds[k] * xs[k];
+                ys[k] = 0.f;
+            }
+            if (tb + g + GROUP < t1) request(tb + g + GROUP);
+            auto token = [&](int k) {
+                float dt = ds[k / L], u = us[k / L];
+                if (L > 1) {
+                    dt = __shfl_sync(0xffffffffu, dt, base + k % L);
+                    u = __shfl_sync(0xffffffffu, u, base + k % L);
+                }
+                const float* B = bc_s + buf * BUF + (g + k) * 2 * NP + n0;
+                const uint64_t dt2 = pair_f32(dt, dt), u2 = pair_f32(u, u);
+                uint64_t y2 = 0;
+#pragma unroll
+                for (int i = 0; i < NS; i += 4) {
+                    const ulonglong2 b4 = *reinterpret_cast<const ulonglong2*>(B + i), c4 = *reinterpret_cast<const ulonglong2*>(B + NP + i);
+                    const uint64_t bb[2] = {b4.x, b4.y}, cc2[2] = {c4.x, c4.y};
+#pragma unroll
+                    for (int j = 0; j < 2; j++) {
+                        uint64_t& s2 = S2[i / 2 + j];
+                        float lo, hi;
+                        unpair_f32(mul_f32x2(dt2, A2[i / 2 + j]), lo, hi);
+                        s2 = fma_f32x2(pair_f32(exp2_approx(lo), exp2_approx(hi)), s2, mul_f32x2(u2, bb[j]));
+                        y2 = fma_f32x2(s2, cc2[j], y2);
+                    }
+                }
+                float y, y_hi;
+                unpair_f32(y2, y, y_hi);
+                y += y_hi;
+#pragma unroll
+                for (int off = L >> 1; off >= 1; off >>= 1) y += __shfl_xor_sync(0xffffffffu, y, off);
+                if (k % L == ln) ys[k / L] = y;
+            };
+            if (nt - g >= GROUP) {
+#pragma unroll
+                for (int k = 0; k < GROUP; k++) token(k);
+            } else {
+#pragma unroll
+                for (int k = 0; k < GROUP; k++)
+                    if (g + k < nt) token(k);
+            }
+#pragma unroll
+            for (int k = 0; k < OWN; k++) {
+                const int tk = ln + k * L;
+                if (on && g + tk < nt) Y[(size_t)(tb + g + tk) * p.C] = from_f32<T>(fmaf(D, xs[k], ys[k]) * silu_for<T>(zs[k]));
+            }
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < NS; i += 2) unpair_f32(S2[i / 2], S[i], S[i + 1]);
+    if (!on) return;
+    if (vec) {
+#pragma unroll
+        for (int i = 0; i < NS; i += 4)
+            if (n0 + i < N) *reinterpret_cast<float4*>(slot + i) = make_float4(S[i], S[i + 1], S[i + 2], S[i + 3]);
+    } else {
+#pragma unroll
+        for (int i = 0; i < NS; i++)
+            if (n0 + i < N) slot[i] = S[i];
+    }
+}
+
 // One token per span: four states per lane straight from and to memory, a few spans in turn per CTA so that A is read
 // once for them, everything of the next span requested before this one is worked on.
 template <typename T, int L, bool VEC>
@@ -558,8 +714,26 @@ ScanShape scan_shape(const ca_spans& sp, int channels, int n_states) {
     return best;
 }
 
-// CTAs that share the spans.  One each, or, of short spans, several: a CTA's beginning costs as much as about 7 tokens (200 spans of 3
-// tokens, 8192 channels: 133 us with one each, 90 so; 64 of 20: 107 and 81), and the next span's rows arrive under the present one.
+// Whether whole spans go to the kernel of short ones.  Staged inputs, and lanes with fewer or more states, cost a CTA its beginning and the SM
+// the CTAs that would hide it.  Spans of equal length, this kernel | the other one, us: 8192 channels of 16 states, fp32, 200 spans of 3 tokens
+// 103 | 124, 64 of 33 144 | 164, of 64 248 | 272, of 96 365 | 388, 16 of 128 134 | 133, 8 of 33 25 | 25, of 64 40 | 39; bf16, 200 of 3 99 | 121, 64 of
+// 33 134 | 144, of 64 228 | 233, of 96 334 | 331; 2048 channels, fp32, 16 of 3 6 | 6, of 40 19 | 17, 64 of 33 42 | 44; bf16, 64 of 40 44 | 42.
+// 8192 channels of 8 states, bf16, 64 of 5 28 | 32, of 12 49 | 39; fp32, of 5 29 | 32, of 8 39 | 34; 24 states, fp32, 64 of 5 72 | 90, of 17 148 | 174, of
+// 64 444 | 472, bf16, of 17 150 | 156, of 20 165 | 155; 32 states, 64 of 5 79 | 93, of 8 95 | 95.  4096 of 64 states: 64 of 33 249 | 155, 200 of 3 283 | 156.
+bool scan_short(const ca_spans& sp, int channels, int n_states, bool bits16) {
+    if (n_states <= 4 || n_states > 32 || sp.max_tokens > 128) return false;
+    const int per_block = SCAN_THREADS / scan_lanes(n_states, 8);
+    const double ctas = (double)((channels + per_block - 1) / per_block) * sp.n_entries, mean = (double)sp.n_tokens / sp.n_entries;
+    if (n_states <= 8) return bits16 && mean <= 6;
+    if (n_states > 24) return mean <= 6;
+    if (mean <= 9) return true;
+    if (n_states > 16) return ctas >= 1024 && mean <= (bits16 ? 18 : 64);
+    return bits16 ? ctas >= 4096 && mean <= 56 : (ctas >= 1024 && mean <= 36) || (ctas >= 2048 && mean <= 100);
+}
+
+// CTAs of the kernel with staged inputs that share the spans.  One each, or, of short spans, several: a CTA's beginning costs as much as about 7
+// tokens (200 spans of 3 tokens, 8192 channels of 16 states: 133 us with one each, 90 so; 64 of 20: 107 and 81), and the next span's rows arrive
+// under the present one.
 int scan_rows(const ca_spans& sp, int blocks, int resident) {
     constexpr int SHORT = 40, BEGIN = 7;
     const int E = sp.n_entries;
@@ -793,6 +967,11 @@ template <typename T>
 int selective_scan(const ScanParams& p, int per_lane, cudaStream_t stream) {
     if (p.sp.max_tokens == 1 && p.N <= 128)
         by_lanes(scan_lanes(p.N, 4), [&](auto l) { launch_scan_step<T, decltype(l)::value>(p, stream); });
+    else if (p.run == 0 && scan_short(p.sp, p.C, p.N, sizeof(T) == 2))
+        by_lanes(scan_lanes(p.N, 8), [&](auto l) {
+            constexpr int L = decltype(l)::value;
+            if constexpr (L <= 4) scan_short_kernel<T, L><<<dim3((p.C * L + SCAN_THREADS - 1) / SCAN_THREADS, p.sp.n_entries), SCAN_THREADS, 0, stream>>>(p);
+        });
     else
         by_lanes(scan_lanes(p.N, per_lane), [&](auto l) {
             constexpr int L = decltype(l)::value;

@@ -41,7 +41,10 @@ def scan(lens, channels, states, dtype, A=None):
     (EDGES, 40, 3), (EDGES, 33, 6), (EDGES, 136, 8), (EDGES, 72, 16), (EDGES, 72, 18), (EDGES, 40, 64), (EDGES, 17, 129), (EDGES, 24, 256),
     ([40] * 20, 4096, 16), ([33] * 8, 4096, 64), ([300, 257], 200, 4), ([300, 257], 200, 16), ([400], 136, 128), ([400, 31], 130, 160),
     ([33] * 130, 64, 16),  # more spans than are put into order
-    ([3, 32, 1, 9] * 60, 1024, 16), ([3, 32, 1, 9] * 60, 264, 100)])  # short ones: several by a CTA
+    ([3, 32, 1, 9] * 60, 1024, 16), ([3, 32, 1, 9] * 60, 264, 100),  # short ones: several by a CTA
+    # the kernel of short spans: one to four lanes a channel, some without states, rows that are not read four at a time
+    ([1, 7, 8, 2, 9, 1, 17, 3], 40, 5), ([1, 7, 8, 2, 9, 1, 17, 3], 33, 8), ([1, 7, 8, 2, 9, 1, 33, 3], 72, 16), ([1, 7, 8, 2, 9, 1, 33, 3], 36, 13),
+    ([1, 7, 8, 2, 9, 1, 17, 3], 72, 18), ([1, 7, 8, 2, 9, 1, 17, 3], 40, 32), ([33, 64, 65, 8] * 16, 4096, 16), ([33, 64, 65, 8] * 8, 1100, 20), ([128] + [1] * 15, 70, 16)])
 def test_scan_shapes(lens, channels, states, dtype):
     y, state, want, ends = scan(lens, channels, states, dtype)
     close(y, np.concatenate(want), dtype)
@@ -83,11 +86,12 @@ class Spans(C.Structure):
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
-@pytest.mark.parametrize("lens,channels", [([3, 0, 5] * 100, 8192), ([0, 0, 9, 33, 0] * 25, 4096), ([0, 40], 64)])
-def test_spans_without_tokens(lens, channels, dtype):
+@pytest.mark.parametrize("lens,channels", [([3, 0, 5] * 100, 8192), ([0, 0, 9, 33, 0] * 40, 4096), ([0, 40], 64)])
+@pytest.mark.parametrize("N", [16, 64])   # the kernel of short spans, and the one whose CTAs have several
+def test_spans_without_tokens(lens, channels, N, dtype):
     # batches that the C interface takes: a CTA that has several spans goes on behind one without tokens, whose state stays (or, at a
     # sequence's beginning, becomes zero).  Compared with the batch without those spans, bit by bit
-    N, E, n = 16, len(lens), sum(lens)
+    E, n = len(lens), sum(lens)
     bf16 = dtype == torch.bfloat16
     x, z, dt, bc = rnd(1, n, channels).to(dtype).to(DEV), rnd(2, n, channels).to(dtype).to(DEV), rnd(3, n, channels).to(DEV), rnd(4, n, 2 * N).to(DEV)
     A, D, bias = (-torch.exp(rnd(5, channels, N))).to(DEV), rnd(6, channels).to(DEV), (rnd(7, channels) - 2).to(DEV)
@@ -112,6 +116,7 @@ def test_spans_without_tokens(lens, channels, dtype):
 
     y, state = run(list(range(E)))
     want_y, want = run([e for e in range(E) if lens[e]])
+    assert bool(torch.isfinite(want_y).all())
     for e in range(E):
         if not lens[e] and e % 2 == 0:
             want[e] = 0
