@@ -135,7 +135,7 @@ struct ca_context {
         int max_item_tiles = 0;
         bool gaps = false;             // Plan::gaps
         int32_t short_slot_base = 0;
-        int64_t tail_rounds = 0;       // 8-token rounds of all tails at the refresh
+        int64_t tail_rounds = 0, tail_tokens = 0;  // 8-token rounds and tokens of all tails at the refresh
         int direct_cluster = 0, direct_blocks = 0, direct_rows = 0;  // Plan::direct_*
         ca_plan_stats stats{};
     } meta;
@@ -571,8 +571,11 @@ static int upload_plan(ca_context* c, const ca::Plan& pl, cudaStream_t stream) {
     c->meta.max_item_tiles = 0;
     for (const ca::PlanItem& it : pl.items) c->meta.max_item_tiles = std::max(c->meta.max_item_tiles, (int)it.n_tiles);
     c->meta.short_slot_base = pl.short_slot_base;
-    c->meta.tail_rounds = 0;
-    for (int32_t t : pl.tail_tokens) c->meta.tail_rounds += (t + 7) / 8;
+    c->meta.tail_rounds = c->meta.tail_tokens = 0;
+    for (int32_t t : pl.tail_tokens) {
+        c->meta.tail_rounds += (t + 7) / 8;
+        c->meta.tail_tokens += t;
+    }
     c->meta.direct_cluster = pl.direct_cluster;
     c->meta.direct_rows = pl.direct_rows;
     c->meta.direct_blocks = (int)(pl.direct_blocks.size() / 2);
@@ -634,18 +637,26 @@ static bool tails_can_finish(const ca_context* c) {
 }
 
 // True when the wide-runs kernel does the whole step: all rows are in one run, cut into at most two pieces, and have nothing
-// beside it but a short tail; and where that is faster.  A CTA's tails are walked by few warps, so they must be few beside its tiles, and
-// every SM needs its CTAs.  32 heads, steps back to back, two or three kernels -> one, in us: 1000 rows of 2048 shared and 4 / 20 / 40 own
-// tokens 67 / 105 / 153 -> 58 / 93 / 153; of 512 shared and 4 / 20 (8 tiles a CTA, 3 rounds of 8 tokens a row) 41 / 78 -> 36 / 79; 560 rows of
-// 2048 and 20 (160 CTAs on 148 SMs) 68 -> 76; 830 (224 CTAs) 92 -> 85; 400 of 512 and 4 (4 tiles) 23 -> 25.
+// beside it but a short tail; and where that is faster.  A CTA's tails are walked by few warps, so they must be few beside its tiles; every
+// SM needs its CTAs, the last wave its share of them, and the tails must be long enough for the kernel of their own to take its time.
+// Steps back to back, two or three kernels -> one, in us, by CTAs of 148 SMs that hold two each.  One piece, 32 heads, 2048 shared tokens and 1 | 8 own:
+// 192 CTAs 51 -> 55 | 59 -> 57, 224 55 -> 56 | 63 -> 57, 256 58 -> 55 | 68 -> 60, 288 66 -> 55 | 85 -> 64, 320 96 -> 91 | 115 -> 95, 384 108 -> 92 |
+// 130 -> 96, 576 128 -> 110 | 165 -> 129; 512 shared: 224 33 -> 34 | 43 -> 39, 256 36 -> 34 | 47 -> 41, 320 54 -> 59 | 75 -> 67, 384 61 -> 59 | 87 -> 76.
+// Two pieces, 16 heads, 1536 shared: 224 29 -> 34 | 33 -> 35, 256 31 -> 34 | 36 -> 35, 288 32 -> 34 | 40 -> 36; 3776 shared: 320 76 -> 84 | 86 -> 87,
+// 448 88 -> 96 | 100 -> 98, 576 102 -> 100 | 122 -> 105, 768 145 -> 146 | 170 -> 149.  1000 rows of 2048 and 20 | 40 own (one piece, 256) 105 -> 93 |
+// 153 -> 153; of 512 and 20 (8 tiles a CTA, 3 rounds of 8 tokens a row) 78 -> 79.
 static bool wide_can_finish(const ca_context* c) {
     if (!c->fast || !c->opt_finish_in_tails || !c->opt_finish_in_wide || c->opt_overlap || c->trace || c->meta.split_phases || c->meta.n_items_wide == 0 ||
         c->meta.n_items_short != c->meta.n_seqs || c->meta.n_items_short + c->meta.n_items_wide != c->meta.n_items || c->meta.wide_pieces < 1 ||
         c->meta.wide_pieces > 2)
         return false;
-    const double H = c->geo.n_heads, ctas = c->meta.n_items_wide * H, tiles = (double)c->meta.n_wide_chunks / c->meta.wide_pieces,
-                 rounds = (c->meta.tail_rounds + c->meta.n_seqs * (c->delta_tokens / 8.0)) * H / (128 * ctas);
-    return c->opt_finish_in_wide == 2 || (tiles >= 8 && tiles >= 4 * rounds && (ctas >= 1.46 * c->num_sms));
+    if (c->opt_finish_in_wide == 2) return true;
+    const double H = c->geo.n_heads, n = c->meta.n_seqs, ctas = c->meta.n_items_wide * H, tiles = (double)c->meta.n_wide_chunks / c->meta.wide_pieces,
+                 rounds = (c->meta.tail_rounds + n * (c->delta_tokens / 8.0)) * H / (128 * ctas), own = c->meta.tail_tokens / n + c->delta_tokens,
+                 waves = ctas / (2.0 * c->num_sms);
+    if (tiles < 8 || tiles < (waves < 0.95 ? 5 : 4) * rounds) return false;  // 256 CTAs of 18 tiles and 4 rounds 112 -> 116, 288 of 15 129 -> 118
+    if (c->meta.wide_pieces == 2) return own >= 4 && (waves <= 1 ? waves >= 0.95 : waves >= 1.85);
+    return waves <= 1 ? waves >= (own >= 3 ? 0.73 : 0.85) : tiles >= 24 || waves >= 1.28 || own >= 4;
 }
 
 // The partial results of a step.  finish != null and tails_can_finish(): the short-tails kernel goes LAST and stores the

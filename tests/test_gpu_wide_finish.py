@@ -114,3 +114,17 @@ def test_where_it_is_taken():
     assert eng.ctx.stats()["kernels_per_step"] == 3
     with pytest.raises(cabi.CAError):
         eng.ctx.set_option(cabi.CA_OPT_FINISH_IN_WIDE, 3)
+
+
+@pytest.mark.parametrize("H,n,shared,own,one", [(16, 856, 1536, 1, False),   # two pieces, 224 CTAs: 29 us in three kernels, 34 in one
+                                                (16, 856, 1536, 8, False), (16, 1112, 1536, 8, True),
+                                                (32, 600, 3776, 1, False),  # more CTAs than a wave, most of the last one idle: 78 and 85
+                                                (32, 984, 1024, 8, True), (32, 856, 1024, 1, False)])
+def test_rule(H, n, shared, own, one):
+    # the work list alone says which way a step goes: no tokens are stored here
+    eng = CabiEngine(H, 128, C, torch.float16, max_chunks=shared // C + n + 4)
+    for i in range(n):
+        eng.tree.add_seq_detailed(list(range(shared)) + [10_000 * (i + 1) + j for j in range(own)])
+    eng.refresh()
+    st = eng.ctx.stats()
+    assert st["n_items_wide"] > 0 and (st["kernels_per_step"] == 1) == one
