@@ -190,6 +190,8 @@ double waves(double ctas, double slots) {
 // 12.1 -> 8.4, of 4000 16.9 -> 14.1; 32 heads, 4 rows of 256 shared and 200 own 10.9 -> 8.7; 16 rows over 256 shared 11.7 -> 9.0;
 // 12 heads of 64, 16 rows of 500 shared and 250 own 11.5 -> 8.1.  Larger steps belong to the items: 64 rows of 1100 tokens, 8 heads,
 // 52 against 59 (CTAs of units that differ cannot take over from each other), 16 rows of 2048 shared and 1100 own, 32 heads, 62 against 69.
+// The items' times are of steps launched by the host, which takes 7.8 us for two kernels.  Replayed from a graph, 16 of 260 steps are more than
+// 3 % slower here than by items, those of one head over 2048 shared tokens most (20 rows 6.9 -> 9.7); all together take 0.84 of the time.
 void build_direct(Plan& plan, int mode, int d_head, bool items, int group) {
     const int columns = std::max(1, group);  // of a row
     plan.direct_cluster = 0;
@@ -264,15 +266,23 @@ void build_direct(Plan& plan, int mode, int d_head, bool items, int group) {
         other = 9.0 + 0.16 * mb + 2.2e-3 * (double)(pairs * group) + 0.13 * plan.max_merge_len;
     } else if (items) {  // two launches, K/V at HBM rate; shared runs bring a partial result per row and piece
         other = 7.8 + (double)plan.stats.unique_kv_bytes / 6.9e6 + (plan.stats.n_runs > 0 ? 3.5e-3 * (double)pairs + 0.03 * plan.max_merge_len : 0.0);
-    } else {      // the any-geometry kernel: every row walks its whole path
-        const int block = d_head <= 32 ? 32 : 16;
+    } else {
+        // The any-geometry kernel: every row walks its whole path, in blocks of tokens that end where a chunk does.  Fitted to steps replayed from
+        // a captured graph, 420 of them (heads of 16 to 128 in chunks of 16 to 64, 1 to 64 rows, 0 to 2048 shared and 3 to 2000 own tokens), where
+        // no launch hides what the smallest take; of 420 others 8 are more than 3 % slower than there, and all together take 0.84 of the time.
+        // That kernel -> this one: 1 head of 64, 7 rows of 128 shared and 21 own 4.0 -> 5.4 us, 8 heads of 64, 7 rows of 10 2.9 -> 3.3, 12 of 16, 32
+        // rows of 500 and 419 22.1 -> 10.8, 16 of 64, 54 rows of 1024 and 49 38.4 -> 11.1.
+        const int size = d_head <= 32 ? 0 : (small ? 1 : 2), block = size == 0 ? 32 : 16, C = plan.chunk_size;
         int64_t c = 1, total = 0;
         while (c < 8 && pairs * c * 2 <= 4 * B200_SMS && c * 4 * block < plan.max_path_tokens) c *= 2;
         for (int32_t n : plan.path_tokens) total += n;
-        const double per_warp = (double)(((plan.max_path_tokens + block - 1) / block + 4 * c - 1) / (4 * c));
-        const double W = waves((double)(pairs * c), B200_SMS * (small ? 7.0 : 4.0));
-        if (d_head > 32) margin = small ? 1.3 : (any_shared ? 1.05 : 0.95);
-        other = 3.0 + W * (1.0 + (small ? 0.5 : 1.1) * per_warp) + (c > 1 ? 0.7 : 0.0) + (double)(total * H) * d_head * 4 / 20e6;
+        const int64_t blocks = (int64_t)(plan.max_path_tokens / C) * ((C + block - 1) / block) + (plan.max_path_tokens % C + block - 1) / block;
+        const double per_warp = (double)((blocks + 4 * c - 1) / (4 * c)), x = (double)(pairs * c) / (B200_SMS * (2.5 + 0.5 * size));
+        const double W = x <= 1 ? 1 : x + (size == 0 ? 0.5 : 0.3);
+        constexpr double FIT[3][5] = {{1.7, 0.48, 0.78, 1.35, 0.0}, {1.14, 0.97, 0.87, 1.38, 0.75}, {0.0, 2.3, 1.12, 1.43, 1.52}};
+        const double* f = FIT[size];
+        margin = 0.97;
+        other = f[0] + W * (f[1] + f[2] * per_warp) + (c > 1 ? f[3] : 0.0) + f[4] * (double)(total * H) * d_head * 4 / 20e6;
     }
     if (mode == 2 || best < margin * other) cut_direct(plan, rows, cluster, columns);
 }

@@ -85,6 +85,13 @@ def test_which_way():
     assert large.direct(1, 128) == 0 and large.direct(2, 128) > 0
     tails, _ = plan_of(build_tree(shared_spec(300, 128, 4)), 8)
     assert tails.stats()["n_items_short"] > 0 and tails.direct(1, 128) == 0
+    # where the any-geometry kernel is the alternative, the smallest steps are its own
+    least, _ = plan_of(build_tree(shared_spec(7, 128, 21), chunk_size=16), 1)
+    assert least.direct(1, 64, against_items=False) == 0 and least.direct(2, 64, against_items=False) > 0
+    few, _ = plan_of(build_tree(shared_spec(7, 0, 10)), 8)
+    assert few.direct(1, 64, against_items=False) == 0
+    over, _ = plan_of(build_tree(shared_spec(54, 1024, 49), chunk_size=16), 16)
+    assert over.direct(1, 64, against_items=False) > 0
     with pytest.raises(cabi.CAError):
         small.direct(1, 256)
     with pytest.raises(cabi.CAError):
