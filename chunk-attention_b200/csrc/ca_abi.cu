@@ -908,8 +908,14 @@ int ca_peer_barrier(void* const* flag_arrays, int n_peers, int rank, uint32_t ep
 }
 
 // The step goes to the one-launch kernel: the work list has its form, no option looks at the kernels of the item lists, and rows
-// can be moved in whole granules.
+// can be moved in whole granules.  A call that brings its queries from the host and waits for its rows pays for the kernel's chain and not for a
+// second launch, which the first kernel covers: few rows by clusters of CTAs are faster by items there (us a call, items | here: 4 heads, 1 row of
+// 1373 tokens 18.7 | 20.4, 16 heads, 1 of 864 19.5 | 21.8, 2 heads, 10 rows of 339 19.3 | 20.8, 8 heads, 2 of 339 19.6 | 20.5; in the mean of 25
+// such calls 0.96; but 4 heads, 8 rows of 381 21.7 | 21.1, 32 heads, 10 rows of 77 shared and 22 30.0 | 23.8; in the mean of 31 calls of 21 to 64
+// rows and heads by clusters of 8 CTAs 1.04, of 20 of more than 100 1.11, and without clusters 1.00 to 1.23).
 static bool goes_direct(const ca_context* c, const void* q = nullptr, const void* out = nullptr) {
+    constexpr int64_t HOST_MIN_PAIRS = 21;
+    if (c->out_is_host && c->fast && c->opt_direct != 2 && c->meta.direct_cluster > 1 && (int64_t)c->meta.n_seqs * c->geo.n_heads < HOST_MIN_PAIRS) return false;
     return c->meta.direct_cluster > 0 && c->opt_withhold_item < 0 && !c->trace && !c->opt_overlap &&
            (reinterpret_cast<uintptr_t>(c->pool) | reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(out)) % 16 == 0;
 }

@@ -183,6 +183,24 @@ def test_the_same_as_the_other_kernels():
             assert (res.float() - out[0]).abs().max() < TOL
 
 
+@pytest.mark.parametrize("H,lens,items", [(4, [400], True), (2, [339] * 10, True), (8, [64], False), (32, [400], False)])
+def test_host_calls_of_few_rows(H, lens, items):
+    # calls on host buffers: few rows that would take clusters of CTAs go by items, bit by bit as with the one-launch kernel off
+    g = torch.Generator().manual_seed(H)
+    eng = engine(H, 128, 64, max_chunks=sum(n // 64 + 3 for n in lens), mode=1)
+    ctx = fill(eng, g, 0, lens)
+    q = torch.randn(len(lens), H, 128, generator=g).half()
+    out = {}
+    for mode in (0, 1, 2):
+        eng.ctx.set_option(cabi.CA_OPT_DIRECT, mode)
+        eng.valid = False
+        eng.refresh()
+        out[mode] = torch.empty_like(q)
+        eng.ctx.attention_host(q, out[mode])
+        assert (out[mode].double() - dense(q, ctx, 128 ** -0.5)).abs().max() < TOL
+    assert not torch.equal(out[0], out[2]) and torch.equal(out[1], out[0 if items else 2])
+
+
 def test_captured_and_replayed():
     H, d, chunk, g = 4, 64, 32, torch.Generator().manual_seed(1)
     eng = engine(H, d, chunk, max_chunks=40)
