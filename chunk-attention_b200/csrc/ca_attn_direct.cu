@@ -1,8 +1,8 @@
 // Decode attention of small steps in ONE launch: fp16 caches with rows of whole 16-byte granules and d_head <= 128, and bf16 caches of
 // grouped heads (1, 2, 4 or 8 query heads to a key/value head) of 64 or 128 elements.
 //
-// A unit is a key/value head and a block of up to 8 columns: consecutive rows, each with the query heads of the group; its work is the list of chunks that any of the rows
-// sees, each with the set of columns that see it, so a shared chunk is read once for the block.  The list is cut into steps of 16
+// A unit is a key/value head and a block of up to 8 columns: consecutive rows, each with the query heads of the group; its work is the list
+// of chunks that any of the rows sees, each with the set of columns that see it, so a shared chunk is read once for the block.  The list is cut into steps of 16
 // tokens, dealt in consecutive ranges to the warps of a CLUSTER of 1 to 8 CTAs per unit (cut by the host, ca_plan.h).  A
 // warp takes K and V from global memory straight into registers, as the operands of mma.sync:
 //   S^T = K Q^T          lane (g, c) = (lane / 4, lane % 4) holds granules 4 j + c of tokens g and g + 8: their four registers are
@@ -22,8 +22,9 @@
 // scheduler's time, 20 until the result is there) and one trip to memory; maxima are exchanged between lanes only when a score
 // exceeds the reference in use by 2^8, as in the other kernels.
 // Measured (B200, steps back to back, partial results and merge or any-geometry kernel -> here): 32 heads of 128, one row of 1500
-// tokens 12.1 -> 8.5 us; 8 heads, 4 rows of 300 tokens 8.0 -> 5.8; 12 heads of 64, 16 rows of 500 shared and up to 333 own tokens
-// 11.5 -> 8.2.  Errors against 64 bits are the rounding of the result alone (2.1e-4 of its norm; weights of 11 bits: 2.8e-4).
+// tokens 12.3 -> 9.0 us; 8 heads, 4 rows of 300 tokens 9.6 -> 7.5; 12 heads of 64, 16 rows of 500 shared and up to 333 own tokens
+// 12.8 -> 8.7 (8.8, 7.3 and 8.7 without the second look at infinite values and with a reference at the maximum).  Errors against 64 bits are the
+// rounding of the result alone (2.1e-4 of its norm; weights of 11 bits: 2.8e-4).
 // Tried and slower: a ring of three steps per warp in shared memory, filled by cp.async (8 warps on an SM instead of 12, a third more
 // instructions): one row of 1500 tokens 9.3 -> 10.5 us.
 #include <cooperative_groups.h>

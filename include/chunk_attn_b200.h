@@ -123,11 +123,13 @@ CA_API int ca_context_create_shaped(ca_context** out, int device, const ca_head_
 #define CA_OPT_SEQ_FIRST_TENSOR 3
 /* 1: the attention kernel records per-CTA nanosecond timestamps, read with ca_context_read_trace;
  * 2: as 1, but the tcgen05 kernel for wide runs accounts for the cycles of its two serial roles instead
- * (see ca_context_read_trace) */
+ * (see ca_context_read_trace).  While a trace is on, every step goes by the kernels of the item lists: those that do a step in one
+ * launch (CA_OPT_DIRECT, CA_OPT_FINISH_IN_WIDE) stand aside. */
 #define CA_OPT_TRACE 4
 /* programmatic dependent launches: bit 0, the merge kernel is set up while the attention kernel
  * drains; bit 1, the attention kernel is set up while the kernel before it in the stream finishes
- * (it waits for that kernel's completion before it touches global memory).  Default 3. */
+ * (it waits for that kernel's completion before it touches global memory; the item kernel of grouped heads
+ * is always launched in the ordinary way).  Default 3. */
 #define CA_OPT_DEPENDENT_LAUNCH 5
 /* Shared runs on the tcgen05 / TMEM kernel (tensor memory accumulators, tcgen05.mma fed by descriptor from the
  * staged tiles): 0 never, 1 (default) when walking the step's wide runs (more than 32 rows) with mma.sync would
@@ -157,8 +159,9 @@ CA_API int ca_context_create_shaped(ca_context** out, int device, const ca_head_
 /* Decode steps of latent caches whose sequences share nothing: a CTA or two for every sequence, one launch, instead of items whose
  * partial results a second kernel combines: 1 (default) where that is faster, 0 never, 2 always. */
 #define CA_OPT_LATENT_ROWS 14
-/* Steps of fp16 caches with d_head <= 128 in one launch instead of partial results and their combination: 1 (default) where
- * that is faster, 0 never, 2 always. */
+/* Steps of fp16 caches with d_head <= 128, and decode steps of bf16 caches of grouped heads (1, 2, 4 or 8 query heads to a key/value head
+ * of 64 or 128 elements), in one launch instead of partial results and their combination: 1 (default) where that is faster, 0 never,
+ * 2 always. */
 #define CA_OPT_DIRECT 12
 /* Failure-path tests only: the CTA that draws item `value` of the next launches (portions of prompts on tcgen05: piece
  * `value`, key/value heads fastest) stops feeding its consumer warps, whose bounded wait then runs out (status 1; portions:

@@ -2,7 +2,8 @@
     python tests/wide_cycle_accounting.py
 sets CA_OPT_TRACE = 2, runs a few decode steps of three shapes whose shared runs the planner routes to that kernel,
 and prints, per K/V tile, the SM cycles of the CTA's two serial roles: the thread that issues the MMAs (issuing,
-waiting for P, waiting for the K tile) and a softmax thread (waiting for a score tile, from scores to P)."""
+waiting for P, waiting for the K tile) and a softmax thread (waiting for a score tile, from scores to P).  A traced step takes
+the kernel without the tails (a trace keeps the finishing form, which serves steps of short tails over one prompt, aside)."""
 import sys, os
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 for p in (ROOT, os.path.join(ROOT, "chunk-attention_b200"), os.path.join(ROOT, "oracle"), os.path.join(ROOT, "tests")):
