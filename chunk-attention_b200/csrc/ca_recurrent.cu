@@ -721,7 +721,7 @@ ScanShape scan_shape(const ca_spans& sp, int channels, int n_states) {
 // 8192 channels of 8 states, bf16, 64 of 5 28 | 32, of 12 49 | 39; fp32, of 5 29 | 32, of 8 39 | 34; 24 states, fp32, 64 of 5 72 | 90, of 17 148 | 174, of
 // 64 444 | 472, bf16, of 17 150 | 156, of 20 165 | 155; 32 states, 64 of 5 79 | 93, of 8 95 | 95.  4096 of 64 states: 64 of 33 249 | 155, 200 of 3 283 | 156.
 bool scan_short(const ca_spans& sp, int channels, int n_states, bool bits16) {
-    if (n_states <= 4 || n_states > 32 || sp.max_tokens > 128) return false;
+    if (n_states <= 4 || n_states > 32 || sp.max_tokens > 128 || sp.n_entries > 65535) return false;  // a span is a row of the grid
     const int per_block = SCAN_THREADS / scan_lanes(n_states, 8);
     const double ctas = (double)((channels + per_block - 1) / per_block) * sp.n_entries, mean = (double)sp.n_tokens / sp.n_entries;
     if (n_states <= 8) return bits16 && mean <= 6;
