@@ -15,15 +15,15 @@
 // dropped, so a row's infinities never meet another row.  Areas are combined per CTA, and the CTAs' results through
 // distributed shared memory: no partial results in global memory, no second launch.
 // Infinite values of an fp16 cache: a weight's hi part times infinity is the result, its lo part times infinity is NaN or the other
-// infinity.  Elements that come out as NaN are computed once more, with fp32 weights in fp32 products (redo below): what is not a number
-// then is none.
+// infinity.  A row with an element that is not finite in any CTA is computed once more, with fp32 weights in fp32 products (redo): what
+// is not a number then is none.  The rows' marks travel with what the CTAs tell each other anyway.
 // Bound: latency (launch, work list, tokens, meeting), and the bytes in flight: 8 KiB a warp, K of the next step requested
 // as soon as K of this one is used, V likewise; 12 warps of an SM have 96 KiB under way.  A step is 16 MMAs (8 cycles each of a
 // scheduler's time, 20 until the result is there) and one trip to memory; maxima are exchanged between lanes only when a score
 // exceeds the reference in use by 2^8, as in the other kernels.
 // Measured (B200, steps back to back, partial results and merge or any-geometry kernel -> here): 32 heads of 128, one row of 1500
-// tokens 12.3 -> 9.0 us; 8 heads, 4 rows of 300 tokens 9.6 -> 7.5; 12 heads of 64, 16 rows of 500 shared and up to 333 own tokens
-// 12.8 -> 8.7 (8.8, 7.3 and 8.7 without the second look at infinite values and with a reference at the maximum).  Errors against 64 bits are the
+// tokens 12.3 -> 8.9 us; 8 heads, 4 rows of 300 tokens 9.6 -> 7.5; 12 heads of 64, 16 rows of 500 shared and up to 333 own tokens
+// 12.8 -> 8.8 (8.8, 7.5 and 8.7 without the second look at infinite values).  Errors against 64 bits are the
 // rounding of the result alone (2.1e-4 of its norm; weights of 11 bits: 2.8e-4).
 // Tried and slower: a ring of three steps per warp in shared memory, filled by cp.async (8 warps on an SM instead of 12, a third more
 // instructions): one row of 1500 tokens 9.3 -> 10.5 us.
@@ -95,16 +95,119 @@ template <> struct Reference<__half> {
 template <int VG> struct DirectSmem {
     static constexpr int DV = VG * 64, PITCH = DV + 4;             // floats of a row
     static __host__ __device__ constexpr int stats(int rows) { return D_WARPS * rows * PITCH * 4; }
-    static __host__ __device__ constexpr int again(int rows) { return stats(rows) + D_WARPS * rows * 8 + D_WARPS * 4; }  // [3][D_ROWS]
-    static __host__ __device__ constexpr int bytes(int rows) { return again(rows) + 3 * D_ROWS * 4; }
+    static __host__ __device__ constexpr int again(int rows) { return stats(rows) + D_WARPS * rows * 8 + D_WARPS * 4; }  // [2] rows, [2][D_ROWS]
+    static __host__ __device__ constexpr int bytes(int rows) { return again(rows) + (2 + 2 * D_ROWS) * 4; }
 };
+
+// fp16 elements d .. d + 7 of column n, where its row goes
+template <bool PEERS> __device__ __forceinline__ void store_half8(const DirectParams& p, int row, int head, int d, const uint4& packed) {
+    if (!PEERS) {
+        *reinterpret_cast<uint4*>(static_cast<__half*>(p.out) + ((size_t)row * p.n_heads + head) * p.d + d) = packed;
+    } else {  // head-sharded: into every rank's full-width output, by the switch or by plain stores over NVLink
+        const size_t to = ((size_t)row * p.total_heads + p.head_offset + head) * p.d + d;
+        if (p.mc_out) {
+            asm volatile("multimem.st.weak.global.v4.f16x2 [%0], {%1, %2, %3, %4};" ::"l"(static_cast<__half*>(p.mc_out) + to), "r"(packed.x),
+                         "r"(packed.y), "r"(packed.z), "r"(packed.w)
+                         : "memory");
+        } else {
+            for (int k = 0; k < p.n_peers; k++) *reinterpret_cast<uint4*>(static_cast<__half*>(p.peer_out[k]) + to) = packed;
+        }
+    }
+}
+
+// Rows of an fp16 block once more over all of their tokens, row by row, a half-warp per token, a lane per granule.  A function of its own: as
+// a part of the kernel it cost every step time, by what the compiler made of the rest (32 heads, 1 row of 1500 tokens 8.8 without it, 9.1 as a
+// part, 8.9 so; 4 rows of 256 shared and 200 own 9.4, 9.8, 9.5; 12 heads of 64, 16 rows of 500 and 333 8.7, 8.8, 8.8).
+template <int VG, bool PANELS, bool PEERS> __device__ __noinline__ void redo(const DirectParams& p, uint8_t* smem, int rows_again) {
+    using Smem = DirectSmem<VG>;
+    constexpr int DV = Smem::DV, PITCH = Smem::PITCH;
+    float* const area = reinterpret_cast<float*>(smem);
+    const float* const again_m = reinterpret_cast<const float*>(smem + Smem::again(p.block_rows)) + 2;
+    const float* const again_inv = again_m + D_ROWS;
+    const int unit = blockIdx.x / p.cluster, block = unit / p.n_heads, head = unit - block * p.n_heads;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, C = p.chunk_size;
+    const int2 rows = __ldg(p.blocks + block);
+    const int row_begin = rows.x, n_rows = rows.y;
+    int e_begin = 0, e_end = -1;  // the block's entries
+    for (int w = 0; w < p.cluster * D_WARPS; w++) {
+        const int4 of = __ldg(p.ranges + (size_t)block * (p.cluster * D_WARPS) + w);
+        if (of.x > of.z) continue;
+        if (e_end < 0) e_begin = of.x;
+        e_end = of.z;
+    }
+    const int G = lane & 15;
+    for (int n = 0; n < n_rows; n++) {
+        if (!((rows_again >> n) & 1)) continue;
+        const float mm = again_m[n], ref = mm == -INFINITY ? 0.f : mm;
+        uint4 qn = make_uint4(0u, 0u, 0u, 0u);
+        if (G < p.gpr) qn = __ldg(reinterpret_cast<const uint4*>(p.q) + ((size_t)(row_begin + n) * p.n_heads + head) * p.gpr + G);
+        float acc[8];
+#pragma unroll
+        for (int k = 0; k < 8; k++) acc[k] = 0.f;
+        for (int e = e_begin; e <= e_end; e++) {
+            const int4 of = __ldg(p.entries + e);
+            if (!((of.z >> n) & 1) || of.x < 0 || of.x >= p.max_chunks) continue;
+            const int tokens = min(C, of.y + (of.w ? p.delta_tokens : 0));
+            const uint8_t* const base = p.pool + ((size_t)of.x * p.n_heads + head) * (size_t)p.pair_bytes;
+            for (int t0 = 0; t0 < tokens; t0 += 2 * D_WARPS) {
+                const int t = t0 + 2 * warp + (lane >> 4);
+                const bool on = t < tokens && G < p.gpr;
+                const size_t at = PANELS ? (size_t)((((G >> 3) * C + t) * 8 + ((G & 7) ^ (t & 7))) * 16) : (size_t)((t * p.gpr + G) * 16);
+                float x = 0.f;
+                uint4 vn = make_uint4(0u, 0u, 0u, 0u);
+                if (on) {
+                    const uint4 kn = __ldg(reinterpret_cast<const uint4*>(base + at));
+                    vn = __ldg(reinterpret_cast<const uint4*>(base + p.v_offset + at));
+#pragma unroll
+                    for (int k = 0; k < 4; k++) {
+                        const float2 a = half2_of((&qn.x)[k]), b = half2_of((&kn.x)[k]);
+                        x = fmaf(a.x, b.x, x);
+                        x = fmaf(a.y, b.y, x);
+                    }
+                }
+#pragma unroll
+                for (int off = 8; off >= 1; off >>= 1) x += __shfl_xor_sync(0xffffffffu, x, off);
+                if (on) {
+                    const float w = exp2f(x * p.scale_log2 - ref);
+#pragma unroll
+                    for (int k = 0; k < 4; k++) {
+                        const float2 b = half2_of((&vn.x)[k]);
+                        acc[2 * k] = fmaf(w, b.x, acc[2 * k]);
+                        acc[2 * k + 1] = fmaf(w, b.y, acc[2 * k + 1]);
+                    }
+                }
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < 8; k++) acc[k] += __shfl_xor_sync(0xffffffffu, acc[k], 16);
+        if (lane < 16 && 8 * lane < DV) {
+            float4* const dst = reinterpret_cast<float4*>(area + warp * PITCH + 8 * lane);
+            dst[0] = make_float4(acc[0], acc[1], acc[2], acc[3]);
+            dst[1] = make_float4(acc[4], acc[5], acc[6], acc[7]);
+        }
+        __syncthreads();
+        if (threadIdx.x < DV / 8 && 8 * (int)threadIdx.x < p.d) {
+            float v[8];
+#pragma unroll
+            for (int k = 0; k < 8; k++) {
+                v[k] = 0.f;
+#pragma unroll
+                for (int w = 0; w < D_WARPS; w++) v[k] += area[w * PITCH + 8 * threadIdx.x + k];
+            }
+            const float inv = again_inv[n];
+            store_half8<PEERS>(p, row_begin + n, head, 8 * (int)threadIdx.x,
+                               make_uint4(pack_half2(v[0] * inv, v[1] * inv), pack_half2(v[2] * inv, v[3] * inv), pack_half2(v[4] * inv, v[5] * inv), pack_half2(v[6] * inv, v[7] * inv)));
+        }
+        __syncthreads();
+    }
+}
 
 // KQ: groups of 4 granules of a K row; VG: groups of 8 granules of a V row; PANELS: the pool's swizzled layout (ca_layout.h).
 // LO: 0 weights as one fp16 number; 1 hi and lo in two products; 2 blocks of up to 4 rows, columns 4 .. 7 repeat the rows and take
 // the lo parts, so that one product does both.
 // T bf16: grouped heads, with the sink and the values' turn of their layers.
 template <typename T, int KQ, int VG, bool PANELS, int LO, bool PEERS>
-__global__ void __launch_bounds__(D_WARPS * 32, VG == 2 ? 3 : 4) attn_direct_kernel(const DirectParams p) {
+__global__ void __launch_bounds__(D_WARPS * 32, VG == 2 ? 3 : 4) attn_direct_kernel(const __grid_constant__ DirectParams p) {
     using Smem = DirectSmem<VG>;
     constexpr int DV = Smem::DV, PITCH = Smem::PITCH;
     extern __shared__ __align__(16) uint8_t smem[];
@@ -112,12 +215,12 @@ __global__ void __launch_bounds__(D_WARPS * 32, VG == 2 ? 3 : 4) attn_direct_ker
     float* const area_m = reinterpret_cast<float*>(smem + Smem::stats(p.block_rows));  // [warps][block_rows]
     float* const area_l = area_m + D_WARPS * p.block_rows;
     int* const area_have = reinterpret_cast<int*>(area_l + D_WARPS * p.block_rows);    // [warps]: rows of which the warp saw a token
-    // elements that came out as NaN, of which infinite values may be the cause: a row's granules, its reference and its factor
+    // rows with an element that is not finite, in this CTA and among those that it stores; a row's reference and its factor
     constexpr bool REDO = LO != 0 && std::is_same_v<T, __half>;
     int* const again = reinterpret_cast<int*>(smem + Smem::again(p.block_rows));
-    float* const again_m = reinterpret_cast<float*>(again + D_ROWS);
+    float* const again_m = reinterpret_cast<float*>(again + 2);
     float* const again_inv = again_m + D_ROWS;
-    if (REDO && threadIdx.x < D_ROWS) again[threadIdx.x] = 0;
+    if (REDO && threadIdx.x < 2) again[threadIdx.x] = 0;
 
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
@@ -382,6 +485,7 @@ __global__ void __launch_bounds__(D_WARPS * 32, VG == 2 ? 3 : 4) attn_direct_ker
                 acc.w = fmaf(a[w], v.w, acc.w);
             }
         *reinterpret_cast<float4*>(area + n * PITCH + d) = acc;
+        if (REDO && ((acc.x + acc.y) + (acc.z + acc.w)) * 0.f != 0.f) atomicOr(again, 1 << n);  // infinity and NaN times zero are NaN
     }
     float m_here = -INFINITY, l_here = 0.f;
     if (threadIdx.x < n_rows) {
@@ -393,7 +497,7 @@ __global__ void __launch_bounds__(D_WARPS * 32, VG == 2 ? 3 : 4) attn_direct_ker
         area_m[threadIdx.x] = m_here;
         area_l[threadIdx.x] = l_here;
     }
-    if (threadIdx.x == 0) area_have[0] = any;
+    if (threadIdx.x == 0) area_have[0] = REDO ? any | again[0] << D_ROWS : any;
     const cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
     if (p.cluster > 1) cl.sync();
     else __syncthreads();
@@ -402,33 +506,6 @@ __global__ void __launch_bounds__(D_WARPS * 32, VG == 2 ? 3 : 4) attn_direct_ker
     const int r = threadIdx.x & (p.cluster - 1), mine = (n_rows - rank + p.cluster - 1) / p.cluster;
     const float* from = p.cluster > 1 ? cl.map_shared_rank(area, r) : area;
     const float* from_m = from + (area_m - area);
-    auto store = [&](int n, int d, float (&v)[8], float inv) {
-        if (GROUPED && p.value_freq) {  // values were cached turned by their position: back by the row's
-            const float pos = (float)__ldg(p.positions + row_begin + n / p.group);
-#pragma unroll
-            for (int k = 0; k < 8; k += 2) {
-                float sn, cs;
-                fast_sincos(pos * __ldg(p.value_freq + (d + k) / 2), &sn, &cs);
-                const float x = v[k] * cs + v[k + 1] * sn;
-                v[k + 1] = v[k + 1] * cs - v[k] * sn;
-                v[k] = x;
-            }
-        }
-        const uint4 packed = make_uint4(pack_pair<T>(v[0] * inv, v[1] * inv), pack_pair<T>(v[2] * inv, v[3] * inv), pack_pair<T>(v[4] * inv, v[5] * inv),
-                                        pack_pair<T>(v[6] * inv, v[7] * inv));
-        if (!PEERS) {
-            *reinterpret_cast<uint4*>(static_cast<T*>(p.out) + pair_of(n) * p.d + d) = packed;
-        } else {  // head-sharded: into every rank's full-width output, by the switch or by plain stores over NVLink
-            const size_t to = ((size_t)(row_begin + n) * p.total_heads + p.head_offset + head) * p.d + d;
-            if (p.mc_out) {
-                asm volatile("multimem.st.weak.global.v4.f16x2 [%0], {%1, %2, %3, %4};" ::"l"(static_cast<__half*>(p.mc_out) + to), "r"(packed.x),
-                             "r"(packed.y), "r"(packed.z), "r"(packed.w)
-                             : "memory");
-            } else {
-                for (int k = 0; k < p.n_peers; k++) *reinterpret_cast<uint4*>(static_cast<__half*>(p.peer_out[k]) + to) = packed;
-            }
-        }
-    };
     const uint32_t group = ((1u << p.cluster) - 1) << (lane - r);  // the lanes of a row's other elements may have left the loop
     for (int i = threadIdx.x / p.cluster; i < mine * (DV / 8); i += D_WARPS * 32 / p.cluster) {
         const int n = rank + (i / (DV / 8)) * p.cluster, d = 8 * (i % (DV / 8));
@@ -462,95 +539,44 @@ __global__ void __launch_bounds__(D_WARPS * 32, VG == 2 ? 3 : 4) attn_direct_ker
             inv = mm == -INFINITY ? (((seen >> n) & 1) && !p.zero_if_none ? nanf("") : 0.f) : 1.f / sum;
         }
         if (r > 0 || d >= p.d) continue;
-        if (REDO) {
-            const float any_nan = ((v[0] + v[1]) + (v[2] + v[3])) + ((v[4] + v[5]) + (v[6] + v[7]));  // or infinities of both signs
-            if (any_nan != any_nan) {
-                atomicOr(again + n, 1 << (d >> 3));
+        if (REDO && ((seen >> (D_ROWS + n)) & 1)) {
+            if (d == 0) {
+                atomicOr(again + 1, 1 << n);
                 again_m[n] = mm;
                 again_inv[n] = inv;
-                continue;
+            }
+            continue;
+        }
+        if (GROUPED && p.value_freq) {  // values were cached turned by their position: back by the row's
+            const float pos = (float)__ldg(p.positions + row_begin + n / p.group);
+#pragma unroll
+            for (int k = 0; k < 8; k += 2) {
+                float sn, cs;
+                fast_sincos(pos * __ldg(p.value_freq + (d + k) / 2), &sn, &cs);
+                const float x = v[k] * cs + v[k + 1] * sn;
+                v[k + 1] = v[k + 1] * cs - v[k] * sn;
+                v[k] = x;
             }
         }
-        store(n, d, v, inv);
+        const uint4 packed = make_uint4(pack_pair<T>(v[0] * inv, v[1] * inv), pack_pair<T>(v[2] * inv, v[3] * inv), pack_pair<T>(v[4] * inv, v[5] * inv),
+                                        pack_pair<T>(v[6] * inv, v[7] * inv));
+        if (GROUPED)
+            *reinterpret_cast<uint4*>(static_cast<T*>(p.out) + pair_of(n) * p.d + d) = packed;
+        else
+            store_half8<PEERS>(p, row_begin + n, head, d, packed);
     }
     if (p.cluster > 1) cl.sync();  // the other CTAs' shared memory is read until here
     if (!REDO) return;
-    if (p.cluster == 1) __syncthreads();
-    int rows_again = 0;
-#pragma unroll
-    for (int n = 0; n < D_ROWS; n++) rows_again |= again[n] ? 1 << n : 0;
-    if (rows_again == 0) return;
-    // ---- redo: row by row over all of its tokens, a half-warp per token, a lane per granule
-    int e_begin = 0, e_end = -1;  // the block's entries
-    for (int w = 0; w < p.cluster * D_WARPS; w++) {
-        const int4 of = __ldg(p.ranges + (size_t)block * (p.cluster * D_WARPS) + w);
-        if (of.x > of.z) continue;
-        if (e_end < 0) e_begin = of.x;
-        e_end = of.z;
-    }
-    const int G = lane & 15;
-    for (int n = 0; n < n_rows; n++) {
-        if (!((rows_again >> n) & 1)) continue;
-        const float mm = again_m[n], ref = mm == -INFINITY ? 0.f : mm;
-        uint4 qn = make_uint4(0u, 0u, 0u, 0u);
-        if (G < p.gpr) qn = __ldg(reinterpret_cast<const uint4*>(p.q) + pair_of(n) * p.gpr + G);
-        float acc[8];
-#pragma unroll
-        for (int k = 0; k < 8; k++) acc[k] = 0.f;
-        for (int e = e_begin; e <= e_end; e++) {
-            const int4 of = __ldg(p.entries + e);
-            if (!((of.z >> n) & 1) || of.x < 0 || of.x >= p.max_chunks) continue;
-            const int tokens = min(C, of.y + (of.w ? p.delta_tokens : 0));
-            const uint8_t* const base = p.pool + ((size_t)of.x * p.n_heads + head) * (size_t)p.pair_bytes;
-            for (int t0 = 0; t0 < tokens; t0 += 2 * D_WARPS) {
-                const int t = t0 + 2 * warp + (lane >> 4);
-                const bool on = t < tokens && G < p.gpr;
-                const size_t at = PANELS ? (size_t)((((G >> 3) * C + t) * 8 + ((G & 7) ^ (t & 7))) * 16) : (size_t)((t * p.gpr + G) * 16);
-                float x = 0.f;
-                uint4 vn = make_uint4(0u, 0u, 0u, 0u);
-                if (on) {
-                    const uint4 kn = __ldg(reinterpret_cast<const uint4*>(base + at));
-                    vn = __ldg(reinterpret_cast<const uint4*>(base + p.v_offset + at));
-#pragma unroll
-                    for (int k = 0; k < 4; k++) {
-                        const float2 a = half2_of((&qn.x)[k]), b = half2_of((&kn.x)[k]);
-                        x = fmaf(a.x, b.x, x);
-                        x = fmaf(a.y, b.y, x);
-                    }
-                }
-#pragma unroll
-                for (int off = 8; off >= 1; off >>= 1) x += __shfl_xor_sync(0xffffffffu, x, off);
-                if (on) {
-                    const float w = exp2f(x * p.scale_log2 - ref);
-#pragma unroll
-                    for (int k = 0; k < 4; k++) {
-                        const float2 b = half2_of((&vn.x)[k]);
-                        acc[2 * k] = fmaf(w, b.x, acc[2 * k]);
-                        acc[2 * k + 1] = fmaf(w, b.y, acc[2 * k + 1]);
-                    }
-                }
-            }
-        }
-#pragma unroll
-        for (int k = 0; k < 8; k++) acc[k] += __shfl_xor_sync(0xffffffffu, acc[k], 16);
-        if (lane < 16 && 8 * lane < DV) {
-            float4* const dst = reinterpret_cast<float4*>(area + warp * PITCH + 8 * lane);
-            dst[0] = make_float4(acc[0], acc[1], acc[2], acc[3]);
-            dst[1] = make_float4(acc[4], acc[5], acc[6], acc[7]);
-        }
+    int rows_again;
+    if (p.cluster == 1) {
+        rows_again = area_have[0] >> D_ROWS;
+        if (rows_again == 0) return;
         __syncthreads();
-        if (threadIdx.x < DV / 8 && ((again[n] >> threadIdx.x) & 1)) {
-            float v[8];
-#pragma unroll
-            for (int k = 0; k < 8; k++) {
-                v[k] = 0.f;
-#pragma unroll
-                for (int w = 0; w < D_WARPS; w++) v[k] += area[w * PITCH + 8 * threadIdx.x + k];
-            }
-            store(n, 8 * (int)threadIdx.x, v, again_inv[n]);
-        }
-        __syncthreads();
+    } else {
+        rows_again = again[1];
+        if (rows_again == 0) return;
     }
+    if constexpr (REDO) redo<VG, PANELS, PEERS>(p, smem, rows_again);
 }
 
 template <typename T, int KQ, int VG, bool PANELS, int LO, bool PEERS = false> cudaError_t launch(const DirectParams& p, cudaStream_t stream) {

@@ -186,9 +186,9 @@ double waves(double ctas, double slots) {
 // Which way a step goes, by estimates of its time in us.  Their constants are fits to steps back to back on a B200, 340 of them
 // (heads of 32 to 128, 1 to 256 rows, 0 to 2048 shared and 4 to 4000 own tokens, every shape of blocks and clusters): the shape they
 // pick is 1 % from the best one in the mean, and the way they pick loses at most a few per cent.
-// Some of them, items or any-geometry kernel -> here: 32 heads of 128, 1 row of 1500 tokens 12.3 -> 9.0, of 4000 16.8 -> 14.5, 4 rows of 256
-// shared and 200 own 11.1 -> 9.7, 16 rows over 256 shared 11.9 -> 8.2; 8 heads, 4 rows of 300 9.6 -> 7.5; 12 heads of 64, 16 rows of 500 shared and up
-// to 333 own 12.8 -> 8.7.  Larger steps belong to the items: 64 rows of 1100 tokens, 8 heads, 52 against 59 (CTAs of units that differ cannot take
+// Some of them, items or any-geometry kernel -> here: 32 heads of 128, 1 row of 1500 tokens 12.3 -> 8.9, of 4000 16.8 -> 14.1, 4 rows of 256
+// shared and 200 own 11.1 -> 9.5, 16 rows over 256 shared 11.9 -> 8.2; 8 heads, 4 rows of 300 9.6 -> 7.5; 12 heads of 64, 16 rows of 500 shared and up
+// to 333 own 12.8 -> 8.8.  Larger steps belong to the items: 64 rows of 1100 tokens, 8 heads, 52 against 59 (CTAs of units that differ cannot take
 // over from each other), 16 rows of 2048 shared and 1100 own, 32 heads, 62 against 69.
 // The items' times are of steps launched by the host, which takes 7.8 us for two kernels.  Replayed from a graph, 16 of 260 steps are more than
 // 3 % slower here than by items, those of one head over 2048 shared tokens most (20 rows 6.9 -> 9.7); all together take 0.84 of the time.
